@@ -203,11 +203,10 @@ struct SingleArgs {
   uint64_t nprimes;
   uint64_t p_lim;
   unsigned long long* ctr;  // [0] work, [1] found, [2] max p
+  uint32_t warp_queries;  // set by the launch: queries a warp holds at a time
 };
-// Batches below kLaneBatchMin queries take the warp-per-query kernel (latency),
-// larger ones the lane-per-query kernel (throughput).
-constexpr uint64_t kLaneBatchMin = 8192;
-cudaError_t launch_single(const SingleArgs& a, int grid, cudaStream_t s);
+// The batch's CTAs fill at most share_pct percent of sm_count SMs.
+cudaError_t launch_single(const SingleArgs& a, int sm_count, uint32_t share_pct, cudaStream_t s);
 // Arguments of segment_reduce_kernel, kept together for a graph's kernel node.
 struct SegReduceArgs {
   const uint64_t* p;
@@ -217,8 +216,8 @@ struct SegReduceArgs {
 };
 // Kernel-node parameters of the launches launch_single / launch_segment_reduce
 // would make (argv: caller storage for the argument pointers; a, r and argv
-// must stay alive until the node is added or updated).
-void single_kernel_node(const SingleArgs& a, int grid, void** argv, cudaKernelNodeParams* kp);
+// must stay alive until the node is added or updated; a's shape is set).
+void single_kernel_node(SingleArgs& a, int sm_count, void** argv, cudaKernelNodeParams* kp);
 void segment_reduce_node(const SegReduceArgs& r, void** argv, cudaKernelNodeParams* kp);
 cudaError_t launch_is_prime(const uint64_t* n, uint64_t count, uint8_t* out, cudaStream_t s);
 cudaError_t launch_win_expand(const gb_window* w, const uint64_t* off, uint32_t nw, uint64_t* n,

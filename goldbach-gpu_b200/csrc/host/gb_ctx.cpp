@@ -531,9 +531,7 @@ gb_status single_impl(gb_ctx* c, Workspace& w, Arena* arena, const uint64_t* n, 
     a.nprimes = np;
     a.p_lim = o.p_limit;
     a.ctr = w.ctr;
-    uint64_t grid = (uint64_t)c->sm_count * 6;
-    grid = std::min<uint64_t>(grid, (count + 7) / 8);
-    chk(launch_single(a, (int)std::max<uint64_t>(grid, 1), s));
+    chk(launch_single(a, c->sm_count, 100, s));
     ++launches;
   }
   if (!o.on_device && count) {

@@ -179,8 +179,9 @@ void poll_queue(gb_server* S, int ln) {
 // single-n kernel, the per-request reduction, two downloads) as one CUDA
 // graph, built once with the lane's fixed buffers; each batch updates the
 // copy sizes and the two kernels' arguments and launches it.  Only batches
-// of fewer than kLaneBatchMin n use it (the kernel node is the
-// warp-per-query kernel).
+// of fewer than kGraphBatchMax n use it (beyond, the kernel's time hides the
+// launches).
+constexpr uint64_t kGraphBatchMax = 8192;
 struct SingleGraph {
   cudaGraph_t g = nullptr;
   cudaGraphExec_t x = nullptr;
@@ -197,7 +198,7 @@ struct SingleBufs {
   unsigned long long* d_agg;
 };
 
-bool build_single_graph(gb_server* S, const SingleBufs& B, const SingleArgs& a0,
+bool build_single_graph(gb_server* S, const SingleBufs& B, SingleArgs a0,
                         SingleGraph* G) {
   Lane& L = S->lane[0];
   if (cudaGraphCreate(&G->g, 0) != cudaSuccess) return false;
@@ -218,7 +219,7 @@ bool build_single_graph(gb_server* S, const SingleBufs& B, const SingleArgs& a0,
   prev = G->reset;
   void* argv[4];
   cudaKernelNodeParams kp;
-  single_kernel_node(a0, 1, argv, &kp);
+  single_kernel_node(a0, S->c->sm_count, argv, &kp);
   ok = ok && cudaGraphAddKernelNode(&G->ks, G->g, &prev, 1, &kp) == cudaSuccess;
   prev = G->ks;
   const SegReduceArgs r0{B.d_p, B.d_off, 1, B.d_agg};
@@ -236,8 +237,8 @@ bool build_single_graph(gb_server* S, const SingleBufs& B, const SingleArgs& a0,
 }
 
 // One batch through the graph: pos n, nreq requests, args a (count = pos).
-cudaError_t run_single_graph(gb_server* S, const SingleBufs& B, const SingleArgs& a, int grid,
-                             uint32_t nreq, SingleGraph* G) {
+cudaError_t run_single_graph(gb_server* S, const SingleBufs& B, SingleArgs a, uint32_t nreq,
+                             SingleGraph* G) {
   Lane& L = S->lane[0];
   const uint64_t pos = a.count;
   cudaError_t e;
@@ -253,7 +254,7 @@ cudaError_t run_single_graph(gb_server* S, const SingleBufs& B, const SingleArgs
     return e;
   void* argv[4];
   cudaKernelNodeParams kp;
-  single_kernel_node(a, grid, argv, &kp);
+  single_kernel_node(a, S->c->sm_count, argv, &kp);
   if ((e = cudaGraphExecKernelNodeSetParams(G->x, G->ks, &kp)) != cudaSuccess) return e;
   const SegReduceArgs r{B.d_p, B.d_off, nreq, B.d_agg};
   segment_reduce_node(r, argv, &kp);
@@ -323,14 +324,13 @@ void single_lane(gb_server* S) {
     };
     SingleArgs a = base;
     a.count = pos;
-    const uint64_t grid = std::max<uint64_t>(1, std::min<uint64_t>((uint64_t)c->sm_count * 6, (pos + 7) / 8));
-    if (graph && pos < kLaneBatchMin) {
-      chk(run_single_graph(S, B, a, (int)grid, (uint32_t)take.size(), &G));
+    if (graph && pos < kGraphBatchMax) {
+      chk(run_single_graph(S, B, a, (uint32_t)take.size(), &G));
     } else {
       chk(cudaMemcpyAsync(d_n, S->h_n, pos * 8, cudaMemcpyHostToDevice, L.stream));
       chk(cudaMemcpyAsync(d_off, S->h_off, (take.size() + 1) * 8, cudaMemcpyHostToDevice, L.stream));
       chk(cudaMemsetAsync(L.ws.ctr, 0, 4 * 8, L.stream));
-      chk(launch_single(a, (int)grid, L.stream));
+      chk(launch_single(a, c->sm_count, 100, L.stream));
       chk(launch_segment_reduce(d_p, d_off, (uint32_t)take.size(), d_agg, L.stream));
       chk(cudaMemcpyAsync(S->h_p, d_p, pos * 8, cudaMemcpyDeviceToHost, L.stream));
       chk(cudaMemcpyAsync(S->h_agg, d_agg, take.size() * 32, cudaMemcpyDeviceToHost, L.stream));

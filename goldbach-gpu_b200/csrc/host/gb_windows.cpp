@@ -372,10 +372,7 @@ static gb_status windows_mr_impl(gb_ctx* c, Workspace& ws, Arena* arena, const g
     a.p_out = (uint64_t*)d_p + b;
     a.q_out = (uint64_t*)d_q + b;
     chk(cudaMemsetAsync(ws.ctr, 0, 4 * 8, s));
-    const uint64_t share = o.gpu_share_pct ? o.gpu_share_pct : 100;
-    const uint64_t gcap = std::max<uint64_t>(1, (uint64_t)c->sm_count * 6 * share / 100);
-    const uint64_t grid = std::max<uint64_t>(1, std::min<uint64_t>(gcap, (n + 7) / 8));
-    chk(launch_single(a, (int)grid, s));
+    chk(launch_single(a, c->sm_count, o.gpu_share_pct ? o.gpu_share_pct : 100, s));
     ++launches;
   }
   chk(launch_segment_reduce((const uint64_t*)d_p, (const uint64_t*)d_off, (uint32_t)count,

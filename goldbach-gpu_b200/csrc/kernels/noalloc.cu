@@ -173,8 +173,6 @@ extern "C" gb_status gb_check_single_batch_noalloc(const uint64_t* n, size_t cou
   a.ctr = ctr;
   int sm = 148;
   cudaDeviceGetAttribute(&sm, cudaDevAttrMultiProcessorCount, dev);
-  uint64_t grid = (uint64_t)sm * 6;
-  if (grid > (count + 7) / 8) grid = (count + 7) / 8;
-  if (launch_single(a, (int)(grid ? grid : 1), s) != cudaSuccess) return GB_ECUDA;
+  if (launch_single(a, sm, 100, s) != cudaSuccess) return GB_ECUDA;
   return GB_OK;
 }

@@ -4,37 +4,31 @@
 // 95-282).  The reference sieves p in chunks of 1e8 on the CPU, copies them
 // to the GPU, runs one thread per p with a 128-bit-remainder Miller-Rabin
 // and keeps whichever thread finishes first, so its p is not the minimal
-// one.  Here every lane of a warp owns one query n (taken from a device work
-// counter as it frees up) and walks the candidate primes p = 3, 5, 7, ...
-// in order until q = n - p is prime:
-//   1. candidates come in batches of 32 consecutive primes, filtered by the
-//      whole warp for the query that needs them (lane i tests the i-th
-//      prime): q is dropped when a prime r <= 61 divides it, tested on
-//      x = q mod M for three products M of those primes (x = n mod M - p
-//      mod M, n mod M computed once per query) by exact-division checks;
-//   2. each lane runs one strong probable-prime test per round on its own
-//      next survivor: base 2 first, then, for a base-2 pass, the six other
-//      bases of the deterministic set one per round, so a query takes about
-//      12 rounds (about 5.7 base-2 tests for n near 2^63) and every lane
-//      does useful work in every round;
-//   3. a round's exponentiation is uniform across the warp: a fixed 2-bit
-//      window (squaring twice, then one product with 1, a, a^2 or a^3 picked
-//      by the two exponent bits) over the warp's longest exponent, so lanes
-//      with different q and bases never diverge.
-// Queries n < 2^21 (where q may be a prime <= 61) take a warp-cooperative
-// scan with the full test per candidate instead.  Small batches, where
-// latency rather than throughput sets the time, take single_warp_kernel
-// (one warp per query).
+// one.  Here a query n walks the candidate primes p = 3, 5, 7, ... in order
+// until q = n - p is prime:
+//   1. the first 64 candidates (p <= 313) are sieved at once: for each odd
+//      prime r <= 617, the residue of n mod r picks a 64-bit mask of the
+//      candidates whose q r does not divide (SieveTab), and the masks are
+//      ANDed; about 3.8 survivors are then tested per query near 2^63;
+//   2. a survivor's q takes the base-2 strong test, 32 lanes at once with the
+//      loops uniform across the warp (prp64.cuh);
+//   3. a pass takes the extra strong Lucas test, which makes it a proof.
+// A warp holds up to 32 queries and deals its lanes out to them: with 32
+// queries each has one lane (throughput), with fewer each has several, which
+// test that many of its survivors at once (latency, and the tail of a large
+// batch).  Queries n < 2^21 (where q may be a prime <= 617) take a
+// warp-cooperative scan with the full test per candidate.
 #include <cuda_runtime.h>
 
 #include <cstdint>
+#include <type_traits>
 
 #include "../gb_device.cuh"
 #include "../gb_internal.h"
+#include "prp64.cuh"
 
 namespace gb {
 
-constexpr int kSingleThreads = 256;
 constexpr uint64_t kSmallN = 1ull << 21;  // below this, q may be tiny: plain path
 constexpr uint32_t kFull = 0xffffffffu;
 
@@ -44,15 +38,17 @@ __device__ __forceinline__ uint32_t lanemask_lt() {
   return m;
 }
 
-// Lane-parallel ascending scan with the full primality test per lane (the
-// whole warp serves one n).
-__device__ uint32_t minp_plain(const SingleArgs& a, uint64_t n, uint64_t lim) {
+// Lane-parallel ascending scan over the primes above p_after with the full
+// primality test per lane (the whole warp serves one n).
+__device__ __noinline__ uint32_t minp_plain(const SingleArgs& a, uint64_t n, uint32_t p_after) {
   const int lane = threadIdx.x & 31;
+  const uint64_t half = n >> 1;
+  const uint64_t lim = half < a.p_lim ? half : a.p_lim;
   for (uint64_t k = 1;; k += 32) {
     const uint64_t kk = k + lane;
     const uint32_t p = kk < a.nprimes ? a.primes[kk] : 0xffffffffu;
     const bool valid = kk < a.nprimes && p <= lim;
-    const bool ok = valid && is_prime_u64(n - p);
+    const bool ok = valid && p > p_after && is_prime_u64(n - p);
     const uint32_t b = __ballot_sync(kFull, ok);
     if (b) return __shfl_sync(kFull, p, __ffs(b) - 1);
     if (__ballot_sync(kFull, valid) != kFull) return 0;
@@ -93,189 +89,401 @@ __device__ __forceinline__ bool no_small_factor(uint32_t nm1, uint32_t nm2, uint
   return !f;
 }
 
-// Montgomery context for mont_mul32: the modulus, -n^-1 mod 2^32 and R mod n.
-struct Mont32 {
-  uint64_t n;
-  uint64_t one;
-  uint32_t ni;
-};
-
-// R mod n without a 64-bit division: 2^(k+1) - n for the top bit k of n,
-// then doubled up to 2^64 (no doubling for n >= 2^63).
-__device__ __forceinline__ Mont32 mont32_init(uint64_t n) {
-  Mont32 M;
-  M.n = n;
-  M.ni = 0u - inv32((uint32_t)n);
-  const int k = 63 - __clzll(n);
-  uint64_t x = k == 63 ? 0 - n : (2ull << k) - n;
-  for (int j = k + 1; j < 64; ++j) x = mod_dbl(x, n);
-  M.one = x;
-  return M;
+// The candidate sieve.  Bit k of a mask stands for the k-th odd prime p (3, 5,
+// ..., 313).  For each of the first kSieveMods moduli R -- a prime up to 313, or a
+// product of a few small ones -- a table gives the mask of x = n mod R: bit k
+// is clear when a prime factor f of R divides x - p, that is when f divides
+// q = n - p.  A prime r above 313 strikes at most the candidate p = n mod r
+// itself, so those up to 617 share one table of 315 masks (kSieveOnes; the
+// last entry strikes nothing).  617 is about where one more prime (15 clocks
+// a lane) stops paying for the base-2 tests it saves (4 x 3900 / r clocks).
+constexpr int kSieveMods = 57;
+__host__ __device__ constexpr uint32_t sieve_mod(int i) {
+  constexpr uint16_t kMods[kSieveMods] = {
+      1155, 221, 437, 899, 1517, 43,  47,  53,  59,  61,  67,  71,  73,  79,  83,  89,  97,  101, 103,
+      107,  109, 113, 127, 131,  137, 139, 149, 151, 157, 163, 167, 173, 179, 181, 191, 193, 197, 199,
+      211,  223, 227, 229, 233,  239, 241, 251, 257, 263, 269, 271, 277, 281, 283, 293, 307, 311, 313};
+  return kMods[i];
 }
+__host__ __device__ constexpr uint32_t sieve_offset(int i) {
+  uint32_t o = 0;
+  for (int j = 0; j < i; ++j) o += sieve_mod(j);
+  return o;
+}
+constexpr uint32_t kSieveOnes = sieve_offset(kSieveMods);
+constexpr uint32_t kSieveEntries = kSieveOnes + 315;
 
-// Strong probable-prime test of every lane's odd modulus M.n = d 2^s + 1 to
-// its base a1 (Montgomery form), the loop lengths set by the warp's longest
-// exponent and largest s (lanes with act false only run along).
-__device__ __forceinline__ bool sprp_warp(const Mont32& M, uint64_t a1, uint64_t d, int s, bool act) {
-  const uint32_t ni = M.ni;
-  const uint64_t a2 = mont_mul32(a1, a1, M.n, ni);
-  const uint64_t a3 = mont_mul32(a2, a1, M.n, ni);
-  const int top = 63 - __clzll(d);  // d >= 1
-  const int T = (int)__reduce_max_sync(kFull, act ? (uint32_t)top : 0u) | 1;  // odd
-  // bit pairs (i+1, i) from i = T-1 down to 0; the first pair starts x
-  uint32_t b = (uint32_t)(d >> (T - 1)) & 3u;
-  uint64_t x = b == 0 ? M.one : b == 1 ? a1 : b == 2 ? a2 : a3;
-  for (int i = T - 3; i >= 0; i -= 2) {
-    x = mont_mul32(x, x, M.n, ni);
-    x = mont_mul32(x, x, M.n, ni);
-    b = (uint32_t)(d >> i) & 3u;
-    x = mont_mul32(x, b == 0 ? M.one : b == 1 ? a1 : b == 2 ? a2 : a3, M.n, ni);
-  }
-  const uint64_t mone = M.n - M.one;
-  bool ok = x == M.one || x == mone;
-  bool done = ok;
-  const int S = (int)__reduce_max_sync(kFull, act ? (uint32_t)s : 0u);
-  for (int i = 1; i < S; ++i) {
-    x = mont_mul32(x, x, M.n, ni);
-    if (!done && i < s) {
-      if (x == mone) ok = done = true;
-      else if (x == M.one) done = true;
+struct SieveTab {
+  uint64_t m[kSieveEntries];
+  uint64_t m2[kSieveOnes];  // the same for the next 64 odd primes (317, ..., 727)
+  uint32_t mod[kSieveMods], off[kSieveMods];
+  constexpr SieveTab() : m(), m2(), mod(), off() {
+    uint32_t odd_primes[128] = {};
+    int np = 0;
+    for (uint32_t v = 3; np < 128; v += 2) {
+      bool prime = true;
+      for (int k = 0; k < np && prime; ++k) prime = v % odd_primes[k] != 0;
+      if (prime) odd_primes[np++] = v;
     }
+    for (uint32_t i = 0; i < kSieveEntries; ++i) m[i] = ~0ull;
+    for (uint32_t i = 0; i < kSieveOnes; ++i) m2[i] = ~0ull;
+    uint32_t o = 0;
+    for (int i = 0; i < kSieveMods; ++i) {
+      const uint32_t R = sieve_mod(i);
+      mod[i] = R;
+      off[i] = o;
+      for (int j = 0; j < 64; ++j) {  // prime factors of R (all <= 313)
+        const uint32_t f = odd_primes[j];
+        if (R % f) continue;
+        for (int k = 0; k < 64; ++k)
+          for (uint32_t x = odd_primes[k] % f; x < R; x += f) m[o + x] &= ~(1ull << k);
+        for (int k = 0; k < 64; ++k)
+          for (uint32_t x = odd_primes[64 + k] % f; x < R; x += f) m2[o + x] &= ~(1ull << k);
+      }
+      o += R;
+    }
+    for (int k = 0; k < 64; ++k) m[kSieveOnes + odd_primes[k]] &= ~(1ull << k);
   }
-  return ok;
+};
+__device__ const SieveTab g_sieve{};
+
+// n mod M for a constant 2^13 < M < 2^31 from one FMA of n as a double: the
+// conversion, 1/M and the product are each within 2^-53 of exact, so the
+// estimate is within 2^-4 of n / M < 2^51 and rounds to floor(n / M) or one
+// more; the low 32 bits of the sum with 1.5 * 2^52 are that quotient's.
+template <uint32_t M>
+__device__ __forceinline__ uint32_t mod_const(double nd, uint32_t nl) {
+  static_assert(M > (1u << 13) && M < (1u << 31), "quotient estimate");
+  constexpr double kInv = 1.0 / M;
+  const uint32_t qt = (uint32_t)__double_as_longlong(fma(nd, kInv, 6755399441055744.0));
+  const uint32_t r = nl - qt * M;
+  return min(r, r + M);
 }
 
-__global__ void __launch_bounds__(kSingleThreads) single_kernel(SingleArgs a) {
+// The masks of C moduli from index I on, by way of n mod their product.
+template <int I, int C>
+__device__ __forceinline__ uint64_t sieve_group(const uint64_t* tab, double nd, uint32_t nl) {
+  constexpr uint32_t M = sieve_mod(I) * (C > 1 ? sieve_mod(I + (C > 1)) : 1u) *
+                         (C > 2 ? sieve_mod(I + 2 * (C > 2)) : 1u) *
+                         (C > 3 ? sieve_mod(I + 3 * (C > 3)) : 1u);
+  const uint32_t x = mod_const<M>(nd, nl);
+  uint64_t m = tab[sieve_offset(I) + x % sieve_mod(I)];
+  if constexpr (C > 1) m &= tab[sieve_offset(I + 1) + x % sieve_mod(I + 1)];
+  if constexpr (C > 2) m &= tab[sieve_offset(I + 2) + x % sieve_mod(I + 2)];
+  if constexpr (C > 3) m &= tab[sieve_offset(I + 3) + x % sieve_mod(I + 3)];
+  return m;
+}
+// The same for three primes above 313.
+template <uint32_t A, uint32_t B, uint32_t C>
+__device__ __forceinline__ uint64_t sieve_ones(const uint64_t* tab, double nd, uint32_t nl) {
+  const uint32_t x = mod_const<A * B * C>(nd, nl);
+  const uint64_t* t = tab + kSieveOnes;
+  return t[min(x % A, 314u)] & t[min(x % B, 314u)] & t[min(x % C, 314u)];
+}
+
+__device__ __forceinline__ uint64_t sieve_all(const uint64_t* tab, uint64_t n) {
+  const double nd = __ull2double_rn(n);
+  const uint32_t nl = (uint32_t)n;
+  uint64_t m = sieve_group<0, 3>(tab, nd, nl) & sieve_group<3, 3>(tab, nd, nl) &
+               sieve_group<6, 4>(tab, nd, nl) & sieve_group<10, 4>(tab, nd, nl) &
+               sieve_group<14, 4>(tab, nd, nl) & sieve_group<18, 4>(tab, nd, nl) &
+               sieve_group<22, 4>(tab, nd, nl) & sieve_group<26, 4>(tab, nd, nl) &
+               sieve_group<30, 4>(tab, nd, nl) & sieve_group<34, 4>(tab, nd, nl) &
+               sieve_group<38, 3>(tab, nd, nl) & sieve_group<41, 3>(tab, nd, nl) &
+               sieve_group<44, 3>(tab, nd, nl) & sieve_group<47, 3>(tab, nd, nl) &
+               sieve_group<50, 3>(tab, nd, nl) & sieve_group<53, 2>(tab, nd, nl) &
+               sieve_group<55, 2>(tab, nd, nl);
+  m &= sieve_ones<317, 331, 337>(tab, nd, nl) & sieve_ones<347, 349, 353>(tab, nd, nl) &
+       sieve_ones<359, 367, 373>(tab, nd, nl) & sieve_ones<379, 383, 389>(tab, nd, nl) &
+       sieve_ones<397, 401, 409>(tab, nd, nl) & sieve_ones<419, 421, 431>(tab, nd, nl) &
+       sieve_ones<433, 439, 443>(tab, nd, nl) & sieve_ones<449, 457, 461>(tab, nd, nl) &
+       sieve_ones<463, 467, 479>(tab, nd, nl) & sieve_ones<487, 491, 499>(tab, nd, nl) &
+       sieve_ones<503, 509, 521>(tab, nd, nl) & sieve_ones<523, 541, 547>(tab, nd, nl) &
+       sieve_ones<557, 563, 569>(tab, nd, nl) & sieve_ones<571, 577, 587>(tab, nd, nl) &
+       sieve_ones<593, 599, 601>(tab, nd, nl) & sieve_ones<607, 613, 617>(tab, nd, nl);
+  return m;
+}
+
+// The warp's sieve of the first 128 candidates of one n (lanes agree on n)
+// over the moduli with tables of their own, for small batches: a query's
+// lanes test more survivors at once than 64 candidates leave (about 17), and
+// the few queries whose minimal p lies beyond 313 (6%) would make the whole
+// batch wait for further rounds (100 queries: 41 -> 28 us).
+struct Mask128 {
+  uint64_t lo, hi;
+};
+__device__ __forceinline__ uint64_t warp_and(uint64_t m) {
+  const uint32_t l = __reduce_and_sync(kFull, (uint32_t)m), h = __reduce_and_sync(kFull, (uint32_t)(m >> 32));
+  return (uint64_t)h << 32 | l;
+}
+__device__ __forceinline__ Mask128 sieve_warp(uint64_t n) {
+  const uint32_t hi = (uint32_t)(n >> 32), lo = (uint32_t)n;
+  Mask128 m{~0ull, ~0ull};
+#pragma unroll 1
+  for (int j = threadIdx.x & 31; j < kSieveMods; j += 32) {
+    const uint32_t R = g_sieve.mod[j];
+    // n mod R from its halves: R < 2^11, so the sum stays below 2^32
+    const uint32_t t = g_sieve.off[j] + ((hi % R) * ((0xffffffffu % R + 1) % R) + lo % R) % R;
+    m.lo &= g_sieve.m[t];
+    m.hi &= g_sieve.m2[t];
+  }
+  return {warp_and(m.lo), warp_and(m.hi)};
+}
+
+// Bits of the 64 candidates from prime index k0 on that are <= p_lim: a whole
+// warp's call, two loads a lane.
+__device__ __forceinline__ uint64_t candidates_below(const SingleArgs& a, uint32_t k0) {
+  const uint32_t k = k0 + (threadIdx.x & 31);
+  const uint32_t lo = __ballot_sync(kFull, k < a.nprimes && a.primes[k] <= a.p_lim);
+  const uint32_t hi = __ballot_sync(kFull, k + 32 < a.nprimes && a.primes[k + 32] <= a.p_lim);
+  return (uint64_t)hi << 32 | lo;
+}
+
+// Every round the warp deals its 32 lanes out to its A <= 32 queries (slots),
+// rank by rank: lane l tests survivor l / A of query l % A.  The lowest rank
+// that passes base 2 holds the query's minimal candidate; it joins the warp's
+// pending list and the slot is free for the next query at once.  Whenever 32
+// candidates are pending, one Lucas test proves them all, so both tests run
+// with (nearly) all lanes at work, and the sieve runs for a whole warp's
+// refill of queries at a time.  A candidate that the Lucas test rejects (a
+// base-2 pseudoprime) sends its query through minp_plain from there on.
+//
+// Bound: the multiplier (prp64.cuh).  One CTA of 16 warps per SM: four warps
+// per quarter cover a product's latency (95 clocks against 54 of issue), and
+// the sieve tables take 108 KB. 
+// Device time of a batch uniform below 2^64, against one strong test to each
+// of 7 bases on a lane (8192 queries or more) or a warp (fewer) per query:
+// 1e6 queries 2.97 -> 0.97 ms, 20000 648 -> 81 us, 8191 107 -> 57, 3001 58 -> 47,
+// 592 and fewer unchanged (36 us, of which about 13 are the launch).
+constexpr int kSingleThreads = 512;
+struct SingleWarp {
+  // slots: query, its index, its survivors not yet tested among 128 candidates,
+  // prime index of mask's bit 0, and of the next block (0: none)
+  uint64_t n[32], qi[32], mask[32], mask2[32];
+  uint32_t cbase[32], kb[32];
+  uint64_t rn[32], rmask[32], rmask2[32], rqi[32];  // sieved queries not yet in a slot
+  uint64_t pq[64], pqi[64];          // pending: q, query index
+  uint32_t pp[64];                   // and p
+  uint32_t slot[32];                 // the occupied slots in order
+};
+constexpr int kSingleWarps = kSingleThreads / 32;
+struct SingleCta {
+  SingleWarp warp[kSingleWarps];
+  uint64_t pq[31 * kSingleWarps], pqi[31 * kSingleWarps];  // pending at the end
+  uint32_t pp[31 * kSingleWarps], npend;
+};
+constexpr size_t kSingleTabBytes = kSieveEntries * sizeof(uint64_t);
+
+// Clears the lowest set bit of hi : lo.
+__device__ __forceinline__ void drop_lowest(uint64_t& lo, uint64_t& hi) {
+  if (lo) lo &= lo - 1;
+  else hi &= hi - 1;
+}
+
+template <bool STAGED>
+__global__ void __launch_bounds__(kSingleThreads, 1) single_kernel(SingleArgs a) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  SingleCta& cta = *reinterpret_cast<SingleCta*>(smem_raw);
+  SingleWarp& w = cta.warp[threadIdx.x >> 5];
+  uint64_t* tab = reinterpret_cast<uint64_t*>(smem_raw + sizeof(SingleCta));
+  if (STAGED)
+    for (uint32_t i = threadIdx.x; i < kSieveEntries; i += kSingleThreads) tab[i] = g_sieve.m[i];
+  if (threadIdx.x == 0) cta.npend = 0;
+  __syncthreads();
   const int lane = threadIdx.x & 31;
-  // the lane's query
-  bool have = false, drained = false;
-  uint64_t qi = 0, n = 0;
-  uint32_t lim = 0, nm1 = 0, nm2 = 0, nm3 = 0;
-  uint32_t kb = 1;      // prime index of the next candidate batch
-  uint32_t cmask = 0;   // the current batch's survivors not yet tested
-  uint32_t cbase = 0;   // prime index of the current batch's bit 0
-  bool last = false;    // the current batch reached the end of the candidates
-  int stage = 0;        // 0: next candidate, base 2; k = 1..6: base k of the set
-  uint32_t p = 0;       // the candidate under test
-  bool ready = false;   // p taken for this round (stage 0)
-  Mont32 M{3, 1, 1};
-  uint64_t d = 1, r2 = 0;
-  int s = 1;
+  const uint64_t mask0 = candidates_below(a, 1), mask1 = STAGED ? 0 : candidates_below(a, 65);
+  // the block after a slot's masks, 0 when p_lim ends among them
+  const uint32_t kb0 = STAGED ? (mask0 == ~0ull ? 65 : 0) : (mask1 == ~0ull ? 129 : 0);
+  const uint32_t chunk = a.warp_queries;  // queries a warp holds, 1 .. 32
+  uint32_t active = 0, nready = 0, npend = 0;
+  bool first = true, drained = false;
   uint32_t found = 0, maxp = 0;
-  auto finish = [&](uint32_t pf) {
-    a.p_out[qi] = pf;
-    a.q_out[qi] = pf ? n - pf : 0;
+  auto finish = [&](uint64_t i, uint32_t pf, uint64_t q) {
+    a.p_out[i] = pf;
+    a.q_out[i] = q;
     if (pf) {
       ++found;
       maxp = pf > maxp ? pf : maxp;
     }
-    have = false;
+  };
+  // Lucas tests of the lanes' q = n - p (PAIR: lanes 2i and 2i + 1 hold the same)
+  auto prove = [&](uint64_t q, uint64_t i, uint32_t p, bool act, auto pair) {
+    constexpr bool PAIR = decltype(pair)::value;
+    const bool ok = PAIR ? lucas_pair_any(q, act) : lucas_any(q, act);
+    if (PAIR && (lane & 1)) act = false;
+    if (act && ok) finish(i, p, q);
+    for (uint32_t bad = __ballot_sync(kFull, act && !ok); bad; bad &= bad - 1) {
+      const int l = __ffs(bad) - 1;
+      const uint64_t n = __shfl_sync(kFull, q + p, l);
+      const uint32_t pl = minp_plain(a, n, __shfl_sync(kFull, p, l));
+      if (lane == l) finish(i, pl, pl ? n - pl : 0);
+    }
+    __syncwarp();
   };
   for (;;) {
-    // every lane gets a query with a candidate ready, or the queue is empty
+    // fill the slots
     for (;;) {
-      const uint32_t need = __ballot_sync(kFull, !have && !drained);
-      if (need) {
+      if (nready == 0 && !drained && (uint32_t)__popc(active) < chunk) {
+        // the first queries by place, the others from the work counter
+        const uint64_t warps = (uint64_t)gridDim.x * kSingleWarps;
         unsigned long long base = 0;
-        if (lane == __ffs(need) - 1) base = atomicAdd(&a.ctr[0], (unsigned long long)__popc(need));
-        base = __shfl_sync(kFull, base, __ffs(need) - 1);
-        if (!have && !drained) {
-          qi = base + __popc(need & lanemask_lt());
-          if (qi >= a.count) {
-            drained = true;
-          } else {
-            n = a.n[qi];
-            have = true;
-            stage = 0;
-            kb = 1;
-            cmask = 0;
-            last = false;
-            const uint64_t half = n >> 1;
-            lim = (uint32_t)(half < a.p_lim ? half : a.p_lim);
-            nm1 = (uint32_t)(n % kM1);
-            nm2 = (uint32_t)(n % kM2);
-            nm3 = (uint32_t)(n % kM3);
-            if (n < 4 || (n & 1)) finish(0);
-            else if (n == 4) finish(2);
+        if (first) {
+          base = ((uint64_t)(threadIdx.x >> 5) * gridDim.x + blockIdx.x) * chunk;
+        } else {
+          if (lane == 0) base = warps * chunk + atomicAdd(&a.ctr[0], (unsigned long long)chunk);
+          base = __shfl_sync(kFull, base, 0);
+        }
+        first = false;
+        drained = base >= a.count;
+        const uint64_t qi = base + lane;
+        bool ready = lane < (int)chunk && qi < a.count;
+        const uint64_t n = ready ? a.n[qi] : 0;
+        if (ready && (n <= 4 || (n & 1))) {
+          finish(qi, n == 4 ? 2 : 0, n == 4 ? 2 : 0);
+          ready = false;
+        }
+        const uint32_t rb = __ballot_sync(kFull, ready);
+        uint64_t m = 0, m2 = 0;
+        if (STAGED) {
+          if (ready && n >= kSmallN) m = sieve_all(tab, n) & mask0;
+        } else {
+          for (uint32_t left = __ballot_sync(kFull, ready && n >= kSmallN); left; left &= left - 1) {
+            const int l = __ffs(left) - 1;
+            const Mask128 ml = sieve_warp(__shfl_sync(kFull, n, l));
+            if (lane == l) {
+              m = ml.lo & mask0;
+              m2 = ml.hi & mask1;
+            }
           }
         }
+        if (ready) {
+          const uint32_t i = __popc(rb & lanemask_lt());
+          w.rn[i] = n;
+          w.rmask[i] = m;
+          if (!STAGED) w.rmask2[i] = m2;
+          w.rqi[i] = qi;
+        }
+        nready = __popc(rb);
+        __syncwarp();
       }
-      // candidate batches for the lanes that ran out, one query at a time
+      // ready queries into free slots (slots 0 .. chunk - 1 are in use)
+      const uint32_t room = ~active & (chunk == 32 ? kFull : (1u << chunk) - 1);
+      const uint32_t k = min((uint32_t)__popc(room), nready);
+      const uint32_t rank = __popc(room & lanemask_lt());
+      const bool take = ((room >> lane) & 1u) && rank < k;
+      if (take) {
+        const uint32_t i = nready - 1 - rank;
+        w.n[lane] = w.rn[i];
+        w.mask[lane] = w.rmask[i];
+        if (!STAGED) w.mask2[lane] = w.rmask2[i];
+        w.qi[lane] = w.rqi[i];
+        w.cbase[lane] = 1;
+        w.kb[lane] = kb0;
+      }
+      nready -= k;
+      active |= __ballot_sync(kFull, take);
+      __syncwarp();
+      // slots without a survivor: further blocks of candidates, and small n
       for (;;) {
-        const uint32_t m = __ballot_sync(kFull, have && stage == 0 && !ready && cmask == 0 && !last);
-        if (!m) break;
-        const int j = __ffs(m) - 1;
-        const uint64_t nj = __shfl_sync(kFull, n, j);
-        const uint32_t limj = __shfl_sync(kFull, lim, j);
-        if (nj < kSmallN) {
-          const uint32_t pj = minp_plain(a, nj, limj);
-          if (lane == j) finish(pj);
+        const uint32_t b = __ballot_sync(kFull, ((active >> lane) & 1u) && (STAGED ? w.mask[lane] : w.mask[lane] | w.mask2[lane]) == 0);
+        if (!b) break;
+        const int j = __ffs(b) - 1;
+        const uint64_t n = w.n[j];
+        const uint32_t kj = w.kb[j];
+        __syncwarp();
+        if (n < kSmallN || kj == 0) {
+          const uint32_t p = n < kSmallN ? minp_plain(a, n, 2) : 0;
+          if (lane == j) finish(w.qi[j], p, p ? n - p : 0);  // kj = 0: every prime p <= p_lim tried
+          active &= ~(1u << j);
           continue;
         }
-        const uint32_t kj = __shfl_sync(kFull, kb, j);
-        const uint32_t m1 = __shfl_sync(kFull, nm1, j);
-        const uint32_t m2 = __shfl_sync(kFull, nm2, j);
-        const uint32_t m3 = __shfl_sync(kFull, nm3, j);
-        const uint64_t k = (uint64_t)kj + lane;
-        const uint32_t pk = k < a.nprimes ? a.primes[k] : 0xffffffffu;
-        const bool valid = k < a.nprimes && pk <= limj;
-        const uint32_t pass = __ballot_sync(kFull, valid && no_small_factor(m1, m2, m3, pk));
-        const uint32_t vb = __ballot_sync(kFull, valid);
+        const uint64_t half = n >> 1;
+        const uint32_t lim = (uint32_t)(half < a.p_lim ? half : a.p_lim);
+        // a block is 64 candidates, or 128 when few queries wait for each other
+        uint64_t blk[2] = {0, 0};
+        uint32_t more = kFull;
+#pragma unroll 1
+        for (int i = 0; i < (STAGED ? 2 : 4) && more == kFull; ++i) {
+          const uint64_t k = (uint64_t)kj + 32 * i + lane;
+          const uint32_t pk = k < a.nprimes ? a.primes[k] : 0xffffffffu;
+          const bool valid = k < a.nprimes && pk <= lim;
+          const uint64_t pass = __ballot_sync(kFull, valid && no_small_factor(n % kM1, n % kM2, n % kM3, pk));
+          more = __ballot_sync(kFull, valid);
+          if (i < 2) blk[0] |= pass << (32 * i);
+          else blk[1] |= pass << (32 * (i - 2));
+        }
         if (lane == j) {
-          cmask = pass;
-          cbase = kj;
-          kb = kj + 32;
-          last = vb != kFull;
+          w.mask[j] = blk[0];
+          if (!STAGED) w.mask2[j] = blk[1];
+          w.cbase[j] = kj;
+          w.kb[j] = more == kFull ? kj + (STAGED ? 64 : 128) : 0;
         }
+        __syncwarp();
       }
-      // set up this round's test
-      if (have && stage == 0 && !ready) {
-        if (cmask == 0) {
-          finish(0);  // every prime p <= min(n/2, p_lim) tried
+      if ((uint32_t)__popc(active) == chunk || (drained && nready == 0)) break;
+    }
+    if (active) {
+      // deal the lanes out
+      const uint32_t A = __popc(active);
+      if ((active >> lane) & 1u) w.slot[__popc(active & lanemask_lt())] = lane;
+      __syncwarp();
+      const uint32_t idx = lane % A, rank = lane / A;
+      const uint32_t j = w.slot[idx];
+      uint64_t m = w.mask[j], m2 = STAGED ? 0 : w.mask2[j];
+      for (uint32_t i = 0; i < 31 / A; ++i)
+        if (i < rank) drop_lowest(m, m2);
+      const bool act = (m | m2) != 0;
+      const uint32_t bit = m ? __ffsll((long long)m) - 1 : 63 + __ffsll((long long)m2);
+      const uint32_t p = act ? a.primes[w.cbase[j] + bit] : 0;
+      const uint64_t q = act ? w.n[j] - p : 3;
+      const bool pass = sprp2_any(q, act) && act;
+      const uint32_t b = __ballot_sync(kFull, pass);
+      uint32_t mine = 0;  // the lanes of this lane's query
+      for (uint32_t i = idx; i < 32; i += A) mine |= 1u << i;
+      const uint32_t win = b & mine;
+      const int l = win ? __ffs(win) - 1 : lane;
+      const uint64_t qw = __shfl_sync(kFull, q, l);
+      const uint32_t pw = __shfl_sync(kFull, p, l);
+      const uint32_t wb = __ballot_sync(kFull, rank == 0 && win);
+      __syncwarp();
+      if (rank == 0) {
+        if (win) {
+          const uint32_t i = npend + __popc(wb & lanemask_lt());
+          w.pq[i] = qw;
+          w.pqi[i] = w.qi[j];
+          w.pp[i] = pw;
         } else {
-          const int bit = __ffs(cmask) - 1;
-          cmask &= cmask - 1;
-          p = a.primes[cbase + bit];
-          ready = true;
+          uint64_t left = w.mask[j], left2 = STAGED ? 0 : w.mask2[j];
+          for (int i = __popc(mine); i > 0; --i) drop_lowest(left, left2);
+          w.mask[j] = left;
+          if (!STAGED) w.mask2[j] = left2;
         }
       }
-      if (!__ballot_sync(kFull, !have && !drained)) break;
+      active &= ~__reduce_or_sync(kFull, rank == 0 && win ? 1u << j : 0u);
+      npend += __popc(wb);
     }
-    if (!__any_sync(kFull, have)) break;
-    // one strong test per lane: base 2 of a new candidate, or base `stage`
-    uint64_t am = 0;
-    bool skip = false;
-    if (have) {
-      if (stage == 0) {
-        const uint64_t q = n - p;
-        d = q - 1;
-        s = __ffsll((long long)d) - 1;
-        d >>= s;
-        M = mont32_init(q);
-        am = mod_dbl(M.one, M.n);  // 2
-      } else {
-        uint64_t b = kMR7Bases[stage];
-        if (b >= M.n) b %= M.n;
-        skip = b == 0;
-        am = mont_mul32(b, r2, M.n, M.ni);
-      }
+    if (npend >= 32) {
+      npend -= 32;
+      __syncwarp();
+      prove(w.pq[npend + lane], w.pqi[npend + lane], w.pp[npend + lane], true, std::false_type{});
     }
-    const bool ok = sprp_warp(M, am, d, s, have) || skip;
-    ready = false;
-    if (have) {
-      if (!ok) {
-        stage = 0;  // composite (a base-2 pseudoprime when stage > 0)
-      } else if (stage == 0) {
-        // R^2 mod q = 2^64 in Montgomery form: 2 squared six times
-        uint64_t t = mod_dbl(M.one, M.n);
-#pragma unroll
-        for (int i = 0; i < 6; ++i) t = mont_mul32(t, t, M.n, M.ni);
-        r2 = t;
-        stage = 1;
-      } else if (++stage == 7) {
-        finish(p);
-      }
-    }
+    if (!active && drained && nready == 0) break;
+  }
+  // what the warps still have pending, proved 16 to a warp with a pair of lanes each
+  uint32_t base = 0;
+  if (lane == 0 && npend) base = atomicAdd(&cta.npend, npend);
+  base = __shfl_sync(kFull, base, 0);
+  if (lane < (int)npend) {
+    cta.pq[base + lane] = w.pq[lane];
+    cta.pqi[base + lane] = w.pqi[lane];
+    cta.pp[base + lane] = w.pp[lane];
+  }
+  __syncthreads();
+  const uint32_t total = cta.npend;
+  for (uint32_t e0 = 16 * (threadIdx.x >> 5); e0 < total; e0 += 16 * kSingleWarps) {
+    const uint32_t e = e0 + (lane >> 1);
+    const bool act = e < total;
+    prove(act ? cta.pq[e] : 3, act ? cta.pqi[e] : 0, act ? cta.pp[e] : 0, act, std::true_type{});
   }
   // the warp's counts, one atomic each
   found = __reduce_add_sync(kFull, found);
@@ -286,125 +494,48 @@ __global__ void __launch_bounds__(kSingleThreads) single_kernel(SingleArgs a) {
   }
 }
 
-// Latency path for small batches: one warp per query.  Survivors of the
-// small-prime filter are gathered in order (shared memory) until 32 are
-// pending; each lane runs the base-2 test on one of them, and the lowest
-// lane that passed gets the six other bases, one base per lane.  A lone
-// query then costs about two strong-test latencies instead of the dozen
-// the lane-per-query kernel spends on it one after another.
-__device__ uint32_t minp_warp(const SingleArgs& a, uint64_t n, uint32_t* buf) {
-  const int lane = threadIdx.x & 31;
-  const uint64_t half = n >> 1;
-  const uint32_t lim = (uint32_t)(half < a.p_lim ? half : a.p_lim);
-  const uint32_t nm1 = (uint32_t)(n % kM1), nm2 = (uint32_t)(n % kM2), nm3 = (uint32_t)(n % kM3);
-  uint64_t k = 1;
-  uint32_t nsurv = 0;
-  bool exhausted = false;
-  for (;;) {
-    while (nsurv < 32 && !exhausted) {
-      const uint64_t kk = k + lane;
-      const uint32_t p = kk < a.nprimes ? a.primes[kk] : 0xffffffffu;
-      const bool valid = kk < a.nprimes && p <= lim;
-      const bool pass = valid && no_small_factor(nm1, nm2, nm3, p);
-      const uint32_t b = __ballot_sync(kFull, pass);
-      if (pass) buf[nsurv + __popc(b & lanemask_lt())] = (uint32_t)kk;
-      nsurv += __popc(b);
-      if (__ballot_sync(kFull, valid) != kFull) exhausted = true;
-      k += 32;
-    }
-    __syncwarp();
-    if (nsurv == 0) return 0;
-    const uint32_t take = nsurv < 32 ? nsurv : 32;
-    const bool act = lane < (int)take;
-    uint32_t pk = 0;
-    uint64_t q = 3;
-    if (act) {
-      pk = a.primes[buf[lane]];
-      q = n - pk;
-    }
-    uint64_t d = q - 1;
-    int s = __ffsll((long long)d) - 1;
-    d >>= s;
-    Mont32 M = mont32_init(q);
-    const bool ok2 = sprp_warp(M, mod_dbl(M.one, M.n), d, s, act) && act;
-    uint32_t b = __ballot_sync(kFull, ok2);
-    while (b) {
-      const int l = __ffs(b) - 1;
-      const uint64_t qc = __shfl_sync(kFull, q, l);
-      const uint32_t pc = __shfl_sync(kFull, pk, l);
-      uint64_t dc = qc - 1;
-      const int sc = __ffsll((long long)dc) - 1;
-      dc >>= sc;
-      const Mont32 Mc = mont32_init(qc);
-      uint64_t r2 = mod_dbl(Mc.one, Mc.n);
-#pragma unroll
-      for (int i = 0; i < 6; ++i) r2 = mont_mul32(r2, r2, Mc.n, Mc.ni);
-      uint64_t base = kMR7Bases[lane < 6 ? lane + 1 : 1];
-      if (base >= qc) base %= qc;
-      const bool test = lane < 6 && base != 0;
-      const bool ok = sprp_warp(Mc, mont_mul32(base, r2, Mc.n, Mc.ni), dc, sc, test) || !test;
-      if (__all_sync(kFull, ok)) return pc;
-      b &= b - 1;
-    }
-    // none of the first `take` survivors is prime: drop them
-    __syncwarp();
-    uint32_t keep = 0;
-    if (lane + take < nsurv) keep = buf[lane + take];
-    __syncwarp();
-    if (lane + take < nsurv) buf[lane] = keep;
-    __syncwarp();
-    nsurv -= take;
-  }
+// Shape of a batch on sm_count SMs, of which it may fill share_pct percent: the
+// queries spread over 16 warps per SM, up to 32 each.  From kSingleTabQueries a
+// warp on, the sieve tables are staged in shared memory and every lane sieves
+// its own query: 20000 queries (9 a warp) take 81 us unstaged and 97 staged, 76000
+// (32 a warp) 146 both ways, 40000 (17 a warp) 118 unstaged.
+constexpr uint64_t kSpreadWarps = 16, kSingleTabQueries = 20;
+
+struct SingleShape {
+  void (*kernel)(SingleArgs);
+  int grid;
+  size_t smem;
+};
+static SingleShape single_shape(SingleArgs& a, int sm_count, uint32_t share_pct) {
+  uint64_t sms = (uint64_t)sm_count * share_pct / 100;
+  if (sms < 1) sms = 1;
+  const uint64_t per = (a.count + sms * kSpreadWarps - 1) / (sms * kSpreadWarps);
+  a.warp_queries = per < 1 ? 1 : per > 32 ? 32 : (uint32_t)per;
+  const uint64_t need = (a.count + a.warp_queries - 1) / a.warp_queries;  // warps with a query
+  const bool staged = per >= kSingleTabQueries;
+  SingleShape s;
+  s.kernel = staged ? single_kernel<true> : single_kernel<false>;
+  s.grid = (int)(need < sms ? (need ? need : 1) : sms);
+  s.smem = sizeof(SingleCta) + (staged ? kSingleTabBytes : 0);
+  cudaFuncSetAttribute(s.kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)s.smem);
+  return s;
 }
 
-__global__ void __launch_bounds__(kSingleThreads) single_warp_kernel(SingleArgs a) {
-  __shared__ uint32_t sbuf[kSingleThreads / 32][64];
-  const int lane = threadIdx.x & 31;
-  uint32_t* buf = sbuf[threadIdx.x >> 5];
-  uint32_t found = 0, maxp = 0;
-  for (;;) {
-    unsigned long long qi = 0;
-    if (lane == 0) qi = atomicAdd(&a.ctr[0], 1ull);
-    qi = __shfl_sync(kFull, qi, 0);
-    if (qi >= a.count) break;
-    const uint64_t n = a.n[qi];
-    uint32_t p = 0;
-    if (n >= 4 && !(n & 1)) {
-      const uint64_t half = n >> 1;
-      if (n == 4) p = 2;
-      else if (n < kSmallN) p = minp_plain(a, n, half < a.p_lim ? half : a.p_lim);
-      else p = minp_warp(a, n, buf);
-    }
-    if (lane == 0) {
-      a.p_out[qi] = p;
-      a.q_out[qi] = p ? n - p : 0;
-      if (p) {
-        ++found;
-        maxp = p > maxp ? p : maxp;
-      }
-    }
-  }
-  if (lane == 0) {
-    if (found) atomicAdd(&a.ctr[1], (unsigned long long)found);
-    if (maxp) atomicMax(&a.ctr[2], (unsigned long long)maxp);
-  }
-}
-
-// Batches below kLaneBatchMin queries take the warp-per-query kernel: they
-// fit the GPU's resident warps at once, so the per-query latency (about
-// two strong tests there, a dozen per lane in single_kernel) sets the time.
-cudaError_t launch_single(const SingleArgs& a, int grid, cudaStream_t s) {
-  if (a.count < kLaneBatchMin) single_warp_kernel<<<grid, kSingleThreads, 0, s>>>(a);
-  else single_kernel<<<grid, kSingleThreads, 0, s>>>(a);
+cudaError_t launch_single(const SingleArgs& args, int sm_count, uint32_t share_pct, cudaStream_t s) {
+  SingleArgs a = args;
+  const SingleShape sh = single_shape(a, sm_count, share_pct);
+  sh.kernel<<<sh.grid, kSingleThreads, sh.smem, s>>>(a);
   return cudaGetLastError();
 }
 
-void single_kernel_node(const SingleArgs& a, int grid, void** argv, cudaKernelNodeParams* kp) {
+void single_kernel_node(SingleArgs& a, int sm_count, void** argv, cudaKernelNodeParams* kp) {
+  const SingleShape sh = single_shape(a, sm_count, 100);
   argv[0] = (void*)&a;
   *kp = cudaKernelNodeParams{};
-  kp->func = a.count < kLaneBatchMin ? (void*)single_warp_kernel : (void*)single_kernel;
-  kp->gridDim = dim3((unsigned)grid);
+  kp->func = (void*)sh.kernel;
+  kp->gridDim = dim3((unsigned)sh.grid);
   kp->blockDim = dim3(kSingleThreads);
+  kp->sharedMemBytes = (unsigned)sh.smem;
   kp->kernelParams = argv;
 }
 
