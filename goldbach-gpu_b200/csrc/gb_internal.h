@@ -18,8 +18,9 @@ enum Counter : int {
   kCtrMaxP = 4,       // largest minimal p (atomicMax)
   kCtrQueue = 5,      // entries pushed to the Phase-2 queue
   kCtrQueueOvf = 6,   // set when the queue overflowed
-  kCtrWork2 = 7,      // second work counter (multi-stage pipelines)
-  kCtrCount = 8
+  kCtrPairs = 7,      // (prime, window) pairs of the large-prime pass
+  kCtrTest = 8,       // next run of the tested windows' primality tests
+  kCtrCount = 10      // (an even count: the arrays behind it stay 16-byte aligned)
 };
 
 // Phase-2 queue entry: an even n whose minimal p is beyond the window halo.
@@ -56,7 +57,8 @@ struct SearchParams {
 // lwords words each at word lbase of the mask buffer: bit t of class c <->
 // q = 6(g0 + t) + c, with g0 = floor((start - H - 1) / 6) the first chunk's
 // window base.  A bit is cleared when q is a multiple of a sieving prime
-// above the chunk sieve's bound (other than the prime itself).
+// above the chunk sieve's bound (other than the prime itself) -- or, for a
+// window whose survivors are tested one by one (nsieve 0), when q is not prime.
 struct WinDesc6 {
   uint64_t start;
   uint64_t count;
@@ -66,6 +68,8 @@ struct WinDesc6 {
   uint64_t lbase;    // first word of L1 (L5 follows at lbase + lwords)
   uint32_t lwords;   // words of each class mask
   uint32_t orig;     // index of the window in the caller's order
+  uint32_t ne;       // even n per chunk
+  uint32_t nsieve;   // primes[kWheelPrimeCount+1 .. nsieve) mark its chunks
 };
 
 // What the large-prime pass reads for every (prime, window) pair: the mask
@@ -158,12 +162,32 @@ struct WinLargeArgs {
   const uint2* a15;
   uint32_t k0, k1;
   uint32_t* lmask;
+  unsigned long long* pairs;  // the (prime, window) pairs visited are added here
 };
 cudaError_t launch_win_large(const WinLargeArgs& a, int grid, cudaStream_t s);
-// Adds the (prime, window) pairs the pass visits (primes from index k0 up to
-// isqrt(q_top) of each window) to *pairs.
-cudaError_t launch_win_pairs(const WinDesc6* win, uint32_t nwin, const uint32_t* primes, uint64_t nprimes,
-                             uint32_t k0, unsigned long long* pairs, cudaStream_t s);
+// Windows whose masks come from primality tests: the masks are filled with the
+// q without a prime factor up to a bound, and every q left is tested.
+constexpr uint32_t kTileWordsMax = 2048;  // mask words of a class per presieve tile
+constexpr int kTileLogs = 12;             // ceil(log2) of them, 0 .. 11
+struct WinTestArgs {
+  const WinDesc6* win;       // the tested windows
+  const uint64_t* tile_off;  // nwin + 1 prefix sums of their presieve tiles
+  const uint64_t* run_off;   // nwin + 1 prefix sums of their 32-word runs
+  uint32_t nwin;
+  uint64_t tiles, runs;
+  uint32_t tile_words;
+  uint32_t nsieve[kTileLogs];  // primes up to index nsieve[k] sieve a tile of at most 2^k words
+  uint32_t kcoop;              // ... those below kcoop warp-cooperatively
+  const uint32_t* primes;
+  const uint64_t* magic;
+  const uint2* a15;
+  const uint32_t* wheel6;
+  uint32_t* lmask;
+  unsigned long long* ctr;     // next run
+};
+cudaError_t launch_win_presieve(const WinTestArgs& a, int grid, cudaStream_t s);
+cudaError_t launch_win_test(const WinTestArgs& a, int grid, cudaStream_t s);
+constexpr int kPresieveCtasPerSm = 2, kWinTestCtasPerSm = 3;
 
 // kernels/big.cu: partitions of n beyond 2^64.  One batch of candidates
 // primes[k0 .. k0 + kcount): the filter appends the indices (from k0) whose

@@ -4,10 +4,11 @@
 // offsets in [1e15, 1e18]) in one batch.  The reference has no batch mode:
 // each window would be one `goldbach --start=A LIMIT` process with its own
 // segment loop (src/goldbach.cu:420-485).  GB_WINDOWS_PERSISTENT runs the
-// batch as one CUDA graph of three launches: the large-prime pass over
-// every window's class masks (kernels/windows.cu), range6_kernel in windows
-// mode over every (window, chunk) item from one device work counter, and the
-// device Phase 2.
+// batch as one CUDA graph: the wide windows' class masks come from the
+// large-prime pass, the narrower ones' from a short sieve and a primality test
+// of every q it leaves (kernels/windows.cu); then range6_kernel in windows
+// mode runs over every (window, chunk) item from one device work counter, and
+// the device Phase 2 over what it leaves.
 // GB_WINDOWS_PLAIN runs the same launches window by window (the per-window
 // launch pipeline, kept for comparison).
 #include <algorithm>
@@ -26,8 +27,47 @@ constexpr uint64_t kWinChunkSieveBound = 1ull << 20;
 // CTAs per SM of the large-prime pass (grid-stride over the primes: a fine
 // grid evens out primes that visit many windows and primes that visit few)
 constexpr uint64_t kLargeBlocksPerSM = 64;
-// Default break-even divisor of the Miller-Rabin split (see windows_impl).
-constexpr double kMrBelowDivisor = 2600.0;
+// Halo of the windows' chunks: a minimal p beyond it goes to the device Phase 2.
+// The largest minimal p known below 4e18 is 9781, and a 1024-n window's q-window is
+// mostly halo (32768: 11 numbers of halo to one of the window).
+constexpr uint32_t kWinHalo = 8192;
+// Chunks of the windows are cut so that a small batch still fills the GPU,
+// down to these widths; a tested window's chunks sieve no primes, so they can
+// be narrower.
+constexpr uint64_t kMinSievedChunk = 1ull << 15, kMinTestedChunk = 1ull << 13;
+
+// The path of a window, by what it costs (results do not depend on it).
+//   kPerN: its n one by one through the single-n kernel (about 1 ns per n);
+//   kTested: a short sieve and a primality test of every q left (about 16 ps
+//     per n near 1e18, and some 100 ns for the halo);
+//   kSieved: every sieving prime's first multiple (the large-prime pass: about
+//     0.8 ps per prime).
+// So the line between the last two lies at pi(sqrt(top)) / 20 n, pi(sqrt(top))
+// / mr_divisor where the caller sets it, and below kPerNMax n the first is
+// the cheapest.  mr_below = 1 sieves every window; another mr_below sends
+// narrower windows n by n and sieves the others.
+enum WinPath { kPerN, kTested, kSieved };
+constexpr double kTestDivisor = 20.0;
+constexpr uint64_t kPerNMax = 64;
+
+static WinPath window_path(const gb_window& w, const gb_windows_opts& o) {
+  if (o.mr_below) return w.count < o.mr_below && o.mr_below != 1 ? kPerN : kSieved;
+  const uint64_t last = w.start + 2 * (w.count - 1);
+  const double r = std::sqrt((double)last);
+  if (r <= (double)kWinChunkSieveBound) return kSieved;  // no prime needs the large-prime pass
+  const double div = o.mr_divisor ? (double)o.mr_divisor : kTestDivisor;
+  const double lim = 1.1 * r / std::log(r) / div;  // pi(r) < 1.1 r / ln r here
+  if ((double)w.count >= lim) return kSieved;
+  return w.count < kPerNMax ? kPerN : kTested;
+}
+
+// The largest power of two up to `most` that cuts `total` n into at least
+// `pieces` chunks, but at least `least`.
+static uint32_t chunk_for(uint64_t total, uint64_t pieces, uint64_t least, uint64_t most) {
+  uint64_t ne = most;
+  while (ne > least && total / ne < pieces) ne >>= 1;
+  return (uint32_t)ne;
+}
 
 // floor((A - H - 1) / 6) for A possibly below H (range.cu window_g0)
 static int64_t host_window_g0(uint64_t A, uint32_t H) {
@@ -48,7 +88,7 @@ static gb_status windows_sieve_impl(gb_ctx* c, Workspace& ws, Arena* arena, cons
   if (sum) std::memset(sum, 0, sizeof *sum);
   if (count == 0) return GB_OK;
   if (count > 0xffffffffull) return fail(ws, GB_EINVAL, "too many windows");
-  const uint32_t H = o.halo ? o.halo : 32768u;
+  const uint32_t H = o.halo ? o.halo : kWinHalo;
   if (H < 128 || H > (1u << 17) || (H & 63)) return fail(ws, GB_EINVAL, "halo must be a multiple of 64 in [128, 2^17]");
   uint32_t NE = o.chunk_evens ? o.chunk_evens : (1u << 20);
   if (NE < 8192 || NE > (1u << 20) || (NE & (NE - 1)))
@@ -74,19 +114,41 @@ static gb_status windows_sieve_impl(gb_ctx* c, Workspace& ws, Arena* arena, cons
   const uint64_t root = isqrt_u64(q_max);
   gb_status st = ensure_primes(c, ws, std::max<uint64_t>({p_lim, (uint64_t)H, root + 2, kWinChunkSieveBound}));
   if (st != GB_OK) return st;
-  const uint32_t nbw = range6_words(H, NE);
-  // descriptors, sorted by top q so that a prime visits a suffix of them
+  // descriptors: the sieved windows first, sorted by top q so that a prime
+  // visits a suffix of them, then the tested ones
   std::vector<uint32_t> order(count);
+  std::vector<char> tested(count);
+  uint64_t n_tested = 0;
+  for (size_t i = 0; i < count; ++i) {
+    tested[i] = window_path(w[i], o) == kTested;
+    if (tested[i]) n_tested += w[i].count;
+  }
   std::iota(order.begin(), order.end(), 0u);
   std::sort(order.begin(), order.end(), [&](uint32_t x, uint32_t y) {
+    if (tested[x] != tested[y]) return tested[x] < tested[y];
     return w[x].start + 2 * (w[x].count - 1) < w[y].start + 2 * (w[y].count - 1);
   });
+  const size_t nsw = count - std::count(tested.begin(), tested.end(), 1);  // sieved windows
+  // chunk widths of the two kinds
+  const uint64_t slots = 4ull * c->sm_count;
+  uint32_t ne_s = NE, ne_t = NE;
+  if (!o.chunk_evens) {
+    ne_s = chunk_for(total_n - n_tested, slots, std::min<uint64_t>(kMinSievedChunk, NE), NE);
+    ne_t = chunk_for(n_tested, slots, std::min<uint64_t>(kMinTestedChunk, NE), std::min<uint64_t>(1u << 17, NE));
+    NE = nsw == 0 ? ne_t : nsw == count ? ne_s : std::max(ne_s, ne_t);
+  }
+  const uint32_t nbw = range6_words(H, NE);
   std::vector<uint64_t> out_off(count + 1, 0);
   for (size_t i = 0; i < count; ++i) out_off[i + 1] = out_off[i] + w[i].count;
   std::vector<WinDesc6> desc(count);
   std::vector<WinLarge> wl(count);
   std::vector<uint64_t> chunk_off(count + 1, 0), chunk_one(2 * count, 0);
-  uint64_t lwords_total = 0;
+  std::vector<uint64_t> test_one(4 * (count - nsw), 0);  // plain mode: each tested window's own offsets
+  std::vector<uint64_t> tile_off(count - nsw + 1, 0), run_off(count - nsw + 1, 0);
+  uint64_t nsmall = 0;
+  if ((st = count_le(c, ws, std::min<uint64_t>(kWinChunkSieveBound, root), &nsmall)) != GB_OK) return st;
+  nsmall = std::max<uint64_t>(nsmall, kWheelPrimeCount + 1);
+  uint64_t lwords_total = 0, lwords_sieved = 0;
   for (size_t r = 0; r < count; ++r) {
     const uint32_t i = order[r];
     WinDesc6& d = desc[r];
@@ -96,15 +158,17 @@ static gb_status windows_sieve_impl(gb_ctx* c, Workspace& ws, Arena* arena, cons
     d.q_top = d.start + 2 * (d.count - 1);
     d.g0 = host_window_g0(d.start, H);
     d.orig = i;
-    const uint64_t chunks = (d.count + NE - 1) / NE;
+    d.ne = r < nsw ? ne_s : ne_t;
+    d.nsieve = r < nsw ? (uint32_t)nsmall : 0;
+    const uint64_t chunks = (d.count + d.ne - 1) / d.ne;
     // a chunk reads nwords + 1 mask words from its own base on (nwords as in
     // range6_kernel: the words its search can read for a real n); the mask
     // ends there, so the large-prime pass marks no bit nobody reads
     auto reach = [&](uint64_t ci) {  // mask words chunk ci reads, from the window base
-      const uint64_t cnt = std::min<uint64_t>(NE, d.count - ci * NE);
+      const uint64_t cnt = std::min<uint64_t>(d.ne, d.count - ci * d.ne);
       const uint64_t nbits = H / 6 + cnt / 3 + 96;
       const uint64_t nwords = std::min<uint64_t>(nbw, (nbits + 31) / 32 + 2);
-      const int64_t gc = host_window_g0(d.start + 2 * (uint64_t)NE * ci, H);
+      const int64_t gc = host_window_g0(d.start + 2 * (uint64_t)d.ne * ci, H);
       return ((uint64_t)(gc - d.g0) >> 5) + nwords + 2;
     };
     // the last full chunk or the (possibly short) last one reaches furthest
@@ -113,26 +177,48 @@ static gb_status windows_sieve_impl(gb_ctx* c, Workspace& ws, Arena* arena, cons
     d.lwords = (uint32_t)((lw + 3) & ~3ull);
     d.lbase = lwords_total;
     lwords_total += 2ull * d.lwords;
+    if (r < nsw) lwords_sieved = lwords_total;
     wl[r].gd = (double)d.g0;
     wl[r].gl = (uint32_t)(uint64_t)d.g0;
     wl[r].lbits = d.g0 >= (int64_t)(1ll << 30) ? d.lwords * 32 : 0xffffffffu;
     chunk_off[r + 1] = chunk_off[r] + chunks;
     chunk_one[2 * r + 1] = chunks;
   }
-  uint64_t ns = 0, kf = 0, nsmall = 0, nlarge = 0, kc = 0;
+  // presieve tiles and test runs of the tested windows
+  WinTestArgs ta{};
+  uint64_t tile_words = kTileWordsMax;
+  while (tile_words > 64 && (lwords_total - lwords_sieved) / 2 / tile_words < slots) tile_words >>= 1;
+  ta.tile_words = (uint32_t)tile_words;
+  for (size_t r = nsw; r < count; ++r) {
+    const uint64_t lw = desc[r].lwords;
+    tile_off[r - nsw + 1] = tile_off[r - nsw] + (lw + tile_words - 1) / tile_words;
+    run_off[r - nsw + 1] = run_off[r - nsw] + 2 * ((lw + 31) / 32);
+    test_one[4 * (r - nsw) + 1] = tile_off[r - nsw + 1] - tile_off[r - nsw];
+    test_one[4 * (r - nsw) + 3] = run_off[r - nsw + 1] - run_off[r - nsw];
+  }
+  for (int k = 0; k < kTileLogs; ++k) {
+    // a prime costs a tile about 12 instructions, a q left of the tile's 192
+    // numbers a word about 2400 for its base-2 test: the derivatives meet near
+    // ten primes' reach per number
+    const uint64_t bound = std::min<uint64_t>({root, 1920ull << k, kHostPrimeLimit / 2});
+    uint64_t n = 0;
+    if ((st = count_le(c, ws, bound, &n)) != GB_OK) return st;
+    ta.nsieve[k] = (uint32_t)std::max<uint64_t>(n, kWheelPrimeCount + 1);
+  }
+  uint64_t ns = 0, kf = 0, nlarge = 0, kc = 0, kct = 0;
   if ((st = count_le(c, ws, std::min<uint64_t>(H - 13, p_lim), &ns)) != GB_OK ||
       (st = count_le(c, ws, p_lim, &kf)) != GB_OK ||
-      (st = count_le(c, ws, std::min<uint64_t>(kWinChunkSieveBound, root), &nsmall)) != GB_OK ||
       (st = count_le(c, ws, root, &nlarge)) != GB_OK ||
-      (st = count_le(c, ws, (H / 6 + NE / 3) / 64, &kc)) != GB_OK)
+      (st = count_le(c, ws, (H / 6 + NE / 3) / 64, &kc)) != GB_OK ||
+      (st = count_le(c, ws, tile_words / 2, &kct)) != GB_OK)
     return st;
 
   Temps tmp(c, arena);
   void *d_desc, *d_wl, *d_coff, *d_cone, *d_lmask, *d_fail, *d_maxp, *d_psum, *d_minp = nullptr;
   if ((st = ws_buffer(c, ws, tmp, 0, count * sizeof(WinDesc6), &d_desc)) != GB_OK ||
       (st = ws_buffer(c, ws, tmp, 1, count * sizeof(WinLarge), &d_wl)) != GB_OK ||
-      (st = ws_buffer(c, ws, tmp, 2, (count + 1) * 8, &d_coff)) != GB_OK ||
-      (st = ws_buffer(c, ws, tmp, 3, 2 * count * 8, &d_cone)) != GB_OK ||
+      (st = ws_buffer(c, ws, tmp, 2, (count + 1 + 2 * tile_off.size()) * 8, &d_coff)) != GB_OK ||
+      (st = ws_buffer(c, ws, tmp, 3, (2 * count + test_one.size()) * 8, &d_cone)) != GB_OK ||
       (st = ws_buffer(c, ws, tmp, 4, lwords_total * 4, &d_lmask)) != GB_OK ||
       (st = ws_buffer(c, ws, tmp, 5, count * 4, &d_fail)) != GB_OK ||
       (st = ws_buffer(c, ws, tmp, 6, count * 8, &d_maxp)) != GB_OK ||
@@ -160,7 +246,7 @@ static gb_status windows_sieve_impl(gb_ctx* c, Workspace& ws, Arena* arena, cons
   a.threads = o.block_threads;
   a.nbw = nbw;
   a.magic = c->d_magic;
-  a.nsieve = (uint32_t)std::max<uint64_t>(nsmall, kWheelPrimeCount + 1);
+  a.nsieve = (uint32_t)nsmall;
   a.kcoop = (uint32_t)std::max<uint64_t>(std::min(kc, nsmall), kWheelPrimeCount + 1);
   a.wheel6 = c->d_wheel6;
   a.a15 = c->d_a15;
@@ -173,13 +259,28 @@ static gb_status windows_sieve_impl(gb_ctx* c, Workspace& ws, Arena* arena, cons
   la.win = (const WinDesc6*)d_desc;
   la.wl = (const WinLarge*)d_wl;
   la.w_lo = 0;
-  la.w_hi = (uint32_t)count;
+  la.w_hi = (uint32_t)nsw;
   la.primes = c->d_primes;
   la.magic = c->d_magic;
   la.a15 = c->d_a15;
-  la.k0 = (uint32_t)std::max<uint64_t>(nsmall, kWheelPrimeCount + 1);
+  la.k0 = (uint32_t)nsmall;
   la.k1 = (uint32_t)std::max<uint64_t>(nlarge, la.k0);
   la.lmask = (uint32_t*)d_lmask;
+  la.pairs = sp.ctr + kCtrPairs;
+  const size_t ntw = count - nsw;  // tested windows
+  ta.win = (const WinDesc6*)d_desc + nsw;
+  ta.tile_off = (const uint64_t*)d_coff + count + 1;
+  ta.run_off = ta.tile_off + ntw + 1;
+  ta.nwin = (uint32_t)ntw;
+  ta.tiles = tile_off[ntw];
+  ta.runs = run_off[ntw];
+  ta.kcoop = (uint32_t)std::max<uint64_t>(kct, kWheelPrimeCount + 1);
+  ta.primes = c->d_primes;
+  ta.magic = c->d_magic;
+  ta.a15 = c->d_a15;
+  ta.wheel6 = c->d_wheel6;
+  ta.lmask = (uint32_t*)d_lmask;
+  ta.ctr = sp.ctr + kCtrTest;
 
   const int sm = c->sm_count;
   int bps = range_max_blocks_per_sm(a);
@@ -197,6 +298,8 @@ static gb_status windows_sieve_impl(gb_ctx* c, Workspace& ws, Arena* arena, cons
   // (a few primes each, grid-stride) and free their slots as they finish,
   // where higher-priority work takes them; a capped grid left it with too
   // few warps per SM to hide its loads
+  const int g_pre = (int)std::max<uint64_t>(1, std::min<uint64_t>(ta.tiles, (uint64_t)sm * kPresieveCtasPerSm * share / 100));
+  const int g_test = (int)std::max<uint64_t>(1, std::min<uint64_t>((ta.runs + 7) / 8, (uint64_t)sm * kWinTestCtasPerSm * share / 100));
   const int gl = (int)std::max<uint64_t>(1, std::min<uint64_t>((np + 255) / 256, (uint64_t)sm * large_per_sm));
 
   cudaStream_t s = o.stream ? (cudaStream_t)o.stream : c->stream;
@@ -207,15 +310,18 @@ static gb_status windows_sieve_impl(gb_ctx* c, Workspace& ws, Arena* arena, cons
   chk(cudaMemcpyAsync(d_desc, desc.data(), count * sizeof(WinDesc6), cudaMemcpyHostToDevice, s));
   chk(cudaMemcpyAsync(d_wl, wl.data(), count * sizeof(WinLarge), cudaMemcpyHostToDevice, s));
   chk(cudaMemcpyAsync(d_coff, chunk_off.data(), (count + 1) * 8, cudaMemcpyHostToDevice, s));
+  chk(cudaMemcpyAsync((uint64_t*)d_coff + count + 1, tile_off.data(), tile_off.size() * 8, cudaMemcpyHostToDevice, s));
+  chk(cudaMemcpyAsync((uint64_t*)d_coff + count + 1 + tile_off.size(), run_off.data(), run_off.size() * 8,
+                      cudaMemcpyHostToDevice, s));
   chk(cudaMemcpyAsync(d_cone, chunk_one.data(), 2 * count * 8, cudaMemcpyHostToDevice, s));
+  const uint64_t* d_tone = (const uint64_t*)d_cone + 2 * count;
+  if (ntw) chk(cudaMemcpyAsync((void*)d_tone, test_one.data(), test_one.size() * 8, cudaMemcpyHostToDevice, s));
   chk(cudaMemsetAsync(d_fail, 0, count * 4, s));
   chk(cudaMemsetAsync(d_maxp, 0, count * 8, s));
   chk(cudaMemsetAsync(d_psum, 0, count * 8, s));
   if (d_minp) chk(cudaMemsetAsync(d_minp, 0, total_n * 4, s));
   chk(cudaMemsetAsync(sp.ctr, 0, kCtrCount * 8, s));
   chk(cudaMemsetAsync(sp.ctr + kCtrFirstFail, 0xff, 8, s));
-  chk(launch_win_pairs((const WinDesc6*)d_desc, (uint32_t)count, c->d_primes, c->nprimes, la.k0,
-                       sp.ctr + kCtrWork2, s));
   chk(cudaStreamSynchronize(s));  // host vectors above are pageable and local
   int launches = 0;
   float large_ms = 0, search_ms = 0;
@@ -233,13 +339,17 @@ static gb_status windows_sieve_impl(gb_ctx* c, Workspace& ws, Arena* arena, cons
       chk(graph ? cudaEventRecordWithFlags(ev, s, cudaEventRecordExternal) : cudaEventRecord(ev, s));
     };
     if (graph) chk(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
-    chk(cudaMemsetAsync(d_lmask, 0xff, lwords_total * 4, s));
+    // every launch is there in every batch, with a grid of one where it has no
+    // work: another topology would have the graph instantiated anew
+    chk(cudaMemsetAsync(d_lmask, 0xff, std::max<uint64_t>(lwords_sieved, 1) * 4, s));
     mark(ws.ek0);
-    if (la.k1 > la.k0) {
-      chk(launch_win_large(la, gl, s));
-      ++launches;
-    }
+    WinLargeArgs l = la;
+    if (!nsw) l.k1 = l.k0;
+    chk(launch_win_large(l, nsw ? gl : 1, s));
     mark(ws.ek1);
+    chk(launch_win_presieve(ta, g_pre, s));
+    chk(launch_win_test(ta, g_test, s));
+    launches += 3;
     const int grid = (int)std::max<uint64_t>(1, std::min<uint64_t>(grid_max, a.total_items));
     chk(launch_range(a, grid, s));
     mark(ws.ek2);
@@ -264,15 +374,29 @@ static gb_status windows_sieve_impl(gb_ctx* c, Workspace& ws, Arena* arena, cons
   } else {
     for (uint32_t r = 0; r < count && e == cudaSuccess; ++r) {
       const WinDesc6& d = desc[r];
-      chk(cudaMemsetAsync((uint32_t*)d_lmask + d.lbase, 0xff, 2ull * d.lwords * 4, s));
       chk(cudaMemsetAsync(sp.ctr + kCtrWork, 0, 8, s));
       chk(cudaMemsetAsync(sp.ctr + kCtrQueue, 0, 8, s));
-      WinLargeArgs l1 = la;
-      l1.w_lo = r;
-      l1.w_hi = r + 1;
-      if (l1.k1 > l1.k0 && d.q_top >= kWinChunkSieveBound * kWinChunkSieveBound) {
-        chk(launch_win_large(l1, gl, s));
-        ++launches;
+      if (r < nsw) {
+        chk(cudaMemsetAsync((uint32_t*)d_lmask + d.lbase, 0xff, 2ull * d.lwords * 4, s));
+        WinLargeArgs l1 = la;
+        l1.w_lo = r;
+        l1.w_hi = r + 1;
+        if (l1.k1 > l1.k0 && d.q_top >= kWinChunkSieveBound * kWinChunkSieveBound) {
+          chk(launch_win_large(l1, gl, s));
+          ++launches;
+        }
+      } else {
+        WinTestArgs t1 = ta;  // one window, with offsets of its own
+        t1.win = ta.win + (r - nsw);
+        t1.nwin = 1;
+        t1.tiles = tile_off[r - nsw + 1] - tile_off[r - nsw];
+        t1.runs = run_off[r - nsw + 1] - run_off[r - nsw];
+        t1.tile_off = (const uint64_t*)d_tone + 4 * (r - nsw);
+        t1.run_off = t1.tile_off + 2;
+        chk(cudaMemsetAsync(ta.ctr, 0, 8, s));
+        chk(launch_win_presieve(t1, (int)std::min<uint64_t>(t1.tiles, g_pre), s));
+        chk(launch_win_test(t1, (int)std::min<uint64_t>((t1.runs + 7) / 8, g_test), s));
+        launches += 2;
       }
       RangeArgs a1 = a;
       a1.win = (const WinDesc6*)d_desc + r;
@@ -317,8 +441,8 @@ static gb_status windows_sieve_impl(gb_ctx* c, Workspace& ws, Arena* arena, cons
     sum->failures = ctr[kCtrFailures];
     sum->kernel_launches = launches;
     sum->device_ms = ms;
-    sum->sieved_windows = count;
-    sum->large_pairs = ctr[kCtrWork2];
+    sum->sieved_windows = nsw;
+    sum->large_pairs = ctr[kCtrPairs];
     sum->large_ms = large_ms;
     sum->search_ms = search_ms;
   }
@@ -407,12 +531,9 @@ static gb_status windows_mr_impl(gb_ctx* c, Workspace& ws, Arena* arena, const g
   return GB_OK;
 }
 
-// Splits the batch, trading the sieve bound against Miller-Rabin: windows
-// narrower than the sieve's break-even take the Miller-Rabin path (the
-// sieve's large-prime pass costs about 1.5 ps of GPU time per sieving prime
-// per window, the single-n path about 3 ns per n, so the break-even width
-// is about pi(sqrt(top)) / 2000 even n; 2600 measured best on 4096 windows
-// in [1e15, 1e18]).  Results do not depend on the split.
+// Splits the batch by path (window_path): the windows taken n by n run through
+// the single-n kernel, the others through the sieve pipeline.  Results do not
+// depend on the split.
 gb_status windows_impl(gb_ctx* c, Workspace& ws, Arena* arena, const gb_window* w, size_t count,
                        const gb_windows_opts* opts, gb_window_result* res, uint32_t* min_p_concat,
                        gb_windows_summary* sum) {
@@ -427,13 +548,7 @@ gb_status windows_impl(gb_ctx* c, Workspace& ws, Arena* arena, const gb_window* 
     const uint64_t last = w[i].start + 2 * (w[i].count - 1);
     if (w[i].start < 4 || (w[i].start & 1) || w[i].count == 0 || last < w[i].start)
       return windows_sieve_impl(c, ws, arena, w, count, opts, res, min_p_concat, sum);  // reports it
-    uint64_t lim = o.mr_below;
-    if (!lim) {
-      const double r = std::sqrt((double)last);
-      const double div = o.mr_divisor ? (double)o.mr_divisor : kMrBelowDivisor;
-      lim = r > 1e4 ? (uint64_t)(1.1 * r / std::log(r) / div) : 0;
-    }
-    narrow[i] = w[i].count < lim;
+    narrow[i] = window_path(w[i], o) == kPerN;
     nn += narrow[i];
   }
   if (nn == 0) return windows_sieve_impl(c, ws, arena, w, count, opts, res, min_p_concat, sum);
@@ -492,16 +607,9 @@ gb_status windows_impl(gb_ctx* c, Workspace& ws, Arena* arena, const gb_window* 
 // Miller-Rabin path, of that path's (its n, p, q and a reduction record);
 // arena alignment included.  Used by serving to admit batches by memory.
 uint64_t windows_request_bytes(const gb_window& w, const gb_windows_opts& o) {
-  const uint64_t H = o.halo ? o.halo : 32768u;
-  const uint64_t last = w.start + 2 * (w.count - 1);
-  uint64_t lim = o.mr_below;
-  if (!lim) {
-    const double r = std::sqrt((double)last);
-    const double div = o.mr_divisor ? (double)o.mr_divisor : kMrBelowDivisor;
-    lim = r > 1e4 ? (uint64_t)(1.1 * r / std::log(r) / div) : 0;
-  }
-  const uint64_t fixed = sizeof(WinDesc6) + sizeof(WinLarge) + 24 + 4 + 16 + 16 + 4 * 256;
-  if (w.count < lim) return fixed + w.count * 24 + 64 + 4 * 256;
+  const uint64_t H = o.halo ? o.halo : kWinHalo;
+  const uint64_t fixed = sizeof(WinDesc6) + sizeof(WinLarge) + 88 + 4 + 16 + 16 + 4 * 256;
+  if (window_path(w, o) == kPerN) return fixed + w.count * 24 + 64 + 4 * 256;
   const uint64_t lwords = (w.count / 3 + H / 6 + 96) / 32 + 16;
   return fixed + 2 * lwords * 4;
 }
@@ -546,7 +654,7 @@ gb_status autotune_windows_impl(gb_ctx* c, Workspace& ws, const gb_window* w, si
     uint64_t n = 0;
     for (const gb_window& x : smp) n += x.count;
     double best = -1;
-    for (uint32_t div : {2600u, 1300u, 5200u})
+    for (uint32_t div : {20u, 14u, 28u})
       for (uint32_t chunk : {1u << 20, 1u << 19})
         for (uint32_t large : {64u, 16u})
           for (uint32_t threads : {512u, 256u}) {

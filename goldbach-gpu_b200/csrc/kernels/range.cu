@@ -42,17 +42,6 @@ __device__ __forceinline__ int64_t window_g0(uint64_t A, uint32_t H) {
   return -(int64_t)(((uint64_t)H + 1 - A + 5) / 6);
 }
 
-// last window w with off[w] <= item (off: nwin + 1 ascending prefix sums)
-__device__ __forceinline__ uint32_t find_item_window(const uint64_t* off, uint32_t nwin, uint64_t item) {
-  uint32_t lo = 0, hi = nwin;
-  while (hi - lo > 1) {
-    const uint32_t mid = (lo + hi) >> 1;
-    if (off[mid] <= item) lo = mid;
-    else hi = mid;
-  }
-  return lo;
-}
-
 // WIN: windows mode (a.win set) -- a template parameter so that the range
 // instantiation carries none of its state through the inlined sieve.
 template <bool MINP, int NT, bool WIN>
@@ -62,7 +51,7 @@ __global__ void __launch_bounds__(NT, 1024 / NT) range6_kernel(const __grid_cons
   // windows mode: the item's window and chunk, decoded by thread 0
   __shared__ uint64_t s_wA, s_wbase, s_wunit, s_wlbase;
   __shared__ int64_t s_wg0;
-  __shared__ uint32_t s_wcnt, s_wlwords;
+  __shared__ uint32_t s_wcnt, s_wlwords, s_wnsieve;
   const int tid = threadIdx.x;
   Ctx6& cx = g_cx6;
   uint32_t* pat6 = smem6_pat();
@@ -84,14 +73,15 @@ __global__ void __launch_bounds__(NT, 1024 / NT) range6_kernel(const __grid_cons
       if (WIN && s_item < a.total_items) {
         const uint32_t w = find_item_window(a.chunk_off, a.nwin, s_item);
         const WinDesc6 d = a.win[w];
-        const uint64_t j0 = (s_item - a.chunk_off[w]) * a.chunk_evens;
+        const uint64_t j0 = (s_item - a.chunk_off[w]) * d.ne;
         s_wA = d.start + 2 * j0;
-        s_wcnt = (uint32_t)(d.count - j0 < a.chunk_evens ? d.count - j0 : a.chunk_evens);
+        s_wcnt = (uint32_t)(d.count - j0 < d.ne ? d.count - j0 : d.ne);
         s_wbase = d.out_off + j0;
         s_wunit = d.orig;
         s_wg0 = d.g0;
         s_wlbase = d.lbase;
         s_wlwords = d.lwords;
+        s_wnsieve = d.nsieve;
       }
       cx.fb = 0;
       cx.maxp = 0;
@@ -169,7 +159,7 @@ __global__ void __launch_bounds__(NT, 1024 / NT) range6_kernel(const __grid_cons
     }
     // q <= n - 3: the chunk's last n bounds the sieve (A + 2 cnt could pass 2^64)
     sieve_window6<NT>(Q1, Q5, nwords, nbits, G0, A + 2ull * (cnt - 1), pat6, s.primes,
-                                 a.magic, a.a15, a.nsieve, a.kcoop, L1, L5, lsh);
+                                 a.magic, a.a15, WIN ? s_wnsieve : a.nsieve, a.kcoop, L1, L5, lsh);
     search_chunk6<MINP, NT>(s);
   }
 }

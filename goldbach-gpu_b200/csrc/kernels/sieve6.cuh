@@ -18,6 +18,17 @@
 
 namespace gb {
 
+// last window w with off[w] <= item (off: nwin + 1 ascending prefix sums)
+__device__ __forceinline__ uint32_t find_item_window(const uint64_t* off, uint32_t nwin, uint64_t item) {
+  uint32_t lo = 0, hi = nwin;
+  while (hi - lo > 1) {
+    const uint32_t mid = (lo + hi) >> 1;
+    if (off[mid] <= item) lo = mid;
+    else hi = mid;
+  }
+  return lo;
+}
+
 // First t >= 0 of class c (offset a_c, r = G0 mod p) whose q is >= p^2.
 __device__ __forceinline__ uint64_t first_mark6(int64_t G0, uint32_t p, uint32_t ac, uint32_t r,
                                                uint32_t c) {

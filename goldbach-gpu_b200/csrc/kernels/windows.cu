@@ -1,6 +1,6 @@
 // windows.cu -- batched verification of many independent windows of even n:
-// the large-prime pass, and the expansion of narrow windows for the
-// Miller-Rabin path.
+// the large-prime pass, the tested windows, and the expansion of narrow windows
+// for the single-n kernel.
 //
 // The reference verifies one contiguous range at a time with a host loop of
 // launches per segment (src/goldbach.cu:420-485).  Windows far out (starts
@@ -14,6 +14,8 @@
 //      visited) and clears p's multiples in each window's two class masks
 //      (mod-6 layout, bit t <-> q = 6(g0 + t) + c, c in {1, 5}) with global
 //      atomicAnd;
+//      (narrow windows have their masks made by primality tests instead,
+//      see below);
 //   2. range6_kernel in windows mode: every (window, chunk) item sieves its
 //      q-window in shared memory with the wheel and the primes up to the
 //      bound, ANDs in the window's masks, and runs the levelled search;
@@ -41,6 +43,7 @@
 #include "../gb_device.cuh"
 #include "../gb_internal.h"
 #include "gb/gb.h"
+#include "prp64.cuh"
 #include "sieve6.cuh"
 
 namespace gb {
@@ -149,9 +152,11 @@ __device__ __forceinline__ void large_pair(const WinLargeArgs& a, const WinLarge
 // against 95 ms on the 4096 seeded windows, with 21.7 of 32 lanes active.)
 __global__ void __launch_bounds__(kWinLargeThreads) win_large_kernel(const __grid_constant__ WinLargeArgs a) {
   const uint32_t stride = gridDim.x * kWinLargeThreads;
+  unsigned long long pairs = 0;
   for (uint32_t k = a.k0 + blockIdx.x * kWinLargeThreads + threadIdx.x; k < a.k1; k += stride) {
     const uint32_t p = __ldg(a.primes + k);
     const uint32_t lo = first_window(a, (uint64_t)p * p);
+    pairs += a.w_hi - lo;
     if (p >= 0x80000000u) {  // windows near 2^64 only: every pair exact
       for (uint32_t w = lo; w < a.w_hi; ++w) win_mark_exact(a, w, p, k);
       continue;
@@ -160,39 +165,161 @@ __global__ void __launch_bounds__(kWinLargeThreads) win_large_kernel(const __gri
 #pragma unroll 4
     for (uint32_t w = lo; w < a.w_hi; ++w) large_pair(a, a.wl[w], w, q, k);
   }
+  for (int o = 16; o; o >>= 1) pairs += __shfl_down_sync(0xffffffffu, pairs, o);
+  if ((threadIdx.x & 31) == 0 && pairs) atomicAdd(a.pairs, pairs);
 }
 
 cudaError_t launch_win_large(const WinLargeArgs& a, int grid, cudaStream_t s) {
-  if (a.k1 <= a.k0 || a.w_hi <= a.w_lo || grid < 1) return cudaSuccess;
   win_large_kernel<<<grid, kWinLargeThreads, 0, s>>>(a);
   return cudaGetLastError();
 }
 
-// (prime, window) pairs the large-prime pass visits: for each window the
-// primes in [k0, pi(isqrt(q_top))), summed into *pairs.
-__global__ void win_pairs_kernel(const WinDesc6* __restrict__ win, uint32_t nwin,
-                                 const uint32_t* __restrict__ primes, uint64_t nprimes, uint32_t k0,
-                                 unsigned long long* pairs) {
-  const uint32_t w = blockIdx.x * blockDim.x + threadIdx.x;
-  if (w < nwin) {
-    const uint64_t q = win[w].q_top;
-    uint64_t r = (uint64_t)sqrt((double)q);
-    while (r > 0 && (r > 0xffffffffull || r * r > q)) --r;
-    while (r < 0xffffffffull && (r + 1) * (r + 1) <= q) ++r;
-    uint64_t lo = 0, hi = nprimes;  // first index with primes[i] > r
-    while (lo < hi) {
-      const uint64_t mid = (lo + hi) >> 1;
-      if (primes[mid] <= r) lo = mid + 1;
-      else hi = mid;
+// ---------------------------------------------------------------------------
+// Tested windows.  A window of W even n costs the large-prime pass one pair per
+// sieving prime, however narrow it is: 5e7 pairs near 1e18 (about 40 us of the
+// GPU), of which nearly all miss.  Its 2W / ln(top) primes can be had for less
+// when it is narrow: sieve with the primes up to a few times its width, which
+// leaves about 1.7 times as many q as there are primes, and test those
+// (prp64.cuh).  The tests cost about 16 ps per even n near 1e18, so the line
+// between the two lies near 2e6 n there (gb_windows.cpp, kTestDivisor).
+// 4096 windows at offsets in [1e15, 1e18], widths log-uniform in [2^10, 2^24]:
+// 145 -> 86 ms in all, of which the presieve 3.3, the tests 13.7 ms; 61 windows
+// of at most 2^18 n 6.5 -> 1.9 ms.
+constexpr int kPresieveThreads = 512;
+
+// One tile of one window per step: both classes sieved in shared memory, the
+// bits past the window's last n cleared, and written to the window's masks.
+__global__ void __launch_bounds__(kPresieveThreads, kPresieveCtasPerSm)
+    win_presieve_kernel(const __grid_constant__ WinTestArgs a) {
+  extern __shared__ uint32_t sm_presieve[];
+  uint32_t* pat6 = sm_presieve;
+  uint32_t* Q1 = pat6 + kWheel6Words;
+  uint32_t* Q5 = Q1 + a.tile_words;
+  if (blockIdx.x >= a.tiles) return;
+  for (uint32_t i = threadIdx.x; i < kWheel6Words; i += kPresieveThreads) pat6[i] = a.wheel6[i];
+  __syncthreads();
+  for (uint64_t item = blockIdx.x; item < a.tiles; item += gridDim.x) {
+    const uint32_t w = find_item_window(a.tile_off, a.nwin, item);
+    const WinDesc6 d = a.win[w];
+    const uint32_t wo = (uint32_t)(item - a.tile_off[w]) * a.tile_words;
+    const uint32_t nw = min(a.tile_words, d.lwords - wo);
+    const int64_t G0 = d.g0 + 32 * (int64_t)wo;
+    sieve_window6<kPresieveThreads>(Q1, Q5, nw, 32 * nw, G0, d.q_top, pat6, a.primes, a.magic, a.a15,
+                                    a.nsieve[nw > 1 ? 32 - __clz(nw - 1) : 0], a.kcoop);
+    uint32_t* L = a.lmask + d.lbase + wo;
+    for (uint32_t i = threadIdx.x; i < 2 * nw; i += kPresieveThreads) {
+      const bool c5 = i >= nw;
+      const uint32_t t = c5 ? i - nw : i;
+      // bits left in this word with 6(G0 + t) + c <= q_top
+      const int64_t keep = (int64_t)((d.q_top - (c5 ? 5 : 1)) / 6) - G0 - 32 * (int64_t)t;
+      const uint32_t m = keep < 0 ? 0u : keep >= 31 ? 0xffffffffu : (2u << keep) - 1;
+      L[c5 ? d.lwords + t : t] = (c5 ? Q5 : Q1)[t] & m;
     }
-    if (lo > k0) atomicAdd(pairs, (unsigned long long)(lo - k0));
+    __syncthreads();
   }
 }
 
-cudaError_t launch_win_pairs(const WinDesc6* win, uint32_t nwin, const uint32_t* primes, uint64_t nprimes,
-                             uint32_t k0, unsigned long long* pairs, cudaStream_t s) {
-  if (!nwin) return cudaSuccess;
-  win_pairs_kernel<<<(nwin + 255) / 256, 256, 0, s>>>(win, nwin, primes, nprimes, k0, pairs);
+cudaError_t launch_win_presieve(const WinTestArgs& a, int grid, cudaStream_t s) {
+  const size_t smem = (kWheel6Words + 2 * (size_t)a.tile_words) * sizeof(uint32_t);
+  win_presieve_kernel<<<grid, kPresieveThreads, smem, s>>>(a);
+  return cudaGetLastError();
+}
+
+// The q that the masks hold, 32 at a time per warp: a lane takes a mask word
+// of a run and hands out its bits; whenever 32 q have gathered they take the
+// base-2 test, and whenever 32 have passed it, the Lucas test; the bits of
+// those that fail are cleared.  Both lists carry over from run to run, so the
+// tests run with all lanes at work.  A word is read, and its bits cleared, by
+// one warp only.  Bound: the multiplier (prp64.cuh).
+constexpr int kWinTestThreads = 256;
+struct WinTestWarp {
+  uint64_t cq[64], cat[64];  // to test: q and its bit in the masks
+  uint64_t pq[64], pat[64];  // passed base 2
+};
+
+__global__ void __launch_bounds__(kWinTestThreads, kWinTestCtasPerSm)
+    win_test_kernel(const __grid_constant__ WinTestArgs a) {
+  constexpr uint32_t kAll = 0xffffffffu;
+  __shared__ WinTestWarp s_warp[kWinTestThreads / 32];
+  WinTestWarp& s = s_warp[threadIdx.x >> 5];
+  const int lane = threadIdx.x & 31;
+  const uint32_t below = (1u << lane) - 1;
+  // runs per fetch: enough to spread the runs over the warps eight times
+  const uint64_t warps = (uint64_t)gridDim.x * (kWinTestThreads / 32);
+  const uint64_t step = a.runs / (8 * warps) + 1;
+  uint64_t run = 0, run_end = 0;
+  uint32_t w = 0, word = 0, nc = 0, np = 0;
+  uint64_t q0 = 0, at0 = 0;  // the q and the place of the word's bit 0
+  bool done = false;
+  for (;;) {
+    while (nc < 32 && !done) {
+      if (!__any_sync(kAll, word != 0)) {  // the next run
+        if (run == run_end) {
+          unsigned long long r = 0;
+          if (lane == 0) r = atomicAdd(a.ctr, (unsigned long long)step);
+          run = __shfl_sync(kAll, r, 0);
+          if (run >= a.runs) {
+            done = true;
+            break;
+          }
+          run_end = run + step < a.runs ? run + step : a.runs;
+          w = find_item_window(a.run_off, a.nwin, run);
+        }
+        while (a.run_off[w + 1] <= run) ++w;
+        const WinDesc6& d = a.win[w];
+        const uint32_t lwords = d.lwords, runs = (lwords + 31) / 32;
+        const uint32_t r = (uint32_t)(run - a.run_off[w]);
+        const uint32_t c5 = r >= runs;
+        const uint32_t t = 32 * (c5 ? r - runs : r) + lane;
+        const uint64_t at = d.lbase + (c5 ? lwords : 0) + t;
+        word = t < lwords ? a.lmask[at] : 0;
+        q0 = 6 * ((uint64_t)d.g0 + 32ull * t) + (c5 ? 5 : 1);
+        at0 = 32 * at;
+        ++run;
+        continue;
+      }
+      const uint32_t b = __ballot_sync(kAll, word != 0);
+      if (word) {
+        const int j = __ffs(word) - 1;
+        word &= word - 1;
+        const uint32_t i = nc + __popc(b & below);
+        s.cq[i] = q0 + 6 * j;
+        s.cat[i] = at0 + j;
+      }
+      nc += __popc(b);
+    }
+    if (nc) {
+      const uint32_t m = min(nc, 32u);
+      nc -= m;
+      __syncwarp();
+      const bool act = lane < (int)m;
+      const uint64_t q = act ? s.cq[nc + lane] : 3, at = act ? s.cat[nc + lane] : 0;
+      const bool pass = sprp2_any(q, act) && act;
+      const uint32_t b = __ballot_sync(kAll, pass);
+      if (pass) {
+        const uint32_t i = np + __popc(b & below);
+        s.pq[i] = q;
+        s.pat[i] = at;
+      } else if (act) {
+        atomicAnd(&a.lmask[at >> 5], ~(1u << (at & 31)));
+      }
+      np += __popc(b);
+      __syncwarp();
+    }
+    if (np >= 32 || (done && nc == 0 && np)) {
+      const uint32_t m = min(np, 32u);
+      np -= m;
+      const bool act = lane < (int)m;
+      const uint64_t q = act ? s.pq[np + lane] : 3, at = act ? s.pat[np + lane] : 0;
+      if (!lucas_any(q, act) && act) atomicAnd(&a.lmask[at >> 5], ~(1u << (at & 31)));
+      __syncwarp();
+    }
+    if (done && nc == 0 && np == 0) break;
+  }
+}
+
+cudaError_t launch_win_test(const WinTestArgs& a, int grid, cudaStream_t s) {
+  win_test_kernel<<<grid, kWinTestThreads, 0, s>>>(a);
   return cudaGetLastError();
 }
 

@@ -308,11 +308,12 @@ typedef struct gb_windows_opts {
   int on_device;          /* windows / min_p / res are device pointers      */
   void* stream;
   uint64_t mr_below;      /* windows of fewer even n skip the sieve: their q
-                             are tested by Miller-Rabin (the single-n
+                             are tested for primality (the single-n
                              kernel).  0: automatic, where sieving would
-                             cost more (about pi(sqrt(top)) / mr_divisor
-                             n); 1: never                                  */
-  uint32_t mr_divisor;    /* the automatic split's divisor (0: 2600)        */
+                             cost more (fewer than about pi(sqrt(top)) /
+                             mr_divisor n: a short sieve, then a primality
+                             test of every q it leaves); 1: never           */
+  uint32_t mr_divisor;    /* the automatic split's divisor (0: 20)          */
   uint32_t large_ctas_per_sm; /* grid of the large-prime pass (0: 64)       */
   uint32_t block_threads; /* as gb_range_opts.block_threads (0: 512)        */
   uint32_t gpu_share_pct; /* the persistent kernels of the call (chunk
@@ -334,7 +335,7 @@ typedef struct gb_windows_summary {
   uint64_t failures;
   uint64_t kernel_launches;
   double device_ms;
-  uint64_t sieved_windows; /* windows on the sieve path (the rest: Miller-Rabin)  */
+  uint64_t sieved_windows; /* windows sieved by every prime (the rest: primality tests) */
   uint64_t large_pairs;    /* (prime, window) pairs of the large-prime pass       */
   double large_ms;         /* device time of the large-prime pass (persistent)    */
   double search_ms;        /* device time of the chunk sieve + search (persistent) */
@@ -348,7 +349,7 @@ gb_status gb_verify_windows(gb_ctx* ctx, const gb_window* w, size_t count,
 
 /* Autotuner for gb_verify_windows (no counterpart in the reference): times
  * the persistent pipeline on a sample of the batch (every k-th window, at
- * most 512 windows) for each mr_divisor (1300, 2600, 5200), chunk_evens
+ * most 512 windows) for each mr_divisor (14, 20, 28), chunk_evens
  * (2^19, 2^20), large-prime grid (16, 64 CTAs per SM) and block shape
  * (512, 256 threads), after one warm-up call, and writes the fastest into
  * *tuned (a copy of *base with those four set).  The choice is cached in the
