@@ -73,14 +73,16 @@ struct WinDesc6 {
 };
 
 // What the large-prime pass reads for every (prime, window) pair: the mask
-// base g0 as a double (rounded) and its low 32 bits, and the bits of each
-// class mask -- or ~0u for a window whose q may include a sieving prime
-// itself (g0 < 2^30), which takes the exact path.
+// base g0 as a double (rounded), -g0 mod 2^32, and the bits of each class mask
+// -- or kLargeExact for a window whose q may include a sieving prime itself
+// (g0 < 2^30) or whose masks hold 2^27 bits or more, which takes the exact path.
+constexpr uint32_t kLargeExact = 0xffffffffu;
 struct __align__(16) WinLarge {
   double gd;
-  uint32_t gl;
+  uint32_t ngl;
   uint32_t lbits;
 };
+constexpr uint64_t kLargeGroupBytes = 32ull << 20;
 
 // With per-n output (SearchParams::minp) the chunks hold at most this many
 // even n: a byte per n in shared memory keeps the entry position that

@@ -22,7 +22,9 @@
 namespace gb {
 // Primes up to this bound sieve each chunk's q-window in shared memory; the
 // larger ones go through the large-prime pass (kernels/windows.cu), whose
-// quotient estimate needs p > 2^17.
+// quotient estimate needs p > 2^20.  (2^22, 2^23 and 2^24 move marks from the
+// pass to the chunks and cost there what they save here: 4096 windows 53.7 ms
+// at 2^20, 56.4, 59.3 and 68 ms.)
 constexpr uint64_t kWinChunkSieveBound = 1ull << 20;
 // CTAs per SM of the large-prime pass (grid-stride over the primes: a fine
 // grid evens out primes that visit many windows and primes that visit few)
@@ -41,13 +43,14 @@ constexpr uint64_t kMinSievedChunk = 1ull << 15, kMinTestedChunk = 1ull << 13;
 //   kTested: a short sieve and a primality test of every q left (about 16 ps
 //     per n near 1e18, and some 100 ns for the halo);
 //   kSieved: every sieving prime's first multiple (the large-prime pass: about
-//     0.8 ps per prime).
-// So the line between the last two lies at pi(sqrt(top)) / 20 n, pi(sqrt(top))
-// / mr_divisor where the caller sets it, and below kPerNMax n the first is
+//     0.5 ps per prime, and 3 ps per n for its marks).
+// So the line between the last two lies at pi(sqrt(top)) / 30 n (4096 windows
+// in [1e15, 1e18]: 53.7 ms at 20, 52.8 at 40, 61 at 80), pi(sqrt(top)) /
+// mr_divisor where the caller sets it, and below kPerNMax n the first is
 // the cheapest.  mr_below = 1 sieves every window; another mr_below sends
 // narrower windows n by n and sieves the others.
 enum WinPath { kPerN, kTested, kSieved };
-constexpr double kTestDivisor = 20.0;
+constexpr double kTestDivisor = 30.0;
 constexpr uint64_t kPerNMax = 64;
 
 static WinPath window_path(const gb_window& w, const gb_windows_opts& o) {
@@ -179,8 +182,8 @@ static gb_status windows_sieve_impl(gb_ctx* c, Workspace& ws, Arena* arena, cons
     lwords_total += 2ull * d.lwords;
     if (r < nsw) lwords_sieved = lwords_total;
     wl[r].gd = (double)d.g0;
-    wl[r].gl = (uint32_t)(uint64_t)d.g0;
-    wl[r].lbits = d.g0 >= (int64_t)(1ll << 30) ? d.lwords * 32 : 0xffffffffu;
+    wl[r].ngl = 0u - (uint32_t)(uint64_t)d.g0;
+    wl[r].lbits = d.g0 >= (int64_t)(1ll << 30) && d.lwords < (1u << 27) / 32 ? d.lwords * 32 : kLargeExact;
     chunk_off[r + 1] = chunk_off[r] + chunks;
     chunk_one[2 * r + 1] = chunks;
   }
@@ -343,13 +346,21 @@ static gb_status windows_sieve_impl(gb_ctx* c, Workspace& ws, Arena* arena, cons
     // work: another topology would have the graph instantiated anew
     chk(cudaMemsetAsync(d_lmask, 0xff, std::max<uint64_t>(lwords_sieved, 1) * 4, s));
     mark(ws.ek0);
-    WinLargeArgs l = la;
-    if (!nsw) l.k1 = l.k0;
-    chk(launch_win_large(l, nsw ? gl : 1, s));
+    size_t r = 0;
+    do {  // groups of windows whose masks stay in L2 together
+      WinLargeArgs l = la;
+      l.w_lo = (uint32_t)r;
+      for (uint64_t bytes = 0; r < nsw && (r == l.w_lo || bytes + 8ull * desc[r].lwords <= kLargeGroupBytes); ++r)
+        bytes += 8ull * desc[r].lwords;
+      l.w_hi = (uint32_t)r;
+      if (!nsw) l.k1 = l.k0;
+      chk(launch_win_large(l, nsw ? gl : 1, s));
+      ++launches;
+    } while (r < nsw);
     mark(ws.ek1);
     chk(launch_win_presieve(ta, g_pre, s));
     chk(launch_win_test(ta, g_test, s));
-    launches += 3;
+    launches += 2;
     const int grid = (int)std::max<uint64_t>(1, std::min<uint64_t>(grid_max, a.total_items));
     chk(launch_range(a, grid, s));
     mark(ws.ek2);
@@ -654,7 +665,7 @@ gb_status autotune_windows_impl(gb_ctx* c, Workspace& ws, const gb_window* w, si
     uint64_t n = 0;
     for (const gb_window& x : smp) n += x.count;
     double best = -1;
-    for (uint32_t div : {20u, 14u, 28u})
+    for (uint32_t div : {30u, 20u, 45u})
       for (uint32_t chunk : {1u << 20, 1u << 19})
         for (uint32_t large : {64u, 16u})
           for (uint32_t threads : {512u, 256u}) {

@@ -81,10 +81,12 @@ __device__ __forceinline__ uint32_t isqrt64(uint64_t x) {
 }
 
 // r = G0 mod p from a double-precision quotient estimate, for 0 <= G0 <
-// 2^53 and p < 2^31; gs = G0 / 2^64 (exact), gl = G0 mod 2^32.  With
+// 2^53 and p < 2^31, or G0 < 2^61 and 2^14 < p < 2^31; gs = G0 / 2^64 (as a
+// double), gl = G0 mod 2^32.  With
 // magic = floor((2^64 - 1) / p), G0 magic / 2^64 is within 2 G0 / 2^64 of
-// G0 / p, and rounding magic to a double adds G0 / p * 2^-53 at most, so the
-// estimate is within 1/4 of G0 / p; adding 1.5 * 2^52 rounds it to
+// G0 / p (2^-2 at most), and rounding magic and G0 to doubles adds G0 / p *
+// 2^-52 at most (2^-5 for the wider range), so the
+// estimate is within 5/16 of G0 / p; adding 1.5 * 2^52 rounds it to
 // floor(G0 / p) or one more, held in the double's low bits.  G0 - p q then
 // lies in (-p, p), and 32-bit arithmetic finishes it.
 __device__ __forceinline__ uint32_t near_mod(double gs, uint32_t gl, uint32_t p, uint64_t magic) {
@@ -213,8 +215,9 @@ __device__ void sieve_window6(uint32_t* __restrict__ Q1, uint32_t* __restrict__ 
   const uint32_t plim = isqrt64(q_top);
   const uint32_t psafe = G0 >= 1 ? isqrt64(6 * (uint64_t)G0 - 4) : 0u;
   // r = G0 mod p by the quotient estimate where the window allows it
-  // (every prime used is <= plim)
-  const bool fastr = G0 >= 0 && G0 < (1ll << 53) && plim < 0x80000000u;
+  // (every prime used is <= plim); far windows allow it from p > 2^14 on
+  const bool farr = G0 >= 0 && G0 < (1ll << 61) && plim < 0x80000000u;
+  const bool fastr = farr && G0 < (1ll << 53);
   const double gs = (double)G0 * 0x1p-64;
   const uint32_t gl = (uint32_t)G0;
   {  // the next prime's table entries are loaded one iteration ahead
@@ -255,7 +258,7 @@ __device__ void sieve_window6(uint32_t* __restrict__ Q1, uint32_t* __restrict__ 
       if (k + NT < nsieve) { pn = __ldg(primes + k + NT); mn = __ldg(magic + k + NT); an = __ldg(a15 + k + NT); }
       if (p > plim) break;
       uint32_t j1, j5;  // offsets >= nbits mean no mark
-      window_marks6(fastr, p <= psafe, gs, gl, G0, p, mg, ac, nbits, j1, j5);
+      window_marks6(fastr || (farr && p > (1u << 14)), p <= psafe, gs, gl, G0, p, mg, ac, nbits, j1, j5);
       if (p >= nbits) {  // at most one multiple per class: no loop (no divergent exits)
         if (j1 < nbits) atomicAnd(&Q1[j1 >> 5], ~(1u << (j1 & 31)));
         if (j5 < nbits) atomicAnd(&Q5[j5 >> 5], ~(1u << (j5 & 31)));

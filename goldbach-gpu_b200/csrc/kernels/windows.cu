@@ -22,20 +22,23 @@
 //   3. the device Phase 2 (range.cu fallback_kernel) for minimal p beyond
 //      the halo.
 //
-// Cost of a pair.  With r = g0 mod p, the first marks of the two classes
-// are t_c = (a_c - r) mod p (a_1 = -1/6, a_5 = -5/6 mod p, from the a15
-// table).  r comes from a double-precision quotient estimate: g0 < 2^62 and
-// p > 2^20, so the fused multiply-add of the window's g0 (as a double) by
-// 1/p, added to 1.5 * 2^52, rounds to round(g0 / p) with an error far below
-// 1/2 -- floor(g0 / p) or one more -- and the low 32 bits of that double are
-// round(g0 / p) mod 2^32.  r = low32(g0) - p * round(g0 / p) (mod 2^32) then
-// lies in (-p, p), so 32-bit arithmetic finishes it (p < 2^31).  One 16-byte
-// record per window holds g0 as a double, its low 32 bits and the mask
-// length; the descriptor is read only on a hit.  The pass marks every
-// multiple of p in the window, those below p^2 included (they are
-// composite); only p itself must stay, and it can lie in a window only when
-// the window starts below 2^32, so those windows (g0 < 2^30) take an exact
-// path with the p^2 rule.
+// Cost of a pair.  The first mark of class c is t_c = (a_c - g0) mod p, a_1 =
+// -1/6 and a_5 = -5/6 (mod p).  One fused multiply-add of g0 (as a double) by
+// 1/p onto 1.5 * 2^52 rounds g0 / p to an integer m with an error below 1/4 (g0 <
+// 2^62, p > 2^20), held in the double's low bits, and d = m p - g0 (mod 2^32)
+// is within 3p/4 of zero.  The a_c taken next to zero are within p/6 of it (6
+// divides p - 1 or p + 1), so d + a_c lies in (-p, p), and t_c = min(d + a_c, d +
+// a_c + p) as unsigned 32-bit numbers when p < 2^31; for larger p a sum below
+// zero leaves t_c >= p/12 > 2^27, beyond every mask taken here (< 2^27 bits),
+// and d + a_c itself is compared.  So a pair costs one 16-byte load, one FMA,
+// one multiply-add, two additions, two add-and-minimum, a minimum and a
+// comparison.  (One residue mod p for both classes, the distance from 6 g0 to
+// p's next multiple, costs half of that but hits three times as often, and the
+// hits are what a wide window pays for: it measured 56 ms against 28.)  The pass marks every multiple of p in
+// the window, those below p^2 included (they are composite); only p itself
+// must stay, and it can lie in a window only when the window starts below 2^32,
+// so those windows (g0 < 2^30) take an exact path with the p^2 rule, and so do
+// masks of 2^27 bits or more.
 #include <cuda_runtime.h>
 
 #include <cstdint>
@@ -63,21 +66,8 @@ __device__ __noinline__ void win_mark_exact(const WinLargeArgs& a, uint32_t w, u
   for (uint64_t i = t5; i < lbits; i += p) atomicAnd(&L5[i >> 5], ~(1u << (i & 31)));
 }
 
-// Marks from the fast path's first marks t1, t5 (< p < 2^31) up to lbits.
-__device__ __noinline__ void win_mark_from(const WinLargeArgs& a, uint32_t w, uint32_t p, uint32_t t1,
-                                           uint32_t t5, uint32_t lbits) {
-  const uint64_t lbase = a.win[w].lbase;
-  const uint32_t lwords = a.win[w].lwords;
-  uint32_t* L1 = a.lmask + lbase;
-  uint32_t* L5 = L1 + lwords;
-  for (uint32_t i = t1; i < lbits; i += p) atomicAnd(&L1[i >> 5], ~(1u << (i & 31)));
-  for (uint32_t i = t5; i < lbits; i += p) atomicAnd(&L5[i >> 5], ~(1u << (i & 31)));
-}
-
-// First window w in [w_lo, w_hi) whose top reaches p^2 (windows sorted by
-// q_top).
-__device__ __forceinline__ uint32_t first_window(const WinLargeArgs& a, uint64_t pp) {
-  uint32_t lo = a.w_lo, hi = a.w_hi;
+// First window w in [lo, hi) whose top reaches p^2 (windows sorted by q_top).
+__device__ __forceinline__ uint32_t first_window(const WinLargeArgs& a, uint64_t pp, uint32_t lo, uint32_t hi) {
   while (lo < hi) {
     const uint32_t mid = (lo + hi) >> 1;
     if (a.win[mid].q_top < pp) lo = mid + 1;
@@ -86,87 +76,148 @@ __device__ __forceinline__ uint32_t first_window(const WinLargeArgs& a, uint64_t
   return lo;
 }
 
-// Per-prime constants of the fast path.
+// Marks p's multiples in window w from the first marks t1, t5 on, in ascending
+// order over both classes: most hits are one mark of either class, so a warp's
+// lanes make it together.
+__device__ __forceinline__ void win_mark_from(const WinLargeArgs& a, uint32_t w, uint32_t p, uint32_t t1,
+                                              uint32_t t5, uint32_t lbits) {
+  const WinDesc6& d = a.win[w];
+  uint32_t* L = a.lmask + d.lbase;
+  const uint32_t lwords = d.lwords;
+  for (;;) {
+    const bool c1 = t1 <= t5;
+    const uint32_t t = c1 ? t1 : t5;
+    if (t >= lbits) break;
+    atomicAnd(L + (t >> 5) + (c1 ? 0 : lwords), ~(1u << (t & 31)));
+    const uint32_t next = lbits - t <= p ? lbits : t + p;
+    if (c1) t1 = next;
+    else t5 = next;
+  }
+}
+
+// 1/p to a relative error near 2^-47: the single-precision reciprocal (2^-23
+// with the rounding of p to a float) and one Newton step in double precision.
+// The quotient estimate needs x / p * error < 1/8 with x / p < 2^44; a
+// correctly rounded division costs several times more and is paid once per
+// prime, which dominates when few windows share the pass.
+__device__ __forceinline__ double near_inv(uint32_t p) {
+  const double pd = (double)p;
+  const double r0 = (double)__frcp_rn((float)p);
+  return fma(r0, fma(-pd, r0, 1.0), r0);
+}
+
+// A warp takes 32 consecutive primes, one per lane, through the windows whose
+// top reaches their squares.  A lane keeps its hits in a column of its own in
+// shared memory (two predicated instructions a pair, no vote), and the warp
+// marks them row by row when a column is nearly full: marking each hit at once
+// runs the marking code for one or two lanes at nearly every pair of a wide
+// window.  944 windows of 6e6 n on average near 1e18, 3.0e10 pairs and 1.6e9
+// marks: 27.6 ms; marking at once 86 ms; at once over all windows in one launch
+// (marks missing L2) 57 ms.  What is left is issue: 72% of the slots, about 24
+// instructions a pair, 10 of them arithmetic.  The host launches the pass for groups of windows
+// whose masks stay in L2 (kLargeGroupBytes): a launch over all of them marks a
+// mask of 0.5 GB at random, and every mark reads and writes a sector of HBM.
+constexpr int kHitRows = 12;  // 48 KB a CTA, 4 CTAs per SM
+struct HitQueue {
+  uint4 e[kHitRows][32];  // t1, t5, window, prime index
+};
+
+// A lane's prime and what a pair needs of it.
 struct LargePrime {
-  uint32_t p, a1, dl;  // prime, -1/6 mod p, (a5 - a1) mod p
+  uint32_t k, p, a1, a1p, a5, a5p, lo;
   double inv;
 };
 
-// The class offsets: from the a15 table when many windows share the pass
-// (its cost is per pair), or from p alone when few do (the pass is then paid
-// per prime, and the table's 8 bytes per prime are two thirds of what it
-// streams): 6 divides p - 1 or p + 1, so -1/6 = (p - 1)/6 for p = 1 (mod 6)
-// and p - (p + 1)/6 for p = 5 (mod 6), and a5 - a1 = 4 a1 (mod p).
-// Measured: 1.227 -> 1.073 ms for one 2^26-n window near 1e19, but
-// 119.3 -> 121.7 ms for the 4096 seeded windows without the table.
-constexpr uint32_t kLargeTableWindows = 64;
+constexpr int kPrimesPerLane = 2;  // sharing each window record's load (1: 30.1, 2: 27.6 ms)
 
-__device__ __forceinline__ LargePrime large_prime(const WinLargeArgs& a, uint32_t k) {
-  LargePrime q;
-  q.p = __ldg(a.primes + k);
-  if (a.w_hi - a.w_lo >= kLargeTableWindows) {
-    const uint2 ac = __ldg(a.a15 + k);
-    q.a1 = ac.x;
-    q.dl = ac.y >= ac.x ? ac.y - ac.x : ac.y + q.p - ac.x;
-  } else {
-    const uint32_t q6 = __umulhi(q.p, 0xAAAAAAABu) >> 2;  // floor(p / 6)
-    q.a1 = q.p - 6 * q6 == 1 ? q6 : q.p - q6 - 1;
-    uint32_t d = q.a1 + q.a1;  // 4 a1 mod p in two doublings (p < 2^31)
-    d = min(d, d - q.p);
-    d = d + d;
-    q.dl = min(d, d - q.p);
-  }
-  // 1/p to a relative error near 2^-47: the single-precision reciprocal
-  // (2^-23 with the rounding of p to a float) and one Newton step in double
-  // precision.  The quotient estimate needs |g0/p| * error < 1/4 with
-  // g0/p < 2^42, i.e. 2^-44; a correctly rounded division costs several
-  // times more and is paid once per prime, which dominates when few
-  // windows share the pass.
-  const double pd = (double)q.p;
-  const double r0 = (double)__frcp_rn((float)q.p);
-  q.inv = fma(r0, fma(-pd, r0, 1.0), r0);
-  return q;
-}
-
-// One (prime, window) pair on the fast path (p < 2^31): the first marks of
-// both classes from the quotient estimate, and the marking when one falls
-// inside the mask (or the exact path for a window flagged for it).
-__device__ __forceinline__ void large_pair(const WinLargeArgs& a, const WinLarge& v, uint32_t w,
-                                           const LargePrime& q, uint32_t k) {
-  const double kRound = 6755399441055744.0;  // 1.5 * 2^52
-  const uint32_t qe = (uint32_t)__double_as_longlong(fma(v.gd, q.inv, kRound));
-  uint32_t r = v.gl - qe * q.p;  // g0 - p round(g0 / p), in (-p, p)
-  r = min(r, r + q.p);           // [0, p)
-  uint32_t t1 = q.a1 - r;
-  t1 = min(t1, t1 + q.p);
-  uint32_t t5 = t1 + q.dl;
-  t5 = min(t5, t5 - q.p);
-  if (min(t1, t5) < v.lbits) {  // a mark in the window, or the exact path
-    if (v.lbits == 0xffffffffu) win_mark_exact(a, w, q.p, k);
-    else win_mark_from(a, w, q.p, t1, t5, v.lbits);
-  }
-}
-
-// One thread per prime, grid-stride over the primes.  (Four consecutive
-// primes per thread sharing each window record measured slower: 146.5
-// against 95 ms on the 4096 seeded windows, with 21.7 of 32 lanes active.)
 __global__ void __launch_bounds__(kWinLargeThreads) win_large_kernel(const __grid_constant__ WinLargeArgs a) {
-  const uint32_t stride = gridDim.x * kWinLargeThreads;
-  unsigned long long pairs = 0;
-  for (uint32_t k = a.k0 + blockIdx.x * kWinLargeThreads + threadIdx.x; k < a.k1; k += stride) {
-    const uint32_t p = __ldg(a.primes + k);
-    const uint32_t lo = first_window(a, (uint64_t)p * p);
-    pairs += a.w_hi - lo;
-    if (p >= 0x80000000u) {  // windows near 2^64 only: every pair exact
-      for (uint32_t w = lo; w < a.w_hi; ++w) win_mark_exact(a, w, p, k);
-      continue;
+  constexpr uint32_t kAll = 0xffffffffu;
+  constexpr int P = kPrimesPerLane;
+  __shared__ HitQueue s_queue[kWinLargeThreads / 32];
+  const uint32_t lane = threadIdx.x & 31;
+  uint4* const q0 = &s_queue[threadIdx.x >> 5].e[0][lane];
+  uint4* q = q0;  // the lane's next row
+  auto flush = [&]() {
+    const int n = (int)(q - q0) / 32;
+    const int rows = (int)__reduce_max_sync(kAll, (uint32_t)n);
+    for (int i = 0; i < rows; ++i) {
+      if (i >= n) continue;
+      const uint4 e = q0[32 * i];
+      const uint32_t lbits = a.wl[e.z].lbits, p = __ldg(a.primes + e.w);
+      if (lbits == kLargeExact) win_mark_exact(a, e.z, p, e.w);
+      else win_mark_from(a, e.z, p, e.x, e.y, lbits);
     }
-    const LargePrime q = large_prime(a, k);
-#pragma unroll 4
-    for (uint32_t w = lo; w < a.w_hi; ++w) large_pair(a, a.wl[w], w, q, k);
+    q = q0;
+    __syncwarp();
+  };
+  auto pair = [&](const WinLarge& r, const LargePrime& c, uint32_t w, bool visits) {
+    const uint32_t m = (uint32_t)__double_as_longlong(fma(r.gd, c.inv, 6755399441055744.0));  // + 1.5 * 2^52
+    const uint32_t d = m * c.p + r.ngl;
+    const uint32_t t1 = min(d + c.a1, d + c.a1p), t5 = min(d + c.a5, d + c.a5p);
+    if (min(t1, t5) < r.lbits && visits) {
+      *q = make_uint4(t1, t5, w, c.k);
+      q += 32;
+    }
+  };
+  unsigned long long pairs = 0;
+  const uint64_t stride = (uint64_t)gridDim.x * kWinLargeThreads * P;
+  const uint64_t top0 = a.w_hi > a.w_lo ? a.win[a.w_lo].q_top : 0;
+  const uint64_t first = a.k0 + ((uint64_t)blockIdx.x * kWinLargeThreads + (threadIdx.x & ~31u)) * P;
+  for (uint64_t kb = first; kb < a.k1; kb += stride) {
+    LargePrime c[P];
+    uint32_t lo = a.w_hi, hi = 0;
+#pragma unroll
+    for (int j = 0; j < P; ++j) {
+      const uint64_t kk = kb + 32 * j + lane;
+      const bool in = kk < a.k1;
+      c[j].k = in ? (uint32_t)kk : a.k1 - 1;
+      const uint32_t p = c[j].p = __ldg(a.primes + c[j].k);
+      const uint64_t pp = (uint64_t)p * p;
+      c[j].lo = !in ? a.w_hi : pp <= top0 ? a.w_lo : first_window(a, pp, a.w_lo, a.w_hi);
+      pairs += a.w_hi - c[j].lo;
+      lo = min(lo, c[j].lo);
+      hi = max(hi, c[j].lo);
+      c[j].inv = near_inv(p);
+      // a_1, a_5 next to zero: (p - 1) / 6 and -(p + 5) / 6 for p = 1 (mod 6),
+      // -(p + 1) / 6 and (p - 5) / 6 for p = 5 (mod 6)
+      const uint32_t p6 = __umulhi(p, 0xAAAAAAABu) >> 2;  // floor(p / 6)
+      const bool one = p - 6 * p6 == 1;
+      c[j].a1 = one ? p6 : 0u - p6 - 1;
+      c[j].a5 = one ? 0u - p6 - 1 : p6;
+      const uint32_t padd = p < 0x80000000u ? p : 0;
+      c[j].a1p = c[j].a1 + padd;
+      c[j].a5p = c[j].a5 + padd;
+    }
+    const uint32_t wlo = __reduce_min_sync(kAll, lo), whi = __reduce_max_sync(kAll, hi);
+    if (wlo >= a.w_hi) break;  // no window reaches these primes' squares, nor later ones'
+    uint4* const near_full = q0 + 32 * (kHitRows - 4 * P);
+    uint32_t w = wlo;
+    for (; w < whi; ++w) {  // windows that only some of the lanes' primes visit
+      if (__any_sync(kAll, q > near_full)) flush();
+      const WinLarge r = a.wl[w];
+#pragma unroll
+      for (int j = 0; j < P; ++j) pair(r, c[j], w, w >= c[j].lo);
+    }
+#pragma unroll 1
+    for (; w + 4 <= a.w_hi; w += 4) {
+      if (__any_sync(kAll, q > near_full)) flush();
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const WinLarge r = a.wl[w + i];
+#pragma unroll
+        for (int j = 0; j < P; ++j) pair(r, c[j], w + i, true);
+      }
+    }
+    for (; w < a.w_hi; ++w) {
+      if (__any_sync(kAll, q > near_full)) flush();
+      const WinLarge r = a.wl[w];
+#pragma unroll
+      for (int j = 0; j < P; ++j) pair(r, c[j], w, true);
+    }
   }
-  for (int o = 16; o; o >>= 1) pairs += __shfl_down_sync(0xffffffffu, pairs, o);
-  if ((threadIdx.x & 31) == 0 && pairs) atomicAdd(a.pairs, pairs);
+  flush();
+  for (int o = 16; o; o >>= 1) pairs += __shfl_down_sync(kAll, pairs, o);
+  if (lane == 0 && pairs) atomicAdd(a.pairs, pairs);
 }
 
 cudaError_t launch_win_large(const WinLargeArgs& a, int grid, cudaStream_t s) {
@@ -177,11 +228,11 @@ cudaError_t launch_win_large(const WinLargeArgs& a, int grid, cudaStream_t s) {
 // ---------------------------------------------------------------------------
 // Tested windows.  A window of W even n costs the large-prime pass one pair per
 // sieving prime, however narrow it is: 5e7 pairs near 1e18 (about 40 us of the
-// GPU), of which nearly all miss.  Its 2W / ln(top) primes can be had for less
+// GPU at first, 25 now), of which nearly all miss.  Its 2W / ln(top) primes can be had for less
 // when it is narrow: sieve with the primes up to a few times its width, which
 // leaves about 1.7 times as many q as there are primes, and test those
 // (prp64.cuh).  The tests cost about 16 ps per even n near 1e18, so the line
-// between the two lies near 2e6 n there (gb_windows.cpp, kTestDivisor).
+// between the two lies near 1.5e6 n there (gb_windows.cpp, kTestDivisor).
 // 4096 windows at offsets in [1e15, 1e18], widths log-uniform in [2^10, 2^24]:
 // 145 -> 86 ms in all, of which the presieve 3.3, the tests 13.7 ms; 61 windows
 // of at most 2^18 n 6.5 -> 1.9 ms.

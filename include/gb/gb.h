@@ -313,7 +313,7 @@ typedef struct gb_windows_opts {
                              cost more (fewer than about pi(sqrt(top)) /
                              mr_divisor n: a short sieve, then a primality
                              test of every q it leaves); 1: never           */
-  uint32_t mr_divisor;    /* the automatic split's divisor (0: 20)          */
+  uint32_t mr_divisor;    /* the automatic split's divisor (0: 30)          */
   uint32_t large_ctas_per_sm; /* grid of the large-prime pass (0: 64)       */
   uint32_t block_threads; /* as gb_range_opts.block_threads (0: 512)        */
   uint32_t gpu_share_pct; /* the persistent kernels of the call (chunk
@@ -349,7 +349,7 @@ gb_status gb_verify_windows(gb_ctx* ctx, const gb_window* w, size_t count,
 
 /* Autotuner for gb_verify_windows (no counterpart in the reference): times
  * the persistent pipeline on a sample of the batch (every k-th window, at
- * most 512 windows) for each mr_divisor (14, 20, 28), chunk_evens
+ * most 512 windows) for each mr_divisor (20, 30, 45), chunk_evens
  * (2^19, 2^20), large-prime grid (16, 64 CTAs per SM) and block shape
  * (512, 256 threads), after one warm-up call, and writes the fastest into
  * *tuned (a copy of *base with those four set).  The choice is cached in the
