@@ -298,6 +298,26 @@ gb_status ensure_primes(gb_ctx* c, Workspace& w, uint64_t limit) {
   return GB_OK;
 }
 
+// Chunk width of a range of `count` even n when the caller leaves it open: the
+// power of two from 2^13 to `most` with the least time on the fullest SM.
+// Measured, two CTAs per SM: a chunk takes 232 us per 2^20 n near 1e12 (250 near
+// 1e9) and 24 us beside, 0.75 ns more for each of its sieving primes: 1e5 n and
+// 4.7 n a prime.  A CTA alone on its SM takes 0.77 of a pair's time.
+static uint32_t range_chunk(uint64_t count, uint64_t nprimes, int sm_count, uint32_t most) {
+  const double fixed = 1e5 + 4.7 * (double)nprimes;
+  double best = 0;
+  uint32_t ne = most;
+  for (uint32_t x = most; x >= 8192; x >>= 1) {
+    const uint64_t per_sm = ((count + x - 1) / x + sm_count - 1) / sm_count;
+    const double t = (x + fixed) * (0.5 * (double)per_sm + (per_sm & 1 ? 0.27 : 0.0));
+    if (x == most || t < best) {
+      best = t;
+      ne = x;
+    }
+  }
+  return ne;
+}
+
 // ---------------------------------------------------------------------------
 gb_status range_impl(gb_ctx* c, Workspace& w, Arena* arena, uint64_t start, uint64_t limit,
                      const gb_range_opts* opts, gb_range_result* res, const gb_range_out* out) {
@@ -319,11 +339,13 @@ gb_status range_impl(gb_ctx* c, Workspace& w, Arena* arena, uint64_t start, uint
   const uint32_t H = o.halo ? o.halo : 32768u;
   if (H < 128 || H > (1u << 17) || (H & 63))
     return fail(w, GB_EINVAL, "halo must be a multiple of 64 in [128, 2^17]");
+  const uint64_t root = isqrt_u64(limit);
   uint32_t NE = o.chunk_evens;
   if (!NE) {
-    // 2^20 n: two CTAs per SM (the two class bitsets hold 2^20 / 3 bits each)
-    NE = 1u << 20;
-    while (NE > 8192 && NE / 2 >= count) NE >>= 1;
+    // at most 2^20 n: two CTAs per SM (the two class bitsets hold 2^20 / 3 bits each)
+    const uint64_t shard = count / (o.shard_count ? o.shard_count : 1) + 1;
+    NE = range_chunk(std::min(shard, count), (uint64_t)(1.1 * (double)root / std::log((double)root + 2.0)),
+                     c->sm_count, out && out->min_p ? kMinpChunk : 1u << 20);
   }
   if (NE < 8192 || NE > (1u << 20) || (NE & (NE - 1)))
     return fail(w, GB_EINVAL, "chunk_evens must be a power of two in [2^13, 2^20]");
@@ -336,7 +358,6 @@ gb_status range_impl(gb_ctx* c, Workspace& w, Arena* arena, uint64_t start, uint
   const uint64_t my_segs = nseg > o.shard_index ? (nseg - o.shard_index + sc - 1) / sc : 0;
   const uint64_t cps = (o.seg_size + NE - 1) / NE;
   const uint64_t p_lim = std::max(o.p_small, o.phase2_limit);
-  const uint64_t root = isqrt_u64(limit);
   gb_status st = ensure_primes(c, w, std::max<uint64_t>({p_lim, (uint64_t)H, root + 2}));
   if (st != GB_OK) return st;
 
@@ -428,17 +449,30 @@ gb_status range_impl(gb_ctx* c, Workspace& w, Arena* arena, uint64_t start, uint
   if (sp.unit_failures) chk(cudaMemsetAsync(sp.unit_failures, 0, nseg * 4, s));
   if (e != cudaSuccess) return cuda_fail(w, e, "range setup");
   int launches = 0;
-  int bps = range_max_blocks_per_sm(a);
+  const bool masked = my_segs && range_masked_pays(c, start, std::min(count, my_segs * o.seg_size), root, my_segs);
+  if (masked) {
+    std::vector<RangePiece> segs;
+    for (uint64_t g = o.shard_index; g < nseg; g += sc)
+      segs.push_back(RangePiece{start + 2 * g * o.seg_size, std::min<uint64_t>(o.seg_size, count - g * o.seg_size),
+                                g * o.seg_size, (uint32_t)g});
+    if (!o.chunk_evens) a.chunk_evens = od.min_p ? kMinpChunk : 1u << 20;
+    chk(cudaEventRecord(w.ek0, s));
+    if ((st = range_masked(c, w, tmp, slot, segs, a, o.chunk_evens ? NE : 0, root, s, &launches)) != GB_OK) return st;
+    chk(cudaEventRecord(w.ek1, s));
+    chk(launch_fallback(sp, c->sm_count * 4, s));
+    ++launches;
+  }
+  int bps = masked ? 1 : range_max_blocks_per_sm(a);
   if (bps < 1) bps = 1;
   uint64_t grid = (uint64_t)c->sm_count * bps;
   if (a.total_items < grid) grid = std::max<uint64_t>(1, a.total_items);
-  if (a.total_items) {  // survivor lists of the levelled search
+  if (a.total_items && !masked) {  // survivor lists of the levelled search
     a.surv_cap = a.nbw;
     void* p = nullptr;
     if ((st = ws_scratch(c, w, (size_t)grid * 6 * a.surv_cap * sizeof(uint2), &p)) != GB_OK) return st;
     a.surv = (uint2*)p;
   }
-  if (a.total_items) {
+  if (a.total_items && !masked) {
     chk(cudaEventRecord(w.ek0, s));
     chk(launch_range(a, (int)grid, s));
     chk(cudaEventRecord(w.ek1, s));

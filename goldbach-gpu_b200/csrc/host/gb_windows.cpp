@@ -36,6 +36,10 @@ constexpr uint32_t kWinHalo = 8192;
 // Chunks of the windows are cut so that a small batch still fills the GPU,
 // down to these widths; a tested window's chunks sieve no primes, so they can
 // be narrower.
+constexpr uint64_t kMinMaskedChunk = 1ull << 16;
+// Ranges of fewer n than this per SM, or with larger sieving primes, are masked
+// (range_masked_pays).
+constexpr uint64_t kMaskedWidth = 1ull << 18, kMaskedRoot = 6000000;
 constexpr uint64_t kMinSievedChunk = 1ull << 15, kMinTestedChunk = 1ull << 13;
 
 // The path of a window, by what it costs (results do not depend on it).
@@ -49,7 +53,7 @@ constexpr uint64_t kMinSievedChunk = 1ull << 15, kMinTestedChunk = 1ull << 13;
 // mr_divisor where the caller sets it, and below kPerNMax n the first is
 // the cheapest.  mr_below = 1 sieves every window; another mr_below sends
 // narrower windows n by n and sieves the others.
-enum WinPath { kPerN, kTested, kSieved };
+enum WinPath { kPerN, kTested, kSieved };  // (ranges: range_masked below)
 constexpr double kTestDivisor = 30.0;
 constexpr uint64_t kPerNMax = 64;
 
@@ -76,6 +80,181 @@ static uint32_t chunk_for(uint64_t total, uint64_t pieces, uint64_t least, uint6
 static int64_t host_window_g0(uint64_t A, uint32_t H) {
   if (A >= (uint64_t)H + 1) return (int64_t)((A - H - 1) / 6);
   return -(int64_t)(((uint64_t)H + 1 - A + 5) / 6);
+}
+
+// ---------------------------------------------------------------------------
+// A range through the windows' kernels (range_impl): its segments, cut into
+// pieces, are the windows of range6_kernel's work items, and runs of adjacent
+// pieces share one mask, so the large-prime pass meets each prime once per run
+// instead of once per chunk.  Runs and batches hold at most kRangeMaskEvens n,
+// whose masks stay in L2.
+constexpr uint64_t kRangeMaskEvens = 1ull << 28;
+constexpr uint64_t kRangeMaskPieces = 1ull << 20;
+
+// Where it pays.  A chunk spends 0.75 ns on each of its sieving primes, whatever
+// its width (range_chunk); the pass spends 7 ps on a mark.  So it pays for
+// ranges that must be cut into narrow chunks to fill the GPU, and for far
+// ones, where the chunk's primes outweigh its n.  Kernel time, chunks alone
+// against masks: 1e7 n near 1e12 108 -> 100 us, 2e5 n 107 -> 70 us, 1e8 n 216 ->
+// 277 us (not masked); 1e9 n near 1e13 1.42 -> 2.11 ms (not masked); 1e8 n near
+// 1e14 0.53 -> 0.35 ms, 4e7 n near 1e15 1.03 -> 0.27, 1e6 and 1e9 n near 1e17
+// 18.6 -> 0.16 and 67 -> 3.2 ms.  The range must start beyond every sieving
+// prime, and the pass's quotient estimates need p > g0 / 2^42 (masked_bound).
+bool range_masked_pays(const gb_ctx* c, uint64_t start, uint64_t count, uint64_t root, uint64_t pieces) {
+  if (start < (8ull << 30) || root < (1ull << 16) || pieces > kRangeMaskPieces) return false;
+  return count < kMaskedWidth * (uint64_t)c->sm_count || root >= kMaskedRoot;
+}
+
+// Largest prime the chunks sieve themselves: about the chunk's own width (a
+// prime above a third of it marks a class less than once), and enough for the
+// pass's quotient estimate of the primes beyond it.
+static uint64_t masked_bound(uint64_t top, uint32_t ne) {
+  return std::min<uint64_t>(kWinChunkSieveBound, std::max<uint64_t>({1ull << 14, (uint64_t)ne, (top / 6) >> 42}));
+}
+
+gb_status range_masked(gb_ctx* c, Workspace& ws, Temps& tmp, int slot, const std::vector<RangePiece>& segs,
+                       RangeArgs a, uint32_t ne, uint64_t root, cudaStream_t s, int* launches) {
+  const uint32_t H = a.s.halo;
+  // pieces and the runs of adjacent ones
+  struct Run {
+    size_t p0, p1;  // pieces
+    WinDesc6 mask;
+  };
+  std::vector<WinDesc6> desc;
+  std::vector<Run> runs;
+  uint64_t run_n = 0, total = 0, top = 0;
+  for (const RangePiece& g : segs)
+    for (uint64_t j = 0; j < g.count; j += kRangeMaskEvens) {
+      WinDesc6 d{};
+      d.start = g.start + 2 * j;
+      d.count = std::min(kRangeMaskEvens, g.count - j);
+      d.out_off = g.out_off + j;
+      d.q_top = d.start + 2 * (d.count - 1);
+      d.orig = g.unit;
+      const bool joins = !desc.empty() && desc.back().q_top + 2 == d.start && run_n + d.count <= kRangeMaskEvens;
+      if (!joins) {
+        runs.push_back(Run{desc.size(), desc.size(), WinDesc6{}});
+        run_n = 0;
+      }
+      run_n += d.count;
+      total += d.count;
+      top = std::max(top, d.q_top);
+      desc.push_back(d);
+      runs.back().p1 = desc.size();
+    }
+  if (!ne) ne = chunk_for(std::min(total, kRangeMaskEvens), 2ull * c->sm_count, kMinMaskedChunk, a.chunk_evens);
+  a.chunk_evens = ne;
+  a.nbw = range6_words(H, ne);
+  const uint64_t bound = masked_bound(top, ne);
+  uint64_t nsmall = 0, nlarge = 0, kc = 0;
+  gb_status st;
+  if ((st = count_le(c, ws, std::min(bound, root), &nsmall)) != GB_OK || (st = count_le(c, ws, root, &nlarge)) != GB_OK ||
+      (st = count_le(c, ws, (H / 6 + ne / 3) / 32, &kc)) != GB_OK)
+    return st;
+  nsmall = std::max<uint64_t>(nsmall, kWheelPrimeCount + 1);
+  a.kcoop = (uint32_t)std::max<uint64_t>(std::min(kc, nsmall), kWheelPrimeCount + 1);
+  // masks, batch by batch in the same buffer
+  struct Batch {
+    size_t r0, r1;
+    uint64_t words, items, off0;  // off0: first entry of its chunk offsets
+  };
+  std::vector<Batch> batches;
+  std::vector<WinDesc6> masks;
+  std::vector<WinLarge> wl;
+  std::vector<uint64_t> coff;
+  uint64_t batch_n = 0, max_words = 0;
+  for (size_t r = 0; r < runs.size(); ++r) {
+    Run& u = runs[r];
+    uint64_t n = 0;
+    for (size_t p = u.p0; p < u.p1; ++p) n += desc[p].count;
+    if (batches.empty() || batch_n + n > kRangeMaskEvens) {
+      batches.push_back(Batch{r, r, 0, 0, coff.size()});
+      coff.push_back(0);
+      batch_n = 0;
+    }
+    Batch& b = batches.back();
+    batch_n += n;
+    b.r1 = r + 1;
+    const int64_t g0 = host_window_g0(desc[u.p0].start, H);
+    uint64_t lw = 0;
+    for (size_t p = u.p0; p < u.p1; ++p) {
+      WinDesc6& d = desc[p];
+      d.g0 = g0;
+      d.lbase = b.words;
+      d.ne = ne;
+      d.nsieve = (uint32_t)nsmall;
+      const uint64_t chunks = (d.count + ne - 1) / ne;
+      // the mask words the last two chunks read, from the mask's base on (as in
+      // windows_sieve_impl)
+      for (uint64_t ci = chunks >= 2 ? chunks - 2 : 0; ci < chunks; ++ci) {
+        const uint64_t cnt = std::min<uint64_t>(ne, d.count - ci * ne);
+        const uint64_t nwords = std::min<uint64_t>(a.nbw, (H / 6 + cnt / 3 + 96 + 31) / 32 + 2);
+        const int64_t gc = host_window_g0(d.start + 2 * (uint64_t)ne * ci, H);
+        lw = std::max(lw, ((uint64_t)(gc - g0) >> 5) + nwords + 2);
+      }
+      b.items += chunks;
+      coff.push_back(b.items);
+    }
+    u.mask = desc[u.p0];
+    u.mask.lwords = (uint32_t)((lw + 3) & ~3ull);
+    u.mask.q_top = desc[u.p1 - 1].q_top;
+    for (size_t p = u.p0; p < u.p1; ++p) desc[p].lwords = u.mask.lwords;
+    b.words += 2ull * u.mask.lwords;
+    max_words = std::max(max_words, b.words);
+    masks.push_back(u.mask);
+    wl.push_back(WinLarge{(double)g0, 0u - (uint32_t)(uint64_t)g0, u.mask.lwords * 32});
+  }
+  // one upload: descriptors, masks, records, chunk offsets
+  const size_t o_mask = desc.size() * sizeof(WinDesc6), o_wl = (o_mask + masks.size() * sizeof(WinDesc6) + 15) & ~size_t(15);
+  const size_t o_off = o_wl + wl.size() * sizeof(WinLarge), bytes = o_off + coff.size() * 8;
+  std::vector<char> up(bytes);
+  std::memcpy(up.data(), desc.data(), desc.size() * sizeof(WinDesc6));
+  std::memcpy(up.data() + o_mask, masks.data(), masks.size() * sizeof(WinDesc6));
+  std::memcpy(up.data() + o_wl, wl.data(), wl.size() * sizeof(WinLarge));
+  std::memcpy(up.data() + o_off, coff.data(), coff.size() * 8);
+  void *d_up, *d_mask;
+  if ((st = ws_buffer(c, ws, tmp, slot, bytes, &d_up)) != GB_OK ||
+      (st = ws_buffer(c, ws, tmp, slot + 1, max_words * 4, &d_mask)) != GB_OK)
+    return st;
+  int bps = range_max_blocks_per_sm(a);
+  if (bps < 1) bps = 1;
+  const uint64_t grid_max = (uint64_t)c->sm_count * bps;
+  a.surv_cap = a.nbw;
+  void* scratch = nullptr;
+  if ((st = ws_scratch(c, ws, (size_t)grid_max * 6 * a.surv_cap * sizeof(uint2), &scratch)) != GB_OK) return st;
+  a.surv = (uint2*)scratch;
+  a.lmask = (const uint32_t*)d_mask;
+  WinLargeArgs la{};
+  la.primes = c->d_primes;
+  la.magic = c->d_magic;
+  la.a15 = c->d_a15;
+  la.k0 = (uint32_t)nsmall;
+  la.k1 = (uint32_t)std::max<uint64_t>(nlarge, nsmall);
+  la.lmask = (uint32_t*)d_mask;
+  la.pairs = a.s.ctr + kCtrPairs;
+  const uint64_t np = la.k1 - la.k0;
+  const int gl = (int)std::max<uint64_t>(1, std::min<uint64_t>((np + 511) / 512, (uint64_t)c->sm_count * kLargeBlocksPerSM));
+  cudaError_t e = cudaMemcpyAsync(d_up, up.data(), bytes, cudaMemcpyHostToDevice, s);  // pageable: staged at the call
+  auto chk = [&](cudaError_t x) {
+    if (e == cudaSuccess && x != cudaSuccess) e = x;
+  };
+  const WinDesc6* dd = (const WinDesc6*)d_up;
+  for (const Batch& b : batches) {
+    chk(cudaMemsetAsync(d_mask, 0xff, b.words * 4, s));
+    if (&b != &batches[0]) chk(cudaMemsetAsync(a.s.ctr + kCtrWork, 0, 8, s));
+    la.win = (const WinDesc6*)((char*)d_up + o_mask) + b.r0;
+    la.wl = (const WinLarge*)((char*)d_up + o_wl) + b.r0;
+    la.w_lo = 0;
+    la.w_hi = (uint32_t)(b.r1 - b.r0);
+    if (np) chk(launch_win_large(la, gl, s));
+    a.win = dd + runs[b.r0].p0;
+    a.nwin = (uint32_t)(runs[b.r1 - 1].p1 - runs[b.r0].p0);
+    a.chunk_off = (const uint64_t*)((char*)d_up + o_off) + b.off0;
+    a.total_items = b.items;
+    chk(launch_range(a, (int)std::min(grid_max, b.items), s));
+    *launches += np ? 2 : 1;
+  }
+  return e == cudaSuccess ? GB_OK : cuda_fail(ws, e, "range (masked)");
 }
 
 // The sieve pipeline over windows w[0..count).

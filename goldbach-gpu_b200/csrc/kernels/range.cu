@@ -62,7 +62,7 @@ __global__ void __launch_bounds__(NT, 1024 / NT) range6_kernel(const __grid_cons
     cx.surv_cap = a.surv_cap;
   }
   __syncthreads();
-  load_tables6(s);
+  load_tables6<NT>(s);
   uint32_t* Q1 = smem6_q(0);
   uint32_t* Q5 = smem6_q(1);
   uint32_t* HIST = smem6_hist();
@@ -158,7 +158,7 @@ __global__ void __launch_bounds__(NT, 1024 / NT) range6_kernel(const __grid_cons
       lsh = (uint32_t)(d & 31);
     }
     // q <= n - 3: the chunk's last n bounds the sieve (A + 2 cnt could pass 2^64)
-    sieve_window6<NT>(Q1, Q5, nwords, nbits, G0, A + 2ull * (cnt - 1), pat6, s.primes,
+    sieve_window6<NT, WIN>(Q1, Q5, nwords, nbits, G0, A + 2ull * (cnt - 1), pat6, s.primes,
                                  a.magic, a.a15, WIN ? s_wnsieve : a.nsieve, a.kcoop, L1, L5, lsh);
     search_chunk6<MINP, NT>(s);
   }

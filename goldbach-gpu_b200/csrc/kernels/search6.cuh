@@ -551,53 +551,71 @@ __device__ __forceinline__ void search_chunk6(const SearchParams& s) {
 // Fills the CTA's lockstep tables (kLockSteps6 entries each at most) from
 // primes[2 .. nsearch):
 //   E0: every p >= 5;  E2: 3, then p = 1 (mod 6);  E4: 3, then p = 5 (mod 6);
-// and sets g_cx6.len / kend.  g_cx6.nbw must be set.  One warp; ends with
-// __syncthreads().
+// and sets g_cx6.len / kend.  g_cx6.nbw must be set.  The whole CTA, NT primes
+// at a time (one warp's 32 at a time left the CTA waiting 8 us for its loads);
+// ends with __syncthreads().
+template <int NT>
 __device__ __forceinline__ void load_tables6(const SearchParams& s) {
-  if (threadIdx.x < 32) {
-    uint32_t* E0 = smem6_etab(0);
-    uint32_t* E2 = smem6_etab(1);
-    uint32_t* E4 = smem6_etab(2);
-    const int lane = threadIdx.x;
-    const uint32_t ns = s.nsearch;
-    constexpr uint32_t L = kLockEntries6;
-    uint32_t n0 = 0, n2 = 1, n4 = 1, k0end = 2, k2end = 2, k4end = 2;
-    for (uint32_t kb = 2; kb < ns && (n0 < L || n2 < L || n4 < L); kb += 32) {
-      const uint32_t k = kb + lane;
-      const bool in = k < ns;
-      const uint32_t p = in ? s.primes[k] : 0;
-      const bool p1 = p - 6 * div6(p) == 1;
-      const uint32_t e = div6(p) | (k << kE6UBits);
-      const uint32_t lt = (1u << lane) - 1;
-      // E0: class bit = q in class 5 = (p = 1 mod 6)
-      if (in && k - 2 < L) E0[k - 2] = e | ((uint32_t)p1 << 31);
-      const uint32_t b2 = __ballot_sync(0xffffffffu, in && p1);
-      const uint32_t b4 = __ballot_sync(0xffffffffu, in && !p1);
-      const uint32_t i2 = n2 + __popc(b2 & lt), i4 = n4 + __popc(b4 & lt);
-      if (in && p1 && i2 < L) E2[i2] = e;                  // q in class 1
-      if (in && !p1 && i4 < L) E4[i4] = e | 0x80000000u;  // q in class 5
-      // prime index after the last stored entry of each table
-      const uint32_t last2 = __reduce_max_sync(0xffffffffu, in && p1 && i2 < L ? k + 1 : 0u);
-      const uint32_t last4 = __reduce_max_sync(0xffffffffu, in && !p1 && i4 < L ? k + 1 : 0u);
-      const uint32_t last0 = __reduce_max_sync(0xffffffffu, in && k - 2 < L ? k + 1 : 0u);
-      if (last2) k2end = last2;
-      if (last4) k4end = last4;
-      if (last0) k0end = last0;
-      n0 = min(L, n0 + __popc(__ballot_sync(0xffffffffu, in)));
-      n2 = min(L, n2 + __popc(b2));
-      n4 = min(L, n4 + __popc(b4));
-    }
+  constexpr uint32_t kAll = 0xffffffffu;
+  constexpr uint32_t L = kLockEntries6;
+  __shared__ uint32_t s_cnt[2][NT / 32];  // this round's primes = 1 and = 5 (mod 6), per warp
+  __shared__ uint32_t s_end[3];
+  uint32_t* E0 = smem6_etab(0);
+  uint32_t* E2 = smem6_etab(1);
+  uint32_t* E4 = smem6_etab(2);
+  const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const uint32_t ns = s.nsearch;
+  if (threadIdx.x < 3) s_end[threadIdx.x] = 2;
+  uint32_t n0 = 0, n2 = 1, n4 = 1;
+  for (uint32_t kb = 2; kb < ns && (n0 < L || n2 < L || n4 < L); kb += NT) {
+    const uint32_t k = kb + threadIdx.x;
+    const bool in = k < ns;
+    const uint32_t p = in ? s.primes[k] : 0;
+    const bool p1 = p - 6 * div6(p) == 1;
+    const uint32_t e = div6(p) | (k << kE6UBits);
+    const uint32_t b2 = __ballot_sync(kAll, in && p1), b4 = __ballot_sync(kAll, in && !p1);
     if (lane == 0) {
-      E2[0] = (1u << kE6UBits) | (1u << 31);  // rho 2: p = 3 (u = 0), q in class 5
-      E4[0] = 1u << kE6UBits;                 // rho 4: p = 3, q in class 1
-      g_cx6.len[0] = n0;
-      g_cx6.len[1] = n2;
-      g_cx6.len[2] = n4;
-      g_cx6.kend[0] = k0end;
-      g_cx6.kend[1] = k2end;
-      g_cx6.kend[2] = k4end;
+      s_cnt[0][warp] = __popc(b2);
+      s_cnt[1][warp] = __popc(b4);
     }
+    __syncthreads();
+    uint32_t i2 = n2, i4 = n4;  // this prime's entry, the round's totals after the loop
+    for (uint32_t w = 0; w < NT / 32; ++w) {
+      const uint32_t c2 = s_cnt[0][w], c4 = s_cnt[1][w];
+      i2 += w < warp ? c2 : 0;
+      i4 += w < warp ? c4 : 0;
+      n2 += c2;
+      n4 += c4;
+    }
+    const uint32_t lt = (1u << lane) - 1;
+    i2 += __popc(b2 & lt);
+    i4 += __popc(b4 & lt);
+    // E0: class bit = q in class 5 = (p = 1 mod 6); prime index after each
+    // table's last stored entry
+    if (in && k - 2 < L) {
+      E0[k - 2] = e | ((uint32_t)p1 << 31);
+      atomicMax(&s_end[0], k + 1);
+    }
+    if (in && p1 && i2 < L) {
+      E2[i2] = e;  // q in class 1
+      atomicMax(&s_end[1], k + 1);
+    }
+    if (in && !p1 && i4 < L) {
+      E4[i4] = e | 0x80000000u;  // q in class 5
+      atomicMax(&s_end[2], k + 1);
+    }
+    n0 = min(ns, kb + NT) - 2;
+    __syncthreads();
   }
+  if (threadIdx.x == 0) {
+    E2[0] = (1u << kE6UBits) | (1u << 31);  // rho 2: p = 3 (u = 0), q in class 5
+    E4[0] = 1u << kE6UBits;                 // rho 4: p = 3, q in class 1
+    g_cx6.len[0] = min(n0, L);
+    g_cx6.len[1] = min(n2, L);
+    g_cx6.len[2] = min(n4, L);
+  }
+  __syncthreads();
+  if (threadIdx.x < 3) g_cx6.kend[threadIdx.x] = s_end[threadIdx.x];
   __syncthreads();
 }
 

@@ -130,7 +130,7 @@ __device__ __forceinline__ void window_marks6(bool fastr, bool near, double gs, 
 // from bit lsh of word t of L1 / L5 (the multiples of the primes beyond
 // nsieve, cleared by the windows' large-prime pass); the mask must hold
 // nwords + 1 words from there.  Ends with __syncthreads().
-template <int NT>
+template <int NT, bool FAR>
 __device__ void sieve_window6(uint32_t* __restrict__ Q1, uint32_t* __restrict__ Q5,
                               uint32_t nwords, uint32_t nbits, int64_t G0, uint64_t q_top,
                               const uint32_t* __restrict__ pat6,
@@ -215,8 +215,9 @@ __device__ void sieve_window6(uint32_t* __restrict__ Q1, uint32_t* __restrict__ 
   const uint32_t plim = isqrt64(q_top);
   const uint32_t psafe = G0 >= 1 ? isqrt64(6 * (uint64_t)G0 - 4) : 0u;
   // r = G0 mod p by the quotient estimate where the window allows it
-  // (every prime used is <= plim); far windows allow it from p > 2^14 on
-  const bool farr = G0 >= 0 && G0 < (1ll << 61) && plim < 0x80000000u;
+  // (every prime used is <= plim); with FAR, windows beyond 2^53 take it from p
+  // > 2^14 on (one more comparison per prime: 0.3% of the range [4, 1e12])
+  const bool farr = G0 >= 0 && G0 < (1ll << (FAR ? 61 : 53)) && plim < 0x80000000u;
   const bool fastr = farr && G0 < (1ll << 53);
   const double gs = (double)G0 * 0x1p-64;
   const uint32_t gl = (uint32_t)G0;
@@ -258,7 +259,7 @@ __device__ void sieve_window6(uint32_t* __restrict__ Q1, uint32_t* __restrict__ 
       if (k + NT < nsieve) { pn = __ldg(primes + k + NT); mn = __ldg(magic + k + NT); an = __ldg(a15 + k + NT); }
       if (p > plim) break;
       uint32_t j1, j5;  // offsets >= nbits mean no mark
-      window_marks6(fastr || (farr && p > (1u << 14)), p <= psafe, gs, gl, G0, p, mg, ac, nbits, j1, j5);
+      window_marks6(fastr || (FAR && farr && p > (1u << 14)), p <= psafe, gs, gl, G0, p, mg, ac, nbits, j1, j5);
       if (p >= nbits) {  // at most one multiple per class: no loop (no divergent exits)
         if (j1 < nbits) atomicAnd(&Q1[j1 >> 5], ~(1u << (j1 & 31)));
         if (j5 < nbits) atomicAnd(&Q5[j5 >> 5], ~(1u << (j5 & 31)));

@@ -255,7 +255,7 @@ __global__ void __launch_bounds__(kPresieveThreads, kPresieveCtasPerSm)
     const uint32_t wo = (uint32_t)(item - a.tile_off[w]) * a.tile_words;
     const uint32_t nw = min(a.tile_words, d.lwords - wo);
     const int64_t G0 = d.g0 + 32 * (int64_t)wo;
-    sieve_window6<kPresieveThreads>(Q1, Q5, nw, 32 * nw, G0, d.q_top, pat6, a.primes, a.magic, a.a15,
+    sieve_window6<kPresieveThreads, true>(Q1, Q5, nw, 32 * nw, G0, d.q_top, pat6, a.primes, a.magic, a.a15,
                                     a.nsieve[nw > 1 ? 32 - __clz(nw - 1) : 0], a.kcoop);
     uint32_t* L = a.lmask + d.lbase + wo;
     for (uint32_t i = threadIdx.x; i < 2 * nw; i += kPresieveThreads) {
