@@ -193,27 +193,32 @@ constexpr int kPresieveCtasPerSm = 2, kWinTestCtasPerSm = 3;
 
 // kernels/big.cu: partitions of n beyond 2^64.  One batch of candidates
 // primes[k0 .. k0 + kcount): the filter appends the indices (from k0) whose
-// q = n - p no trial prime divides; phase 0 runs the base-2 strong test on
-// them and lists the passers; phase 1 runs the 11 other bases, one thread
-// per (passer, base), and marks the passers that fail one.
+// q = n - p no trial prime divides; the base-2 strong test runs on them, lists
+// the passers and keeps the smallest index; the 11 other bases run on one
+// passer and mark *fail if one rejects it.
 struct BigArgs {
-  const uint32_t* n;        // n in `limbs` little-endian 32-bit limbs (zero-padded)
-  uint32_t limbs;           // template width: 4, 8, 16, 32, 64 or 128
-  uint32_t nl;              // n's own limbs (<= limbs): R = 2^(32 nl)
+  const uint32_t* n;        // n in nl little-endian 32-bit limbs
+  uint32_t nl;              // n's limbs
+  uint32_t limbs;           // limbs of R: 2^(32 limbs) >= 4n
+  uint32_t rl;              // big_r_lanes(limbs): the lanes R's limbs fill
   const uint32_t* primes;
   uint64_t p_lim;           // candidates p <= p_lim
   const uint32_t* trial;    // trial primes r
   const uint32_t* nmod;     // n mod r
   uint32_t ntrial;
   uint32_t* surv;           // survivors (candidate index from k0)
-  uint32_t* nsurv;
   uint32_t* pass;           // base-2 passers (candidate index from k0)
-  uint32_t* fail;           // per passer: nonzero once a base fails
+  uint32_t* nsurv;
   uint32_t* npass;
+  uint32_t* minpass;        // smallest of them (~0: none)
+  uint32_t* fail;           // nonzero once a base rejects the passer under test
   unsigned long long* mr_tests;
 };
+uint32_t big_r_lanes(uint32_t limbs);
 cudaError_t launch_big_filter(const BigArgs& a, uint32_t k0, uint32_t kcount, cudaStream_t s);
-cudaError_t launch_big_mr(const BigArgs& a, uint32_t k0, int phase, int grid, cudaStream_t s);
+cudaError_t launch_big_base2(const BigArgs& a, uint32_t k0, int grid, cudaStream_t s);
+// i: the passer's index from k0, ~0u for the smallest
+cudaError_t launch_big_bases(const BigArgs& a, uint32_t k0, uint32_t i, cudaStream_t s);
 
 // kernels/probe.cu: kind 0 = 32-bit ALU ops/s, 1 = shared-memory atomicAnd/s,
 // 2 = 64-bit Montgomery products/s

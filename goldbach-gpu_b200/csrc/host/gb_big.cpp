@@ -6,7 +6,7 @@
 // candidates come from the resident prime table in batches of kBigBatch:
 // the filter kernel drops q = n - p with a factor below kBigTrialBound (from
 // n mod r, computed here once), the base-2 kernel tests the survivors, the
-// bases kernel runs the other 11 bases on the base-2 passers in parallel
+// bases kernel runs the other 11 bases on the smallest base-2 passer
 // (kernels/big.cu), and the smallest passer no base rejects, in the first
 // batch that has one, is the minimal p.
 #include <algorithm>
@@ -50,8 +50,6 @@ gb_status big_impl(gb_ctx* c, Workspace& w, const uint32_t* n_limbs, uint32_t nl
     if (res) *res = r;
     return GB_OK;
   }
-  uint32_t N = 4;
-  while (N < m) N <<= 1;
   gb_status st = ensure_primes(c, w, std::max<uint64_t>(p_limit, kBigTrialBound));
   if (st != GB_OK) return st;
   uint64_t np = 0;
@@ -66,62 +64,83 @@ gb_status big_impl(gb_ctx* c, Workspace& w, const uint32_t* n_limbs, uint32_t nl
     trial.push_back(p);
     nmod.push_back((uint32_t)rem);
   }
-  std::vector<uint32_t> npad(N, 0);
-  std::copy(n_limbs, n_limbs + m, npad.begin());
+  // one upload: n, the trial primes, n mod each
+  std::vector<uint32_t> up(n_limbs, n_limbs + m);
+  up.insert(up.end(), trial.begin(), trial.end());
+  up.insert(up.end(), nmod.begin(), nmod.end());
   Temps tmp(c, nullptr);
-  void *d_n, *d_trial, *d_nmod, *d_surv, *d_pass, *d_small;
-  if ((st = ws_buffer(c, w, tmp, 0, N * 4, &d_n)) != GB_OK ||
-      (st = ws_buffer(c, w, tmp, 1, trial.size() * 4, &d_trial)) != GB_OK ||
-      (st = ws_buffer(c, w, tmp, 2, nmod.size() * 4, &d_nmod)) != GB_OK ||
-      (st = ws_buffer(c, w, tmp, 3, kBigBatch * 4, &d_surv)) != GB_OK ||
-      (st = ws_buffer(c, w, tmp, 4, kBigBatch * 8, &d_pass)) != GB_OK ||
-      (st = ws_buffer(c, w, tmp, 5, 64, &d_small)) != GB_OK)
+  void *d_up, *d_surv, *d_pass, *d_small;
+  if ((st = ws_buffer(c, w, tmp, 0, up.size() * 4, &d_up)) != GB_OK ||
+      (st = ws_buffer(c, w, tmp, 1, kBigBatch * 4, &d_surv)) != GB_OK ||
+      (st = ws_buffer(c, w, tmp, 2, kBigBatch * 4, &d_pass)) != GB_OK ||
+      (st = ws_buffer(c, w, tmp, 3, 64, &d_small)) != GB_OK)
     return st;
+  // the device's figures of a batch, in this order behind the tests' count
+  struct Figures {
+    unsigned long long tests;
+    uint32_t nsurv, npass, fail, minpass;
+  };
+  Figures* fig = (Figures*)d_small;
   BigArgs a{};
-  a.n = (const uint32_t*)d_n;
-  a.limbs = N;
+  a.n = (const uint32_t*)d_up;
   a.nl = m;
+  uint32_t bits = 32 * m;
+  while (!((n_limbs[m - 1] >> ((bits - 1) & 31)) & 1u)) --bits;
+  a.limbs = (bits + 2 + 31) / 32;  // R >= 4n
+  a.rl = big_r_lanes(a.limbs);
   a.primes = c->d_primes;
   a.p_lim = p_limit;
-  a.trial = (const uint32_t*)d_trial;
-  a.nmod = (const uint32_t*)d_nmod;
+  a.trial = a.n + m;
+  a.nmod = a.trial + trial.size();
   a.ntrial = (uint32_t)trial.size();
   a.surv = (uint32_t*)d_surv;
   a.pass = (uint32_t*)d_pass;
-  a.fail = (uint32_t*)d_pass + kBigBatch;
-  a.nsurv = (uint32_t*)d_small;
-  a.npass = (uint32_t*)d_small + 1;
-  a.mr_tests = (unsigned long long*)((char*)d_small + 8);
+  a.nsurv = &fig->nsurv;
+  a.npass = &fig->npass;
+  a.minpass = &fig->minpass;
+  a.fail = &fig->fail;
+  a.mr_tests = &fig->tests;
   cudaStream_t s = c->stream;
   cudaError_t e = cudaSuccess;
   auto chk = [&](cudaError_t x) {
     if (e == cudaSuccess && x != cudaSuccess) e = x;
   };
-  chk(cudaMemcpyAsync(d_n, npad.data(), N * 4, cudaMemcpyHostToDevice, s));
-  chk(cudaMemcpyAsync(d_trial, trial.data(), trial.size() * 4, cudaMemcpyHostToDevice, s));
-  chk(cudaMemcpyAsync(d_nmod, nmod.data(), nmod.size() * 4, cudaMemcpyHostToDevice, s));
-  chk(cudaMemsetAsync(a.mr_tests, 0, 8, s));
+  chk(cudaMemcpyAsync(d_up, up.data(), up.size() * 4, cudaMemcpyHostToDevice, s));
+  chk(cudaMemsetAsync(d_small, 0, 64, s));
   chk(cudaEventRecord(w.ev0, s));
+  Figures* h = (Figures*)w.h_stage;  // pinned
   uint32_t best = 0xffffffffu;
   uint64_t k0 = 1;  // p = 2 leaves q = n - 2 even
   uint32_t pk = 0;
-  std::vector<uint32_t> pass(2 * kBigBatch);
+  auto read = [&]() {
+    chk(cudaMemcpyAsync(h, fig, sizeof(Figures), cudaMemcpyDeviceToHost, s));
+    chk(cudaStreamSynchronize(s));
+  };
   while (k0 < np && e == cudaSuccess) {
     const uint32_t kc = (uint32_t)std::min<uint64_t>(kBigBatch, np - k0);
-    chk(cudaMemsetAsync(a.nsurv, 0, 8, s));  // survivors and passers
+    chk(cudaMemsetAsync(&fig->nsurv, 0, 12, s));  // survivors, passers, fail
+    chk(cudaMemsetAsync(&fig->minpass, 0xff, 4, s));
     chk(launch_big_filter(a, (uint32_t)k0, kc, s));
-    chk(launch_big_mr(a, (uint32_t)k0, 0, c->sm_count * 4, s));
-    chk(launch_big_mr(a, (uint32_t)k0, 1, c->sm_count * 4, s));
-    uint32_t np_ = 0;
-    chk(cudaMemcpyAsync(&np_, a.npass, 4, cudaMemcpyDeviceToHost, s));
-    chk(cudaStreamSynchronize(s));
+    chk(launch_big_base2(a, (uint32_t)k0, c->sm_count * 4, s));
+    chk(launch_big_bases(a, (uint32_t)k0, 0xffffffffu, s));
+    read();
     r.candidates += kc;
-    if (e == cudaSuccess && np_) {
-      chk(cudaMemcpyAsync(pass.data(), a.pass, np_ * 4, cudaMemcpyDeviceToHost, s));
-      chk(cudaMemcpyAsync(pass.data() + kBigBatch, a.fail, np_ * 4, cudaMemcpyDeviceToHost, s));
-      chk(cudaStreamSynchronize(s));
-      for (uint32_t j = 0; j < np_; ++j)
-        if (!pass[kBigBatch + j] && pass[j] < best) best = pass[j];
+    if (e == cudaSuccess && h->npass) {
+      best = h->minpass;
+      if (h->fail) {  // a base rejected it: the other passers, in order
+        std::vector<uint32_t> pass(h->npass);
+        const uint32_t rejected = best;
+        chk(cudaMemcpy(pass.data(), d_pass, pass.size() * 4, cudaMemcpyDeviceToHost));
+        std::sort(pass.begin(), pass.end());
+        best = 0xffffffffu;
+        for (size_t j = 0; j < pass.size() && best == 0xffffffffu && e == cudaSuccess; ++j) {
+          if (pass[j] == rejected) continue;
+          chk(cudaMemsetAsync(&fig->fail, 0, 4, s));
+          chk(launch_big_bases(a, (uint32_t)k0, pass[j], s));
+          read();
+          if (!h->fail) best = pass[j];
+        }
+      }
     }
     if (best != 0xffffffffu) {
       chk(cudaMemcpy(&pk, c->d_primes + k0 + best, 4, cudaMemcpyDeviceToHost));
@@ -130,8 +149,7 @@ gb_status big_impl(gb_ctx* c, Workspace& w, const uint32_t* n_limbs, uint32_t nl
     k0 += kc;
   }
   chk(cudaEventRecord(w.ev1, s));
-  unsigned long long tests = 0;
-  chk(cudaMemcpyAsync(&tests, a.mr_tests, 8, cudaMemcpyDeviceToHost, s));
+  const unsigned long long tests = e == cudaSuccess ? h->tests : 0;
   chk(cudaStreamSynchronize(s));
   if (e != cudaSuccess) return cuda_fail(w, e, "big n");
   float ms = 0;

@@ -5,267 +5,460 @@
 // mpz_probab_prime_p(q, 25) accepts -- a valid partition, not guaranteed
 // the minimal one.  Here the candidates p (ascending, from the resident
 // prime table) are tested in batches (host/gb_big.cpp):
-//   1. big_filter_kernel: one thread per candidate drops q = n - p when a
+//   1. big_filter_kernel: one warp per candidate drops q = n - p when a
 //      trial prime r divides it, from n mod r (computed on the host once per
 //      n) and p mod r, and appends the survivors' indices;
-//   2. big_base2_kernel<N>: one thread per survivor runs the strong
-//      probable-prime test to base 2 and lists the passers (almost all of
-//      them primes);
-//   3. big_bases_kernel<N>: one thread per (passer, base) runs the 11 other
-//      bases 3, 5, ..., 37 -- with base 2 the base set of the reference's
-//      Miller-Rabin (src/goldbach.cu:333-360) -- in parallel, so a prime q
-//      costs two exponentiations of latency, not twelve.
+//   2. big_base2_kernel: one group of lanes per survivor runs the strong
+//      probable-prime test to base 2, lists the passers (almost all of them
+//      primes) and keeps the smallest;
+//   3. big_bases_kernel: one group per base runs the 11 other bases 3, 5, ...,
+//      37 -- with base 2 the base set of the reference's Miller-Rabin
+//      (src/goldbach.cu:333-360) -- on one passer.
 // The smallest passer no base rejects is the minimal p: every smaller
 // candidate was tested and failed.  The test is deterministic for
 // q < 3.3e24 (the 12 prime bases admit no strong pseudoprime below that) and
 // a probable-prime test beyond, like the reference's.
 //
-// The Montgomery product is the coarsely integrated operand-scanning form
-// (CIOS) on 32-bit limbs with 64-bit accumulators, R = 2^(32 nl) for n of
-// nl limbs; the arrays are sized by the template width N (a power of two
-// from 4 to 128, n up to 4096 bits) and the loops run over nl.  Operands
-// live in the thread's local memory for the wide sizes.
+// A batch is a few hundred tests of hundreds to thousands of dependent
+// products each, so the latency of one product is what bounds it, not the
+// multiplier.  A number is therefore spread over G lanes, K limbs of 32 bits
+// per lane (up to 32 limbs one a lane, G = 8, 16 or 32), and a product takes
+// one step per limb of y: every lane multiplies its limbs by it, lane 0's
+// lowest limb gives the reduction's m, and the limbs move down one place.
+// A step is about 70 clocks (two shuffles and two multiply-adds in a row),
+// whatever the width.  The carries stay in 64-bit accumulators until the end,
+// where one pass over the lanes and a carry look-ahead on two ballots settle
+// them; R = 2^(32 L) >= 4q keeps the residues below 2q without a
+// subtraction.  One n of 512 bits: 22.0 -> 1.3 ms (one thread per
+// test with its limbs in local memory took 10.9 ms for each of the two
+// strong-test kernels, 41,000 clocks a product; now 0.47 and 0.56 ms).
 #include <cuda_runtime.h>
 
 #include <cstdint>
+#include <type_traits>
 
 #include "../gb_internal.h"
 
 namespace gb {
 
-constexpr int kBigThreads = 128;
+constexpr uint32_t kAllLanes = 0xffffffffu;
+constexpr int kBigMaxLimbs = GB_BIG_MAX_LIMBS + 1;  // limbs of R
 
 // The 12 prime bases of the strong tests.
 __device__ __constant__ const uint32_t kBigBases[12] = {2, 3, 5, 7, 11, 13, 17, 19, 23, 29, 31, 37};
 
-__global__ void __launch_bounds__(256) big_filter_kernel(const __grid_constant__ BigArgs a, uint32_t k0,
-                                                         uint32_t kcount) {
-  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= kcount) return;
-  const uint32_t k = k0 + i;
-  const uint32_t p = a.primes[k];
-  bool keep = p <= a.p_lim;
-  for (uint32_t j = 0; keep && j < a.ntrial; ++j)
-    if (p % a.trial[j] == a.nmod[j]) keep = false;  // r divides q = n - p (q far above r)
-  if (keep) {
-    const uint32_t slot = atomicAdd(a.nsurv, 1u);
-    a.surv[slot] = i;
-  }
+constexpr int kFilterThreads = 256;
+__global__ void __launch_bounds__(kFilterThreads) big_filter_kernel(const __grid_constant__ BigArgs a, uint32_t k0,
+                                                                    uint32_t kcount) {
+  const uint32_t i = blockIdx.x * (kFilterThreads / 32) + (threadIdx.x >> 5);
+  if (i >= kcount) return;  // warp-uniform
+  const uint32_t p = a.primes[k0 + i];
+  bool drop = p > a.p_lim;
+  for (uint32_t j = threadIdx.x & 31; j < a.ntrial; j += 32)
+    drop |= p % a.trial[j] == a.nmod[j];  // r divides q = n - p (q far above r)
+  if (!__any_sync(kAllLanes, drop) && (threadIdx.x & 31) == 0) a.surv[atomicAdd(a.nsurv, 1u)] = i;
 }
 
-// r = x * y * R^-1 mod q (x, y < q; q odd; R = 2^(32 N)); r may be x or y
-// (it is written after the last read of both).  The inner loops unroll in
-// full for the register-resident sizes only.
-template <int N>
-__device__ void big_mont_mul(uint32_t* r, const uint32_t* x, const uint32_t* y, const uint32_t* q,
-                             uint32_t qinv, int nl) {
-  constexpr int U = N <= 16 ? N : 4;
-  uint32_t t[N + 2];
+// Numbers of G lanes with K limbs each; limb j of lane l is limb l K + j.
+template <int G, int K>
+struct Big {
+  typedef uint32_t Num[K];
+
+  static __device__ __forceinline__ int sub() { return threadIdx.x & (G - 1); }
+  static __device__ __forceinline__ uint32_t up(uint32_t v) {  // from the lane below (0 into lane 0)
+    const uint32_t r = __shfl_up_sync(kAllLanes, v, 1, G);
+    return sub() ? r : 0;
+  }
+  // The carry into this lane, from the lanes that generate one (g) and those
+  // that pass one on (p, not g): the carries of the sum of two numbers whose
+  // bits generate and propagate alike.  out: the carry out of the last lane.
+  static __device__ __forceinline__ uint32_t carry_in(bool g, bool p, bool& out) {
+    uint32_t gb = __ballot_sync(kAllLanes, g), pb = __ballot_sync(kAllLanes, p && !g);
+    if (G < 32) {
+      const int lead = (threadIdx.x & 31) & ~(G - 1);
+      gb = (gb >> lead) & ((1u << (G & 31)) - 1);
+      pb = (pb >> lead) & ((1u << (G & 31)) - 1);
+    }
+    const uint64_t s = (uint64_t)(gb | pb) + gb;
+    out = (s >> G) & 1;
+    return ((uint32_t)s ^ pb) >> sub() & 1;
+  }
+  // r = the number with the 64-bit limbs c (below R): c's high halves go to the
+  // next limb.
+  static __device__ __forceinline__ void settle(Num& r, uint64_t (&c)[K]) {
+    uint64_t carry = 0;
 #pragma unroll
-  for (int j = 0; j < N + 2; ++j) t[j] = 0;
-  for (int i = 0; i < nl; ++i) {
-    const uint32_t yi = y[i];
-    uint64_t c = 0;
-#pragma unroll U
-    for (int j = 0; j < nl; ++j) {
-      const uint64_t v = (uint64_t)x[j] * yi + t[j] + c;
-      t[j] = (uint32_t)v;
-      c = v >> 32;
+    for (int j = 0; j < K; ++j) {
+      c[j] += carry;  // (c stays far below 2^64: high halves of at most a few)
+      r[j] = (uint32_t)c[j];
+      carry = c[j] >> 32;
     }
-    uint64_t v = (uint64_t)t[nl] + c;
-    t[nl] = (uint32_t)v;
-    t[nl + 1] = (uint32_t)(v >> 32);
-    const uint32_t m = t[0] * qinv;
-    v = (uint64_t)m * q[0] + t[0];
-    c = v >> 32;
-#pragma unroll U
-    for (int j = 1; j < nl; ++j) {
-      v = (uint64_t)m * q[j] + t[j] + c;
-      t[j - 1] = (uint32_t)v;
-      c = v >> 32;
+    uint32_t in = up((uint32_t)carry);
+    bool ones = true;
+#pragma unroll
+    for (int j = 0; j < K; ++j) {
+      const uint64_t t = (uint64_t)r[j] + in;
+      r[j] = (uint32_t)t;
+      in = (uint32_t)(t >> 32);
+      ones &= r[j] == 0xffffffffu;
     }
-    v = (uint64_t)t[nl] + c;
-    t[nl - 1] = (uint32_t)v;
-    t[nl] = t[nl + 1] + (uint32_t)(v >> 32);
-  }
-  // t < 2q: subtract q once if t >= q
-  bool ge = t[nl] != 0;
-  if (!ge) {
-    ge = true;  // equal counts as >=
-    for (int j = nl - 1; j >= 0; --j)
-      if (t[j] != q[j]) {
-        ge = t[j] > q[j];
-        break;
-      }
-  }
-  if (ge) {
-    uint64_t b = 0;
-    for (int j = 0; j < nl; ++j) {
-      const uint64_t v = (uint64_t)t[j] - q[j] - b;
-      r[j] = (uint32_t)v;
-      b = (v >> 32) & 1;
+    bool out;
+    in = carry_in(in != 0, ones, out);
+#pragma unroll
+    for (int j = 0; j < K; ++j) {
+      const uint64_t t = (uint64_t)r[j] + in;
+      r[j] = (uint32_t)t;
+      in = (uint32_t)(t >> 32);
     }
-  } else {
-    for (int j = 0; j < nl; ++j) r[j] = t[j];
   }
+  // d = x - y; returns whether x < y (d is then x - y + 2^(32 G K)).
+  static __device__ __forceinline__ bool minus(Num& d, const Num& x, const Num& y) {
+    uint32_t br = 0;
+    bool zero = true;
+#pragma unroll
+    for (int j = 0; j < K; ++j) {
+      const uint64_t t = (uint64_t)x[j] - y[j] - br;
+      d[j] = (uint32_t)t;
+      br = (uint32_t)(t >> 32) & 1;
+      zero &= d[j] == 0;
+    }
+    bool out;
+    br = carry_in(br != 0, zero, out);
+#pragma unroll
+    for (int j = 0; j < K; ++j) {
+      const uint64_t t = (uint64_t)d[j] - br;
+      d[j] = (uint32_t)t;
+      br = (uint32_t)(t >> 32) & 1;
+    }
+    return out;
+  }
+  static __device__ __forceinline__ bool equal(const Num& x, const Num& y) {
+    bool same = true;
+#pragma unroll
+    for (int j = 0; j < K; ++j) same &= x[j] == y[j];
+    const uint32_t b = __ballot_sync(kAllLanes, !same);
+    const int lead = (threadIdx.x & 31) & ~(G - 1);
+    return G == 32 ? b == 0 : ((b >> lead) & ((1u << (G & 31)) - 1)) == 0;
+  }
+  static __device__ __forceinline__ void copy(Num& r, const Num& x) {
+#pragma unroll
+    for (int j = 0; j < K; ++j) r[j] = x[j];
+  }
+  // x mod q for x < 2q
+  static __device__ __forceinline__ void canon(Num& x, const Num& q) {
+    Num d;
+    if (!minus(d, x, q)) copy(x, d);
+  }
+  static __device__ __forceinline__ void dbl(Num& x, const Num& q) {  // 2x mod q for x < q
+    uint32_t in = up(x[K - 1] >> 31);
+#pragma unroll
+    for (int j = 0; j < K; ++j) {
+      const uint32_t o = x[j] >> 31;
+      x[j] = (x[j] << 1) | in;
+      in = o;
+    }
+    canon(x, q);
+  }
+  // One limb of Montgomery reduction: c = (c + m q) / 2^32 with m = c (-q^-1) mod
+  // 2^32; u, h: c's low and high halves.
+  static __device__ __forceinline__ void reduce(uint64_t (&c)[K], const uint32_t (&u)[K], const uint64_t (&h)[K],
+                                                const Num& q, uint32_t qinv) {
+    const uint32_t m = __shfl_sync(kAllLanes, u[0] * qinv, 0, G);
+    uint32_t lo[K];
+#pragma unroll
+    for (int j = 0; j < K; ++j) {
+      const uint64_t t = (uint64_t)q[j] * m + u[j];
+      lo[j] = (uint32_t)t;
+      c[j] = h[j] + (t >> 32);
+    }
+    uint32_t next = __shfl_down_sync(kAllLanes, lo[0], 1, G);
+    if (sub() == G - 1) next = 0;
+#pragma unroll
+    for (int j = 0; j < K; ++j) c[j] += j + 1 < K ? lo[j + 1] : next;
+  }
+  static __device__ __forceinline__ void step(uint64_t (&c)[K], const Num& x, uint32_t yi, const Num& q, uint32_t qinv) {
+    uint32_t u[K];
+    uint64_t h[K];
+#pragma unroll
+    for (int j = 0; j < K; ++j) {
+      const uint64_t t = (uint64_t)x[j] * yi + (uint32_t)c[j];
+      u[j] = (uint32_t)t;
+      h[j] = (t >> 32) + (c[j] >> 32);
+    }
+    reduce(c, u, h, q, qinv);
+  }
+  // x = x y / R mod q below 2q, R = 2^(32 K rl), for x, y < 2q
+  static __device__ __forceinline__ void mul(Num& x, const Num& y, const Num& q, uint32_t qinv, int rl) {
+    uint64_t c[K];
+#pragma unroll
+    for (int j = 0; j < K; ++j) c[j] = 0;
+    for (int l = 0; l < rl; ++l) {
+#pragma unroll
+      for (int j = 0; j < K; ++j) step(c, x, __shfl_sync(kAllLanes, y[j], l, G), q, qinv);
+    }
+    settle(x, c);
+  }
+  // x = x 2^(s - 32) mod q below 2q, 0 <= s < 32, for x < 2q
+  static __device__ __forceinline__ void shift(Num& x, uint32_t s, const Num& q, uint32_t qinv) {
+    uint64_t c[K], h[K];
+    uint32_t u[K];
+#pragma unroll
+    for (int j = 0; j < K; ++j) {
+      const uint64_t t = (uint64_t)x[j] << s;
+      u[j] = (uint32_t)t;
+      h[j] = t >> 32;
+    }
+    reduce(c, u, h, q, qinv);
+    settle(x, c);
+  }
+};
+
+// What a test of q needs: its limbs (in shared memory too, for the exponent's
+// bits), -q^-1 mod 2^32, R mod q.
+template <int G, int K>
+struct BigMod {
+  typedef Big<G, K> B;
+  typename B::Num q, one;
+  uint32_t qinv;
+  int bits, s, rl;  // bit length of q, q - 1 = d 2^s, lanes of R
+
+  // q = n - p; words: this group's q in shared memory (G K words)
+  __device__ __forceinline__ BigMod(const BigArgs& a, uint32_t p, uint32_t* words) : rl((int)a.rl) {
+    typename B::Num n, pn, z;
+#pragma unroll
+    for (int j = 0; j < K; ++j) {
+      const uint32_t i = B::sub() * K + j;
+      n[j] = i < a.nl ? a.n[i] : 0;
+      pn[j] = i == 0 ? p : 0;
+    }
+    B::minus(q, n, pn);
+    __syncwarp();
+#pragma unroll
+    for (int j = 0; j < K; ++j) words[B::sub() * K + j] = q[j];
+    __syncwarp();
+    uint32_t x = words[0];
+    for (int i = 0; i < 4; ++i) x *= 2u - words[0] * x;
+    qinv = 0u - x;
+    int top = (int)a.nl - 1;
+    while (words[top] == 0) --top;
+    bits = 32 * top + 32 - __clz(words[top]);
+    uint32_t low = words[0] & ~1u;
+    int w = 0;
+    while (low == 0) low = words[++w];
+    s = 32 * w + __ffs(low) - 1;
+    // R mod q: 2^bits - q, doubled up to R
+#pragma unroll
+    for (int j = 0; j < K; ++j) {
+      const int i = B::sub() * K + j;
+      z[j] = i == bits / 32 ? 1u << (bits & 31) : 0;
+    }
+    B::minus(one, z, q);
+    // (the groups of a warp may differ by a bit: they run together)
+    const int dbls = 32 * K * rl - bits;
+    const int most = (int)__reduce_max_sync(kAllLanes, (uint32_t)dbls);
+#pragma unroll 1
+    for (int i = 0; i < most; ++i) {
+      B::copy(z, one);
+      B::dbl(z, q);
+      if (i < dbls) B::copy(one, z);
+    }
+  }
+  // The strong test's verdict from x = a^d (in Montgomery form, below 2q).
+  __device__ __forceinline__ bool verdict(typename B::Num& x, int smax) const {
+    typename B::Num mone, y;
+    B::minus(mone, q, one);
+    B::copy(y, x);
+    B::canon(y, q);
+    bool ok = B::equal(y, one) | B::equal(y, mone);
+#pragma unroll 1
+    for (int i = 1; i < smax; ++i) {
+      B::copy(y, x);
+      B::mul(x, y, q, qinv, rl);
+      B::copy(y, x);
+      B::canon(y, q);
+      ok |= B::equal(y, mone) && i < s;
+    }
+    return ok;
+  }
+};
+
+// bits [b, b + w) of the number in words, w <= 8, b + w <= 32 * its words + 24
+__device__ __forceinline__ uint32_t bits_at(const uint32_t* words, int nwords, int b, int w) {
+  const int i = b >> 5;
+  const uint32_t lo = words[i], hi = i + 1 < nwords ? words[i + 1] : 0;
+  return __funnelshift_r(lo, hi, b & 31) & ((1u << w) - 1);
 }
 
-// x = 2x mod q (x < q).
-template <int N>
-__device__ void big_dbl_mod(uint32_t* x, const uint32_t* q, int nl) {
-  uint32_t top = 0;
-  for (int j = 0; j < nl; ++j) {
-    const uint32_t nt = x[j] >> 31;
-    x[j] = (x[j] << 1) | top;
-    top = nt;
-  }
-  bool ge = top != 0;
-  if (!ge) {
-    ge = true;
-    for (int j = nl - 1; j >= 0; --j)
-      if (x[j] != q[j]) {
-        ge = x[j] > q[j];
-        break;
-      }
-  }
-  if (ge) {
-    uint64_t b = 0;
-    for (int j = 0; j < nl; ++j) {
-      const uint64_t v = (uint64_t)x[j] - q[j] - b;
-      x[j] = (uint32_t)v;
-      b = (v >> 32) & 1;
-    }
-  }
-}
+constexpr int kBigThreads = 64;
 
-__device__ __forceinline__ bool big_eq(const uint32_t* x, const uint32_t* y, int nl) {
-  for (int j = 0; j < nl; ++j)
-    if (x[j] != y[j]) return false;
-  return true;
-}
-
-// Strong probable-prime test of odd q (> 2^64, nl limbs) to base kBigBases[bi].
-template <int N>
-__device__ bool big_sprp(const uint32_t* q, int nl, int bi) {
-  uint32_t qinv = q[0];  // -q^-1 mod 2^32 by Newton steps
-  for (int i = 0; i < 4; ++i) qinv *= 2u - q[0] * qinv;
-  qinv = 0u - qinv;
-  // one = R mod q, r2 = R^2 mod q (R = 2^(32 nl)), by doublings of 1
-  uint32_t one[N], r2[N], mone[N], d[N], base[N], x[N];
-  for (int j = 0; j < nl; ++j) one[j] = 0;
-  one[0] = 1;
-  for (int i = 0; i < 32 * nl; ++i) big_dbl_mod<N>(one, q, nl);
-  for (int j = 0; j < nl; ++j) r2[j] = one[j];
-  for (int i = 0; i < 32 * nl; ++i) big_dbl_mod<N>(r2, q, nl);
-  {  // mone = q - one (that is -1 in Montgomery form)
-    uint64_t b = 0;
-    for (int j = 0; j < nl; ++j) {
-      const uint64_t v = (uint64_t)q[j] - one[j] - b;
-      mone[j] = (uint32_t)v;
-      b = (v >> 32) & 1;
-    }
-  }
-  // q - 1 = d 2^s
-  int s = 0;
-  {
-    int lw = 0;
-    while (lw < nl && (q[lw] & ~(lw == 0 ? 1u : 0u)) == 0) ++lw;  // q - 1 has its lowest set bit here
-    const uint32_t low = lw == 0 ? (q[0] & ~1u) : q[lw];
-    s = 32 * lw + __ffs(low) - 1;
-    for (int j = 0; j < nl; ++j) d[j] = q[j];
-    d[0] &= ~1u;  // q - 1 (q odd)
-    const int ws = s >> 5, bs = s & 31;
-    for (int j = 0; j < nl; ++j) {
-      const uint32_t lo = j + ws < nl ? d[j + ws] : 0;
-      const uint32_t hi = j + ws + 1 < nl ? d[j + ws + 1] : 0;
-      d[j] = bs ? (lo >> bs) | (hi << (32 - bs)) : lo;
-    }
-  }
-  int top = nl - 1;
-  while (top > 0 && d[top] == 0) --top;
-  const int nbits = 32 * top + 32 - __clz(d[top]);
-  uint32_t a[N];
-  for (int j = 0; j < nl; ++j) a[j] = 0;
-  a[0] = kBigBases[bi];
-  big_mont_mul<N>(base, a, r2, q, qinv, nl);  // the base in Montgomery form
-  for (int j = 0; j < nl; ++j) x[j] = base[j];
-  for (int b = nbits - 2; b >= 0; --b) {
-    big_mont_mul<N>(x, x, x, q, qinv, nl);
-    if ((d[b >> 5] >> (b & 31)) & 1u) big_mont_mul<N>(x, x, base, q, qinv, nl);
-  }
-  if (big_eq(x, one, nl) || big_eq(x, mone, nl)) return true;
-  for (int i = 1; i < s; ++i) {
-    big_mont_mul<N>(x, x, x, q, qinv, nl);
-    if (big_eq(x, mone, nl)) return true;
-    if (big_eq(x, one, nl)) return false;
-  }
-  return false;
-}
-
-// q = n - p on nl limbs.
-template <int N>
-__device__ __forceinline__ void big_q(const BigArgs& a, uint32_t p, uint32_t* q) {
-  uint32_t borrow = 0;
-  for (int j = 0; j < (int)a.nl; ++j) {
-    const uint64_t v = (uint64_t)a.n[j] - (j == 0 ? p : 0u) - borrow;
-    q[j] = (uint32_t)v;
-    borrow = (uint32_t)(v >> 32) & 1u;
-  }
-}
-
-// Phase 0: base 2 on every survivor; the candidates that pass it join the
-// passers list (each with a slot of 11 later verdicts).
-template <int N>
+// Phase 0: base 2 on every survivor, G lanes each.  The power is taken 5 bits
+// at a time: five squarings take 2^e to 2^(32 e), and a shift by c with one limb
+// of reduction to 2^(32 e + c - 32), so the digits c are those of d + 32 (1 + 32
+// + ... + 32^(m-1)) in base 32: d's own, with one added from the second on and
+// the carries passed up.  What is above the m digits (at most 33) is made by
+// doublings of R mod q.
+template <int G, int K>
 __global__ void __launch_bounds__(kBigThreads) big_base2_kernel(const __grid_constant__ BigArgs a, uint32_t k0) {
-  const uint32_t nsurv = *a.nsurv;
-  for (uint32_t t = blockIdx.x * kBigThreads + threadIdx.x; t < nsurv; t += gridDim.x * kBigThreads) {
-    const uint32_t i = a.surv[t];
-    uint32_t q[N];
-    big_q<N>(a, a.primes[k0 + i], q);
-    atomicAdd(a.mr_tests, 1ull);
-    if (big_sprp<N>(q, (int)a.nl, 0)) {
-      const uint32_t slot = atomicAdd(a.npass, 1u);
-      a.pass[slot] = i;
-      a.fail[slot] = 0;
+  typedef Big<G, K> B;
+  constexpr int kGroups = kBigThreads / G;
+  constexpr int kDigits = (32 * kBigMaxLimbs + 4) / 5;
+  __shared__ uint32_t s_q[kGroups][G * K];
+  __shared__ uint8_t s_dig[kGroups][K == 1 ? 32 * G / 5 + 1 : kDigits];
+  const uint32_t gi = threadIdx.x / G;
+  uint32_t* words = s_q[gi];
+  uint8_t* dig = s_dig[gi];
+  const uint32_t nsurv = *a.nsurv, groups = gridDim.x * kGroups;
+  for (uint32_t t0 = blockIdx.x * kGroups; t0 < nsurv; t0 += groups) {  // uniform in the CTA
+    const uint32_t t = t0 + gi;
+    const bool act = t < nsurv;  // a group past the end runs along on the last survivor
+    const uint32_t i = a.surv[act ? t : nsurv - 1];
+    const BigMod<G, K> M(a, a.primes[k0 + i], words);
+    if (act && B::sub() == 0) atomicAdd(a.mr_tests, 1ull);
+    const int dbits = M.bits - M.s;
+    const int m = dbits > 5 ? (dbits - 1) / 5 : 0;  // at least one bit stays above
+    uint32_t e0 = 0;
+    if (B::sub() == 0) {
+      uint32_t carry = 0;
+      for (int j = 0; j < m; ++j) {
+        const uint32_t v = bits_at(words, G * K, M.s + 5 * j, 5) + (j > 0) + carry;
+        dig[j] = (uint8_t)(v & 31);
+        carry = v >> 5;
+      }
+      e0 = bits_at(words, G * K, M.s + 5 * m, dbits - 5 * m) + (m > 0) + carry;
     }
+    __syncwarp();
+    e0 = __shfl_sync(kAllLanes, e0, 0, G);
+    const int mmax = (int)__reduce_max_sync(kAllLanes, (uint32_t)m);
+    const uint32_t emax = __reduce_max_sync(kAllLanes, e0);
+    typename B::Num x, y;
+    B::copy(x, M.one);
+    for (uint32_t j = 0; j < emax; ++j) {
+      B::copy(y, x);
+      B::dbl(y, M.q);
+      if (j < e0) B::copy(x, y);
+    }
+#pragma unroll 1
+    for (int j = mmax - 1; j >= 0; --j) {
+#pragma unroll 1
+      for (int k = 0; k < 5; ++k) {
+        B::copy(y, x);
+        B::mul(y, x, M.q, M.qinv, M.rl);
+        if (j < m) B::copy(x, y);
+      }
+      B::copy(y, x);
+      B::shift(y, j < m ? dig[j] : 0, M.q, M.qinv);
+      if (j < m) B::copy(x, y);
+    }
+    const bool ok = M.verdict(x, (int)__reduce_max_sync(kAllLanes, (uint32_t)M.s));
+    if (ok && act && B::sub() == 0) {
+      a.pass[atomicAdd(a.npass, 1u)] = i;
+      atomicMin(a.minpass, i);
+    }
+    __syncwarp();
   }
 }
 
-// Phase 1: the 11 other bases, one thread per (passer, base); a failing
-// base marks its passer.
-template <int N>
-__global__ void __launch_bounds__(kBigThreads) big_bases_kernel(const __grid_constant__ BigArgs a, uint32_t k0) {
-  const uint32_t work = *a.npass * 11u;
-  for (uint32_t t = blockIdx.x * kBigThreads + threadIdx.x; t < work; t += gridDim.x * kBigThreads) {
-    const uint32_t slot = t / 11u, bi = 1 + t % 11u;
-    uint32_t q[N];
-    big_q<N>(a, a.primes[k0 + a.pass[slot]], q);
-    if (!big_sprp<N>(q, (int)a.nl, (int)bi)) atomicOr(&a.fail[slot], 1u);
+// Phase 1: bases 3, ..., 37 on one passer (i, or the smallest for ~0u), a warp per
+// base; a failing base marks *fail.  Four exponent bits at a time, the powers
+// base^0 .. base^15 in shared memory.
+template <int G, int K>
+__global__ void __launch_bounds__(32) big_bases_kernel(const __grid_constant__ BigArgs a, uint32_t k0, uint32_t i) {
+  typedef Big<G, K> B;
+  __shared__ uint32_t s_q[G * K], s_all[32 / G][G * K];
+  __shared__ uint32_t s_pow[16][32 * K];
+  if (i == 0xffffffffu) i = *a.minpass;
+  if (i == 0xffffffffu) return;  // no candidate passed base 2
+  const uint32_t lane = threadIdx.x;
+  const BigMod<G, K> M(a, a.primes[k0 + i], s_all[lane / G]);  // every group of the warp holds the same q
+  if (lane < G)
+    for (int j = 0; j < K; ++j) s_q[lane * K + j] = M.q[j];
+  const uint32_t base = kBigBases[1 + blockIdx.x];
+  typename B::Num x, y, b;
+  // base in Montgomery form, from the base's bits
+#pragma unroll
+  for (int j = 0; j < K; ++j) b[j] = 0;
+  for (int k = 5; k >= 0; --k) {
+    B::dbl(b, M.q);
+    if ((base >> k) & 1u) {  // b + one mod q
+      uint64_t c[K];
+#pragma unroll
+      for (int j = 0; j < K; ++j) c[j] = (uint64_t)b[j] + M.one[j];
+      B::settle(b, c);
+      B::canon(b, M.q);
+    }
   }
+  B::copy(x, M.one);
+  for (int k = 0; k < 16; ++k) {
+#pragma unroll
+    for (int j = 0; j < K; ++j) s_pow[k][lane * K + j] = x[j];
+    B::mul(x, b, M.q, M.qinv, M.rl);
+  }
+  __syncwarp();
+  const int dbits = M.bits - M.s;
+  int pos = (dbits - 1) / 4 * 4;  // the lowest bit of the top digit
+  const auto load = [&](uint32_t d) {
+#pragma unroll
+    for (int j = 0; j < K; ++j) y[j] = s_pow[d][lane * K + j];
+  };
+  load(bits_at(s_q, G * K, M.s + pos, dbits - pos));
+  B::copy(x, y);
+#pragma unroll 1
+  while (pos > 0) {
+    pos -= 4;
+#pragma unroll 1
+    for (int k = 0; k < 4; ++k) {
+      B::copy(y, x);
+      B::mul(x, y, M.q, M.qinv, M.rl);
+    }
+    load(bits_at(s_q, G * K, M.s + pos, 4));
+    B::mul(x, y, M.q, M.qinv, M.rl);
+  }
+  const bool ok = M.verdict(x, M.s);
+  if (!ok && lane == 0) atomicOr(a.fail, 1u);
 }
 
 cudaError_t launch_big_filter(const BigArgs& a, uint32_t k0, uint32_t kcount, cudaStream_t s) {
-  big_filter_kernel<<<(kcount + 255) / 256, 256, 0, s>>>(a, k0, kcount);
+  const uint32_t per = kFilterThreads / 32;
+  big_filter_kernel<<<(kcount + per - 1) / per, kFilterThreads, 0, s>>>(a, k0, kcount);
   return cudaGetLastError();
 }
 
-cudaError_t launch_big_mr(const BigArgs& a, uint32_t k0, int phase, int grid, cudaStream_t s) {
-#define GB_BIG_CASE(W)                                                        \
-  case W:                                                                     \
-    if (phase == 0) big_base2_kernel<W><<<grid, kBigThreads, 0, s>>>(a, k0);  \
-    else big_bases_kernel<W><<<grid, kBigThreads, 0, s>>>(a, k0);             \
-    break;
-  switch (a.limbs) {
-    GB_BIG_CASE(4)
-    GB_BIG_CASE(8)
-    GB_BIG_CASE(16)
-    GB_BIG_CASE(32)
-    GB_BIG_CASE(64)
-    GB_BIG_CASE(128)
-    default: return cudaErrorInvalidValue;
-  }
-#undef GB_BIG_CASE
+// Lanes and limbs per lane for R of `limbs` limbs (at most GB_BIG_MAX_LIMBS + 1).
+static void big_shape(uint32_t limbs, int& G, int& K) {
+  G = limbs <= 8 ? 8 : limbs <= 16 ? 16 : 32;
+  K = limbs <= 32 ? 1 : limbs <= 64 ? 2 : limbs <= 96 ? 3 : limbs <= 128 ? 4 : 5;
+}
+
+uint32_t big_r_lanes(uint32_t limbs) {
+  int G, K;
+  big_shape(limbs, G, K);
+  return (limbs + K - 1) / K;
+}
+
+template <typename F>
+static cudaError_t with_big_shape(uint32_t limbs, F f) {
+  int G, K;
+  big_shape(limbs, G, K);
+  if (G == 8) f(std::integral_constant<int, 8>{}, std::integral_constant<int, 1>{});
+  else if (G == 16) f(std::integral_constant<int, 16>{}, std::integral_constant<int, 1>{});
+  else if (K == 1) f(std::integral_constant<int, 32>{}, std::integral_constant<int, 1>{});
+  else if (K == 2) f(std::integral_constant<int, 32>{}, std::integral_constant<int, 2>{});
+  else if (K == 3) f(std::integral_constant<int, 32>{}, std::integral_constant<int, 3>{});
+  else if (K == 4) f(std::integral_constant<int, 32>{}, std::integral_constant<int, 4>{});
+  else f(std::integral_constant<int, 32>{}, std::integral_constant<int, 5>{});
   return cudaGetLastError();
+}
+
+cudaError_t launch_big_base2(const BigArgs& a, uint32_t k0, int grid, cudaStream_t s) {
+  return with_big_shape(a.limbs, [&](auto g, auto k) {
+    big_base2_kernel<decltype(g)::value, decltype(k)::value><<<grid, kBigThreads, 0, s>>>(a, k0);
+  });
+}
+
+cudaError_t launch_big_bases(const BigArgs& a, uint32_t k0, uint32_t i, cudaStream_t s) {
+  return with_big_shape(a.limbs, [&](auto g, auto k) {
+    big_bases_kernel<decltype(g)::value, decltype(k)::value><<<11, 32, 0, s>>>(a, k0, i);
+  });
 }
 
 }  // namespace gb
