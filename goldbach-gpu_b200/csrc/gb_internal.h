@@ -133,8 +133,6 @@ struct SieveArgs {
 // kernels/tables.cu
 cudaError_t launch_wheel_init(uint32_t* wheel, uint32_t* wheel6, cudaStream_t s);
 cudaError_t launch_sieve_bits(const SieveArgs& a, cudaStream_t s);
-cudaError_t launch_counts(const uint32_t* B, uint64_t m_first, uint64_t count, uint32_t splits,
-                          uint64_t wps, unsigned long long* out, cudaStream_t s);
 // Appends the primes of `bits` (odd-only from q_lo) after `prefix` entries of
 // `primes`; writes the new total into *d_total (device) and magic[] for them.
 cudaError_t launch_compact_primes(const uint32_t* bits, uint64_t nbits, uint64_t q_lo,
@@ -143,6 +141,30 @@ cudaError_t launch_compact_primes(const uint32_t* bits, uint64_t nbits, uint64_t
                                   uint32_t* scratch_blocks, uint32_t nblocks_cap,
                                   cudaStream_t s);
 size_t compact_scratch_blocks(uint64_t nbits);
+
+// kernels/counts.cu: partition counts by residue classes mod `modulus`.  Class c's
+// bitset (the c-th residue prime to the modulus) starts `stride` words after
+// class c - 1's, with two zero words in front of the first and after each.
+struct CountPair {     // a pair of classes and the n of one residue
+  uint32_t a, b, half;  // class indices; half: a = b
+  uint64_t count;       // n of the residue
+  uint64_t s0;          // s of the first (as an int64: -1 for an n with no k)
+  uint64_t out;         // output index of the first
+};
+struct CountArgs {
+  const uint32_t* classes;  // class 0's first word (k = 0 .. 31)
+  uint64_t stride;
+  const CountPair* pairs;
+  uint32_t npairs;
+  uint32_t modulus;
+  uint64_t groups;          // of 32 n, the most of any residue
+  uint64_t splits, wps;     // slices of a class's words, and words each
+  uint32_t one;             // 1, unknown to the compiler: keeps multiplications multiplications
+  unsigned long long* out;
+};
+cudaError_t launch_count_classes(const uint32_t* odd, uint64_t nodd, uint32_t modulus, uint32_t* classes,
+                                 uint64_t stride, uint64_t nwords, cudaStream_t s);
+cudaError_t launch_counts(const CountArgs& a, const uint32_t* odd, uint64_t start, uint64_t count, cudaStream_t s);
 
 // kernels/range.cu
 size_t range_smem_bytes(const RangeArgs& a);

@@ -883,10 +883,41 @@ gb_status gb_autotune_windows(gb_ctx* c, const gb_window* w, size_t count, const
   GB_PUBLIC(c, autotune_windows_impl(c, c->ws, w, count, base, tuned, res));
 }
 
-// Partition counts (kernels/counts.cu): the odd-prime bitset of [1, n_max]
-// is sieved into a padded device buffer (two zero words in front, slack
-// behind for the correlation's 64-bit windows), then one warp per 32
-// consecutive n and slice of the bitset's words.
+// The pairs of residue classes mod M that the n of [start, start + 2 (count - 1)]
+// need (kernels/counts.cu), and the work they are: words of 32 n times words of
+// the classes.
+static std::vector<CountPair> count_pairs(uint32_t M, uint64_t start, uint64_t count, double* work) {
+  std::vector<uint32_t> cls, index(M, 0);
+  for (uint32_t a = 1; a < M; a += 2)
+    if ((M % 3 || a % 3) && (M % 5 || a % 5) && (M % 7 || a % 7)) {
+      index[a] = (uint32_t)cls.size();
+      cls.push_back(a);
+    }
+  std::vector<CountPair> pairs;
+  *work = 0;
+  for (uint64_t j = 0; j < M / 2 && j < count; ++j) {  // the first n of each residue
+    const uint64_t n = start + 2 * j;
+    const uint32_t r = (uint32_t)(n % M);
+    CountPair p{};
+    p.count = (count - j - 1) / (M / 2) + 1;
+    p.out = j;
+    for (uint32_t a : cls) {
+      const uint32_t b = (r + M - a) % M;
+      if (b < a || b % 2 == 0 || cls[index[b]] != b) continue;  // each pair once, both prime to M
+      p.a = index[a];
+      p.b = index[b];
+      p.half = a == b;
+      p.s0 = n / M - (a + b - r) / M;
+      pairs.push_back(p);
+      *work += (double)((p.count + 31) / 32) * (double)(n / M / 32 + 1) * (p.half ? 0.5 : 1.0);
+    }
+  }
+  return pairs;
+}
+
+// Partition counts (kernels/counts.cu): the odd-prime bitset of [1, n_max] is
+// sieved, split into the bitsets of the residue classes mod M where that saves
+// more than it costs, and correlated pair by pair.
 static gb_status counts_impl(gb_ctx* c, Workspace& w, uint64_t start, uint64_t count,
                              uint64_t* counts, const gb_count_opts* opts) {
   if (!count) return GB_OK;
@@ -908,6 +939,36 @@ static gb_status counts_impl(gb_ctx* c, Workspace& w, uint64_t start, uint64_t c
   unsigned long long* d_out = (unsigned long long*)counts;
   if ((st = ws_buffer(c, w, tmp, 0, (nwords + 8) * 4, (void**)&buf)) != GB_OK) return st;
   if (!o.on_device && (st = ws_buffer(c, w, tmp, 1, count * 8, (void**)&d_out)) != GB_OK) return st;
+  // the modulus with the least work; building the classes costs about as much
+  // as 6 words of 32 n to each of their words
+  CountArgs ca{};
+  std::vector<CountPair> pairs;
+  double best = 0;
+  for (uint32_t M : {2u, 6u, 30u, 210u}) {
+    double work = 0;
+    std::vector<CountPair> p = count_pairs(M, start, count, &work);
+    if (M > 2) work += 6.0 * (M == 6 ? 2 : M == 30 ? 8 : 48) * ((double)n_max / M / 32);
+    if (M == 2 || work < best) {
+      best = work;
+      pairs.swap(p);
+      ca.modulus = M;
+    }
+  }
+  uint32_t* classes = nullptr;
+  uint64_t stride = 0, cwords = 0;
+  if (ca.modulus > 2) {
+    cwords = n_max / ca.modulus / 32 + 1;
+    stride = (cwords + 2 + 3) & ~3ull;
+    const uint64_t nc = ca.modulus == 6 ? 2 : ca.modulus == 30 ? 8 : 48;
+    if (ws_buffer(c, w, tmp, 2, (nc * stride + 8) * 4, (void**)&classes) != GB_OK) {
+      w.err.clear();  // no room beside the odd bitset: the odd classes alone
+      ca.modulus = 2;
+      pairs = count_pairs(2, start, count, &best);
+    }
+  }
+  CountPair* d_pairs = nullptr;
+  if ((st = ws_buffer(c, w, tmp, 3, std::max<size_t>(pairs.size(), 1) * sizeof(CountPair), (void**)&d_pairs)) != GB_OK)
+    return st;
   const uint32_t tile = 1u << 18;
   const uint64_t root = isqrt_u64(n_max);
   uint64_t ns = 0, kc = 0;
@@ -924,18 +985,34 @@ static gb_status counts_impl(gb_ctx* c, Workspace& w, uint64_t start, uint64_t c
   a.wheel = c->d_wheel;
   a.out = buf + 2;
   // Work split: enough warp tasks to fill the GPU, at most 2^22 words each.
-  const uint64_t groups = (count + 31) / 32;
-  const uint64_t wmax = n_max / 4 / 32 + 1;  // words of i for the largest n
-  uint64_t splits = std::max<uint64_t>(1, ((uint64_t)c->sm_count * 64 + groups - 1) / groups);
-  splits = std::max<uint64_t>(splits, (wmax + (1u << 22) - 1) >> 22);
-  uint64_t wps = (wmax + splits - 1) / splits;
-  wps = std::max<uint64_t>(32, (wps + 31) & ~31ull);
-  splits = (wmax + wps - 1) / wps;
-  cudaError_t e = cudaMemsetAsync(buf, 0, (nwords + 8) * 4, s);
+  ca.classes = ca.modulus > 2 ? classes + 4 : buf + 2;
+  ca.stride = stride;
+  ca.pairs = d_pairs;
+  ca.npairs = (uint32_t)pairs.size();
+  ca.one = 1;
+  ca.out = d_out;
+  for (const CountPair& p : pairs) ca.groups = std::max<uint64_t>(ca.groups, (p.count + 31) / 32);
+  const uint64_t lanes = std::max<uint64_t>(1, ca.groups * pairs.size());
+  const uint64_t wmax = ca.modulus > 2 ? cwords : n_max / 4 / 32 + 1;  // words of k for the largest n
+  ca.splits = std::max<uint64_t>(1, ((uint64_t)c->sm_count * 256 + lanes - 1) / lanes);
+  ca.splits = std::max<uint64_t>(ca.splits, (wmax + (1u << 22) - 1) >> 22);
+  ca.wps = std::max<uint64_t>(224, ((wmax + ca.splits - 1) / ca.splits + 223) / 224 * 224);  // whole rounds of 7 words a lane
+  ca.splits = (wmax + ca.wps - 1) / ca.wps;
+  // the sieve writes words 2 .. nwords + 1; the padding around them is zero
+  cudaError_t e = cudaMemsetAsync(buf, 0, 8, s);
+  if (e == cudaSuccess) e = cudaMemsetAsync(buf + 2 + nwords, 0, 6 * 4, s);
   if (e == cudaSuccess) e = launch_sieve_bits(a, s);
-  if (e == cudaSuccess) e = cudaMemsetAsync(d_out, 0, count * 8, s);
+  if (ca.modulus > 2) {
+    if (e == cudaSuccess) e = cudaMemsetAsync(classes, 0, 16, s);
+    const uint64_t nc = ca.modulus == 6 ? 2 : ca.modulus == 30 ? 8 : 48;
+    if (e == cudaSuccess)  // the words between the classes
+      e = cudaMemset2DAsync(classes + 4 + cwords, stride * 4, 0, (stride - cwords) * 4, nc, s);
+    if (e == cudaSuccess) e = launch_count_classes(buf + 2, nwords, ca.modulus, classes + 4, stride, cwords, s);
+  }
+  if (e == cudaSuccess && !pairs.empty())
+    e = cudaMemcpyAsync(d_pairs, pairs.data(), pairs.size() * sizeof(CountPair), cudaMemcpyHostToDevice, s);
   if (e == cudaSuccess) e = cudaEventRecord(w.ek0, s);
-  if (e == cudaSuccess) e = launch_counts(buf + 2, start / 2 - 1, count, (uint32_t)splits, wps, d_out, s);
+  if (e == cudaSuccess) e = launch_counts(ca, buf + 2, start, count, s);
   if (e == cudaSuccess) e = cudaEventRecord(w.ek1, s);
   if (e == cudaSuccess && !o.on_device) e = cudaMemcpyAsync(counts, d_out, count * 8, cudaMemcpyDeviceToHost, s);
   if (e == cudaSuccess) e = cudaStreamSynchronize(s);
