@@ -9,9 +9,11 @@
 #include "gb_ctx.h"
 
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <cstring>
 #include <new>
+#include <thread>
 
 namespace gb {
 
@@ -86,11 +88,13 @@ void Temps::release() {
 
 gb_status ws_init(gb_ctx* c, Workspace& w, uint32_t queue_cap) {
   gb_status st;
-  if ((st = dev_alloc(c, (void**)&w.ctr, kCtrCount * 8, &w.err)) != GB_OK ||
-      (st = dev_alloc(c, (void**)&w.hist, GB_HIST_BINS * 8, &w.err)) != GB_OK ||
+  // the counters and the histogram in one buffer: one copy reads both back
+  if ((st = dev_alloc(c, (void**)&w.ctr, (kCtrCount + GB_HIST_BINS) * 8, &w.err)) != GB_OK ||
       (st = dev_alloc(c, (void**)&w.queue, (size_t)queue_cap * sizeof(QEntry), &w.err)) != GB_OK)
     return st;
+  w.hist = w.ctr + kCtrCount;
   w.queue_cap = queue_cap;
+  if (cudaMallocHost((void**)&w.h_io, kIoBytes) != cudaSuccess) return fail(w, GB_ENOMEM, "pinned staging buffer");
   if (cudaMallocHost((void**)&w.h_stage, (kCtrCount + GB_HIST_BINS) * 8) != cudaSuccess)
     return fail(w, GB_ENOMEM, "pinned staging buffer");
   if (cudaEventCreate(&w.ev0) != cudaSuccess || cudaEventCreate(&w.ev1) != cudaSuccess ||
@@ -135,9 +139,16 @@ void ws_free(gb_ctx* c, Workspace& w) {
     w.buf_bytes[i] = 0;
   }
   if (w.h_stage) cudaFreeHost(w.h_stage);
+  if (w.h_io) cudaFreeHost(w.h_io);
+  if (w.h_ring) cudaFreeHost(w.h_ring);
   w.h_stage = nullptr;
+  w.h_io = w.h_ring = nullptr;
+  for (cudaEvent_t& e : w.ring_ev)
+    if (e) {
+      cudaEventDestroy(e);
+      e = nullptr;
+    }
   dev_free(c, w.ctr);
-  dev_free(c, w.hist);
   dev_free(c, w.queue);
   dev_free(c, w.scratch);
   w.ctr = nullptr;
@@ -152,6 +163,92 @@ void ws_free(gb_ctx* c, Workspace& w) {
       cudaEventDestroy(*e);
       *e = nullptr;
     }
+}
+
+// A pageable copy of the runtime moves about 6.5 GB/s; the ring's slots come in at
+// the link's rate and four threads empty them (11 MB of minimal p: 1.7 -> 0.6 ms).
+constexpr size_t kRingSlot = 1u << 20;
+constexpr int kRingSlots = 4, kRingThreads = 4;
+
+cudaError_t copy_out(Workspace& w, void* dst, const void* src, size_t bytes, cudaStream_t s) {
+  cudaPointerAttributes at{};
+  if (bytes < 2 * kRingSlot ||
+      (cudaPointerGetAttributes(&at, dst) == cudaSuccess && at.type != cudaMemoryTypeUnregistered))
+    return cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, s);
+  cudaGetLastError();
+  if (!w.h_ring) {
+    if (cudaMallocHost((void**)&w.h_ring, kRingSlot * kRingSlots) != cudaSuccess) {
+      cudaGetLastError();
+      w.h_ring = nullptr;
+      return cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, s);
+    }
+    for (cudaEvent_t& e : w.ring_ev) {
+      cudaError_t x = cudaEventCreateWithFlags(&e, cudaEventDisableTiming);
+      if (x != cudaSuccess) return x;
+    }
+  }
+  const size_t slots = (bytes + kRingSlot - 1) / kRingSlot;
+  auto len = [&](size_t i) { return std::min(kRingSlot, bytes - i * kRingSlot); };
+  auto fill = [&](size_t i) {
+    const int r = (int)(i % kRingSlots);
+    cudaError_t x = cudaMemcpyAsync(w.h_ring + r * kRingSlot, (const char*)src + i * kRingSlot, len(i),
+                                    cudaMemcpyDeviceToHost, s);
+    return x == cudaSuccess ? cudaEventRecord(w.ring_ev[r], s) : x;
+  };
+  // ready: slots that have arrived; taken: the next quarter of a slot to empty;
+  // left: quarters of each ring slot not yet emptied
+  std::atomic<size_t> ready{0}, taken{0};
+  std::atomic<int> left[kRingSlots];
+  constexpr size_t kParts = 4;
+  for (auto& l : left) l.store(0);
+  auto empty_one = [&]() -> bool {  // whether there was a part to take
+    size_t t = taken.load(std::memory_order_relaxed);
+    do {
+      if (t >= ready.load(std::memory_order_acquire) * kParts) return false;
+    } while (!taken.compare_exchange_weak(t, t + 1));
+    const size_t i = t / kParts, part = len(i) / kParts, o = (t % kParts) * part;
+    const size_t n = t % kParts == kParts - 1 ? len(i) - o : part;
+    std::memcpy((char*)dst + i * kRingSlot + o, w.h_ring + (i % kRingSlots) * kRingSlot + o, n);
+    left[i % kRingSlots].fetch_sub(1, std::memory_order_release);
+    return true;
+  };
+  std::atomic<bool> stop{false};
+  std::thread helpers[kRingThreads - 1];
+  int nh = 0;
+  try {
+    for (; nh < kRingThreads - 1; ++nh)
+      helpers[nh] = std::thread([&] {
+        while (!stop.load(std::memory_order_acquire))
+          if (!empty_one()) std::this_thread::yield();
+      });
+  } catch (...) {  // no more threads: fewer helpers
+  }
+  cudaError_t e = cudaSuccess;
+  for (size_t i = 0; i < slots && i < (size_t)kRingSlots && e == cudaSuccess; ++i) e = fill(i);
+  for (size_t i = 0; i < slots && e == cudaSuccess; ++i) {
+    const int r = (int)(i % kRingSlots);
+    while (e == cudaSuccess) {  // slot i's arrival, emptying earlier ones meanwhile
+      const cudaError_t q = cudaEventQuery(w.ring_ev[r]);
+      if (q == cudaSuccess) break;
+      if (q != cudaErrorNotReady) e = q;
+      empty_one();
+    }
+    cudaGetLastError();
+    if (e != cudaSuccess) break;
+    left[r].store((int)kParts, std::memory_order_relaxed);
+    ready.store(i + 1, std::memory_order_release);
+    if (i + 1 >= (size_t)kRingSlots && i + 1 < slots) {  // slot i + 1 goes where slot i + 1 - kRingSlots was
+      while (left[(i + 1) % kRingSlots].load(std::memory_order_acquire) != 0) empty_one();
+      e = fill(i + 1);
+    }
+  }
+  while (e == cudaSuccess && empty_one()) {
+  }
+  for (auto& l : left)
+    while (e == cudaSuccess && l.load(std::memory_order_acquire) != 0) std::this_thread::yield();
+  stop.store(true, std::memory_order_release);
+  for (int h = 0; h < nh; ++h) helpers[h].join();
+  return e;
 }
 
 uint64_t isqrt_u64(uint64_t n) {  // exact floor(sqrt(n)), src/goldbach.cu:637-646
@@ -194,6 +291,15 @@ gb_status count_le(gb_ctx* c, Workspace& w, uint64_t x, uint64_t* out) {
   *out = lo + (std::upper_bound(blk.begin(), blk.end(), (uint32_t)std::min<uint64_t>(x, 0xffffffffu)) -
                blk.begin());
   return GB_OK;
+}
+
+uint64_t count_bound(const gb_ctx* c, uint64_t x) {
+  if (x >= c->primes_limit) return c->nprimes;
+  const uint32_t y = (uint32_t)std::min<uint64_t>(x, 0xffffffffu);
+  if (x <= kHostPrimeLimit || c->nprimes == c->h_primes.size())
+    return std::upper_bound(c->h_primes.begin(), c->h_primes.end(), y) - c->h_primes.begin();
+  const uint64_t b = std::upper_bound(c->h_sample.begin(), c->h_sample.end(), y) - c->h_sample.begin();
+  return std::min<uint64_t>(c->nprimes, b * kSampleStride);
 }
 
 // Builds (or grows) the resident prime table to cover [2, limit] on the
@@ -377,10 +483,10 @@ gb_status range_impl(gb_ctx* c, Workspace& w, Arena* arena, uint64_t start, uint
   a.nbw = range6_words(H, NE);
   const uint64_t search_top = std::min<uint64_t>(H - 13, p_lim);
   const uint64_t window_bits = H / 6 + NE / 3;
-  uint64_t ns = 0, kf = 0, nsv = 0, kc = 0;
+  uint64_t ns = 0, kc = 0;
+  // (kf is compared with window primes only, all below 2^17; the sieve stops at root)
+  const uint64_t kf = count_bound(c, o.p_small), nsv = count_bound(c, root);
   if ((st = count_le(c, w, search_top, &ns)) != GB_OK ||
-      (st = count_le(c, w, o.p_small, &kf)) != GB_OK ||
-      (st = count_le(c, w, root, &nsv)) != GB_OK ||
       (st = count_le(c, w, window_bits / 64, &kc)) != GB_OK)
     return st;
   sp.halo = H;
@@ -418,10 +524,16 @@ gb_status range_impl(gb_ctx* c, Workspace& w, Arena* arena, uint64_t start, uint
   void *d_vbits, *d_minp, *d_shist, *d_sfb, *d_sfail;
   if ((st = dev_out(od.verified_bits, vwords * 4, &d_vbits)) != GB_OK ||
       (st = dev_out(od.min_p, count * 4, &d_minp)) != GB_OK ||
-      (st = dev_out(od.seg_hist, nseg * GB_HIST_BINS * 8, &d_shist)) != GB_OK ||
-      (st = dev_out(od.seg_fallbacks, nseg * 4, &d_sfb)) != GB_OK ||
-      (st = dev_out(od.seg_failures, nseg * 4, &d_sfail)) != GB_OK)
+      (st = dev_out(od.seg_hist, nseg * GB_HIST_BINS * 8, &d_shist)) != GB_OK)
     return st;
+  if (o.on_device) {
+    d_sfb = od.seg_fallbacks;
+    d_sfail = od.seg_failures;
+  } else {  // both in one buffer: one memset and one copy
+    if ((st = dev_out(od.seg_fallbacks ? (void*)od.seg_fallbacks : od.seg_failures, nseg * 8, &d_sfb)) != GB_OK) return st;
+    d_sfail = od.seg_failures ? (uint32_t*)d_sfb + nseg : nullptr;
+    if (!od.seg_fallbacks) d_sfb = nullptr;
+  }
   if (od.minp_hist && o.on_device) sp.hist = (unsigned long long*)od.minp_hist;
   sp.vbits = (uint32_t*)d_vbits;
   sp.minp = (uint32_t*)d_minp;
@@ -435,9 +547,10 @@ gb_status range_impl(gb_ctx* c, Workspace& w, Arena* arena, uint64_t start, uint
   };
   uint32_t last_word = count & 31 ? (1u << (count & 31)) - 1 : 0xffffffffu;
   chk(cudaEventRecord(w.ev0, s));
-  chk(cudaMemsetAsync(sp.ctr, 0, kCtrCount * 8, s));
+  const bool own_hist = sp.hist == w.hist;  // right behind the counters
+  chk(cudaMemsetAsync(sp.ctr, 0, (kCtrCount + (own_hist ? GB_HIST_BINS : 0)) * 8, s));
   chk(cudaMemsetAsync(sp.ctr + kCtrFirstFail, 0xff, 8, s));
-  chk(cudaMemsetAsync(sp.hist, 0, GB_HIST_BINS * 8, s));
+  if (!own_hist) chk(cudaMemsetAsync(sp.hist, 0, GB_HIST_BINS * 8, s));
   if (sp.vbits) {
     chk(cudaMemsetAsync(sp.vbits, 0xff, vwords * 4, s));
     // bits past the last n are zero (pageable source: staged at the call)
@@ -445,8 +558,13 @@ gb_status range_impl(gb_ctx* c, Workspace& w, Arena* arena, uint64_t start, uint
   }
   if (sp.minp) chk(cudaMemsetAsync(sp.minp, 0, count * 4, s));
   if (sp.unit_hist) chk(cudaMemsetAsync(sp.unit_hist, 0, nseg * GB_HIST_BINS * 8, s));
-  if (sp.unit_fallbacks) chk(cudaMemsetAsync(sp.unit_fallbacks, 0, nseg * 4, s));
-  if (sp.unit_failures) chk(cudaMemsetAsync(sp.unit_failures, 0, nseg * 4, s));
+  if (!o.on_device && (sp.unit_fallbacks || sp.unit_failures)) {
+    uint32_t* const both = sp.unit_fallbacks ? sp.unit_fallbacks : sp.unit_failures - nseg;
+    chk(cudaMemsetAsync(both, 0, nseg * 8, s));
+  } else {
+    if (sp.unit_fallbacks) chk(cudaMemsetAsync(sp.unit_fallbacks, 0, nseg * 4, s));
+    if (sp.unit_failures) chk(cudaMemsetAsync(sp.unit_failures, 0, nseg * 4, s));
+  }
   if (e != cudaSuccess) return cuda_fail(w, e, "range setup");
   int launches = 0;
   const bool masked = my_segs && range_masked_pays(c, start, std::min(count, my_segs * o.seg_size), root, my_segs);
@@ -482,20 +600,29 @@ gb_status range_impl(gb_ctx* c, Workspace& w, Arena* arena, uint64_t start, uint
   chk(cudaEventRecord(w.ev1, s));
   unsigned long long ctr[kCtrCount];
   unsigned long long* st_ctr = w.h_stage;  // pinned: the counters, then the histogram
-  chk(cudaMemcpyAsync(st_ctr, sp.ctr, kCtrCount * 8, cudaMemcpyDeviceToHost, s));
   const bool hist_host = od.minp_hist && !o.on_device;
-  if (hist_host)
-    chk(cudaMemcpyAsync(st_ctr + kCtrCount, sp.hist, GB_HIST_BINS * 8, cudaMemcpyDeviceToHost, s));
+  chk(cudaMemcpyAsync(st_ctr, sp.ctr, (kCtrCount + (hist_host ? GB_HIST_BINS : 0)) * 8, cudaMemcpyDeviceToHost, s));
+  const bool seg_host = !o.on_device && (od.seg_fallbacks || od.seg_failures);
+  const bool seg_staged = seg_host && nseg * 8 <= kIoBytes;
   if (!o.on_device) {
-    if (od.verified_bits) chk(cudaMemcpyAsync(od.verified_bits, sp.vbits, vwords * 4, cudaMemcpyDeviceToHost, s));
-    if (od.min_p) chk(cudaMemcpyAsync(od.min_p, sp.minp, count * 4, cudaMemcpyDeviceToHost, s));
-    if (od.seg_hist) chk(cudaMemcpyAsync(od.seg_hist, sp.unit_hist, nseg * GB_HIST_BINS * 8, cudaMemcpyDeviceToHost, s));
-    if (od.seg_fallbacks) chk(cudaMemcpyAsync(od.seg_fallbacks, sp.unit_fallbacks, nseg * 4, cudaMemcpyDeviceToHost, s));
-    if (od.seg_failures) chk(cudaMemcpyAsync(od.seg_failures, sp.unit_failures, nseg * 4, cudaMemcpyDeviceToHost, s));
+    if (seg_staged) {
+      chk(cudaMemcpyAsync(w.h_io, od.seg_fallbacks ? sp.unit_fallbacks : sp.unit_failures - nseg, nseg * 8,
+                          cudaMemcpyDeviceToHost, s));
+    } else if (seg_host) {
+      if (od.seg_fallbacks) chk(copy_out(w, od.seg_fallbacks, sp.unit_fallbacks, nseg * 4, s));
+      if (od.seg_failures) chk(copy_out(w, od.seg_failures, sp.unit_failures, nseg * 4, s));
+    }
+    if (od.verified_bits) chk(copy_out(w, od.verified_bits, sp.vbits, vwords * 4, s));
+    if (od.min_p) chk(copy_out(w, od.min_p, sp.minp, count * 4, s));
+    if (od.seg_hist) chk(copy_out(w, od.seg_hist, sp.unit_hist, nseg * GB_HIST_BINS * 8, s));
   }
   chk(cudaStreamSynchronize(s));
   std::memcpy(ctr, st_ctr, sizeof ctr);
   if (hist_host && e == cudaSuccess) std::memcpy(od.minp_hist, st_ctr + kCtrCount, GB_HIST_BINS * 8);
+  if (seg_staged && e == cudaSuccess) {
+    if (od.seg_fallbacks) std::memcpy(od.seg_fallbacks, w.h_io, nseg * 4);
+    if (od.seg_failures) std::memcpy(od.seg_failures, w.h_io + nseg * 4, nseg * 4);
+  }
   float ms = 0, kms = 0;
   if (e == cudaSuccess) {
     cudaEventElapsedTime(&ms, w.ev0, w.ev1);
@@ -524,6 +651,8 @@ gb_status range_impl(gb_ctx* c, Workspace& w, Arena* arena, uint64_t start, uint
 }
 
 // ---------------------------------------------------------------------------
+constexpr size_t kDirectQueries = 32;
+
 gb_status single_impl(gb_ctx* c, Workspace& w, Arena* arena, const uint64_t* n, size_t count,
                       uint64_t* p_out, uint64_t* q_out, const gb_single_opts* opts,
                       gb_single_result* res) {
@@ -534,26 +663,47 @@ gb_status single_impl(gb_ctx* c, Workspace& w, Arena* arena, const uint64_t* n, 
   if (o.p_limit > 0xfffffffbull) return fail(w, GB_EINVAL, "p_limit above 2^32");
   gb_status st = ensure_primes(c, w, o.p_limit);
   if (st != GB_OK) return st;
-  uint64_t np = 0;
-  if ((st = count_le(c, w, o.p_limit, &np)) != GB_OK) return st;
+  const uint64_t np = count_bound(c, o.p_limit);  // the kernel stops at p_limit itself
   cudaStream_t s = o.stream ? (cudaStream_t)o.stream : c->stream;
   const uint64_t* dn = n;
   uint64_t *dp = p_out, *dq = q_out;
+  unsigned long long* d_ctr = w.ctr;
   Temps tmp(c, arena);
-  if (!o.on_device && count) {
+  // host arrays that fit the pinned staging go up with four zeroed counters in
+  // one copy, and come down with them in one; a handful of queries is read and
+  // written by the kernel in the staging itself (its warps then take their
+  // queries by place, and the counts are made here)
+  const bool host = !o.on_device && count;
+  const bool direct = host && count <= kDirectQueries;
+  const bool staged = host && !direct && (3 * count + 4) * 8 <= kIoBytes;
+  uint64_t* const io = (uint64_t*)w.h_io;
+  if (direct) {
+    std::memcpy(io, n, count * 8);
+    dn = io;
+    dp = io + count;
+    dq = io + 2 * count;
+  } else if (host) {
     void* t;
-    if ((st = ws_buffer(c, w, tmp, 0, count * 8 * 3, &t)) != GB_OK) return st;
-    dn = (const uint64_t*)t;
-    dp = (uint64_t*)t + count;
-    dq = (uint64_t*)t + 2 * count;
+    if ((st = ws_buffer(c, w, tmp, 0, (3 * count + 4) * 8, &t)) != GB_OK) return st;
+    dn = (const uint64_t*)t;  // n, counters, p, q
+    if (staged) d_ctr = (unsigned long long*)t + count;
+    dp = (uint64_t*)t + count + 4;
+    dq = dp + count;
   }
   cudaError_t e = cudaSuccess;
   auto chk = [&](cudaError_t x) {
     if (e == cudaSuccess && x != cudaSuccess) e = x;
   };
   chk(cudaEventRecord(w.ev0, s));
-  if (!o.on_device && count) chk(cudaMemcpyAsync((void*)dn, n, count * 8, cudaMemcpyHostToDevice, s));
-  chk(cudaMemsetAsync(w.ctr, 0, 4 * 8, s));
+  if (direct) {
+  } else if (staged) {
+    std::memcpy(io, n, count * 8);
+    std::memset(io + count, 0, 4 * 8);
+    chk(cudaMemcpyAsync((void*)dn, io, (count + 4) * 8, cudaMemcpyHostToDevice, s));
+  } else {
+    if (host) chk(cudaMemcpyAsync((void*)dn, n, count * 8, cudaMemcpyHostToDevice, s));
+    chk(cudaMemsetAsync(d_ctr, 0, 4 * 8, s));
+  }
   int launches = 0;
   if (count) {
     SingleArgs a{};
@@ -564,18 +714,39 @@ gb_status single_impl(gb_ctx* c, Workspace& w, Arena* arena, const uint64_t* n, 
     a.primes = c->d_primes;
     a.nprimes = np;
     a.p_lim = o.p_limit;
-    a.ctr = w.ctr;
+    a.ctr = d_ctr;
     chk(launch_single(a, c->sm_count, 100, s));
     ++launches;
   }
-  if (!o.on_device && count) {
-    chk(cudaMemcpyAsync(p_out, dp, count * 8, cudaMemcpyDeviceToHost, s));
-    chk(cudaMemcpyAsync(q_out, dq, count * 8, cudaMemcpyDeviceToHost, s));
+  unsigned long long* ctr = w.h_stage;  // pinned
+  if (direct) {
+    chk(cudaEventRecord(w.ev1, s));
+  } else if (staged) {
+    ctr = (unsigned long long*)(io + count);
+    chk(cudaMemcpyAsync(ctr, d_ctr, (2 * count + 4) * 8, cudaMemcpyDeviceToHost, s));
+    chk(cudaEventRecord(w.ev1, s));
+  } else {
+    if (host) {
+      chk(copy_out(w, p_out, dp, count * 8, s));
+      chk(copy_out(w, q_out, dq, count * 8, s));
+    }
+    chk(cudaEventRecord(w.ev1, s));
+    chk(cudaMemcpyAsync(ctr, d_ctr, 4 * 8, cudaMemcpyDeviceToHost, s));
   }
-  chk(cudaEventRecord(w.ev1, s));
-  unsigned long long ctr[4] = {0, 0, 0, 0};
-  chk(cudaMemcpyAsync(ctr, w.ctr, sizeof ctr, cudaMemcpyDeviceToHost, s));
   chk(cudaStreamSynchronize(s));
+  if (direct && e == cudaSuccess) {
+    ctr[1] = ctr[2] = 0;
+    for (size_t i = 0; i < count; ++i) {
+      ctr[1] += dp[i] != 0;
+      ctr[2] = std::max<unsigned long long>(ctr[2], dp[i]);
+    }
+    std::memcpy(p_out, dp, count * 8);
+    std::memcpy(q_out, dq, count * 8);
+  }
+  if (staged && e == cudaSuccess) {
+    std::memcpy(p_out, io + count + 4, count * 8);
+    std::memcpy(q_out, io + 2 * count + 4, count * 8);
+  }
   float ms = 0;
   if (e == cudaSuccess) cudaEventElapsedTime(&ms, w.ev0, w.ev1);
   if (e != cudaSuccess) return cuda_fail(w, e, "single batch");
@@ -764,9 +935,7 @@ static gb_status sieve_bitset_impl(gb_ctx* c, Workspace& w, uint64_t q_lo, uint6
   const uint64_t nwords = (nbits + 31) / 32;
   if (!on_device && (st = ws_buffer(c, w, tmp, 0, nwords * 4, (void**)&d)) != GB_OK) return st;
   const uint32_t tile = 1u << 18;
-  uint64_t ns = 0, kc = 0;
-  if ((st = count_le(c, w, root, &ns)) != GB_OK || (st = count_le(c, w, tile / 64, &kc)) != GB_OK)
-    return st;
+  const uint64_t ns = count_bound(c, root), kc = count_bound(c, tile / 64);  // (the sieve stops at root)
   SieveArgs a{};
   a.q_lo = q_lo;
   a.nbits = nbits;
@@ -971,9 +1140,7 @@ static gb_status counts_impl(gb_ctx* c, Workspace& w, uint64_t start, uint64_t c
     return st;
   const uint32_t tile = 1u << 18;
   const uint64_t root = isqrt_u64(n_max);
-  uint64_t ns = 0, kc = 0;
-  if ((st = count_le(c, w, root, &ns)) != GB_OK || (st = count_le(c, w, tile / 64, &kc)) != GB_OK)
-    return st;
+  const uint64_t ns = count_bound(c, root), kc = count_bound(c, tile / 64);  // (the sieve stops at root)
   SieveArgs a{};
   a.q_lo = 1;
   a.nbits = nbits;

@@ -55,6 +55,11 @@ struct Workspace {
   size_t buf_bytes[kBufSlots] = {};
   // pinned staging for the counters and the histogram read back by each call
   unsigned long long* h_stage = nullptr;  // kCtrCount + GB_HIST_BINS
+  // pinned staging for the small inputs and outputs of a call: a copy between
+  // the device and pageable memory waits for the stream before and after it
+  char* h_io = nullptr;  // kIoBytes
+  char* h_ring = nullptr;  // copy_out's pinned ring, allocated by the first large copy
+  cudaEvent_t ring_ev[4] = {};
   std::string err;
 };
 
@@ -116,9 +121,17 @@ gb_status ws_scratch(gb_ctx* c, Workspace& w, size_t bytes, void** p);
 constexpr size_t kKeptBufferBytes = 256ull << 20;
 struct Temps;
 gb_status ws_buffer(gb_ctx* c, Workspace& w, Temps& t, int slot, size_t bytes, void** p);
+constexpr size_t kIoBytes = 1u << 20;
+// Device -> host copy of `bytes` behind the work queued on s.  Small copies and
+// copies into pinned memory are queued; large ones into pageable memory are
+// complete on return (through a pinned ring, several threads emptying it).
+cudaError_t copy_out(Workspace& w, void* dst, const void* src, size_t bytes, cudaStream_t s);
 gb_status ensure_primes(gb_ctx* c, Workspace& w, uint64_t limit);
 // number of primes <= x in the resident table (x <= primes_limit)
 gb_status count_le(gb_ctx* c, Workspace& w, uint64_t x, uint64_t* out);
+// the same or up to kSampleStride more, from the host's tables alone: for bounds
+// that a kernel checks against the primes again (no copy, no wait)
+uint64_t count_bound(const gb_ctx* c, uint64_t x);
 uint64_t isqrt_u64(uint64_t n);
 
 // Temporary device buffers of one call: from the arena when there is one

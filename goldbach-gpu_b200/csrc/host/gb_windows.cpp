@@ -146,9 +146,10 @@ gb_status range_masked(gb_ctx* c, Workspace& ws, Temps& tmp, int slot, const std
   a.chunk_evens = ne;
   a.nbw = range6_words(H, ne);
   const uint64_t bound = masked_bound(top, ne);
-  uint64_t nsmall = 0, nlarge = 0, kc = 0;
+  uint64_t nsmall = 0, kc = 0;
+  const uint64_t nlarge = count_bound(c, root);  // (the pass stops at each window's top)
   gb_status st;
-  if ((st = count_le(c, ws, std::min(bound, root), &nsmall)) != GB_OK || (st = count_le(c, ws, root, &nlarge)) != GB_OK ||
+  if ((st = count_le(c, ws, std::min(bound, root), &nsmall)) != GB_OK ||
       (st = count_le(c, ws, (H / 6 + ne / 3) / 32, &kc)) != GB_OK)
     return st;
   nsmall = std::max<uint64_t>(nsmall, kWheelPrimeCount + 1);
@@ -207,11 +208,12 @@ gb_status range_masked(gb_ctx* c, Workspace& ws, Temps& tmp, int slot, const std
   // one upload: descriptors, masks, records, chunk offsets
   const size_t o_mask = desc.size() * sizeof(WinDesc6), o_wl = (o_mask + masks.size() * sizeof(WinDesc6) + 15) & ~size_t(15);
   const size_t o_off = o_wl + wl.size() * sizeof(WinLarge), bytes = o_off + coff.size() * 8;
-  std::vector<char> up(bytes);
-  std::memcpy(up.data(), desc.data(), desc.size() * sizeof(WinDesc6));
-  std::memcpy(up.data() + o_mask, masks.data(), masks.size() * sizeof(WinDesc6));
-  std::memcpy(up.data() + o_wl, wl.data(), wl.size() * sizeof(WinLarge));
-  std::memcpy(up.data() + o_off, coff.data(), coff.size() * 8);
+  std::vector<char> up_big(bytes <= kIoBytes ? 0 : bytes);  // pageable: staged at the copy
+  char* const up = up_big.empty() ? ws.h_io : up_big.data();
+  std::memcpy(up, desc.data(), desc.size() * sizeof(WinDesc6));
+  std::memcpy(up + o_mask, masks.data(), masks.size() * sizeof(WinDesc6));
+  std::memcpy(up + o_wl, wl.data(), wl.size() * sizeof(WinLarge));
+  std::memcpy(up + o_off, coff.data(), coff.size() * 8);
   void *d_up, *d_mask;
   if ((st = ws_buffer(c, ws, tmp, slot, bytes, &d_up)) != GB_OK ||
       (st = ws_buffer(c, ws, tmp, slot + 1, max_words * 4, &d_mask)) != GB_OK)
@@ -234,7 +236,7 @@ gb_status range_masked(gb_ctx* c, Workspace& ws, Temps& tmp, int slot, const std
   la.pairs = a.s.ctr + kCtrPairs;
   const uint64_t np = la.k1 - la.k0;
   const int gl = (int)std::max<uint64_t>(1, std::min<uint64_t>((np + 511) / 512, (uint64_t)c->sm_count * kLargeBlocksPerSM));
-  cudaError_t e = cudaMemcpyAsync(d_up, up.data(), bytes, cudaMemcpyHostToDevice, s);  // pageable: staged at the call
+  cudaError_t e = cudaMemcpyAsync(d_up, up, bytes, cudaMemcpyHostToDevice, s);
   auto chk = [&](cudaError_t x) {
     if (e == cudaSuccess && x != cudaSuccess) e = x;
   };
@@ -387,26 +389,49 @@ static gb_status windows_sieve_impl(gb_ctx* c, Workspace& ws, Arena* arena, cons
     if ((st = count_le(c, ws, bound, &n)) != GB_OK) return st;
     ta.nsieve[k] = (uint32_t)std::max<uint64_t>(n, kWheelPrimeCount + 1);
   }
-  uint64_t ns = 0, kf = 0, nlarge = 0, kc = 0, kct = 0;
+  uint64_t ns = 0, kc = 0, kct = 0;
+  const uint64_t kf = count_bound(c, p_lim), nlarge = count_bound(c, root);
   if ((st = count_le(c, ws, std::min<uint64_t>(H - 13, p_lim), &ns)) != GB_OK ||
-      (st = count_le(c, ws, p_lim, &kf)) != GB_OK ||
-      (st = count_le(c, ws, root, &nlarge)) != GB_OK ||
       (st = count_le(c, ws, (H / 6 + NE / 3) / 64, &kc)) != GB_OK ||
       (st = count_le(c, ws, tile_words / 2, &kct)) != GB_OK)
     return st;
 
+  // one upload: descriptors, records, chunk offsets, the tested windows' tile
+  // and run offsets, and the plain mode's offsets of single windows
+  const bool plain = o.mode == GB_WINDOWS_PLAIN;
+  const size_t o_wl = (count * sizeof(WinDesc6) + 15) & ~size_t(15);
+  const size_t o_coff = o_wl + count * sizeof(WinLarge);
+  const size_t o_tile = o_coff + (count + 1) * 8, o_run = o_tile + tile_off.size() * 8;
+  const size_t o_cone = o_run + run_off.size() * 8, o_tone = o_cone + (plain ? 2 * count * 8 : 0);
+  const size_t up_bytes = o_tone + (plain ? test_one.size() * 8 : 0);
+  // results: sum and largest minimal p and failures of each window
+  const size_t res_bytes = count * 20;
   Temps tmp(c, arena);
-  void *d_desc, *d_wl, *d_coff, *d_cone, *d_lmask, *d_fail, *d_maxp, *d_psum, *d_minp = nullptr;
-  if ((st = ws_buffer(c, ws, tmp, 0, count * sizeof(WinDesc6), &d_desc)) != GB_OK ||
-      (st = ws_buffer(c, ws, tmp, 1, count * sizeof(WinLarge), &d_wl)) != GB_OK ||
-      (st = ws_buffer(c, ws, tmp, 2, (count + 1 + 2 * tile_off.size()) * 8, &d_coff)) != GB_OK ||
-      (st = ws_buffer(c, ws, tmp, 3, (2 * count + test_one.size()) * 8, &d_cone)) != GB_OK ||
-      (st = ws_buffer(c, ws, tmp, 4, lwords_total * 4, &d_lmask)) != GB_OK ||
-      (st = ws_buffer(c, ws, tmp, 5, count * 4, &d_fail)) != GB_OK ||
-      (st = ws_buffer(c, ws, tmp, 6, count * 8, &d_maxp)) != GB_OK ||
-      (st = ws_buffer(c, ws, tmp, 7, count * 8, &d_psum)) != GB_OK ||
-      (min_p_concat && (st = ws_buffer(c, ws, tmp, 8, total_n * 4, &d_minp)) != GB_OK))
+  void *d_up, *d_lmask, *d_res, *d_minp = nullptr;
+  if ((st = ws_buffer(c, ws, tmp, 0, up_bytes, &d_up)) != GB_OK ||
+      (st = ws_buffer(c, ws, tmp, 1, res_bytes, &d_res)) != GB_OK ||
+      (st = ws_buffer(c, ws, tmp, 2, lwords_total * 4, &d_lmask)) != GB_OK ||
+      (min_p_concat && (st = ws_buffer(c, ws, tmp, 3, total_n * 4, &d_minp)) != GB_OK))
     return st;
+  std::vector<char> up_big(up_bytes <= kIoBytes ? 0 : up_bytes);  // pageable: staged at the copy
+  char* const up = up_big.empty() ? ws.h_io : up_big.data();
+  std::memcpy(up, desc.data(), count * sizeof(WinDesc6));
+  std::memcpy(up + o_wl, wl.data(), count * sizeof(WinLarge));
+  std::memcpy(up + o_coff, chunk_off.data(), (count + 1) * 8);
+  std::memcpy(up + o_tile, tile_off.data(), tile_off.size() * 8);
+  std::memcpy(up + o_run, run_off.data(), run_off.size() * 8);
+  if (plain) {
+    std::memcpy(up + o_cone, chunk_one.data(), 2 * count * 8);
+    if (!test_one.empty()) std::memcpy(up + o_tone, test_one.data(), test_one.size() * 8);
+  }
+  const void* d_desc = d_up;
+  const void* d_wl = (char*)d_up + o_wl;
+  const uint64_t* d_coff = (const uint64_t*)((char*)d_up + o_coff);
+  const uint64_t* d_cone = (const uint64_t*)((char*)d_up + o_cone);
+  const uint64_t* d_tone = (const uint64_t*)((char*)d_up + o_tone);
+  void* const d_psum = d_res;
+  void* const d_maxp = (char*)d_res + count * 8;
+  void* const d_fail = (char*)d_res + count * 16;
 
   RangeArgs a{};
   SearchParams& sp = a.s;
@@ -433,7 +458,7 @@ static gb_status windows_sieve_impl(gb_ctx* c, Workspace& ws, Arena* arena, cons
   a.wheel6 = c->d_wheel6;
   a.a15 = c->d_a15;
   a.win = (const WinDesc6*)d_desc;
-  a.chunk_off = (const uint64_t*)d_coff;
+  a.chunk_off = d_coff;
   a.nwin = (uint32_t)count;
   a.lmask = (const uint32_t*)d_lmask;
   a.total_items = chunk_off[count];
@@ -451,8 +476,8 @@ static gb_status windows_sieve_impl(gb_ctx* c, Workspace& ws, Arena* arena, cons
   la.pairs = sp.ctr + kCtrPairs;
   const size_t ntw = count - nsw;  // tested windows
   ta.win = (const WinDesc6*)d_desc + nsw;
-  ta.tile_off = (const uint64_t*)d_coff + count + 1;
-  ta.run_off = ta.tile_off + ntw + 1;
+  ta.tile_off = (const uint64_t*)((char*)d_up + o_tile);
+  ta.run_off = (const uint64_t*)((char*)d_up + o_run);
   ta.nwin = (uint32_t)ntw;
   ta.tiles = tile_off[ntw];
   ta.runs = run_off[ntw];
@@ -489,22 +514,11 @@ static gb_status windows_sieve_impl(gb_ctx* c, Workspace& ws, Arena* arena, cons
   auto chk = [&](cudaError_t x) {
     if (e == cudaSuccess && x != cudaSuccess) e = x;
   };
-  chk(cudaMemcpyAsync(d_desc, desc.data(), count * sizeof(WinDesc6), cudaMemcpyHostToDevice, s));
-  chk(cudaMemcpyAsync(d_wl, wl.data(), count * sizeof(WinLarge), cudaMemcpyHostToDevice, s));
-  chk(cudaMemcpyAsync(d_coff, chunk_off.data(), (count + 1) * 8, cudaMemcpyHostToDevice, s));
-  chk(cudaMemcpyAsync((uint64_t*)d_coff + count + 1, tile_off.data(), tile_off.size() * 8, cudaMemcpyHostToDevice, s));
-  chk(cudaMemcpyAsync((uint64_t*)d_coff + count + 1 + tile_off.size(), run_off.data(), run_off.size() * 8,
-                      cudaMemcpyHostToDevice, s));
-  chk(cudaMemcpyAsync(d_cone, chunk_one.data(), 2 * count * 8, cudaMemcpyHostToDevice, s));
-  const uint64_t* d_tone = (const uint64_t*)d_cone + 2 * count;
-  if (ntw) chk(cudaMemcpyAsync((void*)d_tone, test_one.data(), test_one.size() * 8, cudaMemcpyHostToDevice, s));
-  chk(cudaMemsetAsync(d_fail, 0, count * 4, s));
-  chk(cudaMemsetAsync(d_maxp, 0, count * 8, s));
-  chk(cudaMemsetAsync(d_psum, 0, count * 8, s));
+  chk(cudaMemcpyAsync(d_up, up, up_bytes, cudaMemcpyHostToDevice, s));
+  chk(cudaMemsetAsync(d_res, 0, res_bytes, s));
   if (d_minp) chk(cudaMemsetAsync(d_minp, 0, total_n * 4, s));
   chk(cudaMemsetAsync(sp.ctr, 0, kCtrCount * 8, s));
   chk(cudaMemsetAsync(sp.ctr + kCtrFirstFail, 0xff, 8, s));
-  chk(cudaStreamSynchronize(s));  // host vectors above are pageable and local
   int launches = 0;
   float large_ms = 0, search_ms = 0;
   chk(cudaEventRecord(ws.ev0, s));
@@ -581,7 +595,7 @@ static gb_status windows_sieve_impl(gb_ctx* c, Workspace& ws, Arena* arena, cons
         t1.nwin = 1;
         t1.tiles = tile_off[r - nsw + 1] - tile_off[r - nsw];
         t1.runs = run_off[r - nsw + 1] - run_off[r - nsw];
-        t1.tile_off = (const uint64_t*)d_tone + 4 * (r - nsw);
+        t1.tile_off = d_tone + 4 * (r - nsw);
         t1.run_off = t1.tile_off + 2;
         chk(cudaMemsetAsync(ta.ctr, 0, 8, s));
         chk(launch_win_presieve(t1, (int)std::min<uint64_t>(t1.tiles, g_pre), s));
@@ -590,7 +604,7 @@ static gb_status windows_sieve_impl(gb_ctx* c, Workspace& ws, Arena* arena, cons
       }
       RangeArgs a1 = a;
       a1.win = (const WinDesc6*)d_desc + r;
-      a1.chunk_off = (const uint64_t*)d_cone + 2 * r;
+      a1.chunk_off = d_cone + 2 * r;
       a1.nwin = 1;
       a1.total_items = chunk_one[2 * r + 1];
       chk(launch_range(a1, (int)std::min<uint64_t>(grid_max, a1.total_items), s));
@@ -599,15 +613,16 @@ static gb_status windows_sieve_impl(gb_ctx* c, Workspace& ws, Arena* arena, cons
     }
   }
   chk(cudaEventRecord(ws.ev1, s));
-  std::vector<uint32_t> fails(count);
-  std::vector<uint64_t> maxp(count), psum(count);
-  unsigned long long ctr[kCtrCount];
-  chk(cudaMemcpyAsync(fails.data(), d_fail, count * 4, cudaMemcpyDeviceToHost, s));
-  chk(cudaMemcpyAsync(maxp.data(), d_maxp, count * 8, cudaMemcpyDeviceToHost, s));
-  chk(cudaMemcpyAsync(psum.data(), d_psum, count * 8, cudaMemcpyDeviceToHost, s));
-  chk(cudaMemcpyAsync(ctr, sp.ctr, sizeof ctr, cudaMemcpyDeviceToHost, s));
-  if (d_minp) chk(cudaMemcpyAsync(min_p_concat, d_minp, total_n * 4, cudaMemcpyDeviceToHost, s));
+  std::vector<char> res_big(res_bytes <= kIoBytes ? 0 : res_bytes);
+  char* const h_res = res_big.empty() ? ws.h_io : res_big.data();
+  unsigned long long* const ctr = ws.h_stage;  // pinned
+  chk(cudaMemcpyAsync(h_res, d_res, res_bytes, cudaMemcpyDeviceToHost, s));
+  chk(cudaMemcpyAsync(ctr, sp.ctr, kCtrCount * 8, cudaMemcpyDeviceToHost, s));
+  if (d_minp) chk(copy_out(ws, min_p_concat, d_minp, total_n * 4, s));
   chk(cudaStreamSynchronize(s));
+  const uint64_t* psum = (const uint64_t*)h_res;
+  const uint64_t* maxp = psum + count;
+  const uint32_t* fails = (const uint32_t*)(maxp + count);
   float ms = 0;
   if (e == cudaSuccess) {
     cudaEventElapsedTime(&ms, ws.ev0, ws.ev1);
@@ -652,15 +667,16 @@ static gb_status windows_mr_impl(gb_ctx* c, Workspace& ws, Arena* arena, const g
   std::vector<uint64_t> off(count + 1, 0);
   for (size_t i = 0; i < count; ++i) off[i + 1] = off[i] + w[i].count;
   total = off[count];
-  uint64_t np = 0;
-  gb_status st = count_le(c, ws, p_lim, &np);
-  if (st != GB_OK) return st;
+  const uint64_t np = count_bound(c, p_lim);  // the kernel stops at p_lim itself
+  gb_status st;
   Temps tmp(c, arena);
   void *d_w, *d_off, *d_n, *d_p, *d_q, *d_agg;
-  if ((st = tmp.get(count * sizeof(gb_window), &d_w, ws)) != GB_OK ||
-      (st = tmp.get((count + 1) * 8, &d_off, ws)) != GB_OK ||
-      (st = tmp.get(total * 8, &d_n, ws)) != GB_OK || (st = tmp.get(total * 8, &d_p, ws)) != GB_OK ||
-      (st = tmp.get(total * 8, &d_q, ws)) != GB_OK || (st = tmp.get(count * 32, &d_agg, ws)) != GB_OK)
+  if ((st = ws_buffer(c, ws, tmp, 0, count * sizeof(gb_window), &d_w)) != GB_OK ||
+      (st = ws_buffer(c, ws, tmp, 1, (count + 1) * 8, &d_off)) != GB_OK ||
+      (st = ws_buffer(c, ws, tmp, 2, total * 8, &d_n)) != GB_OK ||
+      (st = ws_buffer(c, ws, tmp, 3, total * 8, &d_p)) != GB_OK ||
+      (st = ws_buffer(c, ws, tmp, 4, total * 8, &d_q)) != GB_OK ||
+      (st = ws_buffer(c, ws, tmp, 5, count * 32, &d_agg)) != GB_OK)
     return st;
   cudaStream_t s = o.stream ? (cudaStream_t)o.stream : c->stream;
   cudaError_t e = cudaSuccess;
