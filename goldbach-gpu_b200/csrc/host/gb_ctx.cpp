@@ -71,12 +71,30 @@ void dev_free(gb_ctx* c, void* p) {
   cudaFree(p);
 }
 
+// dev_alloc for a workspace's call: when there is no room, the kept buffers
+// the call has not asked for are given back first.
+static gb_status ws_alloc(gb_ctx* c, Workspace& w, size_t bytes, void** p) {
+  gb_status st = dev_alloc(c, p, bytes, &w.err);
+  if (st != GB_ENOMEM) return st;
+  bool freed = false;
+  for (int i = 0; i < 2 * Workspace::kBufSlots; ++i)
+    if (w.buf[i] && !((w.buf_used >> i) & 1u)) {
+      dev_free(c, w.buf[i]);
+      w.buf[i] = nullptr;
+      w.buf_bytes[i] = 0;
+      freed = true;
+    }
+  if (!freed) return st;
+  w.err.clear();
+  return dev_alloc(c, p, bytes, &w.err);
+}
+
 gb_status Temps::get(size_t bytes, void** p, Workspace& w) {
   if (arena) {
     *p = arena->take(bytes);
     return *p ? GB_OK : fail(w, GB_ENOMEM, "serving arena exhausted");
   }
-  gb_status st = dev_alloc(c, p, bytes, &w.err);
+  gb_status st = ws_alloc(c, w, bytes, p);
   if (st == GB_OK) owned.push_back(*p);
   return st;
 }
@@ -109,7 +127,7 @@ gb_status ws_scratch(gb_ctx* c, Workspace& w, size_t bytes, void** p) {
     dev_free(c, w.scratch);
     w.scratch = nullptr;
     w.scratch_bytes = 0;
-    gb_status st = dev_alloc(c, &w.scratch, bytes, &w.err);
+    gb_status st = ws_alloc(c, w, bytes, &w.scratch);
     if (st != GB_OK) return st;
     w.scratch_bytes = bytes;
   }
@@ -119,21 +137,23 @@ gb_status ws_scratch(gb_ctx* c, Workspace& w, size_t bytes, void** p) {
 
 gb_status ws_buffer(gb_ctx* c, Workspace& w, Temps& t, int slot, size_t bytes, void** p) {
   if (t.arena || bytes > kKeptBufferBytes || slot >= Workspace::kBufSlots) return t.get(bytes, p, w);
+  if (bytes > kBigBufferBytes) slot += Workspace::kBufSlots;
   if (bytes > w.buf_bytes[slot]) {
     dev_free(c, w.buf[slot]);
     w.buf[slot] = nullptr;
     w.buf_bytes[slot] = 0;
     const size_t grow = std::max<size_t>(bytes, 64 << 10);
-    gb_status st = dev_alloc(c, &w.buf[slot], grow, &w.err);
+    gb_status st = ws_alloc(c, w, grow, &w.buf[slot]);
     if (st != GB_OK) return st;
     w.buf_bytes[slot] = grow;
   }
+  w.buf_used |= 1u << slot;
   *p = w.buf[slot];
   return GB_OK;
 }
 
 void ws_free(gb_ctx* c, Workspace& w) {
-  for (int i = 0; i < Workspace::kBufSlots; ++i) {
+  for (int i = 0; i < 2 * Workspace::kBufSlots; ++i) {
     dev_free(c, w.buf[i]);
     w.buf[i] = nullptr;
     w.buf_bytes[i] = 0;
@@ -325,9 +345,9 @@ gb_status ensure_primes(gb_ctx* c, Workspace& w, uint64_t limit) {
   uint32_t *bits, *blocks;
   unsigned long long* total;
   gb_status st;
-  if ((st = dev_alloc(c, (void**)&primes, cap * 4, &w.err)) != GB_OK) return st;
-  if ((st = dev_alloc(c, (void**)&magic, cap * 8, &w.err)) != GB_OK ||
-      (st = dev_alloc(c, (void**)&a15, cap * 8, &w.err)) != GB_OK ||
+  if ((st = ws_alloc(c, w, cap * 4, (void**)&primes)) != GB_OK) return st;
+  if ((st = ws_alloc(c, w, cap * 8, (void**)&magic)) != GB_OK ||
+      (st = ws_alloc(c, w, cap * 8, (void**)&a15)) != GB_OK ||
       (st = t.get(((nbits_max + 31) / 32 + 4) * 4, (void**)&bits, w)) != GB_OK ||
       (st = t.get((nblk + 1) * 4, (void**)&blocks, w)) != GB_OK ||
       (st = t.get(8, (void**)&total, w)) != GB_OK) {
@@ -895,6 +915,7 @@ uint64_t gb_num_segments(uint64_t start, uint64_t limit, uint64_t seg_size) {
     std::lock_guard<std::mutex> lk(ctx->mu);  \
     cudaSetDevice(ctx->device);               \
     ctx->ws.err.clear();                      \
+    ctx->ws.buf_used = 0;                     \
     const gb_status st_ = (call);             \
     ctx->err = ctx->ws.err;                   \
     return st_;                               \

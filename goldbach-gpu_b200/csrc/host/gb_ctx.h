@@ -50,9 +50,12 @@ struct Workspace {
   size_t scratch_bytes = 0;
   // per-call device buffers of the public entry points (slot i grown on
   // demand and kept, up to kKeptBufferBytes; larger ones are per call)
+  // (entries kBufSlots and up: the slots' buffers above kBigBufferBytes, so that
+  // a call with small needs does not hold on to another's large buffers)
   static constexpr int kBufSlots = 8;
-  void* buf[kBufSlots] = {};
-  size_t buf_bytes[kBufSlots] = {};
+  void* buf[2 * kBufSlots] = {};
+  size_t buf_bytes[2 * kBufSlots] = {};
+  uint32_t buf_used = 0;  // slots handed out in the current call
   // pinned staging for the counters and the histogram read back by each call
   unsigned long long* h_stage = nullptr;  // kCtrCount + GB_HIST_BINS
   // pinned staging for the small inputs and outputs of a call: a copy between
@@ -117,8 +120,10 @@ void ws_free(gb_ctx* c, Workspace& w);
 gb_status ws_scratch(gb_ctx* c, Workspace& w, size_t bytes, void** p);
 // Per-call device buffers kept between calls (no cudaMalloc / cudaFree per
 // call for the usual sizes): slot `slot` of the workspace, grown to `bytes`;
-// above kKeptBufferBytes the buffer comes from `t` and is freed with it.
-constexpr size_t kKeptBufferBytes = 256ull << 20;
+// above kKeptBufferBytes the buffer comes from `t` and is freed with it.  Kept
+// buffers the current call has not asked for are given back when an
+// allocation fails for want of memory or budget.
+constexpr size_t kKeptBufferBytes = 1ull << 30, kBigBufferBytes = 32ull << 20;
 struct Temps;
 gb_status ws_buffer(gb_ctx* c, Workspace& w, Temps& t, int slot, size_t bytes, void** p);
 constexpr size_t kIoBytes = 1u << 20;

@@ -62,3 +62,21 @@ def test_wide_window_agrees_with_the_full_sieve(ctx):
     a, _, sa = ctx.verify_windows(starts, counts, mr_divisor=1)
     b, _, sb = ctx.verify_windows(starts, counts, mr_below=1)
     assert a == b and sa["sieved_windows"] == 0 and sb["sieved_windows"] == 2
+
+
+def test_kept_buffers_are_given_back(gbmod):
+    """A context whose budget the masks of a wide batch nearly fill: later calls
+    that need the room get it, and the same results as in a roomy context."""
+    starts = np.array([10**13 + 2], dtype=np.uint64)
+    counts = np.array([2 * 10**9], dtype=np.uint64)  # 170 MB of masks
+    want = None
+    for budget in (0, 720 << 20):  # the range call alone holds 684 MB
+        with gbmod.Context(0, budget=budget) as c:
+            a, _, _ = c.verify_windows(starts, counts)
+            r = c.verify_range(10**12, 10**12 + 2 * (10**8 - 1), want_minp=True)  # 400 MB out
+            b, _, _ = c.verify_windows(starts, counts)
+            got = (a, b, int(r.min_p.astype(np.uint64).sum()))
+            held, room = c.mem_info()
+            assert held <= room
+        want = want or got
+        assert got == want and a == b
