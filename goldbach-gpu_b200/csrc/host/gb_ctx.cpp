@@ -576,7 +576,8 @@ gb_status range_impl(gb_ctx* c, Workspace& w, Arena* arena, uint64_t start, uint
     // bits past the last n are zero (pageable source: staged at the call)
     if (count & 31) chk(cudaMemcpyAsync(sp.vbits + vwords - 1, &last_word, 4, cudaMemcpyHostToDevice, s));
   }
-  if (sp.minp) chk(cudaMemsetAsync(sp.minp, 0, count * 4, s));
+  // (the chunks write every n of their segments; other shards' stay 0)
+  if (sp.minp && sc > 1) chk(cudaMemsetAsync(sp.minp, 0, count * 4, s));
   if (sp.unit_hist) chk(cudaMemsetAsync(sp.unit_hist, 0, nseg * GB_HIST_BINS * 8, s));
   if (!o.on_device && (sp.unit_fallbacks || sp.unit_failures)) {
     uint32_t* const both = sp.unit_fallbacks ? sp.unit_fallbacks : sp.unit_failures - nseg;

@@ -516,7 +516,6 @@ static gb_status windows_sieve_impl(gb_ctx* c, Workspace& ws, Arena* arena, cons
   };
   chk(cudaMemcpyAsync(d_up, up, up_bytes, cudaMemcpyHostToDevice, s));
   chk(cudaMemsetAsync(d_res, 0, res_bytes, s));
-  if (d_minp) chk(cudaMemsetAsync(d_minp, 0, total_n * 4, s));
   chk(cudaMemsetAsync(sp.ctr, 0, kCtrCount * 8, s));
   chk(cudaMemsetAsync(sp.ctr + kCtrFirstFail, 0xff, 8, s));
   int launches = 0;

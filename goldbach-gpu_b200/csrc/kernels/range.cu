@@ -58,6 +58,7 @@ __global__ void __launch_bounds__(NT, 1024 / NT) range6_kernel(const __grid_cons
   for (uint32_t i = tid; i < kWheel6Words; i += NT) pat6[i] = a.wheel6[i];
   if (tid == 0) {
     cx.nbw = a.nbw;
+    cx.xbytes = MINP ? eidx6_class_bytes(a.chunk_evens) : 0;
     cx.surv = a.surv + (size_t)blockIdx.x * 6 * a.surv_cap;
     cx.surv_cap = a.surv_cap;
   }
@@ -93,10 +94,6 @@ __global__ void __launch_bounds__(NT, 1024 / NT) range6_kernel(const __grid_cons
       cx.maxk = 0;
     }
     for (uint32_t i = tid; i < kSmemHistBins; i += NT) HIST[i] = 0;
-    if (MINP) {  // no n resolved yet
-      uint32_t* X = reinterpret_cast<uint32_t*>(smem6_eidx());
-      for (uint32_t i = tid; i < a.chunk_evens / 4; i += NT) X[i] = 0xffffffffu;
-    }
     __syncthreads();
     const unsigned long long item = s_item;
     if (item >= a.total_items) break;

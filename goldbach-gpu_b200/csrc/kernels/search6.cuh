@@ -68,12 +68,14 @@ constexpr int kWT6 = 8;                      // U words per lane per warp task (
                                              // paired levels and the faster sieve,
                                              // 7: 449.7, 8: 436.9, 9: 437.9 ms)
 constexpr uint32_t kTaskWords6 = 32 * kWT6;  // words per warp task
+constexpr int kWTM6 = 4;  // the same with per-n output, whose level 0 holds 5 bit planes a word
 
 // Per-CTA search context (static shared memory): the class tables' lengths
 // (fixed for the kernel) and the current chunk (written by one thread
 // before the sieve).
 struct Ctx6 {
   uint32_t nbw;      // words of each class bitset
+  uint32_t xbytes;   // per-n output: bytes of each class's entry positions
   uint32_t len[3];   // lockstep entries of each class (<= kLockSteps6)
   uint32_t kend[3];  // prime index after each class's last lockstep entry
   // the chunk
@@ -120,12 +122,17 @@ __device__ __forceinline__ uint32_t* smem6_etab(int ri) {
   return smem6_hist() + kSmemHistBins + ri * kLockSteps6;
 }
 // per-n output: the entry position of each n of the chunk resolved in the
-// lockstep (0xFF: resolved elsewhere, its minimal p written directly)
-__device__ __forceinline__ uint8_t* smem6_eidx() {
-  return reinterpret_cast<uint8_t*>(smem6_etab(0) + 3 * kLockSteps6);
+// lockstep (0xFF: resolved elsewhere, its minimal p written directly), class
+// by class, 32 bytes per U word
+__host__ __device__ constexpr uint32_t eidx6_class_bytes(uint32_t chunk) { return 32 * ((chunk / 3 + 2 + 31) / 32); }
+__device__ __forceinline__ uint8_t* smem6_eidx(int ri) {
+  const uint32_t words = kWheel6Words + 2 * g_cx6.nbw + kSmemHistBins + 3 * kLockSteps6;
+  return reinterpret_cast<uint8_t*>(g_smem6 + ((words + 3) & ~3u)) + ri * g_cx6.xbytes;
 }
-__host__ __device__ constexpr size_t range6_smem_words(uint32_t nbw, uint32_t eidx_bytes = 0) {
-  return kWheel6Words + 2 * (size_t)nbw + kSmemHistBins + 3 * kLockSteps6 + (eidx_bytes + 3) / 4;
+// chunk: even n per chunk with per-n output, 0 without
+__host__ __device__ constexpr size_t range6_smem_words(uint32_t nbw, uint32_t chunk = 0) {
+  return kWheel6Words + 2 * (size_t)nbw + kSmemHistBins + 3 * kLockSteps6 +
+         (chunk ? 3 + 3 * eidx6_class_bytes(chunk) / 4 : 0);
 }
 
 __device__ __forceinline__ uint32_t e6_u(uint32_t e) { return e & ((1u << kE6UBits) - 1); }
@@ -177,6 +184,7 @@ __device__ __noinline__ void tail_one6(const SearchParams& s, int ri, uint32_t m
   }
   // every window prime p <= n/2 tried: the Phase-2 queue or a failure
   const uint64_t lim = half < s.p_lim ? half : s.p_lim;
+  if (MINP) s.minp[idx] = 0;  // until the Phase 2 finds one
   if (past_half || s.nsearch >= s.nprimes || s.primes[s.nsearch] > lim) {
     atomicAdd(&s.ctr[kCtrFailures], 1ull);
     atomicMin(&s.ctr[kCtrFirstFail], (unsigned long long)n);
@@ -235,37 +243,60 @@ struct Cache6 {
   }
 };
 
-// One lockstep step: the U words of a lane against one prime p.  No mask
-// for p > n/2 is needed: a partition n = p + q
-// with q < p would have been found at the smaller prime q, which is in the
-// same class sequence, and every q < 5 reads a cleared bit.
-// With per-n output (MINP) the entry position pos of every n the step
-// resolves goes to the chunk's byte array at the n's index in the chunk
-// (jbase + 3 m for bit m of the class); the chunk writes the minimal p out
-// in n order at its end (search_chunk6).
-template <bool MINP, int WT, typename Words>
+// One lockstep step of the later levels with per-n output: the U words of a lane
+// against one prime p.  No mask for p > n/2 is needed (here and in level 0): a
+// partition n = p + q with q < p would have been found at the smaller prime q,
+// which is in the same class sequence, and every q < 5 reads a cleared bit.
+// The entry position pos of every n the step resolves goes to the class's
+// bytes X; the chunk writes the minimal p out in n order at its end.
+template <int WT, typename Words>
 __device__ __forceinline__ uint32_t step6(uint32_t (&U)[WT], const uint32_t (&lo)[WT],
                                           const uint32_t (&hi)[WT], uint32_t sh, uint32_t pos,
-                                          const Words& W, uint32_t jbase) {  // pos, jbase: MINP only
+                                          const Words& W, uint8_t* X) {
   uint32_t cnt = 0;
-  uint8_t* X = smem6_eidx();
 #pragma unroll
   for (int i = 0; i < WT; ++i) {
     uint32_t h = U[i] & __funnelshift_r(lo[i], hi[i], sh);
     U[i] ^= h;
     cnt += __popc(h);
-    if (MINP) {
-      if (h) {
-        const uint32_t m0 = 32 * W[i];
-        while (h) {
-          const int b = __ffs(h) - 1;
-          h &= h - 1;
-          X[jbase + 3 * (m0 + b)] = (uint8_t)pos;
-        }
-      }
+    while (h) {
+      const int b = __ffs(h) - 1;
+      h &= h - 1;
+      X[32 * W[i] + b] = (uint8_t)pos;
     }
   }
   return cnt;
+}
+
+// 8 bit planes of 32 n to 32 bytes: a 4 x 4 byte transposition, then 8 x 8 bit
+// transpositions (three swaps each, Warren, "Hacker's Delight", 7-3).  out[2k],
+// out[2k + 1] hold the n 8k .. 8k + 7.
+__device__ __forceinline__ void planes_to_bytes(const uint32_t (&p)[8], uint32_t (&out)[8]) {
+  uint32_t col[2][4];  // byte k of planes 0..3 and of planes 4..7
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    const uint32_t a = __byte_perm(p[4 * h], p[4 * h + 1], 0x5140), c = __byte_perm(p[4 * h], p[4 * h + 1], 0x7362);
+    const uint32_t b = __byte_perm(p[4 * h + 2], p[4 * h + 3], 0x5140);
+    const uint32_t d = __byte_perm(p[4 * h + 2], p[4 * h + 3], 0x7362);
+    col[h][0] = __byte_perm(a, b, 0x5410);
+    col[h][1] = __byte_perm(a, b, 0x7632);
+    col[h][2] = __byte_perm(c, d, 0x5410);
+    col[h][3] = __byte_perm(c, d, 0x7632);
+  }
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    uint32_t x[2] = {col[0][k], col[1][k]};
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      uint32_t t = (x[h] ^ (x[h] >> 7)) & 0x00AA00AAu;
+      x[h] ^= t ^ (t << 7);
+      t = (x[h] ^ (x[h] >> 14)) & 0x0000CCCCu;
+      x[h] ^= t ^ (t << 14);
+    }
+    const uint32_t t = (x[0] ^ (x[1] << 4)) & 0xF0F0F0F0u;
+    out[2 * k] = x[0] ^ t;
+    out[2 * k + 1] = x[1] ^ (t >> 4);
+  }
 }
 
 // One warp task of class ri (rho = 2 ri) at level L, through the entries
@@ -281,17 +312,19 @@ __device__ __forceinline__ uint32_t step6(uint32_t (&U)[WT], const uint32_t (&lo
 // loop around it keeps nothing live across the call), and it calls nothing.
 template <bool MINP, bool LISTED>
 __device__ __noinline__ void search_task6(const SearchParams& s, int ri, uint32_t task, int L) {
+  constexpr int WT = MINP ? kWTM6 : kWT6;
+  constexpr uint32_t TW = 32 * WT;  // words of the task
   const Ctx6& cx = g_cx6;
   const int lane = threadIdx.x & 31;
   const uint64_t n0 = cx.n[ri];
-  uint32_t U[kWT6];
-  typename std::conditional<LISTED, WordsListed<kWT6>, WordsStrided>::type W;
+  uint32_t U[WT];
+  typename std::conditional<LISTED, WordsListed<WT>, WordsStrided>::type W;
   if constexpr (!LISTED) {
     const uint32_t M = cx.M[ri];
     const uint32_t nuw = (M + 31) >> 5;
-    W.base = task * kTaskWords6 + lane;
+    W.base = task * TW + lane;
 #pragma unroll
-    for (int i = 0; i < kWT6; ++i) {
+    for (int i = 0; i < WT; ++i) {
       const uint32_t w = W[i];
       uint32_t mk = 0;
       if (w < nuw) {
@@ -310,8 +343,8 @@ __device__ __noinline__ void search_task6(const SearchParams& s, int ri, uint32_
     const uint2* in = surv6_list((L - 1) & 1, ri);
     const uint32_t cnt_in = cx.scnt[L - 1][ri];
 #pragma unroll
-    for (int i = 0; i < kWT6; ++i) {
-      const uint32_t j = task * kTaskWords6 + lane + 32 * i;
+    for (int i = 0; i < WT; ++i) {
+      const uint32_t j = task * TW + lane + 32 * i;
       const uint2 v = j < cnt_in ? in[j] : make_uint2(0u, 0u);
       W.w[i] = v.x;
       U[i] = v.y;
@@ -322,20 +355,19 @@ __device__ __noinline__ void search_task6(const SearchParams& s, int ri, uint32_
   const uint32_t* __restrict__ Q5 = smem6_q(1);
   uint32_t* HIST = smem6_hist();
   const uint32_t K1 = cx.K[ri][0], K5 = cx.K[ri][1];
-  const uint32_t jbase = (uint32_t)((n0 - cx.A) >> 1);  // index of n0 in the chunk
-  Cache6<kWT6> ca;
+  Cache6<WT> ca;
   // without per-n output the step clears bits with one operation per word
   // and counts the lane's unresolved n: resolved = live before - live after
   uint32_t live = 0;
   if (!MINP) {
 #pragma unroll
-    for (int i = 0; i < kWT6; ++i) live += __popc(U[i]);
+    for (int i = 0; i < WT; ++i) live += __popc(U[i]);
   }
   const uint32_t pos0 = level6_start(L), pend = level6_end(ri, L);
   if constexpr (!MINP) {
     // Without per-n output every level steps in pairs (its span starts at
     // an even entry: 0, 32, 44 or 60): the two steps' counts, at most
-    // kWT6 * 32 * 32 = 8192 each, share one warp reduction packed in the
+    // WT * 32 * 32 = 8192 each, share one warp reduction packed in the
     // halves of a word, and the early-exit vote comes every fourth pair.
     // Each step clears the q-prime bits of the lane's words and counts the
     // lane's unresolved n: resolved = live before - live after.
@@ -347,7 +379,7 @@ __device__ __noinline__ void search_task6(const SearchParams& s, int ri, uint32_
       const uint32_t sh = off & 31;
       uint32_t now = 0;
 #pragma unroll
-      for (int i = 0; i < kWT6; ++i) {
+      for (int i = 0; i < WT; ++i) {
         U[i] &= ~__funnelshift_r(ca.lo[i], ca.hi[i], sh);
         now += __popc(U[i]);
       }
@@ -362,7 +394,7 @@ __device__ __noinline__ void search_task6(const SearchParams& s, int ri, uint32_
       if (((pos - pos0) & 7) == 0) {
         uint32_t any = 0;
 #pragma unroll
-        for (int i = 0; i < kWT6; ++i) any |= U[i];
+        for (int i = 0; i < WT; ++i) any |= U[i];
         if (!__any_sync(0xffffffffu, any)) {
           done = true;
           break;
@@ -382,7 +414,93 @@ __device__ __noinline__ void search_task6(const SearchParams& s, int ri, uint32_
       const uint32_t v = __reduce_add_sync(0xffffffffu, step(e));
       if (lane == 0 && v) atomicAdd(&HIST[e6_k(e)], v);
     }
-  } else {  // per-n output: one step at a time, each recording its entry position
+  } else if constexpr (!LISTED) {
+    // Per-n output, level 0: the entry position (0 .. 31) that resolved each n,
+    // as 5 bit planes per word.  Four entries at a time: bit 0 of the position
+    // is collected at the odd steps, bit 1 over the second half, and the higher
+    // bits, the same for the four, from what the four resolved.
+    static_assert(level6_start(1) <= 32, "level 0's positions take 5 bits");
+    uint32_t P0[WT], P1[WT], P2[WT], P3[WT], P4[WT];
+    uint32_t live = 0;
+#pragma unroll
+    for (int i = 0; i < WT; ++i) {
+      P0[i] = P1[i] = P2[i] = P3[i] = P4[i] = 0;
+      live += __popc(U[i]);
+    }
+    auto step = [&](uint32_t pos, bool odd) -> uint32_t {  // returns e's prime index and the count
+      const uint32_t e = E[pos];
+      const uint32_t q5 = e >> 31;
+      const uint32_t off = (q5 ? K5 : K1) - e6_u(e);
+      const uint32_t wo = off >> 5;
+      ca.at(q5 ? Q5 : Q1, wo, wo | (q5 << 31), W);
+      const uint32_t sh = off & 31;
+      uint32_t now = 0;
+#pragma unroll
+      for (int i = 0; i < WT; ++i) {
+        const uint32_t f = __funnelshift_r(ca.lo[i], ca.hi[i], sh);
+        if (odd) P0[i] |= U[i] & f;
+        U[i] &= ~f;
+        now += __popc(U[i]);
+      }
+      const uint32_t c = live - now;
+      live = now;
+      return c;
+    };
+    uint32_t U0[WT];  // before any entry
+#pragma unroll
+    for (int i = 0; i < WT; ++i) U0[i] = U[i];
+#pragma unroll 1
+    for (uint32_t pos = pos0; pos < pend; pos += 4) {
+      if ((pos & 7) == 0) {
+        uint32_t any = 0;
+#pragma unroll
+        for (int i = 0; i < WT; ++i) any |= U[i];
+        if (!__any_sync(0xffffffffu, any)) break;
+      }
+      uint32_t Ua[WT], Ub[WT];
+#pragma unroll
+      for (int i = 0; i < WT; ++i) Ua[i] = U[i];
+      uint32_t c01 = step(pos, false);
+      if (pos + 1 < pend) c01 |= step(pos + 1, true) << 16;
+#pragma unroll
+      for (int i = 0; i < WT; ++i) Ub[i] = U[i];
+      uint32_t c23 = 0;
+      if (pos + 2 < pend) c23 = step(pos + 2, false);
+      if (pos + 3 < pend) c23 |= step(pos + 3, true) << 16;
+      const uint32_t m2 = pos & 4 ? ~0u : 0u, m3 = pos & 8 ? ~0u : 0u, m4 = pos & 16 ? ~0u : 0u;
+#pragma unroll
+      for (int i = 0; i < WT; ++i) {
+        P1[i] |= Ub[i] & ~U[i];
+        const uint32_t g = Ua[i] & ~U[i];
+        P2[i] |= g & m2;
+        P3[i] |= g & m3;
+        P4[i] |= g & m4;
+      }
+      const uint32_t v = __reduce_add_sync(0xffffffffu, c01), u = __reduce_add_sync(0xffffffffu, c23);
+      if (lane == 0) {
+        if (v & 0xffffu) atomicAdd(&HIST[e6_k(E[pos])], v & 0xffffu);
+        if (v >> 16) atomicAdd(&HIST[e6_k(E[pos + 1])], v >> 16);
+        if (u & 0xffffu) atomicAdd(&HIST[e6_k(E[pos + 2])], u & 0xffffu);
+        if (u >> 16) atomicAdd(&HIST[e6_k(E[pos + 3])], u >> 16);
+      }
+    }
+    // the positions as bytes, 0xFF where level 0 resolved nothing
+    uint8_t* X = smem6_eidx(ri);
+    const uint32_t nuw = (cx.M[ri] + 31) >> 5;
+#pragma unroll
+    for (int i = 0; i < WT; ++i) {
+      const uint32_t none = ~(U0[i] & ~U[i]);
+      const uint32_t p[8] = {P0[i] | none, P1[i] | none, P2[i] | none, P3[i] | none, P4[i] | none, none, none, none};
+      uint32_t o[8];
+      planes_to_bytes(p, o);
+      if (W[i] < nuw) {
+        uint4* x = reinterpret_cast<uint4*>(X + 32 * W[i]);
+        x[0] = make_uint4(o[0], o[1], o[2], o[3]);
+        x[1] = make_uint4(o[4], o[5], o[6], o[7]);
+      }
+    }
+  } else {  // per-n output, later levels: one step at a time, each recording its entry position
+    uint8_t* X = smem6_eidx(ri);
     uint32_t held = 0, kheld = 0;  // a step's count waiting for the next step's
     bool pending = false;          // (warp-uniform)
 #pragma unroll 1
@@ -390,7 +508,7 @@ __device__ __noinline__ void search_task6(const SearchParams& s, int ri, uint32_
       if (((pos - pos0) & 7) == 0) {
         uint32_t any = 0;
 #pragma unroll
-        for (int i = 0; i < kWT6; ++i) any |= U[i];
+        for (int i = 0; i < WT; ++i) any |= U[i];
         if (!__any_sync(0xffffffffu, any)) break;
       }
       const uint32_t e = E[pos];
@@ -398,9 +516,9 @@ __device__ __noinline__ void search_task6(const SearchParams& s, int ri, uint32_
       const uint32_t off = (q5 ? K5 : K1) - e6_u(e);
       const uint32_t wo = off >> 5;
       ca.at(q5 ? Q5 : Q1, wo, wo | (q5 << 31), W);
-      const uint32_t cnt = step6<MINP, kWT6>(U, ca.lo, ca.hi, off & 31, pos, W, jbase);
-      // two steps' counts (at most kWT6 * 32 * 32 = 8192 each) share one warp
-      // reduction, packed in the two halves of a word
+      const uint32_t cnt = step6<WT>(U, ca.lo, ca.hi, off & 31, pos, W, X);
+      // two steps' counts (at most 32 WT 32 each) share one warp reduction,
+      // packed in the two halves of a word
       if (pending) {
         const uint32_t v = __reduce_add_sync(0xffffffffu, held | (cnt << 16));
         if (lane == 0) {
@@ -424,7 +542,7 @@ __device__ __noinline__ void search_task6(const SearchParams& s, int ri, uint32_
     uint32_t* out_cnt = &g_cx6.scnt[L][ri];
     const uint32_t lt = (1u << lane) - 1;
 #pragma unroll
-    for (int i = 0; i < kWT6; ++i) {
+    for (int i = 0; i < WT; ++i) {
       const uint32_t alive = __ballot_sync(0xffffffffu, U[i] != 0);
       if (alive) {
         uint32_t base = 0;
@@ -437,8 +555,8 @@ __device__ __noinline__ void search_task6(const SearchParams& s, int ri, uint32_
     uint2* in = surv6_list((L - 1) & 1, ri);
     const uint32_t cnt_in = cx.scnt[L - 1][ri];
 #pragma unroll
-    for (int i = 0; i < kWT6; ++i) {
-      const uint32_t j = task * kTaskWords6 + lane + 32 * i;
+    for (int i = 0; i < WT; ++i) {
+      const uint32_t j = task * TW + lane + 32 * i;
       if (j < cnt_in) in[j].y = U[i];
     }
   }
@@ -453,19 +571,20 @@ __device__ __noinline__ void search_task6(const SearchParams& s, int ri, uint32_
 // argument: one call site per level made ptxas spill in every task.)
 template <bool MINP, int NT>
 __device__ __forceinline__ void search_chunk6(const SearchParams& s) {
+  constexpr uint32_t TW = 32 * (MINP ? kWTM6 : kWT6);  // words per warp task
   const int tid = threadIdx.x;
   const int lane = tid & 31;
 #pragma unroll 1
   for (int l = 0; l < kLevels6; ++l) {
     uint32_t b0, b2, b4;
     if (l == 0) {  // every word of the chunk
-      b0 = (((g_cx6.M[0] + 31) >> 5) + kTaskWords6 - 1) / kTaskWords6;
-      b2 = (((g_cx6.M[1] + 31) >> 5) + kTaskWords6 - 1) / kTaskWords6;
-      b4 = (((g_cx6.M[2] + 31) >> 5) + kTaskWords6 - 1) / kTaskWords6;
+      b0 = (((g_cx6.M[0] + 31) >> 5) + TW - 1) / TW;
+      b2 = (((g_cx6.M[1] + 31) >> 5) + TW - 1) / TW;
+      b4 = (((g_cx6.M[2] + 31) >> 5) + TW - 1) / TW;
     } else {  // the survivor lists of the level before
-      b0 = (g_cx6.scnt[l - 1][0] + kTaskWords6 - 1) / kTaskWords6;
-      b2 = (g_cx6.scnt[l - 1][1] + kTaskWords6 - 1) / kTaskWords6;
-      b4 = (g_cx6.scnt[l - 1][2] + kTaskWords6 - 1) / kTaskWords6;
+      b0 = (g_cx6.scnt[l - 1][0] + TW - 1) / TW;
+      b2 = (g_cx6.scnt[l - 1][1] + TW - 1) / TW;
+      b4 = (g_cx6.scnt[l - 1][2] + TW - 1) / TW;
     }
     for (;;) {
       uint32_t task = 0;
@@ -496,17 +615,17 @@ __device__ __forceinline__ void search_chunk6(const SearchParams& s) {
   // the chunk's figures: the tails' (in g_cx6) plus fallbacks, largest and
   // summed minimal p read off the histogram
   __syncthreads();
-  if (MINP) {  // the lockstep's minimal p of every n, written out in n order
-    const uint8_t* X = smem6_eidx();
-    const uint32_t cnt = g_cx6.cnt;
-    const uint32_t amod = (uint32_t)(g_cx6.A % 6);
+  if (MINP) {  // the lockstep's minimal p of every n, three neighbours (one of each class) per thread
     uint32_t* out = s.minp + g_cx6.base_idx;
-    for (uint32_t j = tid; j < cnt; j += NT) {
-      const uint32_t e = X[j];
-      if (e != 0xFFu) {
-        const int ri = (int)(((amod + 2 * (j % 3)) % 6) >> 1);  // (A + 2j) mod 6 = 2 ri
-        const uint32_t en = smem6_etab(ri)[e];
-        out[j] = 6 * e6_u(en) + e6_pmod(ri, en >> 31);
+    const uint32_t most = max(g_cx6.M[0], max(g_cx6.M[1], g_cx6.M[2]));
+    for (uint32_t m = tid; m < most; m += NT) {
+#pragma unroll
+      for (int ri = 0; ri < 3; ++ri) {
+        const uint32_t e = m < g_cx6.M[ri] ? smem6_eidx(ri)[m] : 0xFFu;
+        if (e != 0xFFu) {
+          const uint32_t en = smem6_etab(ri)[e];
+          out[(uint32_t)((g_cx6.n[ri] - g_cx6.A) >> 1) + 3 * m] = 6 * e6_u(en) + e6_pmod(ri, en >> 31);
+        }
       }
     }
   }
