@@ -68,7 +68,9 @@ constexpr int kWT6 = 8;                      // U words per lane per warp task (
                                              // paired levels and the faster sieve,
                                              // 7: 449.7, 8: 436.9, 9: 437.9 ms)
 constexpr uint32_t kTaskWords6 = 32 * kWT6;  // words per warp task
-constexpr int kWTM6 = 4;  // the same with per-n output, whose level 0 holds 5 bit planes a word
+constexpr int kWTM6 = 4;   // the same with per-n output, whose level 0 holds 5 bit planes a word,
+constexpr int kWTML6 = 1;  // and its later levels: the 2^16-n chunks leave them few words (2^28
+                           // n near 1e9: 4: 1072, 3: 1065, 2: 1049, 1: 1010 us)
 
 // Per-CTA search context (static shared memory): the class tables' lengths
 // (fixed for the kernel) and the current chunk (written by one thread
@@ -312,7 +314,7 @@ __device__ __forceinline__ void planes_to_bytes(const uint32_t (&p)[8], uint32_t
 // loop around it keeps nothing live across the call), and it calls nothing.
 template <bool MINP, bool LISTED>
 __device__ __noinline__ void search_task6(const SearchParams& s, int ri, uint32_t task, int L) {
-  constexpr int WT = MINP ? kWTM6 : kWT6;
+  constexpr int WT = !MINP ? kWT6 : LISTED ? kWTML6 : kWTM6;
   constexpr uint32_t TW = 32 * WT;  // words of the task
   const Ctx6& cx = g_cx6;
   const int lane = threadIdx.x & 31;
@@ -571,20 +573,20 @@ __device__ __noinline__ void search_task6(const SearchParams& s, int ri, uint32_
 // argument: one call site per level made ptxas spill in every task.)
 template <bool MINP, int NT>
 __device__ __forceinline__ void search_chunk6(const SearchParams& s) {
-  constexpr uint32_t TW = 32 * (MINP ? kWTM6 : kWT6);  // words per warp task
   const int tid = threadIdx.x;
   const int lane = tid & 31;
 #pragma unroll 1
   for (int l = 0; l < kLevels6; ++l) {
     uint32_t b0, b2, b4;
+    constexpr uint32_t TW0 = 32 * (MINP ? kWTM6 : kWT6), TWL = 32 * (MINP ? kWTML6 : kWT6);  // words per task
     if (l == 0) {  // every word of the chunk
-      b0 = (((g_cx6.M[0] + 31) >> 5) + TW - 1) / TW;
-      b2 = (((g_cx6.M[1] + 31) >> 5) + TW - 1) / TW;
-      b4 = (((g_cx6.M[2] + 31) >> 5) + TW - 1) / TW;
+      b0 = (((g_cx6.M[0] + 31) >> 5) + TW0 - 1) / TW0;
+      b2 = (((g_cx6.M[1] + 31) >> 5) + TW0 - 1) / TW0;
+      b4 = (((g_cx6.M[2] + 31) >> 5) + TW0 - 1) / TW0;
     } else {  // the survivor lists of the level before
-      b0 = (g_cx6.scnt[l - 1][0] + TW - 1) / TW;
-      b2 = (g_cx6.scnt[l - 1][1] + TW - 1) / TW;
-      b4 = (g_cx6.scnt[l - 1][2] + TW - 1) / TW;
+      b0 = (g_cx6.scnt[l - 1][0] + TWL - 1) / TWL;
+      b2 = (g_cx6.scnt[l - 1][1] + TWL - 1) / TWL;
+      b4 = (g_cx6.scnt[l - 1][2] + TWL - 1) / TWL;
     }
     for (;;) {
       uint32_t task = 0;
