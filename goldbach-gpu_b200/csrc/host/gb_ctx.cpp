@@ -424,24 +424,51 @@ gb_status ensure_primes(gb_ctx* c, Workspace& w, uint64_t limit) {
   return GB_OK;
 }
 
-// Chunk width of a range of `count` even n when the caller leaves it open: the
-// power of two from 2^13 to `most` with the least time on the fullest SM.
-// Measured, two CTAs per SM: a chunk takes 232 us per 2^20 n near 1e12 (250 near
-// 1e9) and 24 us beside, 0.75 ns more for each of its sieving primes: 1e5 n and
-// 4.7 n a prime.  A CTA alone on its SM takes 0.77 of a pair's time.
-static uint32_t range_chunk(uint64_t count, uint64_t nprimes, int sm_count, uint32_t most) {
-  const double fixed = 1e5 + 4.7 * (double)nprimes;
-  double best = 0;
-  uint32_t ne = most;
-  for (uint32_t x = most; x >= 8192; x >>= 1) {
-    const uint64_t per_sm = ((count + x - 1) / x + sm_count - 1) / sm_count;
-    const double t = (x + fixed) * (0.5 * (double)per_sm + (per_sm & 1 ? 0.27 : 0.0));
-    if (x == most || t < best) {
-      best = t;
-      ne = x;
+// Chunk width when the caller leaves it open: the one with the least time on
+// the fullest SM, for pieces cut into chunks each by itself (`pieces` of `len`
+// n and one of `tail`).  A chunk costs ne + fixed, in n; an SM runs two CTAs at
+// once, and one alone takes 0.77 of a pair's time.  For a few numbers of chunks
+// per SM the narrowest width that needs no more is tried, in steps of 512 n.
+// Powers of two left a last wave of a few chunks: 2e8 n near 1e12 329 -> 257
+// us, 5e8 n near 1e9 469 -> 396, 4e7 n near 1e15 (masked) 237 -> 189.  With five or
+// more chunks of the widest per SM, an odd number, the last one overlaps the
+// uneven ends of the others and narrower chunks only add their fixed cost:
+// 6e8 and 1e9 n near 1e12 689 and 1045 us at the widest, 717 and 1105 narrower.
+uint32_t balanced_chunk(uint64_t pieces, uint64_t len, uint64_t tail, double fixed, int sm_count, uint32_t least,
+                        uint32_t most) {
+  auto chunks = [&](uint64_t ne) { return pieces * ((len + ne - 1) / ne) + (tail + ne - 1) / ne; };
+  const double total = (double)pieces * (double)len + (double)tail;
+  double best = -1;
+  uint32_t pick = most;
+  const uint64_t at_most = (chunks(most) + sm_count - 1) / sm_count;  // chunks per SM at the widest
+  if (at_most >= 5 && (at_most & 1)) return most;
+  for (uint64_t k = std::max<uint64_t>(1, at_most); k <= at_most + 5; ++k) {
+    // the narrowest width (a multiple of 512) with at most k sm_count chunks
+    uint64_t lo = std::max<uint64_t>(least, (uint64_t)(total / (double)(k * sm_count)) & ~511ull), hi = most;
+    if (chunks(hi) > k * sm_count) continue;
+    if (lo > hi) lo = hi;
+    lo = (lo + 511) & ~511ull;
+    while (lo < hi) {
+      const uint64_t mid = (lo + hi) / 1024 * 512;
+      if (chunks(mid) <= k * sm_count) hi = mid;
+      else lo = mid + 512;
     }
+    const double t = ((double)hi + fixed) * (0.5 * (double)k + (k & 1 ? 0.27 : 0.0));
+    if (best < 0 || t < best) {
+      best = t;
+      pick = (uint32_t)hi;
+    }
+    if (hi <= least) break;
   }
-  return ne;
+  return pick;
+}
+
+// The same for a range whose chunks sieve with nprimes primes.  Measured, two
+// CTAs per SM: a chunk takes 232 us per 2^20 n near 1e12 (250 near 1e9) and 24 us
+// beside, 0.75 ns more for each of its sieving primes: 1e5 n and 4.7 n a prime.
+static uint32_t range_chunk(uint64_t pieces, uint64_t len, uint64_t tail, uint64_t nprimes, int sm_count,
+                            uint32_t most) {
+  return balanced_chunk(pieces, len, tail, 1e5 + 4.7 * (double)nprimes, sm_count, 8192, most);
 }
 
 // ---------------------------------------------------------------------------
@@ -469,12 +496,13 @@ gb_status range_impl(gb_ctx* c, Workspace& w, Arena* arena, uint64_t start, uint
   uint32_t NE = o.chunk_evens;
   if (!NE) {
     // at most 2^20 n: two CTAs per SM (the two class bitsets hold 2^20 / 3 bits each)
-    const uint64_t shard = count / (o.shard_count ? o.shard_count : 1) + 1;
-    NE = range_chunk(std::min(shard, count), (uint64_t)(1.1 * (double)root / std::log((double)root + 2.0)),
+    const uint64_t shards = o.shard_count ? o.shard_count : 1;
+    const uint64_t full = count / o.seg_size / shards, rest = full ? count % o.seg_size : count;
+    NE = range_chunk(full, o.seg_size, rest, (uint64_t)(1.1 * (double)root / std::log((double)root + 2.0)),
                      c->sm_count, out && out->min_p ? kMinpChunk : 1u << 20);
-  }
-  if (NE < 8192 || NE > (1u << 20) || (NE & (NE - 1)))
+  } else if (NE < 8192 || NE > (1u << 20) || (NE & (NE - 1))) {
     return fail(w, GB_EINVAL, "chunk_evens must be a power of two in [2^13, 2^20]");
+  }
   if (out && out->min_p && NE > kMinpChunk) NE = kMinpChunk;  // per-n output: smaller chunks
   if (o.block_threads && o.block_threads != 256 && o.block_threads != 512 && o.block_threads != 1024)
     return fail(w, GB_EINVAL, "block_threads must be 256, 512 or 1024");

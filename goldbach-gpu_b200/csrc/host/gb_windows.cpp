@@ -37,6 +37,7 @@ constexpr uint32_t kWinHalo = 8192;
 // down to these widths; a tested window's chunks sieve no primes, so they can
 // be narrower.
 constexpr uint64_t kMinMaskedChunk = 1ull << 16;
+constexpr double kMaskedFixed = 1e5;  // n that a masked range's chunk costs beside its own (balanced_chunk)
 // Ranges of fewer n than this per SM, or with larger sieving primes, are masked
 // (range_masked_pays).
 constexpr uint64_t kMaskedWidth = 1ull << 18, kMaskedRoot = 6000000;
@@ -95,10 +96,10 @@ constexpr uint64_t kRangeMaskPieces = 1ull << 20;
 // its width (range_chunk); the pass spends 7 ps on a mark.  So it pays for
 // ranges that must be cut into narrow chunks to fill the GPU, and for far
 // ones, where the chunk's primes outweigh its n.  Kernel time, chunks alone
-// against masks: 1e7 n near 1e12 108 -> 100 us, 2e5 n 107 -> 70 us, 1e8 n 216 ->
+// against masks: 1e7 n near 1e12 108 -> 95 us, 2e5 n 107 -> 70 us, 1e8 n 174 ->
 // 277 us (not masked); 1e9 n near 1e13 1.42 -> 2.11 ms (not masked); 1e8 n near
-// 1e14 0.53 -> 0.35 ms, 4e7 n near 1e15 1.03 -> 0.27, 1e6 and 1e9 n near 1e17
-// 18.6 -> 0.16 and 67 -> 3.2 ms.  The range must start beyond every sieving
+// 1e14 0.53 -> 0.35 ms, 4e7 n near 1e15 1.03 -> 0.19, 1e6 and 1e9 n near 1e17
+// 18.6 -> 0.15 and 67 -> 3.2 ms.  The range must start beyond every sieving
 // prime, and the pass's quotient estimates need p > g0 / 2^42 (masked_bound).
 bool range_masked_pays(const gb_ctx* c, uint64_t start, uint64_t count, uint64_t root, uint64_t pieces) {
   if (start < (8ull << 30) || root < (1ull << 16) || pieces > kRangeMaskPieces) return false;
@@ -142,7 +143,12 @@ gb_status range_masked(gb_ctx* c, Workspace& ws, Temps& tmp, int slot, const std
       desc.push_back(d);
       runs.back().p1 = desc.size();
     }
-  if (!ne) ne = chunk_for(std::min(total, kRangeMaskEvens), 2ull * c->sm_count, kMinMaskedChunk, a.chunk_evens);
+  if (!ne) {
+    // one batch's pieces: its segments, or its share of a longer one
+    const uint64_t n = std::min(total, kRangeMaskEvens);
+    const uint64_t len = std::min<uint64_t>(segs[0].count, kRangeMaskEvens);
+    ne = balanced_chunk(n / len, len, n % len, kMaskedFixed, c->sm_count, kMinMaskedChunk, a.chunk_evens);
+  }
   a.chunk_evens = ne;
   a.nbw = range6_words(H, ne);
   const uint64_t bound = masked_bound(top, ne);
