@@ -25,13 +25,14 @@
 // per lane (up to 32 limbs one a lane, G = 8, 16 or 32), and a product takes
 // one step per limb of y: every lane multiplies its limbs by it, lane 0's
 // lowest limb gives the reduction's m, and the limbs move down one place.
-// A step is about 70 clocks (two shuffles and two multiply-adds in a row),
-// whatever the width.  The carries stay in 64-bit accumulators until the end,
-// where one pass over the lanes and a carry look-ahead on two ballots settle
-// them; R = 2^(32 L) >= 4q keeps the residues below 2q without a
-// subtraction.  One n of 512 bits: 22.0 -> 1.3 ms (one thread per
-// test with its limbs in local memory took 10.9 ms for each of the two
-// strong-test kernels, 41,000 clocks a product; now 0.47 and 0.56 ms).
+// A step is about 70 clocks (one round of shuffles, then two multiplications
+// and the sums in a row), whatever the width.  The carries stay in 64-bit
+// accumulators until the end, where one pass over the lanes and a carry
+// look-ahead on two ballots settle them; R = 2^(32 L) >= 4q keeps the residues below 2q without a
+// subtraction.  One n of 512 bits: 22.0 -> 0.84 ms (one thread per test with its
+// limbs in local memory took 10.9 ms for each of the two strong-test kernels,
+// 41,000 clocks a product; moving m, then the limbs, in two rounds of shuffles
+// took 1.22 ms where this takes 1.03, both in batches of 8192 candidates).
 #include <cuda_runtime.h>
 
 #include <cstdint>
@@ -159,56 +160,61 @@ struct Big {
     }
     canon(x, q);
   }
-  // One limb of Montgomery reduction: c = (c + m q) / 2^32 with m = c (-q^-1) mod
-  // 2^32; u, h: c's low and high halves.
-  static __device__ __forceinline__ void reduce(uint64_t (&c)[K], const uint32_t (&u)[K], const uint64_t (&h)[K],
-                                                const Num& q, uint32_t qinv) {
-    const uint32_t m = __shfl_sync(kAllLanes, u[0] * qinv, 0, G);
-    uint32_t lo[K];
+  // One limb of Montgomery reduction of the number with the 64-bit limbs c, and
+  // the limbs of another number added: c = (c + m q) / 2^32 + add with m = c (-q^-1)
+  // mod 2^32.  qn: the lowest limb of q in the next lane; top: what c holds beyond
+  // the last lane.  Every lane makes m itself, from lane 0's lowest limb, and
+  // takes both the low half of its own products and the high half of those one
+  // limb below, so the only exchange is the one that hands out that limb and
+  // moves the limbs down.
+  static __device__ __forceinline__ void reduce(uint64_t (&c)[K], const uint64_t (&add)[K], uint32_t top,
+                                                const Num& q, uint32_t qn, uint32_t qinv) {
+    const uint32_t t = __shfl_sync(kAllLanes, (uint32_t)c[0], 0, G);
+    const uint32_t next = __shfl_down_sync(kAllLanes, (uint32_t)c[0], 1, G);
+    const uint32_t m = t * qinv;
+    uint64_t d[K];
+#pragma unroll
+    for (int j = 0; j < K; ++j)
+      d[j] = (c[j] >> 32) + (j + 1 < K ? (uint32_t)c[j + 1] : sub() == G - 1 ? top : next) + add[j];
+    d[0] += sub() == 0 && t != 0;  // t + (m q mod 2^32) is 0 or 2^32
 #pragma unroll
     for (int j = 0; j < K; ++j) {
-      const uint64_t t = (uint64_t)q[j] * m + u[j];
-      lo[j] = (uint32_t)t;
-      c[j] = h[j] + (t >> 32);
+      const uint32_t hi = __umulhi(q[j], m), lo = (j + 1 < K ? q[j + 1] : qn) * m;
+      c[j] = d[j] + hi + lo;
     }
-    uint32_t next = __shfl_down_sync(kAllLanes, lo[0], 1, G);
-    if (sub() == G - 1) next = 0;
-#pragma unroll
-    for (int j = 0; j < K; ++j) c[j] += j + 1 < K ? lo[j + 1] : next;
   }
-  static __device__ __forceinline__ void step(uint64_t (&c)[K], const Num& x, uint32_t yi, const Num& q, uint32_t qinv) {
-    uint32_t u[K];
-    uint64_t h[K];
+  // z = x v limb by limb (64-bit limbs); xb: the highest limb of x in the lane below
+  static __device__ __forceinline__ void times(uint64_t (&z)[K], const Num& x, uint32_t xb, uint32_t v) {
 #pragma unroll
-    for (int j = 0; j < K; ++j) {
-      const uint64_t t = (uint64_t)x[j] * yi + (uint32_t)c[j];
-      u[j] = (uint32_t)t;
-      h[j] = (t >> 32) + (c[j] >> 32);
-    }
-    reduce(c, u, h, q, qinv);
+    for (int j = 0; j < K; ++j) z[j] = (uint64_t)(x[j] * v) + __umulhi(j ? x[j - 1] : xb, v);
   }
   // x = x y / R mod q below 2q, R = 2^(32 K rl), for x, y < 2q
-  static __device__ __forceinline__ void mul(Num& x, const Num& y, const Num& q, uint32_t qinv, int rl) {
-    uint64_t c[K];
-#pragma unroll
-    for (int j = 0; j < K; ++j) c[j] = 0;
+  static __device__ __forceinline__ void mul(Num& x, const Num& y, const Num& q, uint32_t qn, uint32_t qinv, int rl) {
+    const uint32_t xb = up(x[K - 1]);
+    uint64_t c[K], z[K];
+    uint32_t v = __shfl_sync(kAllLanes, y[0], 0, G);
+    times(c, x, xb, v);
     for (int l = 0; l < rl; ++l) {
 #pragma unroll
-      for (int j = 0; j < K; ++j) step(c, x, __shfl_sync(kAllLanes, y[j], l, G), q, qinv);
+      for (int j = 0; j < K; ++j) {
+        const uint32_t top = __umulhi(x[K - 1], v);
+        v = __shfl_sync(kAllLanes, y[j + 1 < K ? j + 1 : 0], j + 1 < K ? l : l + 1, G);
+        if (j + 1 == K && l + 1 == rl) v = 0;  // past y
+        times(z, x, xb, v);
+        reduce(c, z, top, q, qn, qinv);
+      }
     }
     settle(x, c);
   }
   // x = x 2^(s - 32) mod q below 2q, 0 <= s < 32, for x < 2q
-  static __device__ __forceinline__ void shift(Num& x, uint32_t s, const Num& q, uint32_t qinv) {
-    uint64_t c[K], h[K];
-    uint32_t u[K];
+  static __device__ __forceinline__ void shift(Num& x, uint32_t s, const Num& q, uint32_t qn, uint32_t qinv) {
+    uint64_t c[K], z[K];
 #pragma unroll
     for (int j = 0; j < K; ++j) {
-      const uint64_t t = (uint64_t)x[j] << s;
-      u[j] = (uint32_t)t;
-      h[j] = t >> 32;
+      c[j] = (uint64_t)x[j] << s;
+      z[j] = 0;
     }
-    reduce(c, u, h, q, qinv);
+    reduce(c, z, 0, q, qn, qinv);
     settle(x, c);
   }
 };
@@ -219,7 +225,7 @@ template <int G, int K>
 struct BigMod {
   typedef Big<G, K> B;
   typename B::Num q, one;
-  uint32_t qinv;
+  uint32_t qn, qinv;  // q's lowest limb in the next lane; -q^-1 mod 2^32
   int bits, s, rl;  // bit length of q, q - 1 = d 2^s, lanes of R
 
   // q = n - p; words: this group's q in shared memory (G K words)
@@ -232,6 +238,8 @@ struct BigMod {
       pn[j] = i == 0 ? p : 0;
     }
     B::minus(q, n, pn);
+    qn = __shfl_down_sync(kAllLanes, q[0], 1, G);
+    if (B::sub() == G - 1) qn = 0;
     __syncwarp();
 #pragma unroll
     for (int j = 0; j < K; ++j) words[B::sub() * K + j] = q[j];
@@ -273,7 +281,7 @@ struct BigMod {
 #pragma unroll 1
     for (int i = 1; i < smax; ++i) {
       B::copy(y, x);
-      B::mul(x, y, q, qinv, rl);
+      B::mul(x, y, q, qn, qinv, rl);
       B::copy(y, x);
       B::canon(y, q);
       ok |= B::equal(y, mone) && i < s;
@@ -342,11 +350,11 @@ __global__ void __launch_bounds__(kBigThreads) big_base2_kernel(const __grid_con
 #pragma unroll 1
       for (int k = 0; k < 5; ++k) {
         B::copy(y, x);
-        B::mul(y, x, M.q, M.qinv, M.rl);
+        B::mul(y, x, M.q, M.qn, M.qinv, M.rl);
         if (j < m) B::copy(x, y);
       }
       B::copy(y, x);
-      B::shift(y, j < m ? dig[j] : 0, M.q, M.qinv);
+      B::shift(y, j < m ? dig[j] : 0, M.q, M.qn, M.qinv);
       if (j < m) B::copy(x, y);
     }
     const bool ok = M.verdict(x, (int)__reduce_max_sync(kAllLanes, (uint32_t)M.s));
@@ -391,7 +399,7 @@ __global__ void __launch_bounds__(32) big_bases_kernel(const __grid_constant__ B
   for (int k = 0; k < 16; ++k) {
 #pragma unroll
     for (int j = 0; j < K; ++j) s_pow[k][lane * K + j] = x[j];
-    B::mul(x, b, M.q, M.qinv, M.rl);
+    B::mul(x, b, M.q, M.qn, M.qinv, M.rl);
   }
   __syncwarp();
   const int dbits = M.bits - M.s;
@@ -408,10 +416,10 @@ __global__ void __launch_bounds__(32) big_bases_kernel(const __grid_constant__ B
 #pragma unroll 1
     for (int k = 0; k < 4; ++k) {
       B::copy(y, x);
-      B::mul(x, y, M.q, M.qinv, M.rl);
+      B::mul(x, y, M.q, M.qn, M.qinv, M.rl);
     }
     load(bits_at(s_q, G * K, M.s + pos, 4));
-    B::mul(x, y, M.q, M.qinv, M.rl);
+    B::mul(x, y, M.q, M.qn, M.qinv, M.rl);
   }
   const bool ok = M.verdict(x, M.s);
   if (!ok && lane == 0) atomicOr(a.fail, 1u);

@@ -60,3 +60,12 @@ def test_base2_pseudoprime_beyond_64_bits(ctx, B, p):
     assert B.sprp(s, 2) and not B.is_probable_prime(s)
     got, q, _ = ctx.check_big(s + p)
     assert got == B.minimal_p(s + p, primes=B.PR) and q == s + p - got
+
+
+@pytest.mark.parametrize("bits,d", [(200, 798), (256, 908), (400, 196), (512, 660)])
+def test_minimal_p_beyond_the_first_batch(ctx, B, bits, d):
+    """Every candidate of the first batch (two for each bit of n, at least 512) fails."""
+    n = 2 ** (bits - 1) + d
+    p, q, r = ctx.check_big(n)
+    assert p == B.minimal_p(n, primes=B.PR) and q == n - p
+    assert p > B.PR[max(512, 2 * bits)] and r["candidates"] > max(512, 2 * bits)
