@@ -228,10 +228,11 @@ struct BigArgs {
   const uint32_t* trial;    // trial primes r
   const uint32_t* nmod;     // n mod r
   uint32_t ntrial;
-  uint32_t* surv;           // survivors (candidate index from k0)
+  uint32_t* surv;           // survivors of the trial primes, a bit per candidate from k0
+  uint32_t words;           // words of them
   uint32_t* pass;           // base-2 passers (candidate index from k0)
-  uint32_t* nsurv;
   uint32_t* npass;
+  uint32_t* specfail;       // bit r: a base rejects survivor r (the first of them, big.cu)
   uint32_t* minpass;        // smallest of them (~0: none)
   uint32_t* fail;           // nonzero once a base rejects the passer under test
   unsigned long long* mr_tests;

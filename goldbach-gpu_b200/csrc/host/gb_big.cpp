@@ -77,14 +77,14 @@ gb_status big_impl(gb_ctx* c, Workspace& w, const uint32_t* n_limbs, uint32_t nl
   Temps tmp(c, nullptr);
   void *d_up, *d_surv, *d_pass, *d_small;
   if ((st = ws_buffer(c, w, tmp, 0, up.size() * 4, &d_up)) != GB_OK ||
-      (st = ws_buffer(c, w, tmp, 1, kBigBatch * 4, &d_surv)) != GB_OK ||
+      (st = ws_buffer(c, w, tmp, 1, kBigBatch / 8, &d_surv)) != GB_OK ||
       (st = ws_buffer(c, w, tmp, 2, kBigBatch * 4, &d_pass)) != GB_OK ||
       (st = ws_buffer(c, w, tmp, 3, 64, &d_small)) != GB_OK)
     return st;
   // the device's figures of a batch, in this order behind the tests' count
   struct Figures {
     unsigned long long tests;
-    uint32_t nsurv, npass, fail, minpass;
+    uint32_t npass, specfail, fail, minpass;
   };
   Figures* fig = (Figures*)d_small;
   BigArgs a{};
@@ -101,9 +101,9 @@ gb_status big_impl(gb_ctx* c, Workspace& w, const uint32_t* n_limbs, uint32_t nl
   a.ntrial = (uint32_t)trial.size();
   a.surv = (uint32_t*)d_surv;
   a.pass = (uint32_t*)d_pass;
-  a.nsurv = &fig->nsurv;
   a.npass = &fig->npass;
   a.minpass = &fig->minpass;
+  a.specfail = &fig->specfail;
   a.fail = &fig->fail;
   a.mr_tests = &fig->tests;
   cudaStream_t s = c->stream;
@@ -125,7 +125,8 @@ gb_status big_impl(gb_ctx* c, Workspace& w, const uint32_t* n_limbs, uint32_t nl
   const uint32_t batch = std::min<uint32_t>(kBigBatch, std::max<uint32_t>(512, kBatchPerBit * bits));
   while (k0 < np && e == cudaSuccess) {
     const uint32_t kc = (uint32_t)std::min<uint64_t>(batch, np - k0);
-    chk(cudaMemsetAsync(&fig->nsurv, 0, 12, s));  // survivors, passers, fail
+    a.words = (kc + 31) / 32;
+    chk(cudaMemsetAsync(&fig->npass, 0, 12, s));  // passers, specfail, fail
     chk(cudaMemsetAsync(&fig->minpass, 0xff, 4, s));
     chk(launch_big_filter(a, (uint32_t)k0, kc, s));
     chk(launch_big_base2(a, (uint32_t)k0, c->sm_count * 4, s));

@@ -7,11 +7,12 @@
 // prime table) are tested in batches (host/gb_big.cpp):
 //   1. big_filter_kernel: one warp per candidate drops q = n - p when a
 //      trial prime r divides it, from n mod r (computed on the host once per
-//      n) and p mod r, and appends the survivors' indices;
+//      n) and p mod r; the survivors are a bitmap;
 //   2. big_base2_kernel: one group of lanes per survivor runs the strong
 //      probable-prime test to base 2, lists the passers (almost all of them
-//      primes) and keeps the smallest;
-//   3. big_bases_kernel: one group per base runs the 11 other bases 3, 5, ...,
+//      primes) and keeps the smallest; up to 1024 bits, more CTAs run the other
+//      bases on the first survivors meanwhile;
+//   3. big_bases_kernel: one warp per base runs the 11 other bases 3, 5, ...,
 //      37 -- with base 2 the base set of the reference's Miller-Rabin
 //      (src/goldbach.cu:333-360) -- on one passer.
 // The smallest passer no base rejects is the minimal p: every smaller
@@ -29,7 +30,7 @@
 // and the sums in a row), whatever the width.  The carries stay in 64-bit
 // accumulators until the end, where one pass over the lanes and a carry
 // look-ahead on two ballots settle them; R = 2^(32 L) >= 4q keeps the residues below 2q without a
-// subtraction.  One n of 512 bits: 22.0 -> 0.84 ms (one thread per test with its
+// subtraction.  One n of 512 bits: 22.0 -> 0.6 ms (one thread per test with its
 // limbs in local memory took 10.9 ms for each of the two strong-test kernels,
 // 41,000 clocks a product; moving m, then the limbs, in two rounds of shuffles
 // took 1.22 ms where this takes 1.03, both in batches of 8192 candidates).
@@ -48,16 +49,76 @@ constexpr int kBigMaxLimbs = GB_BIG_MAX_LIMBS + 1;  // limbs of R
 // The 12 prime bases of the strong tests.
 __device__ __constant__ const uint32_t kBigBases[12] = {2, 3, 5, 7, 11, 13, 17, 19, 23, 29, 31, 37};
 
-constexpr int kFilterThreads = 256;
+// A warp per candidate, a word of a.surv per CTA.
+constexpr int kFilterThreads = 1024;
 __global__ void __launch_bounds__(kFilterThreads) big_filter_kernel(const __grid_constant__ BigArgs a, uint32_t k0,
                                                                     uint32_t kcount) {
-  const uint32_t i = blockIdx.x * (kFilterThreads / 32) + (threadIdx.x >> 5);
-  if (i >= kcount) return;  // warp-uniform
-  const uint32_t p = a.primes[k0 + i];
-  bool drop = p > a.p_lim;
-  for (uint32_t j = threadIdx.x & 31; j < a.ntrial; j += 32)
-    drop |= p % a.trial[j] == a.nmod[j];  // r divides q = n - p (q far above r)
-  if (!__any_sync(kAllLanes, drop) && (threadIdx.x & 31) == 0) a.surv[atomicAdd(a.nsurv, 1u)] = i;
+  __shared__ uint32_t s_drop[32];
+  const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const uint32_t i = blockIdx.x * 32 + warp;
+  bool drop = i >= kcount;  // warp-uniform
+  if (!drop) {
+    const uint32_t p = a.primes[k0 + i];
+    drop = p > a.p_lim;
+    for (uint32_t j = lane; j < a.ntrial; j += 32)
+      drop |= p % a.trial[j] == a.nmod[j];  // r divides q = n - p (q far above r)
+  }
+  drop = __any_sync(kAllLanes, drop);
+  if (lane == 0) s_drop[warp] = drop;
+  __syncthreads();
+  if (warp == 0) {
+    const uint32_t w = __ballot_sync(kAllLanes, !s_drop[lane]);
+    if (lane == 0) a.surv[blockIdx.x] = w;
+  }
+}
+
+// The survivors by rank, from their bits: lane l holds the words [l per, (l + 1) per).
+struct Survivors {
+  const uint32_t* bits;
+  uint32_t words, per, upto;  // upto: survivors up to this lane's words, included
+  uint32_t total;
+
+  __device__ __forceinline__ Survivors(const BigArgs& a)
+      : bits(a.surv), words(a.words), per((a.words + 31) / 32), upto(0) {
+    const uint32_t lane = threadIdx.x & 31;
+    for (uint32_t j = lane * per; j < min((lane + 1) * per, words); ++j) upto += __popc(bits[j]);
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+      const uint32_t v = __shfl_up_sync(kAllLanes, upto, d);
+      if (lane >= (uint32_t)d) upto += v;
+    }
+    total = __shfl_sync(kAllLanes, upto, 31);
+  }
+  // candidate index of survivor t (below total; t may differ between lanes)
+  __device__ __forceinline__ uint32_t nth(uint32_t t) const {
+    uint32_t own = 0, before = 0;  // the lane whose words hold it, the survivors below those
+    for (int l = 0; l < 31; ++l) {
+      const uint32_t v = __shfl_sync(kAllLanes, upto, l);
+      if (t >= v) {
+        own = l + 1;
+        before = v;
+      }
+    }
+    uint32_t j = own * per, w = bits[j];
+    t -= before;
+    for (uint32_t c; t >= (c = __popc(w)); w = bits[++j]) t -= c;
+    for (; t; --t) w &= w - 1;
+    return 32 * j + __ffs(w) - 1;
+  }
+  __device__ __forceinline__ uint32_t rank(uint32_t i) const {  // survivors below candidate i
+    uint32_t c = 0;
+    for (uint32_t j = threadIdx.x & 31; j <= i >> 5; j += 32)
+      c += __popc(j < i >> 5 ? bits[j] : bits[j] & ((1u << (i & 31)) - 1));
+    return __reduce_add_sync(kAllLanes, c);
+  }
+};
+
+// candidate index of survivor t, or of the last one; ~0u without any (t may
+// differ between lanes).  A call, so that a test's registers are its own (inlined:
+// 4096 bits 104.5 -> 106.5 ms).
+__device__ __noinline__ uint32_t nth_survivor(const BigArgs& a, uint32_t t) {
+  const Survivors S(a);
+  return S.total ? S.nth(min(t, S.total - 1)) : 0xffffffffu;
 }
 
 // Numbers of G lanes with K limbs each; limb j of lane l is limb l K + j.
@@ -298,6 +359,69 @@ __device__ __forceinline__ uint32_t bits_at(const uint32_t* words, int nwords, i
 }
 
 constexpr int kBigThreads = 64;
+// Up to 32 limbs (K = 1) the other bases of the first survivors run beside base
+// 2, in CTAs of the same launch: at 512 bits 85% of the n have their first prime
+// among 32 (n of 512 bits 0.81 -> 0.53 ms, of 96 0.11 -> 0.086, of 1024 3.44 -> 3.38;
+// longer n find it there less often than not, and their tests fill the lanes).
+constexpr uint32_t kBigSpec = 32;
+constexpr uint32_t kSpecCtas = kBigSpec * 11 / (kBigThreads / 32);
+
+// The strong test of q = n - p to `base` by one warp.  Four exponent bits at a time,
+// the powers base^0 .. base^15 in shared memory.
+template <int G, int K>
+struct BasesShared {
+  uint32_t q[G * K], all[32 / G][G * K];
+  uint32_t pow[16][32 * K];
+};
+template <int G, int K>
+__device__ __forceinline__ bool big_strong(const BigArgs& a, uint32_t p, uint32_t base, BasesShared<G, K>& sm) {
+  typedef Big<G, K> B;
+  const uint32_t lane = threadIdx.x & 31;
+  const BigMod<G, K> M(a, p, sm.all[lane / G]);  // every group of the warp holds the same q
+  if (lane < G)
+    for (int j = 0; j < K; ++j) sm.q[lane * K + j] = M.q[j];
+  typename B::Num x, y, b;
+  // base in Montgomery form, from the base's bits
+#pragma unroll
+  for (int j = 0; j < K; ++j) b[j] = 0;
+  for (int k = 5; k >= 0; --k) {
+    B::dbl(b, M.q);
+    if ((base >> k) & 1u) {  // b + one mod q
+      uint64_t c[K];
+#pragma unroll
+      for (int j = 0; j < K; ++j) c[j] = (uint64_t)b[j] + M.one[j];
+      B::settle(b, c);
+      B::canon(b, M.q);
+    }
+  }
+  B::copy(x, M.one);
+  for (int k = 0; k < 16; ++k) {
+#pragma unroll
+    for (int j = 0; j < K; ++j) sm.pow[k][lane * K + j] = x[j];
+    B::mul(x, b, M.q, M.qn, M.qinv, M.rl);
+  }
+  __syncwarp();
+  const int dbits = M.bits - M.s;
+  int pos = (dbits - 1) / 4 * 4;  // the lowest bit of the top digit
+  const auto load = [&](uint32_t d) {
+#pragma unroll
+    for (int j = 0; j < K; ++j) y[j] = sm.pow[d][lane * K + j];
+  };
+  load(bits_at(sm.q, G * K, M.s + pos, dbits - pos));
+  B::copy(x, y);
+#pragma unroll 1
+  while (pos > 0) {
+    pos -= 4;
+#pragma unroll 1
+    for (int k = 0; k < 4; ++k) {
+      B::copy(y, x);
+      B::mul(x, y, M.q, M.qn, M.qinv, M.rl);
+    }
+    load(bits_at(sm.q, G * K, M.s + pos, 4));
+    B::mul(x, y, M.q, M.qn, M.qinv, M.rl);
+  }
+  return M.verdict(x, M.s);
+}
 
 // Phase 0: base 2 on every survivor, G lanes each.  The power is taken 5 bits
 // at a time: five squarings take 2^e to 2^(32 e), and a shift by c with one limb
@@ -308,6 +432,18 @@ constexpr int kBigThreads = 64;
 template <int G, int K>
 __global__ void __launch_bounds__(kBigThreads) big_base2_kernel(const __grid_constant__ BigArgs a, uint32_t k0) {
   typedef Big<G, K> B;
+  if constexpr (K == 1) {  // the first CTAs: a warp per base of the first survivors
+    if (blockIdx.x < kSpecCtas) {
+      __shared__ BasesShared<G, 1> sm[kBigThreads / 32];
+      const uint32_t w = threadIdx.x >> 5, job = blockIdx.x * (kBigThreads / 32) + w;
+      const uint32_t r = job / 11;
+      if (r >= Survivors(a).total) return;
+      if (!big_strong<G, 1>(a, a.primes[k0 + nth_survivor(a, r)], kBigBases[1 + job % 11], sm[w]) && (threadIdx.x & 31) == 0)
+        atomicOr(a.specfail, 1u << r);
+      return;
+    }
+  }
+  const uint32_t cta = blockIdx.x - (K == 1 ? kSpecCtas : 0), ctas = gridDim.x - (K == 1 ? kSpecCtas : 0);
   constexpr int kGroups = kBigThreads / G;
   constexpr int kDigits = (32 * kBigMaxLimbs + 4) / 5;
   __shared__ uint32_t s_q[kGroups][G * K];
@@ -315,11 +451,11 @@ __global__ void __launch_bounds__(kBigThreads) big_base2_kernel(const __grid_con
   const uint32_t gi = threadIdx.x / G;
   uint32_t* words = s_q[gi];
   uint8_t* dig = s_dig[gi];
-  const uint32_t nsurv = *a.nsurv, groups = gridDim.x * kGroups;
-  for (uint32_t t0 = blockIdx.x * kGroups; t0 < nsurv; t0 += groups) {  // uniform in the CTA
+  const uint32_t nsurv = Survivors(a).total, groups = ctas * kGroups;
+  for (uint32_t t0 = cta * kGroups; t0 < nsurv; t0 += groups) {  // uniform in the CTA
     const uint32_t t = t0 + gi;
     const bool act = t < nsurv;  // a group past the end runs along on the last survivor
-    const uint32_t i = a.surv[act ? t : nsurv - 1];
+    const uint32_t i = nth_survivor(a, t);
     const BigMod<G, K> M(a, a.primes[k0 + i], words);
     if (act && B::sub() == 0) atomicAdd(a.mr_tests, 1ull);
     const int dbits = M.bits - M.s;
@@ -367,67 +503,26 @@ __global__ void __launch_bounds__(kBigThreads) big_base2_kernel(const __grid_con
 }
 
 // Phase 1: bases 3, ..., 37 on one passer (i, or the smallest for ~0u), a warp per
-// base; a failing base marks *fail.  Four exponent bits at a time, the powers
-// base^0 .. base^15 in shared memory.
+// base; a failing base sets *fail.  A passer among the first kBigSpec survivors
+// has been through them beside base 2.
 template <int G, int K>
 __global__ void __launch_bounds__(32) big_bases_kernel(const __grid_constant__ BigArgs a, uint32_t k0, uint32_t i) {
-  typedef Big<G, K> B;
-  __shared__ uint32_t s_q[G * K], s_all[32 / G][G * K];
-  __shared__ uint32_t s_pow[16][32 * K];
+  __shared__ BasesShared<G, K> sm;
   if (i == 0xffffffffu) i = *a.minpass;
   if (i == 0xffffffffu) return;  // no candidate passed base 2
-  const uint32_t lane = threadIdx.x;
-  const BigMod<G, K> M(a, a.primes[k0 + i], s_all[lane / G]);  // every group of the warp holds the same q
-  if (lane < G)
-    for (int j = 0; j < K; ++j) s_q[lane * K + j] = M.q[j];
-  const uint32_t base = kBigBases[1 + blockIdx.x];
-  typename B::Num x, y, b;
-  // base in Montgomery form, from the base's bits
-#pragma unroll
-  for (int j = 0; j < K; ++j) b[j] = 0;
-  for (int k = 5; k >= 0; --k) {
-    B::dbl(b, M.q);
-    if ((base >> k) & 1u) {  // b + one mod q
-      uint64_t c[K];
-#pragma unroll
-      for (int j = 0; j < K; ++j) c[j] = (uint64_t)b[j] + M.one[j];
-      B::settle(b, c);
-      B::canon(b, M.q);
+  if constexpr (K == 1) {
+    const uint32_t r = Survivors(a).rank(i);
+    if (r < kBigSpec) {
+      if (blockIdx.x == 0 && threadIdx.x == 0 && (*a.specfail >> r & 1)) *a.fail = 1;
+      return;
     }
   }
-  B::copy(x, M.one);
-  for (int k = 0; k < 16; ++k) {
-#pragma unroll
-    for (int j = 0; j < K; ++j) s_pow[k][lane * K + j] = x[j];
-    B::mul(x, b, M.q, M.qn, M.qinv, M.rl);
-  }
-  __syncwarp();
-  const int dbits = M.bits - M.s;
-  int pos = (dbits - 1) / 4 * 4;  // the lowest bit of the top digit
-  const auto load = [&](uint32_t d) {
-#pragma unroll
-    for (int j = 0; j < K; ++j) y[j] = s_pow[d][lane * K + j];
-  };
-  load(bits_at(s_q, G * K, M.s + pos, dbits - pos));
-  B::copy(x, y);
-#pragma unroll 1
-  while (pos > 0) {
-    pos -= 4;
-#pragma unroll 1
-    for (int k = 0; k < 4; ++k) {
-      B::copy(y, x);
-      B::mul(x, y, M.q, M.qn, M.qinv, M.rl);
-    }
-    load(bits_at(s_q, G * K, M.s + pos, 4));
-    B::mul(x, y, M.q, M.qn, M.qinv, M.rl);
-  }
-  const bool ok = M.verdict(x, M.s);
-  if (!ok && lane == 0) atomicOr(a.fail, 1u);
+  const bool ok = big_strong<G, K>(a, a.primes[k0 + i], kBigBases[1 + blockIdx.x], sm);
+  if (!ok && threadIdx.x == 0) atomicOr(a.fail, 1u);
 }
 
 cudaError_t launch_big_filter(const BigArgs& a, uint32_t k0, uint32_t kcount, cudaStream_t s) {
-  const uint32_t per = kFilterThreads / 32;
-  big_filter_kernel<<<(kcount + per - 1) / per, kFilterThreads, 0, s>>>(a, k0, kcount);
+  big_filter_kernel<<<(kcount + 31) / 32, kFilterThreads, 0, s>>>(a, k0, kcount);
   return cudaGetLastError();
 }
 
@@ -459,7 +554,8 @@ static cudaError_t with_big_shape(uint32_t limbs, F f) {
 
 cudaError_t launch_big_base2(const BigArgs& a, uint32_t k0, int grid, cudaStream_t s) {
   return with_big_shape(a.limbs, [&](auto g, auto k) {
-    big_base2_kernel<decltype(g)::value, decltype(k)::value><<<grid, kBigThreads, 0, s>>>(a, k0);
+    constexpr int K = decltype(k)::value;
+    big_base2_kernel<decltype(g)::value, K><<<grid + (K == 1 ? kSpecCtas : 0), kBigThreads, 0, s>>>(a, k0);
   });
 }
 

@@ -69,3 +69,13 @@ def test_minimal_p_beyond_the_first_batch(ctx, B, bits, d):
     p, q, r = ctx.check_big(n)
     assert p == B.minimal_p(n, primes=B.PR) and q == n - p
     assert p > B.PR[max(512, 2 * bits)] and r["candidates"] > max(512, 2 * bits)
+
+
+@pytest.mark.parametrize("bits,d,p", [(96, 1778, 2333), (96, 45472, 691), (250, 774, 3217), (250, 1452, 2473),
+                                      (512, 356, 2357), (512, 492, 1753)])
+def test_first_prime_at_the_end_of_the_spread_bases(ctx, B, bits, d, p):
+    """The first prime n - p is the 32nd or the 33rd candidate without a factor
+    below 4096: the other bases run beside base 2 on 32 of them."""
+    n = 2 ** (bits - 1) + d
+    assert B.minimal_p(n, primes=B.PR) == p
+    assert ctx.check_big(n)[:2] == (p, n - p)
