@@ -154,7 +154,8 @@ struct CountPair {     // a pair of classes and the n of one residue
 struct CountArgs {
   const uint32_t* classes;  // class 0's first word (k = 0 .. 31)
   uint64_t stride;
-  const CountPair* pairs;
+  const CountPair* pairs;   // (not read for one pair: first)
+  CountPair first;
   uint32_t npairs;
   uint32_t modulus;
   uint64_t groups;          // of 32 n, the most of any residue

@@ -1108,7 +1108,7 @@ gb_status gb_autotune_windows(gb_ctx* c, const gb_window* w, size_t count, const
 // The pairs of residue classes mod M that the n of [start, start + 2 (count - 1)]
 // need (kernels/counts.cu), and the work they are: words of 32 n times words of
 // the classes.
-static std::vector<CountPair> count_pairs(uint32_t M, uint64_t start, uint64_t count, double* work) {
+static std::vector<CountPair> count_pairs(uint32_t M, uint64_t start, uint64_t count) {
   std::vector<uint32_t> cls, index(M, 0);
   for (uint32_t a = 1; a < M; a += 2)
     if ((M % 3 || a % 3) && (M % 5 || a % 5) && (M % 7 || a % 7)) {
@@ -1116,7 +1116,6 @@ static std::vector<CountPair> count_pairs(uint32_t M, uint64_t start, uint64_t c
       cls.push_back(a);
     }
   std::vector<CountPair> pairs;
-  *work = 0;
   for (uint64_t j = 0; j < M / 2 && j < count; ++j) {  // the first n of each residue
     const uint64_t n = start + 2 * j;
     const uint32_t r = (uint32_t)(n % M);
@@ -1131,7 +1130,6 @@ static std::vector<CountPair> count_pairs(uint32_t M, uint64_t start, uint64_t c
       p.half = a == b;
       p.s0 = n / M - (a + b - r) / M;
       pairs.push_back(p);
-      *work += (double)((p.count + 31) / 32) * (double)(n / M / 32 + 1) * (p.half ? 0.5 : 1.0);
     }
   }
   return pairs;
@@ -1161,18 +1159,19 @@ static gb_status counts_impl(gb_ctx* c, Workspace& w, uint64_t start, uint64_t c
   unsigned long long* d_out = (unsigned long long*)counts;
   if ((st = ws_buffer(c, w, tmp, 0, (nwords + 8) * 4, (void**)&buf)) != GB_OK) return st;
   if (!o.on_device && (st = ws_buffer(c, w, tmp, 1, count * 8, (void**)&d_out)) != GB_OK) return st;
-  // the modulus with the least work; building the classes costs about as much
-  // as 6 words of 32 n to each of their words
+  // the modulus with the least work, in words of 32 n times words of the classes:
+  // half of the ordered pairs of classes, phi(M)^2 over all residues; building
+  // the classes costs about as much as 6 of them to each of their words, and its
+  // launches as much as 2e6 (15 us)
   CountArgs ca{};
-  std::vector<CountPair> pairs;
   double best = 0;
-  for (uint32_t M : {2u, 6u, 30u, 210u}) {
-    double work = 0;
-    std::vector<CountPair> p = count_pairs(M, start, count, &work);
-    if (M > 2) work += 6.0 * (M == 6 ? 2 : M == 30 ? 8 : 48) * ((double)n_max / M / 32);
+  for (const auto& [M, phi] : {std::pair<uint32_t, uint32_t>{2, 1}, {30, 8}, {210, 48}}) {
+    const uint64_t res = std::min<uint64_t>(M / 2, count);  // residues among the n
+    const double words = (double)n_max / M / 32 + 1;
+    double work = 0.5 * phi * phi * ((double)res / (M / 2)) * (double)((count / res + 31) / 32) * words;
+    if (M > 2) work += 6.0 * phi * words + 2e6;
     if (M == 2 || work < best) {
       best = work;
-      pairs.swap(p);
       ca.modulus = M;
     }
   }
@@ -1181,13 +1180,13 @@ static gb_status counts_impl(gb_ctx* c, Workspace& w, uint64_t start, uint64_t c
   if (ca.modulus > 2) {
     cwords = n_max / ca.modulus / 32 + 1;
     stride = (cwords + 2 + 3) & ~3ull;
-    const uint64_t nc = ca.modulus == 6 ? 2 : ca.modulus == 30 ? 8 : 48;
+    const uint64_t nc = ca.modulus == 30 ? 8 : 48;
     if (ws_buffer(c, w, tmp, 2, (nc * stride + 8) * 4, (void**)&classes) != GB_OK) {
       w.err.clear();  // no room beside the odd bitset: the odd classes alone
       ca.modulus = 2;
-      pairs = count_pairs(2, start, count, &best);
     }
   }
+  const std::vector<CountPair> pairs = count_pairs(ca.modulus, start, count);
   CountPair* d_pairs = nullptr;
   if ((st = ws_buffer(c, w, tmp, 3, std::max<size_t>(pairs.size(), 1) * sizeof(CountPair), (void**)&d_pairs)) != GB_OK)
     return st;
@@ -1204,7 +1203,6 @@ static gb_status counts_impl(gb_ctx* c, Workspace& w, uint64_t start, uint64_t c
   a.kcoop = (uint32_t)std::max<uint64_t>(std::min(kc, ns), kWheelPrimeCount + 1);
   a.wheel = c->d_wheel;
   a.out = buf + 2;
-  // Work split: enough warp tasks to fill the GPU, at most 2^22 words each.
   ca.classes = ca.modulus > 2 ? classes + 4 : buf + 2;
   ca.stride = stride;
   ca.pairs = d_pairs;
@@ -1214,9 +1212,20 @@ static gb_status counts_impl(gb_ctx* c, Workspace& w, uint64_t start, uint64_t c
   for (const CountPair& p : pairs) ca.groups = std::max<uint64_t>(ca.groups, (p.count + 31) / 32);
   const uint64_t lanes = std::max<uint64_t>(1, ca.groups * pairs.size());
   const uint64_t wmax = ca.modulus > 2 ? cwords : n_max / 4 / 32 + 1;  // words of k for the largest n
-  ca.splits = std::max<uint64_t>(1, ((uint64_t)c->sm_count * 256 + lanes - 1) / lanes);
-  ca.splits = std::max<uint64_t>(ca.splits, (wmax + (1u << 22) - 1) >> 22);
-  ca.wps = std::max<uint64_t>(224, ((wmax + ca.splits - 1) / ca.splits + 223) / 224 * 224);  // whole rounds of 7 words a lane
+  // Work split, at most 2^22 words a task.  Less than a round of 7 words a lane
+  // for each warp the SMs hold (16): single words, spread over those; else whole
+  // rounds, up to four (the end of a task, 31 shuffles, costs about one: 32 n near
+  // 1e9 in tasks of one round 477 us, of four 384), in 64 tasks per SM, and more
+  // than four in 256.
+  const auto per_task = [&](uint64_t tasks) {
+    const uint64_t splits = std::max((tasks + lanes - 1) / lanes, (wmax + (1u << 22) - 1) >> 22);
+    return (wmax + splits - 1) / splits;
+  };
+  ca.wps = (per_task((uint64_t)c->sm_count * 16) + 31) / 32 * 32;
+  if (ca.wps >= 224) {
+    ca.wps = std::min<uint64_t>(896, per_task((uint64_t)c->sm_count * 64));
+    ca.wps = (std::max(ca.wps, per_task((uint64_t)c->sm_count * 256)) + 223) / 224 * 224;
+  }
   ca.splits = (wmax + ca.wps - 1) / ca.wps;
   // the sieve writes words 2 .. nwords + 1; the padding around them is zero
   cudaError_t e = cudaMemsetAsync(buf, 0, 8, s);
@@ -1224,13 +1233,18 @@ static gb_status counts_impl(gb_ctx* c, Workspace& w, uint64_t start, uint64_t c
   if (e == cudaSuccess) e = launch_sieve_bits(a, s);
   if (ca.modulus > 2) {
     if (e == cudaSuccess) e = cudaMemsetAsync(classes, 0, 16, s);
-    const uint64_t nc = ca.modulus == 6 ? 2 : ca.modulus == 30 ? 8 : 48;
+    const uint64_t nc = ca.modulus == 30 ? 8 : 48;
     if (e == cudaSuccess)  // the words between the classes
       e = cudaMemset2DAsync(classes + 4 + cwords, stride * 4, 0, (stride - cwords) * 4, nc, s);
     if (e == cudaSuccess) e = launch_count_classes(buf + 2, nwords, ca.modulus, classes + 4, stride, cwords, s);
   }
-  if (e == cudaSuccess && !pairs.empty())
-    e = cudaMemcpyAsync(d_pairs, pairs.data(), pairs.size() * sizeof(CountPair), cudaMemcpyHostToDevice, s);
+  if (!pairs.empty()) ca.first = pairs[0];
+  if (e == cudaSuccess && pairs.size() > 1) {
+    const size_t bytes = pairs.size() * sizeof(CountPair);
+    const void* up = pairs.data();
+    if (bytes <= kIoBytes) up = std::memcpy(w.h_io, up, bytes);  // pinned
+    e = cudaMemcpyAsync(d_pairs, up, bytes, cudaMemcpyHostToDevice, s);
+  }
   if (e == cudaSuccess) e = cudaEventRecord(w.ek0, s);
   if (e == cudaSuccess) e = launch_counts(ca, buf + 2, start, count, s);
   if (e == cudaSuccess) e = cudaEventRecord(w.ek1, s);

@@ -3,14 +3,14 @@
 // c(n) = #{p <= n/2 : p and n - p prime}, the reference's goldbach_count
 // (src/cpu_goldbach.cpp:29-36, a scalar scan over a byte table on the CPU;
 // "partition counting c(n) at scale" is its open roadmap item,
-// RESULTS.md:169).  The primes are split by residue: for a modulus M (2, 6, 30
-// or 210) and a residue a prime to it, C_a is the bitset of the primes M k + a.
+// RESULTS.md:169).  The primes are split by residue: for a modulus M (2, 30 or
+// 210) and a residue a prime to it, C_a is the bitset of the primes M k + a.
 // With n = M t + r, p = a and q = b (mod M) need a + b = r (mod M), so
 //     c(n) = sum over the pairs {a, b} of sum_k C_a[k] C_b[s - k]
 //            + #{p | M : p <= n/2, n - p prime},     s = t - (a + b - r) / M,
 // k over 0 .. s, or 0 .. s/2 for a = b.  A larger M leaves fewer pairs to test
-// (n/4 of them per n for M = 2, 0.11, 0.071 and 0.052 n on average for 6, 30 and
-// 210) but takes more n to fill the groups of 32 n of one residue below; the
+// (n/4 of them per n for M = 2, 0.071 and 0.052 n on average for 30 and 210; 6,
+// with 0.11, is never the cheapest) but takes more n to fill the groups of 32 n of one residue below; the
 // host picks the M with the least work (counts_impl).
 //
 // A warp takes one pair {a, b}, 32 consecutive n of one residue (s0 .. s0 + 31)
@@ -50,7 +50,7 @@ __global__ void __launch_bounds__(kCountThreads, 2) counts_kernel(const __grid_c
   task /= a.splits;
   const uint64_t g = task % a.groups;
   if (task / a.groups >= a.npairs) return;  // warp-uniform, like the exits below
-  const CountPair pr = a.pairs[task / a.groups];
+  const CountPair pr = a.npairs == 1 ? a.first : a.pairs[task / a.groups];
   if (g * 32 >= pr.count) return;
   const int64_t s0 = (int64_t)(pr.s0 + 32 * g);
   const int64_t last = pr.half ? (s0 + 31) / 2 : s0 + 31;  // largest k of any d
@@ -168,7 +168,7 @@ __global__ void __launch_bounds__(kGatherThreads) gather_kernel(const uint32_t* 
   const uint32_t* t = tile + threadIdx.x * H;
   int c = 0;
   for (int a = 1; a < M; a += 2) {
-    if (a % 3 == 0 || (M % 5 == 0 && a % 5 == 0) || (M % 7 == 0 && a % 7 == 0)) continue;
+    if (a % 3 == 0 || a % 5 == 0 || (M % 7 == 0 && a % 7 == 0)) continue;
     uint32_t v = 0;
 #pragma unroll 8
     for (int b = 0; b < 32; ++b) {
@@ -184,7 +184,6 @@ cudaError_t launch_count_classes(const uint32_t* odd, uint64_t nodd, uint32_t mo
   const uint64_t blocks = (nwords + kGatherThreads - 1) / kGatherThreads;
   if (blocks > 0x7fffffffull) return cudaErrorInvalidValue;
   switch (modulus) {
-    case 6: gather_kernel<6><<<(unsigned)blocks, kGatherThreads, 0, s>>>(odd, nodd, classes, stride, nwords); break;
     case 30: gather_kernel<30><<<(unsigned)blocks, kGatherThreads, 0, s>>>(odd, nodd, classes, stride, nwords); break;
     case 210: {
       gather_kernel<210><<<(unsigned)blocks, kGatherThreads, 0, s>>>(odd, nodd, classes, stride, nwords);
