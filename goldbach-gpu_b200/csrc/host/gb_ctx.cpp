@@ -619,18 +619,28 @@ gb_status range_impl(gb_ctx* c, Workspace& w, Arena* arena, uint64_t start, uint
   }
   if (e != cudaSuccess) return cuda_fail(w, e, "range setup");
   int launches = 0;
-  const bool masked = my_segs && range_masked_pays(c, start, std::min(count, my_segs * o.seg_size), root, my_segs);
+  bool masked = my_segs && range_masked_pays(c, start, std::min(count, my_segs * o.seg_size), root, my_segs);
   if (masked) {
     std::vector<RangePiece> segs;
     for (uint64_t g = o.shard_index; g < nseg; g += sc)
       segs.push_back(RangePiece{start + 2 * g * o.seg_size, std::min<uint64_t>(o.seg_size, count - g * o.seg_size),
                                 g * o.seg_size, (uint32_t)g});
-    if (!o.chunk_evens) a.chunk_evens = od.min_p ? kMinpChunk : 1u << 20;
+    RangeArgs m = a;
+    if (!o.chunk_evens) m.chunk_evens = od.min_p ? kMinpChunk : 1u << 20;
     chk(cudaEventRecord(w.ek0, s));
-    if ((st = range_masked(c, w, tmp, slot, segs, a, o.chunk_evens ? NE : 0, root, s, &launches)) != GB_OK) return st;
-    chk(cudaEventRecord(w.ek1, s));
-    chk(launch_fallback(sp, c->sm_count * 4, s));
-    ++launches;
+    st = range_masked(c, w, tmp, slot, segs, m, o.chunk_evens ? NE : 0, root, s, &launches);
+    if (st == GB_ENOMEM && launches == 0) {  // no room for the masks (nothing launched yet): the chunks alone
+      masked = false;
+      w.err.clear();
+      const uint32_t slots = 3u << slot;
+      w.buf_used &= ~(slots | slots << Workspace::kBufSlots);
+    } else if (st != GB_OK) {
+      return st;
+    } else {
+      chk(cudaEventRecord(w.ek1, s));
+      chk(launch_fallback(sp, c->sm_count * 4, s));
+      ++launches;
+    }
   }
   int bps = masked ? 1 : range_max_blocks_per_sm(a);
   if (bps < 1) bps = 1;

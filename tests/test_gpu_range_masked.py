@@ -65,3 +65,17 @@ def test_wide_masked_range_agrees_with_windows(ctx):
     assert r.result["verified"] == per[0]["verified"] == count
     assert r.result["max_minp"] == per[0]["max_minp"]
     assert int((r.hist * primes).sum()) == per[0]["minp_sum"]
+
+
+def test_without_room_for_the_masks(gbmod):
+    """A budget that holds the chunks' lists (157 MB) but not the masks (22 MB)
+    beside them: the chunks sieve every prime, with the same results."""
+    start, count = 10**15 + 2, 1 << 28
+    with gbmod.Context(0) as c:
+        room = c.mem_info()[0] + (163 << 20)
+        want = c.verify_range(start, start + 2 * (count - 1), chunk=1 << 20)
+    with gbmod.Context(0, budget=room) as c:
+        got = c.verify_range(start, start + 2 * (count - 1), chunk=1 << 20)
+    np.testing.assert_array_equal(got.hist, want.hist)
+    assert got.result["verified"] == want.result["verified"] == count
+    assert got.result["kernel_launches"] < want.result["kernel_launches"]
