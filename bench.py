@@ -292,52 +292,46 @@ def measure_windows(gb, ctx, nwin=4096, plain=True, tune=True):
 
 
 _MR7_BASES = (2, 325, 9375, 28178, 450775, 9780504, 1795265022)
-_SMALL = (2, 3, 5, 7, 11, 13, 17, 19, 23, 29, 31)
 
 
-def _mr7_products(q):
-    """(is q prime, modular products) of the oracle's 7-base Miller-Rabin
-    (trial division by the primes <= 31, then per base a binary powmod of
-    bitlen(d) squarings and popcount(d) products, then the squaring tail with
-    its early exit, stopping at the first failing base)."""
-    if q < 2:
-        return False, 0
-    for sp in _SMALL:
-        if q == sp:
-            return True, 0
-        if q % sp == 0:
-            return False, 0
-    if q < 37 * 37:
-        return True, 0
+def _strong(q, b):
+    """(passes the strong test to base b, squarings of its power and tail)."""
     d, s = q - 1, 0
     while d % 2 == 0:
         d //= 2
         s += 1
-    work = 0
-    for b in _MR7_BASES:
-        a = b % q
-        if a == 0:
-            continue
-        work += d.bit_length() + bin(d).count("1")
-        x = pow(a, d, q)
-        if x == 1 or x == q - 1:
-            continue
-        ok = False
-        for _ in range(1, s):
-            work += 1
-            x = x * x % q
-            if x == q - 1:
-                ok = True
-                break
-        if not ok:
-            return False, work
-    return True, work
+    work = d.bit_length()
+    x = pow(b % q, d, q)
+    if x in (0, 1, q - 1):
+        return True, work
+    for _ in range(1, s):
+        work += 1
+        x = x * x % q
+        if x == q - 1:
+            return True, work
+    return False, work
 
 
-def single_mr_products(ns, primes):
-    """Mean modular products per query of the oracle's minimal-p scan (p
-    ascending from 3, q = n - p by the 7-base test): the Miller-Rabin work
-    unit, one Montgomery product each."""
+def _prime_products(q, trial):
+    """(is q prime, modular products) of the least work this build knows: trial
+    division (no products), the strong test to base 2 (its squarings; doublings
+    are not counted), and on a pass the Lucas test's two products per bit.  The
+    verdict itself is the deterministic 7-base test's."""
+    for r in trial:
+        if q % r == 0:
+            return q == r, 0
+    if q < trial[-1] ** 2:
+        return q > 1, 0
+    ok, work = _strong(q, 2)
+    if not ok:
+        return False, work
+    return all(_strong(q, b)[0] for b in _MR7_BASES[1:]), work + 2 * q.bit_length()
+
+
+def single_products(ns, primes):
+    """Mean modular products per query of the minimal-p scan (p ascending from 3,
+    q = n - p sieved by the primes to 617, then tested)."""
+    trial = [int(r) for r in primes if r <= 617]
     tot = 0
     for n in ns:
         n = int(n)
@@ -347,7 +341,7 @@ def single_mr_products(ns, primes):
             p = int(p)
             if p > n // 2:
                 break
-            ok, w = _mr7_products(n - p)
+            ok, w = _prime_products(n - p, trial)
             tot += w
             if ok:
                 break
@@ -385,10 +379,10 @@ def measure_single(gb, ctx, count=10**6):
         p, q, r2 = ctx.check_single(n)
         walls.append(time.perf_counter() - t0)
     e2e = statistics.mean(walls)
-    # roofline: Montgomery products of the oracle's scan (seeded sample of
-    # the batch) against the measured Montgomery-product peak
+    # roofline: Montgomery products of the scan (seeded sample of the batch)
+    # against the measured Montgomery-product peak
     sample = n[np.random.default_rng(5).choice(count, size=1 << 13, replace=False)]
-    per_q = single_mr_products(sample, ctx.primes_upto(100000))
+    per_q = single_products(sample, ctx.primes_upto(100000))
     mont = ctx.probe_mont_products()
     achieved = per_q * count / (ms / 1e3)
     return {"queries": count, "ms": ms, "value": count / (ms / 1e3), "unit": "queries/s",
@@ -398,8 +392,9 @@ def measure_single(gb, ctx, count=10**6):
             "roofline": {"bound": "int-mul", "kernel": "single_kernel",
                          "achieved": achieved / 1e9, "peak": mont / 1e9, "unit": "G Montgomery products/s",
                          "frac": achieved / mont, "products_per_query": per_q,
-                         "work_source": "modular products of the oracle's 7-base scan (base order, "
-                                        "early exit) on 8192 seeded queries of the batch",
+                         "work_source": "modular products of a base-2 strong test per candidate the "
+                                        "primes to 617 leave and a Lucas test per base-2 pass, on "
+                                        "8192 seeded queries of the batch",
                          "peak_source": "measured in-process: gb_probe_mont_products"}}
 
 
