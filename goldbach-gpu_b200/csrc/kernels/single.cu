@@ -461,10 +461,12 @@ __global__ void __launch_bounds__(kSingleThreads, 1) single_kernel(SingleArgs a)
       }
       active &= ~__reduce_or_sync(kFull, rank == 0 && win ? 1u << j : 0u);
       npend += __popc(wb);
+      // the rank-0 lanes' entries and masks before other lanes read them: the proof
+      // below, the refill above, and the copy of what is left after the loop
+      __syncwarp();
     }
     if (npend >= 32) {
       npend -= 32;
-      __syncwarp();
       prove(w.pq[npend + lane], w.pqi[npend + lane], w.pp[npend + lane], true, std::false_type{});
     }
     if (!active && drained && nready == 0) break;
