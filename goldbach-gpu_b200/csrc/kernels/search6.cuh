@@ -105,7 +105,9 @@ struct Ctx6 {
 __shared__ Ctx6 g_cx6;
 // dynamic shared memory of range6_kernel:
 //   class wheel patterns | Q1 | Q5 (nbw words each) | HIST | E0 | E2 | E4
-extern __shared__ uint32_t g_smem6[];
+// and with per-n output the entry positions, which level 0 stores 16 bytes at a time
+extern __shared__ __align__(16) uint32_t g_smem6[];
+static_assert(__alignof__(g_smem6) >= 16, "smem6_eidx rounds its offset, not its address");
 
 __device__ __forceinline__ uint2* surv6_list(int b, int ri) {
   return g_cx6.surv + (size_t)(3 * b + ri) * g_cx6.surv_cap;
