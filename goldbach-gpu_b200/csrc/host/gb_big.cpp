@@ -115,6 +115,7 @@ gb_status big_impl(gb_ctx* c, Workspace& w, const uint32_t* n_limbs, uint32_t nl
   chk(cudaMemsetAsync(d_small, 0, 64, s));
   chk(cudaEventRecord(w.ev0, s));
   Figures* h = (Figures*)w.h_stage;  // pinned
+  *h = Figures{};  // (it holds an earlier call's figures, and np <= 1 reads none)
   uint32_t best = 0xffffffffu;
   uint64_t k0 = 1;  // p = 2 leaves q = n - 2 even
   uint32_t pk = 0;
