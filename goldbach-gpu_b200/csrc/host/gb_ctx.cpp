@@ -9,11 +9,9 @@
 #include "gb_ctx.h"
 
 #include <algorithm>
-#include <atomic>
 #include <cmath>
 #include <cstring>
 #include <new>
-#include <thread>
 
 namespace gb {
 
@@ -183,92 +181,6 @@ void ws_free(gb_ctx* c, Workspace& w) {
       cudaEventDestroy(*e);
       *e = nullptr;
     }
-}
-
-// A pageable copy of the runtime moves about 6.5 GB/s; the ring's slots come in at
-// the link's rate and four threads empty them (11 MB of minimal p: 1.7 -> 0.6 ms).
-constexpr size_t kRingSlot = 1u << 20;
-constexpr int kRingSlots = 4, kRingThreads = 4;
-
-cudaError_t copy_out(Workspace& w, void* dst, const void* src, size_t bytes, cudaStream_t s) {
-  cudaPointerAttributes at{};
-  if (bytes < 2 * kRingSlot ||
-      (cudaPointerGetAttributes(&at, dst) == cudaSuccess && at.type != cudaMemoryTypeUnregistered))
-    return cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, s);
-  cudaGetLastError();
-  if (!w.h_ring) {
-    if (cudaMallocHost((void**)&w.h_ring, kRingSlot * kRingSlots) != cudaSuccess) {
-      cudaGetLastError();
-      w.h_ring = nullptr;
-      return cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, s);
-    }
-    for (cudaEvent_t& e : w.ring_ev) {
-      cudaError_t x = cudaEventCreateWithFlags(&e, cudaEventDisableTiming);
-      if (x != cudaSuccess) return x;
-    }
-  }
-  const size_t slots = (bytes + kRingSlot - 1) / kRingSlot;
-  auto len = [&](size_t i) { return std::min(kRingSlot, bytes - i * kRingSlot); };
-  auto fill = [&](size_t i) {
-    const int r = (int)(i % kRingSlots);
-    cudaError_t x = cudaMemcpyAsync(w.h_ring + r * kRingSlot, (const char*)src + i * kRingSlot, len(i),
-                                    cudaMemcpyDeviceToHost, s);
-    return x == cudaSuccess ? cudaEventRecord(w.ring_ev[r], s) : x;
-  };
-  // ready: slots that have arrived; taken: the next quarter of a slot to empty;
-  // left: quarters of each ring slot not yet emptied
-  std::atomic<size_t> ready{0}, taken{0};
-  std::atomic<int> left[kRingSlots];
-  constexpr size_t kParts = 4;
-  for (auto& l : left) l.store(0);
-  auto empty_one = [&]() -> bool {  // whether there was a part to take
-    size_t t = taken.load(std::memory_order_relaxed);
-    do {
-      if (t >= ready.load(std::memory_order_acquire) * kParts) return false;
-    } while (!taken.compare_exchange_weak(t, t + 1));
-    const size_t i = t / kParts, part = len(i) / kParts, o = (t % kParts) * part;
-    const size_t n = t % kParts == kParts - 1 ? len(i) - o : part;
-    std::memcpy((char*)dst + i * kRingSlot + o, w.h_ring + (i % kRingSlots) * kRingSlot + o, n);
-    left[i % kRingSlots].fetch_sub(1, std::memory_order_release);
-    return true;
-  };
-  std::atomic<bool> stop{false};
-  std::thread helpers[kRingThreads - 1];
-  int nh = 0;
-  try {
-    for (; nh < kRingThreads - 1; ++nh)
-      helpers[nh] = std::thread([&] {
-        while (!stop.load(std::memory_order_acquire))
-          if (!empty_one()) std::this_thread::yield();
-      });
-  } catch (...) {  // no more threads: fewer helpers
-  }
-  cudaError_t e = cudaSuccess;
-  for (size_t i = 0; i < slots && i < (size_t)kRingSlots && e == cudaSuccess; ++i) e = fill(i);
-  for (size_t i = 0; i < slots && e == cudaSuccess; ++i) {
-    const int r = (int)(i % kRingSlots);
-    while (e == cudaSuccess) {  // slot i's arrival, emptying earlier ones meanwhile
-      const cudaError_t q = cudaEventQuery(w.ring_ev[r]);
-      if (q == cudaSuccess) break;
-      if (q != cudaErrorNotReady) e = q;
-      empty_one();
-    }
-    cudaGetLastError();
-    if (e != cudaSuccess) break;
-    left[r].store((int)kParts, std::memory_order_relaxed);
-    ready.store(i + 1, std::memory_order_release);
-    if (i + 1 >= (size_t)kRingSlots && i + 1 < slots) {  // slot i + 1 goes where slot i + 1 - kRingSlots was
-      while (left[(i + 1) % kRingSlots].load(std::memory_order_acquire) != 0) empty_one();
-      e = fill(i + 1);
-    }
-  }
-  while (e == cudaSuccess && empty_one()) {
-  }
-  for (auto& l : left)
-    while (e == cudaSuccess && l.load(std::memory_order_acquire) != 0) std::this_thread::yield();
-  stop.store(true, std::memory_order_release);
-  for (int h = 0; h < nh; ++h) helpers[h].join();
-  return e;
 }
 
 uint64_t isqrt_u64(uint64_t n) {  // exact floor(sqrt(n)), src/goldbach.cu:637-646
