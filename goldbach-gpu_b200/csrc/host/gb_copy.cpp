@@ -1,7 +1,10 @@
 // gb_copy.cpp -- device -> host copies of a call's large outputs.
 #include <algorithm>
 #include <atomic>
+#include <chrono>
+#include <condition_variable>
 #include <cstring>
+#include <mutex>
 #include <thread>
 
 #include "gb_ctx.h"
@@ -63,19 +66,42 @@ cudaError_t copy_out(Workspace& w, void* dst, const void* src, size_t bytes, cud
     left[i % kRingSlots].fetch_sub(1, std::memory_order_release);
     return true;
   };
+  // The kernels that make the bytes may run for long: until they are behind, this
+  // thread waits in the runtime, and the helpers go to sleep after a millisecond.
+  // (Asleep from the start they wake 45 us late: 61 windows with per-n output
+  // 1.16 ms instead of 1.11.)
+  std::mutex mu;
+  std::condition_variable cv;
+  std::atomic<bool> behind{false};
   std::atomic<bool> stop{false};
   std::thread helpers[kRingThreads - 1];
   int nh = 0;
   try {
     for (; nh < kRingThreads - 1; ++nh)
       helpers[nh] = std::thread([&] {
+        const auto until = std::chrono::steady_clock::now() + std::chrono::milliseconds(1);
+        while (!behind.load(std::memory_order_acquire) && std::chrono::steady_clock::now() < until)
+          std::this_thread::yield();
+        if (!behind.load(std::memory_order_acquire)) {
+          std::unique_lock<std::mutex> lk(mu);
+          cv.wait(lk, [&] { return behind.load(); });
+        }
         while (!stop.load(std::memory_order_acquire))
           if (!empty_one()) std::this_thread::yield();
       });
   } catch (...) {  // no more threads: fewer helpers
   }
-  cudaError_t e = cudaSuccess;
-  for (size_t i = 0; i < slots && i < (size_t)kRingSlots && e == cudaSuccess; ++i) e = fill(i);
+  // (the last ring slot's event stands in front of the copies until then)
+  const size_t last = kRingSlots - 1;
+  cudaError_t e = cudaEventRecord(w.ring_ev[last], s);
+  for (size_t i = 0; i < slots && i < last && e == cudaSuccess; ++i) e = fill(i);
+  if (e == cudaSuccess) e = cudaEventSynchronize(w.ring_ev[last]);
+  {
+    std::lock_guard<std::mutex> lk(mu);
+    behind.store(true, std::memory_order_release);
+  }
+  cv.notify_all();
+  if (slots > last && e == cudaSuccess) e = fill(last);
   for (size_t i = 0; i < slots && e == cudaSuccess; ++i) {
     const int r = (int)(i % kRingSlots);
     while (e == cudaSuccess) {  // slot i's arrival, emptying earlier ones meanwhile

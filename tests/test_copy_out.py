@@ -1,8 +1,9 @@
 """copy_out (goldbach-gpu_b200/csrc/host/gb_copy.cpp) on the host, over a small
 stand-in for the CUDA runtime: one stream whose work a thread runs in order,
 behind a kernel of a given length, and calls that can be made to fail.  The
-pinned ring's copies arrive whole, and a ring that could not be set up leaves
-nothing behind that a later copy trips over."""
+pinned ring's copies arrive whole, a ring that could not be set up leaves
+nothing behind that a later copy trips over, and the threads that empty the
+ring sleep while the kernel in front of the copy runs."""
 import os
 import shutil
 import subprocess
@@ -161,6 +162,14 @@ int main(int argc, char** argv) {
       check(events == ev + 4 && pinned == pin + 1, "the ring");
     }
   }
+  if (mode == "kernel") {  // a kernel of 0.4 s in front: the host waits, it does not work
+    gb::Workspace w;
+    check(copies(w, 5 << 20, 1), "the first copy");
+    push([] { std::this_thread::sleep_for(std::chrono::milliseconds(400)); });
+    const std::clock_t c0 = std::clock();  // of all threads
+    check(copies(w, 5 << 20, 2), "the copy behind it");
+    check((double)(std::clock() - c0) / CLOCKS_PER_SEC < 0.2, "processor time");
+  }
   std::printf(fails ? "failed\n" : "ok\n");
   std::fflush(stdout);
   std::_Exit(fails ? 1 : 0);  // (the stream's thread waits for work)
@@ -181,7 +190,7 @@ def harness(tmp_path_factory):
     return str(exe)
 
 
-@pytest.mark.parametrize("mode", ["sizes", "setup"])
+@pytest.mark.parametrize("mode", ["sizes", "setup", "kernel"])
 def test_copy_out(harness, mode):
     r = subprocess.run([harness, mode], capture_output=True, text=True, timeout=60)
     assert r.returncode == 0 and r.stdout.strip().endswith("ok"), r.stdout[-2000:]
