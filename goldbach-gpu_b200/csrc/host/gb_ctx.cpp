@@ -69,11 +69,7 @@ void dev_free(gb_ctx* c, void* p) {
   cudaFree(p);
 }
 
-// dev_alloc for a workspace's call: when there is no room, the kept buffers
-// the call has not asked for are given back first.
-static gb_status ws_alloc(gb_ctx* c, Workspace& w, size_t bytes, void** p) {
-  gb_status st = dev_alloc(c, p, bytes, &w.err);
-  if (st != GB_ENOMEM) return st;
+bool ws_give_back(gb_ctx* c, Workspace& w) {
   bool freed = false;
   for (int i = 0; i < 2 * Workspace::kBufSlots; ++i)
     if (w.buf[i] && !((w.buf_used >> i) & 1u)) {
@@ -82,7 +78,14 @@ static gb_status ws_alloc(gb_ctx* c, Workspace& w, size_t bytes, void** p) {
       w.buf_bytes[i] = 0;
       freed = true;
     }
-  if (!freed) return st;
+  return freed;
+}
+
+// dev_alloc for a workspace's call: when there is no room, the kept buffers
+// the call has not asked for are given back first.
+static gb_status ws_alloc(gb_ctx* c, Workspace& w, size_t bytes, void** p) {
+  gb_status st = dev_alloc(c, p, bytes, &w.err);
+  if (st != GB_ENOMEM || !ws_give_back(c, w)) return st;
   w.err.clear();
   return dev_alloc(c, p, bytes, &w.err);
 }

@@ -126,6 +126,9 @@ gb_status ws_scratch(gb_ctx* c, Workspace& w, size_t bytes, void** p);
 constexpr size_t kKeptBufferBytes = 1ull << 30, kBigBufferBytes = 32ull << 20;
 struct Temps;
 gb_status ws_buffer(gb_ctx* c, Workspace& w, Temps& t, int slot, size_t bytes, void** p);
+// Gives back the kept buffers the current call has not asked for; whether
+// there were any.
+bool ws_give_back(gb_ctx* c, Workspace& w);
 constexpr size_t kIoBytes = 1u << 20;
 // Device -> host copy of `bytes` behind the work queued on s.  Small copies and
 // copies into pinned memory are queued; large ones into pageable memory are

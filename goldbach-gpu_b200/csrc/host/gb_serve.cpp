@@ -509,6 +509,9 @@ gb_status gb_serve_start(gb_ctx* c, const gb_serve_opts* opts) {
     return bail(GB_EINVAL);
   }
   S->nlanes = 1 + (int)S->o.range_lanes;
+  // the server's memory goes before what earlier calls keep
+  c->ws.buf_used = 0;
+  ws_give_back(c, c->ws);
   // resident tables for every n served: sieving primes to sqrt(max_n) and
   // the candidate primes; frozen while the lanes run
   gb_status st = ensure_primes(c, c->ws, std::max<uint64_t>(isqrt_u64(S->o.max_n) + 2,
