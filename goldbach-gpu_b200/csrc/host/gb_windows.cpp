@@ -410,6 +410,7 @@ static gb_status windows_sieve_impl(gb_ctx* c, Workspace& ws, Arena* arena, cons
   const size_t o_tile = o_coff + (count + 1) * 8, o_run = o_tile + tile_off.size() * 8;
   const size_t o_cone = o_run + run_off.size() * 8, o_tone = o_cone + (plain ? 2 * count * 8 : 0);
   const size_t up_bytes = o_tone + (plain ? test_one.size() * 8 : 0);
+  ws.buf_used = 0;  // (the other path's part of the batch is complete, and so is an earlier batch)
   // results: sum and largest minimal p and failures of each window
   const size_t res_bytes = count * 20;
   Temps tmp(c, arena);
@@ -674,6 +675,7 @@ static gb_status windows_mr_impl(gb_ctx* c, Workspace& ws, Arena* arena, const g
   total = off[count];
   const uint64_t np = count_bound(c, p_lim);  // the kernel stops at p_lim itself
   gb_status st;
+  ws.buf_used = 0;  // (as in windows_sieve_impl)
   Temps tmp(c, arena);
   void *d_w, *d_off, *d_n, *d_p, *d_q, *d_agg;
   if ((st = ws_buffer(c, ws, tmp, 0, count * sizeof(gb_window), &d_w)) != GB_OK ||
