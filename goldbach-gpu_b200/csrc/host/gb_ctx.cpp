@@ -12,6 +12,7 @@
 #include <cmath>
 #include <cstring>
 #include <new>
+#include <numeric>
 
 namespace gb {
 
@@ -144,6 +145,10 @@ gb_status ws_buffer(gb_ctx* c, Workspace& w, Temps& t, int slot, size_t bytes, v
     w.buf[slot] = nullptr;
     w.buf_bytes[slot] = 0;
     const size_t grow = std::max<size_t>(bytes, 64 << 10);
+    const auto room = [&] {
+      return std::accumulate(w.buf_bytes, w.buf_bytes + 2 * Workspace::kBufSlots, grow) <= kKeptTotalBytes;
+    };
+    if (!room() && !(ws_give_back(c, w) && room())) return t.get(bytes, p, w);
     gb_status st = ws_alloc(c, w, grow, &w.buf[slot]);
     if (st != GB_OK) return st;
     w.buf_bytes[slot] = grow;

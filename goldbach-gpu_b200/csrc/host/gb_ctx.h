@@ -120,10 +120,11 @@ void ws_free(gb_ctx* c, Workspace& w);
 gb_status ws_scratch(gb_ctx* c, Workspace& w, size_t bytes, void** p);
 // Per-call device buffers kept between calls (no cudaMalloc / cudaFree per
 // call for the usual sizes): slot `slot` of the workspace, grown to `bytes`;
-// above kKeptBufferBytes the buffer comes from `t` and is freed with it.  Kept
-// buffers the current call has not asked for are given back when an
-// allocation fails for want of memory or budget.
-constexpr size_t kKeptBufferBytes = 1ull << 30, kBigBufferBytes = 32ull << 20;
+// above kKeptBufferBytes, or beyond kKeptTotalBytes for the workspace, the
+// buffer comes from `t` and is freed with it.  Kept buffers the current call has
+// not asked for are given back when an allocation fails for want of memory or
+// budget, when the total would pass its bound, and to a server that starts.
+constexpr size_t kKeptBufferBytes = 1ull << 30, kKeptTotalBytes = 2ull << 30, kBigBufferBytes = 32ull << 20;
 struct Temps;
 gb_status ws_buffer(gb_ctx* c, Workspace& w, Temps& t, int slot, size_t bytes, void** p);
 // Gives back the kept buffers the current call has not asked for; whether
