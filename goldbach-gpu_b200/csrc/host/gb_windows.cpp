@@ -291,28 +291,28 @@ static gb_status windows_sieve_impl(gb_ctx* c, Workspace& ws, Arena* arena, cons
   const uint64_t large_per_sm = o.large_ctas_per_sm ? o.large_ctas_per_sm : kLargeBlocksPerSM;
   if (o.gpu_share_pct > 100) return fail(ws, GB_EINVAL, "gpu_share_pct must be <= 100");
   const uint64_t share = o.gpu_share_pct ? o.gpu_share_pct : 100;
-  uint64_t total_n = 0, q_max = 0;
+  std::vector<uint32_t> order(count);
+  std::vector<char> tested(count);
+  uint64_t total_n = 0, n_tested = 0, q_max = 0, q_sieved = 0;
   for (size_t i = 0; i < count; ++i) {
     if (w[i].start < 4 || (w[i].start & 1) || w[i].count == 0)
       return fail(ws, GB_EINVAL, "window start must be even and >= 4, count >= 1");
     const uint64_t last = w[i].start + 2 * (w[i].count - 1);
     if (w[i].count > GB_WINDOW_MAX_COUNT) return fail(ws, GB_EINVAL, "window wider than GB_WINDOW_MAX_COUNT");
     if (last < w[i].start) return fail(ws, GB_EINVAL, "window passes 2^64");
+    tested[i] = window_path(w[i], o) == kTested;
+    if (tested[i]) n_tested += w[i].count;
+    else q_sieved = std::max(q_sieved, last);
     q_max = std::max(q_max, last);
     total_n += w[i].count;
   }
-  const uint64_t root = isqrt_u64(q_max);
-  gb_status st = ensure_primes(c, ws, std::max<uint64_t>({p_lim, (uint64_t)H, root + 2, kWinChunkSieveBound}));
+  // a sieved window needs every prime up to its top's root, a tested one only
+  // those of its presieve (below kHostPrimeLimit, which every table covers)
+  const uint64_t root = isqrt_u64(q_max), root_sieved = isqrt_u64(q_sieved);
+  gb_status st = ensure_primes(c, ws, std::max<uint64_t>({p_lim, (uint64_t)H, root_sieved + 2, kWinChunkSieveBound}));
   if (st != GB_OK) return st;
   // descriptors: the sieved windows first, sorted by top q so that a prime
   // visits a suffix of them, then the tested ones
-  std::vector<uint32_t> order(count);
-  std::vector<char> tested(count);
-  uint64_t n_tested = 0;
-  for (size_t i = 0; i < count; ++i) {
-    tested[i] = window_path(w[i], o) == kTested;
-    if (tested[i]) n_tested += w[i].count;
-  }
   std::iota(order.begin(), order.end(), 0u);
   std::sort(order.begin(), order.end(), [&](uint32_t x, uint32_t y) {
     if (tested[x] != tested[y]) return tested[x] < tested[y];
@@ -396,7 +396,7 @@ static gb_status windows_sieve_impl(gb_ctx* c, Workspace& ws, Arena* arena, cons
     ta.nsieve[k] = (uint32_t)std::max<uint64_t>(n, kWheelPrimeCount + 1);
   }
   uint64_t ns = 0, kc = 0, kct = 0;
-  const uint64_t kf = count_bound(c, p_lim), nlarge = count_bound(c, root);
+  const uint64_t kf = count_bound(c, p_lim), nlarge = count_bound(c, root_sieved);
   if ((st = count_le(c, ws, std::min<uint64_t>(H - 13, p_lim), &ns)) != GB_OK ||
       (st = count_le(c, ws, (H / 6 + NE / 3) / 64, &kc)) != GB_OK ||
       (st = count_le(c, ws, tile_words / 2, &kct)) != GB_OK)
