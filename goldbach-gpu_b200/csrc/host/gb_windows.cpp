@@ -44,29 +44,89 @@ constexpr uint64_t kMaskedWidth = 1ull << 18, kMaskedRoot = 6000000;
 constexpr uint64_t kMinSievedChunk = 1ull << 15, kMinTestedChunk = 1ull << 13;
 
 // The path of a window, by what it costs (results do not depend on it).
-//   kPerN: its n one by one through the single-n kernel (about 1 ns per n);
 //   kTested: a short sieve and a primality test of every q left (about 16 ps
 //     per n near 1e18, and some 100 ns for the halo);
 //   kSieved: every sieving prime's first multiple (the large-prime pass: about
 //     0.5 ps per prime, and 3 ps per n for its marks).
-// So the line between the last two lies at pi(sqrt(top)) / 30 n (4096 windows
+// So the line between the two lies at pi(sqrt(top)) / 30 n (4096 windows
 // in [1e15, 1e18]: 53.7 ms at 20, 52.8 at 40, 61 at 80), pi(sqrt(top)) /
-// mr_divisor where the caller sets it, and below kPerNMax n the first is
-// the cheapest.  mr_below = 1 sieves every window; another mr_below sends
-// narrower windows n by n and sieves the others.
-enum WinPath { kPerN, kTested, kSieved };  // (ranges: range_masked below)
+// mr_divisor where the caller sets it.  A third path takes a window n by n
+// through the single-n kernel (per_n_windows).  mr_below = 1 sieves every window;
+// another mr_below sends narrower windows n by n and sieves the others.
+enum WinPath { kTested, kSieved };  // (ranges: range_masked below)
 constexpr double kTestDivisor = 30.0;
-constexpr uint64_t kPerNMax = 64;
 
 static WinPath window_path(const gb_window& w, const gb_windows_opts& o) {
-  if (o.mr_below) return w.count < o.mr_below && o.mr_below != 1 ? kPerN : kSieved;
+  if (o.mr_below) return kSieved;
   const uint64_t last = w.start + 2 * (w.count - 1);
   const double r = std::sqrt((double)last);
   if (r <= (double)kWinChunkSieveBound) return kSieved;  // no prime needs the large-prime pass
   const double div = o.mr_divisor ? (double)o.mr_divisor : kTestDivisor;
   const double lim = 1.1 * r / std::log(r) / div;  // pi(r) < 1.1 r / ln r here
-  if ((double)w.count >= lim) return kSieved;
-  return w.count < kPerNMax ? kPerN : kTested;
+  return (double)w.count >= lim ? kSieved : kTested;
+}
+
+// The windows that go n by n, which costs 60 us for the batch and 0.75 to 1.2 ns
+// per n.  The other two paths cost 85 us (sieved, near 1e9) to 140 (tested) for
+// the batch, and 0.13 to 0.31 us per window whatever its width.  Measured, n by n
+// against the others, in us: 4096 windows of 100 n 301 / 681 near 1e9, 360 / 1256
+// near 1e12, 474 / 1411 near 1e18, of 256 n 520 / 715, 634 / 1318, 880 / 1487; one
+// window of 1 n near 1e12 65 / 116, of 1000 n near 1e18 72 / 151, of 16000 n 142 /
+// 177, of 30000 193 / 178; 8 windows of 4000 n near 1e18 130 / 176, of 16000 255 /
+// 178; 64 of 1000 n 158 / 181, of 2000 218 / 183.  So:
+//   * a batch goes n by n as a whole when its windows have fewer than kPerNMax n,
+//     or, where they would be tested, up to kPerNWide, and together not more than
+//     kPerNBatch beside kPerNMax for each;
+//   * in another batch the windows of fewer than kPerNMax n do when what they
+//     save (half as much where they would be sieved) is worth kPerNBatch n, the
+//     other path's fixed cost.
+// n below 2^21 take the single-n kernel's plain path, a warp each (4096 windows of
+// 100 n near 1e6 10.3 ms / 0.6): such windows are not taken.
+// With an arena only windows of fewer than kPerNMax n do, for the memory that
+// windows_request_bytes states.  few, and where this takes more than kPerNMost n
+// (24 bytes each): tested windows of fewer than kPerNFew n alone.
+constexpr uint64_t kPerNMax = 256, kPerNWide = 1ull << 14, kPerNBatch = 1ull << 16, kPerNMost = 1ull << 24;
+constexpr uint64_t kPerNFew = 64;
+constexpr uint64_t kPerNLeast = 1ull << 21;
+
+static bool is_narrow(const gb_window& w) { return w.count < kPerNMax && w.start >= kPerNLeast; }
+
+static std::vector<char> per_n_windows(const gb_window* w, size_t count, const gb_windows_opts& o, bool arena,
+                                       bool few) {
+  std::vector<char> per_n(count, 0);
+  if (o.mr_below) {
+    for (size_t i = 0; i < count; ++i) per_n[i] = w[i].count < o.mr_below && o.mr_below != 1;
+    return per_n;
+  }
+  bool all = true;
+  uint64_t total = 0, narrow = 0, saved = 0;  // n: of the batch, of the narrow windows, worth of going n by n
+  for (size_t i = 0; i < count; ++i) {
+    const uint64_t n = w[i].count;
+    const bool tested = window_path(w[i], o) == kTested;
+    per_n[i] = tested && n < kPerNFew;
+    if (!is_narrow(w[i]) && (arena || !tested || n > kPerNWide)) all = false;
+    total += std::min(n, kPerNWide);
+    if (is_narrow(w[i])) {
+      narrow += n;
+      saved += (kPerNMax - n) >> (tested ? 0 : 1);
+    }
+  }
+  all = all && total <= kPerNBatch + kPerNMax * count;
+  if (few || (all ? total : narrow) > kPerNMost) return per_n;
+  for (size_t i = 0; i < count; ++i) per_n[i] = all || (saved >= kPerNBatch && is_narrow(w[i]));
+  return per_n;
+}
+
+// What the pipeline's options do not allow (null: nothing).
+static const char* opts_error(const gb_windows_opts& o) {
+  const uint32_t H = o.halo ? o.halo : kWinHalo, NE = o.chunk_evens ? o.chunk_evens : (1u << 20);
+  if (H < 128 || H > (1u << 17) || (H & 63)) return "halo must be a multiple of 64 in [128, 2^17]";
+  if (NE < 8192 || NE > (1u << 20) || (NE & (NE - 1))) return "chunk_evens must be a power of two in [2^13, 2^20]";
+  if (o.block_threads && o.block_threads != 256 && o.block_threads != 512 && o.block_threads != 1024)
+    return "block_threads must be 256, 512 or 1024";
+  if (o.phase2_limit > GB_P_SMALL_MAX) return "phase2_limit must be <= 4e9";
+  if (o.gpu_share_pct > 100) return "gpu_share_pct must be <= 100";
+  return nullptr;
 }
 
 // The largest power of two up to `most` that cuts `total` n into at least
@@ -279,17 +339,11 @@ static gb_status windows_sieve_impl(gb_ctx* c, Workspace& ws, Arena* arena, cons
   if (count == 0) return GB_OK;
   if (count > 0xffffffffull) return fail(ws, GB_EINVAL, "too many windows");
   const uint32_t H = o.halo ? o.halo : kWinHalo;
-  if (H < 128 || H > (1u << 17) || (H & 63)) return fail(ws, GB_EINVAL, "halo must be a multiple of 64 in [128, 2^17]");
   uint32_t NE = o.chunk_evens ? o.chunk_evens : (1u << 20);
-  if (NE < 8192 || NE > (1u << 20) || (NE & (NE - 1)))
-    return fail(ws, GB_EINVAL, "chunk_evens must be a power of two in [2^13, 2^20]");
+  if (const char* bad = opts_error(o)) return fail(ws, GB_EINVAL, bad);
   if (min_p_concat && NE > kMinpChunk) NE = kMinpChunk;  // per-n output: smaller chunks
-  if (o.block_threads && o.block_threads != 256 && o.block_threads != 512 && o.block_threads != 1024)
-    return fail(ws, GB_EINVAL, "block_threads must be 256, 512 or 1024");
   const uint64_t p_lim = o.phase2_limit ? o.phase2_limit : GB_PHASE2_LIMIT_DEFAULT;
-  if (p_lim > GB_P_SMALL_MAX) return fail(ws, GB_EINVAL, "phase2_limit must be <= 4e9");
   const uint64_t large_per_sm = o.large_ctas_per_sm ? o.large_ctas_per_sm : kLargeBlocksPerSM;
-  if (o.gpu_share_pct > 100) return fail(ws, GB_EINVAL, "gpu_share_pct must be <= 100");
   const uint64_t share = o.gpu_share_pct ? o.gpu_share_pct : 100;
   std::vector<uint32_t> order(count);
   std::vector<char> tested(count);
@@ -744,7 +798,7 @@ static gb_status windows_mr_impl(gb_ctx* c, Workspace& ws, Arena* arena, const g
   return GB_OK;
 }
 
-// Splits the batch by path (window_path): the windows taken n by n run through
+// Splits the batch by path (per_n_windows): the windows taken n by n run through
 // the single-n kernel, the others through the sieve pipeline.  Results do not
 // depend on the split.
 gb_status windows_impl(gb_ctx* c, Workspace& ws, Arena* arena, const gb_window* w, size_t count,
@@ -755,17 +809,18 @@ gb_status windows_impl(gb_ctx* c, Workspace& ws, Arena* arena, const gb_window* 
   if (!count || !w || o.on_device || o.mr_below == 1 ||
       (o.mode != GB_WINDOWS_PERSISTENT && o.mode != GB_WINDOWS_PLAIN))
     return windows_sieve_impl(c, ws, arena, w, count, opts, res, min_p_concat, sum);
-  std::vector<char> narrow(count, 0);
-  size_t nn = 0;
   for (size_t i = 0; i < count; ++i) {
     const uint64_t last = w[i].start + 2 * (w[i].count - 1);
     if (w[i].start < 4 || (w[i].start & 1) || w[i].count == 0 || last < w[i].start)
       return windows_sieve_impl(c, ws, arena, w, count, opts, res, min_p_concat, sum);  // reports it
-    narrow[i] = window_path(w[i], o) == kPerN;
-    nn += narrow[i];
   }
-  if (nn == 0) return windows_sieve_impl(c, ws, arena, w, count, opts, res, min_p_concat, sum);
   const uint64_t p_lim = o.phase2_limit ? o.phase2_limit : GB_PHASE2_LIMIT_DEFAULT;
+  // (options that the pipeline refuses are refused for what it would take, and
+  // its lockstep tries p = 3 whatever the bound)
+  const bool few = opts_error(o) || p_lim < 3;
+  const std::vector<char> narrow = per_n_windows(w, count, o, arena != nullptr, few);
+  const size_t nn = std::count(narrow.begin(), narrow.end(), 1);
+  if (nn == 0) return windows_sieve_impl(c, ws, arena, w, count, opts, res, min_p_concat, sum);
   if (p_lim > GB_P_SMALL_MAX) return fail(ws, GB_EINVAL, "phase2_limit must be <= 4e9");
   gb_status st = ensure_primes(c, ws, std::max<uint64_t>(p_lim, kWinChunkSieveBound));
   if (st != GB_OK) return st;
@@ -784,9 +839,12 @@ gb_status windows_impl(gb_ctx* c, Workspace& ws, Arena* arena, const gb_window* 
   for (const gb_window& x : wb) nb += x.count;
   std::vector<uint32_t> ma(min_p_concat ? na : 0), mb(min_p_concat ? nb : 0);
   gb_windows_summary sa{}, sb{};
-  if ((st = windows_mr_impl(c, ws, arena, wa.data(), wa.size(), o, p_lim, ra.data(),
-                            min_p_concat ? ma.data() : nullptr, &sa)) != GB_OK)
-    return st;
+  st = windows_mr_impl(c, ws, arena, wa.data(), wa.size(), o, p_lim, ra.data(), min_p_concat ? ma.data() : nullptr, &sa);
+  if (st == GB_ENOMEM && !o.mr_below && !few) {  // no room for their n (nothing launched yet): the pipeline alone
+    ws.err.clear();
+    return windows_sieve_impl(c, ws, arena, w, count, opts, res, min_p_concat, sum);
+  }
+  if (st != GB_OK) return st;
   if (!wb.empty() && (st = windows_sieve_impl(c, ws, arena, wb.data(), wb.size(), &o, rb.data(),
                                               min_p_concat ? mb.data() : nullptr, &sb)) != GB_OK)
     return st;
@@ -816,15 +874,15 @@ gb_status windows_impl(gb_ctx* c, Workspace& ws, Arena* arena, const gb_window* 
 
 // Upper bound of the device bytes one window takes from a caller's arena in
 // windows_impl: its share of the sieve path's buffers (descriptor, record,
-// offsets, results, class masks) or, when it is narrow enough for the
-// Miller-Rabin path, of that path's (its n, p, q and a reduction record);
-// arena alignment included.  Used by serving to admit batches by memory.
+// offsets, results, class masks) or, when it is narrow enough to go n by n, of
+// that path's (its n, p, q and a reduction record), whichever is more; arena
+// alignment included.  Used by serving to admit batches by memory.
 uint64_t windows_request_bytes(const gb_window& w, const gb_windows_opts& o) {
   const uint64_t H = o.halo ? o.halo : kWinHalo;
   const uint64_t fixed = sizeof(WinDesc6) + sizeof(WinLarge) + 88 + 4 + 16 + 16 + 4 * 256;
-  if (window_path(w, o) == kPerN) return fixed + w.count * 24 + 64 + 4 * 256;
   const uint64_t lwords = (w.count / 3 + H / 6 + 96) / 32 + 16;
-  return fixed + 2 * lwords * 4;
+  const bool per_n = o.mr_below ? w.count < o.mr_below && o.mr_below != 1 : is_narrow(w);
+  return fixed + std::max(2 * lwords * 4, per_n ? w.count * 24 + 64 + 4 * 256 : 0);
 }
 
 // Autotuner of the windows pipeline: the persistent mode on a sample of the

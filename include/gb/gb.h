@@ -309,11 +309,14 @@ typedef struct gb_windows_opts {
   void* stream;
   uint64_t mr_below;      /* windows of fewer even n skip the sieve: their q
                              are tested for primality (the single-n
-                             kernel).  0: automatic, where sieving would
-                             cost more (fewer than about pi(sqrt(top)) /
-                             mr_divisor n: a short sieve, then a primality
-                             test of every q it leaves); 1: never           */
-  uint32_t mr_divisor;    /* the automatic split's divisor (0: 30)          */
+                             kernel).  0: automatic, by cost: windows of
+                             fewer than about pi(sqrt(top)) / mr_divisor n
+                             take a short sieve, then a primality test of
+                             every q it leaves, and a few n or small batches
+                             of narrow windows go n by n; 1: never          */
+  uint32_t mr_divisor;    /* the automatic split's divisor (0: 30; another
+                             one moves the line between the sieve and the
+                             tests of its short sieve's q)                  */
   uint32_t large_ctas_per_sm; /* grid of the large-prime pass (0: 64)       */
   uint32_t block_threads; /* as gb_range_opts.block_threads (0: 512)        */
   uint32_t gpu_share_pct; /* the persistent kernels of the call (chunk
