@@ -12,8 +12,12 @@
 namespace gb {
 
 // A pageable copy of the runtime moves about 6.5 GB/s; the ring's slots come in at
-// the link's rate and four threads empty them (11 MB of minimal p: 1.7 -> 0.6 ms).
-constexpr size_t kRingSlot = 1u << 20;
+// the link's rate and four threads empty them.  Starting and joining the threads
+// takes up to half a millisecond, so smaller copies stay with the runtime.
+// Range calls with per-n output into a fresh numpy array, median us, runtime / ring: 4 MB 421
+// / 588, 8 MB 714 / 790, 11 MB 916 / 885, 32 MB 7630 / 3420; into one used before:
+// 11 MB 776 / 707, 16 MB 1075 / 1057, 64 MB 4030 / 3156.
+constexpr size_t kRingSlot = 1u << 20, kRingLeast = 10u << 20;
 constexpr int kRingSlots = 4, kRingThreads = 4;
 
 // The ring's memory and events, all of them or none.
@@ -36,7 +40,7 @@ static bool ring_init(Workspace& w) {
 
 cudaError_t copy_out(Workspace& w, void* dst, const void* src, size_t bytes, cudaStream_t s) {
   cudaPointerAttributes at{};
-  if (bytes < 2 * kRingSlot ||
+  if (bytes < kRingLeast ||
       (cudaPointerGetAttributes(&at, dst) == cudaSuccess && at.type != cudaMemoryTypeUnregistered))
     return cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, s);
   cudaGetLastError();

@@ -1,9 +1,9 @@
 """copy_out (goldbach-gpu_b200/csrc/host/gb_copy.cpp) on the host, over a small
 stand-in for the CUDA runtime: one stream whose work a thread runs in order,
 behind a kernel of a given length, and calls that can be made to fail.  The
-pinned ring's copies arrive whole, a ring that could not be set up leaves
-nothing behind that a later copy trips over, and the threads that empty the
-ring sleep while the kernel in front of the copy runs."""
+pinned ring's copies arrive whole, small ones do without it, a ring that could
+not be set up leaves nothing behind that a later copy trips over, and the threads
+that empty the ring sleep while the kernel in front of the copy runs."""
 import os
 import shutil
 import subprocess
@@ -145,29 +145,34 @@ int main(int argc, char** argv) {
     gb::Workspace w;
     const size_t m = 1 << 20;
     unsigned seed = 0;
-    for (size_t n : {size_t(1), m, 2 * m - 1, 2 * m, 2 * m + 1, 4 * m, 4 * m + 3, 5 * m - 1, 37 * m + 12345})
+    for (size_t n : {size_t(1), m, 10 * m - 1}) {
       check(copies(w, n, ++seed), "copy");
+      check(pinned == 0 && events == 0, "a small copy sets up no ring");
+    }
+    for (size_t n : {10 * m, 10 * m + 1, 12 * m - 1, 12 * m + 3, 37 * m + 12345})
+      check(copies(w, n, ++seed), "copy");
+    check(pinned == 1, "the ring");
   } else if (mode == "setup") {
     for (int k = 0; k < 5; ++k) {  // the k-th event, or (4) the memory, cannot be had
       gb::Workspace w;
       const int ev = events, pin = pinned;
       fail_event = k < 4 ? k : -1;
       fail_host = k == 4;
-      check(copies(w, 5 << 20, k), "copy without a ring");
+      check(copies(w, 11 << 20, k), "copy without a ring");
       check(events == ev && pinned == pin, "nothing kept");
       fail_event = -1;
       fail_host = false;
-      check(copies(w, 5 << 20, 10 + k), "the next copy");
-      check(copies(w, 9 << 20, 20 + k), "and the one after");
+      check(copies(w, 11 << 20, 10 + k), "the next copy");
+      check(copies(w, 13 << 20, 20 + k), "and the one after");
       check(events == ev + 4 && pinned == pin + 1, "the ring");
     }
   }
   if (mode == "kernel") {  // a kernel of 0.4 s in front: the host waits, it does not work
     gb::Workspace w;
-    check(copies(w, 5 << 20, 1), "the first copy");
+    check(copies(w, 11 << 20, 1), "the first copy");
     push([] { std::this_thread::sleep_for(std::chrono::milliseconds(400)); });
     const std::clock_t c0 = std::clock();  // of all threads
-    check(copies(w, 5 << 20, 2), "the copy behind it");
+    check(copies(w, 11 << 20, 2), "the copy behind it");
     check((double)(std::clock() - c0) / CLOCKS_PER_SEC < 0.2, "processor time");
   }
   std::printf(fails ? "failed\n" : "ok\n");
