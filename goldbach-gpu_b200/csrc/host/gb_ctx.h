@@ -155,9 +155,6 @@ struct Temps {
   void release();
 };
 
-uint32_t balanced_chunk(uint64_t pieces, uint64_t len, uint64_t tail, double fixed, int sm_count, uint32_t least,
-                        uint32_t most);
-
 // A segment of a range: `unit` is its index, out_off its first output index.
 struct RangePiece {
   uint64_t start, count, out_off;

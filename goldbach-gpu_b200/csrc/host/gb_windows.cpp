@@ -18,6 +18,7 @@
 #include <vector>
 
 #include "gb_ctx.h"
+#include "range_plan.h"
 
 namespace gb {
 // Primes up to this bound sieve each chunk's q-window in shared memory; the
