@@ -501,7 +501,9 @@ gb_status range_impl(gb_ctx* c, Workspace& w, Arena* arena, uint64_t start, uint
   }
   if (e != cudaSuccess) return cuda_fail(w, e, "range setup");
   int launches = 0;
-  bool masked = my_segs && range_masked_pays(c, start, std::min(count, my_segs * o.seg_size), root, my_segs);
+  // (a shard's segments lie apart)
+  bool masked = my_segs && range_masked_pays(c->sm_count, start, std::min(count, my_segs * o.seg_size), root, my_segs,
+                                             sc > 1 ? my_segs : 1, NE);
   if (masked) {
     std::vector<RangePiece> segs;
     for (uint64_t g = o.shard_index; g < nseg; g += sc)

@@ -160,11 +160,9 @@ struct RangePiece {
   uint64_t start, count, out_off;
   uint32_t unit;
 };
-// gb_windows.cpp: whether a range of `count` n from `start` on, with sieving
-// primes up to root, goes through masks of the large-prime pass; and its
-// launches (a: everything but the chunks; ne: chunk width, 0 to pick one of at
-// most a.chunk_evens; slots slot and slot + 1 of the workspace are used).
-bool range_masked_pays(const gb_ctx* c, uint64_t start, uint64_t count, uint64_t root, uint64_t pieces);
+// gb_windows.cpp: the launches of a range through masks of the large-prime pass
+// (a: everything but the chunks; ne: chunk width, 0 to pick one of at most
+// a.chunk_evens; slots slot and slot + 1 of the workspace are used).
 gb_status range_masked(gb_ctx* c, Workspace& ws, Temps& tmp, int slot, const std::vector<RangePiece>& segs,
                        RangeArgs a, uint32_t ne, uint64_t root, cudaStream_t s, int* launches);
 

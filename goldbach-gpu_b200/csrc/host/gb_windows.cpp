@@ -39,9 +39,6 @@ constexpr uint32_t kWinHalo = 8192;
 // be narrower.
 constexpr uint64_t kMinMaskedChunk = 1ull << 16;
 constexpr double kMaskedFixed = 1e5;  // n that a masked range's chunk costs beside its own (balanced_chunk)
-// Ranges of fewer n than this per SM, or with larger sieving primes, are masked
-// (range_masked_pays).
-constexpr uint64_t kMaskedWidth = 1ull << 18, kMaskedRoot = 6000000;
 constexpr uint64_t kMinSievedChunk = 1ull << 15, kMinTestedChunk = 1ull << 13;
 
 // The path of a window, by what it costs (results do not depend on it).
@@ -150,22 +147,6 @@ static int64_t host_window_g0(uint64_t A, uint32_t H) {
 // pieces share one mask, so the large-prime pass meets each prime once per run
 // instead of once per chunk.  Runs and batches hold at most kRangeMaskEvens n,
 // whose masks stay in L2.
-constexpr uint64_t kRangeMaskEvens = 1ull << 28;
-constexpr uint64_t kRangeMaskPieces = 1ull << 20;
-
-// Where it pays.  A chunk spends 0.75 ns on each of its sieving primes, whatever
-// its width (range_chunk); the pass spends 7 ps on a mark.  So it pays for
-// ranges that must be cut into narrow chunks to fill the GPU, and for far
-// ones, where the chunk's primes outweigh its n.  Kernel time, chunks alone
-// against masks: 1e7 n near 1e12 108 -> 95 us, 2e5 n 107 -> 70 us, 1e8 n 174 ->
-// 277 us (not masked); 1e9 n near 1e13 1.42 -> 2.11 ms (not masked); 1e8 n near
-// 1e14 0.53 -> 0.35 ms, 4e7 n near 1e15 1.03 -> 0.19, 1e6 and 1e9 n near 1e17
-// 18.6 -> 0.15 and 67 -> 3.2 ms.  The range must start beyond every sieving
-// prime, and the pass's quotient estimates need p > g0 / 2^42 (masked_bound).
-bool range_masked_pays(const gb_ctx* c, uint64_t start, uint64_t count, uint64_t root, uint64_t pieces) {
-  if (start < (8ull << 30) || root < (1ull << 16) || pieces > kRangeMaskPieces) return false;
-  return count < kMaskedWidth * (uint64_t)c->sm_count || root >= kMaskedRoot;
-}
 
 // Largest prime the chunks sieve themselves: about the chunk's own width (a
 // prime above a third of it marks a class less than once), and enough for the

@@ -50,4 +50,37 @@ inline uint32_t balanced_chunk(uint64_t pieces, uint64_t len, uint64_t tail, dou
   return pick;
 }
 
+// Whether a range of `count` n from `start` on, in `pieces` segments that form
+// `runs` stretches without a gap, goes through masks of the large-prime pass
+// (range_masked); root: its largest sieving prime; ne: the width of its chunks
+// without them.  A chunk spends 0.6 ns on each of its sieving primes, whatever
+// its width, and with two CTAs per SM a wave of chunks as much; the masks leave it the
+// primes up to 2^16.  They cost, in ns: 25000 and 0.05 a prime for the pass,
+// 1.5 per n for its marks, 14000 per further wave (a chunk's window is looked up and its
+// masks read), 400 per run (each prime walks all of them in a row), and 10 per
+// piece on the host.  Chunks alone against masks, us per call: 1e6 n near 1e11 115 /
+// 116, 1e12 132 / 126, 1e13 207 / 126; 1e7 n near 1e12 144 / 153, 4e12 185 / 157; 3e7
+// near 4e12 207 / 208; 1e7 near 1e12 in segments of 1000 n 2379 / 1496; every second of
+// them 1241 / 3059, of 30000 n 157 / 199, near 1e13 243 / 212.
+// From kMaskedWidth n per SM on the chunks are wide, their own cost is below the
+// marks', and the line lies at kMaskedRoot whatever the count: 1e9 n near 1e13 1.46 / 2.11
+// ms, 5e13 2.04 / 1.91, 3e14 3.96 / 2.07, near 1e17 67 / 3.2.
+// The range must start beyond every sieving prime, and the pass's quotient
+// estimates need p > g0 / 2^42 (masked_bound).
+constexpr uint64_t kRangeMaskEvens = 1ull << 28;   // of a run, and of the masks made at a time
+constexpr uint64_t kRangeMaskPieces = 1ull << 20;
+constexpr uint64_t kMaskedWidth = 1ull << 18, kMaskedRoot = 6000000;
+
+inline bool range_masked_pays(int sm_count, uint64_t start, uint64_t count, uint64_t root, uint64_t pieces,
+                              uint64_t runs, uint32_t ne) {
+  if (start < (8ull << 30) || root < (1ull << 16) || pieces > kRangeMaskPieces) return false;
+  if (root >= kMaskedRoot) return true;
+  if (count >= kMaskedWidth * (uint64_t)sm_count) return false;
+  const double primes = 1.1 * (double)root / std::log((double)root) - 6542;  // beyond 2^16
+  const double waves = std::max(1.0, std::max((double)pieces, (double)count / ne) / (2.0 * sm_count));
+  const double cost = 25e3 + 0.05 * primes + 1.5e-3 * (double)count + 14e3 * (waves - 1) + 400.0 * (double)runs +
+                      10.0 * (double)pieces;
+  return cost < 0.6 * primes * waves;
+}
+
 }  // namespace gb

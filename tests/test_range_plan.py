@@ -1,6 +1,7 @@
 """How a range is cut (goldbach-gpu_b200/csrc/host/range_plan.h), compiled on the
 host: chunk widths are multiples of 512 within their bounds and no wider than
-the longest piece, whatever the number of pieces."""
+the longest piece, whatever the number of pieces, and the large-prime masks are
+taken where they were measured to pay."""
 import os
 import shutil
 import subprocess
@@ -35,8 +36,36 @@ static void widths() {
   }
 }
 
+// us per call of the chunks alone and of the masks (B200, 148 SMs): the rule takes
+// the faster one, or one within a tenth of it
+static void masks() {
+  struct Case { double top, count, seg; int shards; double alone, masked; };
+  const Case cases[] = {
+      {9e9, 1e5, 1e7, 1, 93, 114},      {9e9, 1e7, 1e3, 1, 973, 1408},    {9e9, 1e7, 1e3, 2, 532, 3092},
+      {9e9, 1e7, 3e3, 2, 247, 966},     {9e9, 1e7, 1e7, 1, 111, 150},     {1e11, 1e6, 1e7, 1, 115, 117},
+      {1e11, 1e7, 3e3, 2, 330, 971},    {1e12, 1e5, 1e7, 1, 138, 118},    {1e12, 1e6, 1e3, 1, 332, 231},
+      {1e12, 1e7, 1e3, 1, 2379, 1496},  {1e12, 1e7, 1e3, 2, 1241, 3059},  {1e12, 1e7, 3e3, 2, 508, 980},
+      {1e12, 1e7, 1e4, 2, 233, 319},    {1e12, 1e7, 1e7, 1, 144, 152},    {4e12, 1e7, 1e7, 1, 185, 157},
+      {4e12, 3e7, 1e7, 1, 207, 208},    {1e13, 1e6, 1e3, 1, 627, 231},    {1e13, 1e7, 1e3, 2, 2604, 3346},
+      {1e13, 1e7, 3e4, 2, 243, 212},    {1e13, 1e7, 1e7, 1, 220, 165},    {1e13, 1e8, 1e7, 1, 319, 500},
+      {5e13, 1e9, 1e7, 1, 2038, 1906},  {1e14, 1e7, 1e3, 2, 6536, 4118},  {1e14, 1e8, 1e7, 1, 527, 318},
+  };
+  for (const Case& c : cases) {
+    const uint64_t root = (uint64_t)std::sqrt(c.top), segs = (uint64_t)std::ceil(c.count / c.seg);
+    const uint64_t mine = (segs + c.shards - 1) / c.shards;
+    const bool m = gb::range_masked_pays(148, (uint64_t)(c.top - 2 * c.count), (uint64_t)(c.count / c.shards), root, mine,
+                                         c.shards > 1 ? mine : 1, 1u << 20);
+    check((m ? c.masked : c.alone) <= 1.1 * std::min(c.masked, c.alone), "masks", (uint64_t)c.top, (uint64_t)c.count,
+          (uint64_t)c.seg);
+  }
+  // below every sieving prime, and with more segments than the descriptors are meant for
+  check(!gb::range_masked_pays(148, 1u << 30, 1000, 1u << 20, 1, 1, 8192), "low", 0, 0, 0);
+  check(!gb::range_masked_pays(148, 1ull << 60, 1ull << 40, 1u << 30, (1u << 20) + 1, 1, 8192), "pieces", 0, 0, 0);
+}
+
 int main() {
   widths();
+  masks();
   std::printf(fails ? "failed\n" : "ok\n");
   return fails ? 1 : 0;
 }
