@@ -73,7 +73,8 @@ constexpr uint64_t kMaskedWidth = 1ull << 18, kMaskedRoot = 6000000;
 
 inline bool range_masked_pays(int sm_count, uint64_t start, uint64_t count, uint64_t root, uint64_t pieces,
                               uint64_t runs, uint32_t ne) {
-  if (start < (8ull << 30) || root < (1ull << 16) || pieces > kRangeMaskPieces) return false;
+  if (start < (8ull << 30) || root < (1ull << 16)) return false;
+  if (pieces + count / kRangeMaskEvens > kRangeMaskPieces) return false;  // (some 500 bytes each, on the host and the GPU)
   if (root >= kMaskedRoot) return true;
   if (count >= kMaskedWidth * (uint64_t)sm_count) return false;
   const double primes = 1.1 * (double)root / std::log((double)root) - 6542;  // beyond 2^16

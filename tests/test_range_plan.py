@@ -63,9 +63,17 @@ static void masks() {
   check(!gb::range_masked_pays(148, 1ull << 60, 1ull << 40, 1u << 30, (1u << 20) + 1, 1, 8192), "pieces", 0, 0, 0);
 }
 
+// a segment is cut into runs of 2^28 n, each with descriptors of its own
+static void descriptors() {
+  check(gb::range_masked_pays(148, 1ull << 60, 1ull << 47, 1u << 30, 100, 1, 8192), "2^19 runs", 0, 0, 0);
+  for (uint64_t n : {1ull << 49, 1ull << 55, 1ull << 62})
+    check(!gb::range_masked_pays(148, 1ull << 40, n, 0xffffffffu, 1, 1, 8192), "one segment's runs", n, 0, 0);
+}
+
 int main() {
   widths();
   masks();
+  descriptors();
   std::printf(fails ? "failed\n" : "ok\n");
   return fails ? 1 : 0;
 }
