@@ -503,7 +503,7 @@ gb_status range_impl(gb_ctx* c, Workspace& w, Arena* arena, uint64_t start, uint
   int launches = 0;
   // (a shard's segments lie apart)
   bool masked = my_segs && range_masked_pays(c->sm_count, start, std::min(count, my_segs * o.seg_size), root, my_segs,
-                                             sc > 1 ? my_segs : 1, NE);
+                                             sc > 1 ? my_segs : 1, NE, nseg);
   if (masked) {
     std::vector<RangePiece> segs;
     for (uint64_t g = o.shard_index; g < nseg; g += sc)

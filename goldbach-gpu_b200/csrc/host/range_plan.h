@@ -51,7 +51,7 @@ inline uint32_t balanced_chunk(uint64_t pieces, uint64_t len, uint64_t tail, dou
 }
 
 // Whether a range of `count` n from `start` on, in `pieces` segments that form
-// `runs` stretches without a gap, goes through masks of the large-prime pass
+// `runs` stretches without a gap (a shard's share of `segments`), goes through masks of the large-prime pass
 // (range_masked); root: its largest sieving prime; ne: the width of its chunks
 // without them.  A chunk spends 0.6 ns on each of its sieving primes, whatever
 // its width, and with two CTAs per SM a wave of chunks as much; the masks leave it the
@@ -72,8 +72,9 @@ constexpr uint64_t kRangeMaskPieces = 1ull << 20;
 constexpr uint64_t kMaskedWidth = 1ull << 18, kMaskedRoot = 6000000;
 
 inline bool range_masked_pays(int sm_count, uint64_t start, uint64_t count, uint64_t root, uint64_t pieces,
-                              uint64_t runs, uint32_t ne) {
+                              uint64_t runs, uint32_t ne, uint64_t segments) {
   if (start < (8ull << 30) || root < (1ull << 16)) return false;
+  if (segments > 0xffffffffull) return false;  // (a piece's index takes 32 bits)
   if (pieces + count / kRangeMaskEvens > kRangeMaskPieces) return false;  // (some 500 bytes each, on the host and the GPU)
   if (root >= kMaskedRoot) return true;
   if (count >= kMaskedWidth * (uint64_t)sm_count) return false;

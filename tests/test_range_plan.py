@@ -54,26 +54,34 @@ static void masks() {
     const uint64_t root = (uint64_t)std::sqrt(c.top), segs = (uint64_t)std::ceil(c.count / c.seg);
     const uint64_t mine = (segs + c.shards - 1) / c.shards;
     const bool m = gb::range_masked_pays(148, (uint64_t)(c.top - 2 * c.count), (uint64_t)(c.count / c.shards), root, mine,
-                                         c.shards > 1 ? mine : 1, 1u << 20);
+                                         c.shards > 1 ? mine : 1, 1u << 20, segs);
     check((m ? c.masked : c.alone) <= 1.1 * std::min(c.masked, c.alone), "masks", (uint64_t)c.top, (uint64_t)c.count,
           (uint64_t)c.seg);
   }
   // below every sieving prime, and with more segments than the descriptors are meant for
-  check(!gb::range_masked_pays(148, 1u << 30, 1000, 1u << 20, 1, 1, 8192), "low", 0, 0, 0);
-  check(!gb::range_masked_pays(148, 1ull << 60, 1ull << 40, 1u << 30, (1u << 20) + 1, 1, 8192), "pieces", 0, 0, 0);
+  check(!gb::range_masked_pays(148, 1u << 30, 1000, 1u << 20, 1, 1, 8192, 1), "low", 0, 0, 0);
+  check(!gb::range_masked_pays(148, 1ull << 60, 1ull << 40, 1u << 30, (1u << 20) + 1, 1, 8192, (1u << 20) + 1), "pieces", 0, 0, 0);
 }
 
 // a segment is cut into runs of 2^28 n, each with descriptors of its own
 static void descriptors() {
-  check(gb::range_masked_pays(148, 1ull << 60, 1ull << 47, 1u << 30, 100, 1, 8192), "2^19 runs", 0, 0, 0);
+  check(gb::range_masked_pays(148, 1ull << 60, 1ull << 47, 1u << 30, 100, 1, 8192, 100), "2^19 runs", 0, 0, 0);
   for (uint64_t n : {1ull << 49, 1ull << 55, 1ull << 62})
-    check(!gb::range_masked_pays(148, 1ull << 40, n, 0xffffffffu, 1, 1, 8192), "one segment's runs", n, 0, 0);
+    check(!gb::range_masked_pays(148, 1ull << 40, n, 0xffffffffu, 1, 1, 8192, 1), "one segment's runs", n, 0, 0);
+}
+
+// a piece carries its segment's index in the whole range in 32 bits
+static void indexes() {
+  for (int k : {-1, 0, 1})
+    check(gb::range_masked_pays(148, 1ull << 60, 1u << 20, 1u << 30, 1000, 1000, 8192, (1ull << 32) + k) == (k < 0),
+          "segments", k + 1, 0, 0);
 }
 
 int main() {
   widths();
   masks();
   descriptors();
+  indexes();
   std::printf(fails ? "failed\n" : "ok\n");
   return fails ? 1 : 0;
 }
