@@ -147,13 +147,13 @@ struct SieveTab {
 };
 __device__ const SieveTab g_sieve{};
 
-// n mod M for a constant 2^13 < M < 2^31 from one FMA of n as a double: the
-// conversion, 1/M and the product are each within 2^-53 of exact, so the
-// estimate is within 2^-4 of n / M < 2^51 and rounds to floor(n / M) or one
+// n mod M for a constant 2^16 < M < 2^31 from one FMA of n as a double: the
+// conversion and 1/M are each within 2^-53 of exact, so before the sum is rounded
+// the estimate is within 2^-4 of n / M < 2^48 and rounds to floor(n / M) or one
 // more; the low 32 bits of the sum with 1.5 * 2^52 are that quotient's.
 template <uint32_t M>
 __device__ __forceinline__ uint32_t mod_const(double nd, uint32_t nl) {
-  static_assert(M > (1u << 13) && M < (1u << 31), "quotient estimate");
+  static_assert(M > (1u << 16) && M < (1u << 31), "quotient estimate");
   constexpr double kInv = 1.0 / M;
   const uint32_t qt = (uint32_t)__double_as_longlong(fma(nd, kInv, 6755399441055744.0));
   const uint32_t r = nl - qt * M;

@@ -24,9 +24,9 @@
 //
 // Cost of a pair.  The first mark of class c is t_c = (a_c - g0) mod p, a_1 =
 // -1/6 and a_5 = -5/6 (mod p).  One fused multiply-add of g0 (as a double) by
-// 1/p onto 1.5 * 2^52 rounds g0 / p to an integer m with an error below 1/4 (g0 <
-// 2^62, p > 2^20), held in the double's low bits, and d = m p - g0 (mod 2^32)
-// is within 3p/4 of zero.  The a_c taken next to zero are within p/6 of it (6
+// 1/p onto 1.5 * 2^52 rounds g0 / p to an integer m with an error below 1/4 beside the
+// rounding (g0 / p < 2^42, near_inv), held in the double's low bits, and d = m p - g0
+// (mod 2^32) is within 3p/4 of zero.  The a_c taken next to zero are within p/6 of it (6
 // divides p - 1 or p + 1), so d + a_c lies in (-p, p), and t_c = min(d + a_c, d +
 // a_c + p) as unsigned 32-bit numbers when p < 2^31; for larger p a sum below
 // zero leaves t_c >= p/12 > 2^27, beyond every mask taken here (< 2^27 bits),
@@ -34,11 +34,11 @@
 // one multiply-add, two additions, two add-and-minimum, a minimum and a
 // comparison.  (One residue mod p for both classes, the distance from 6 g0 to
 // p's next multiple, costs half of that but hits three times as often, and the
-// hits are what a wide window pays for: it measured 56 ms against 28.)  The pass marks every multiple of p in
-// the window, those below p^2 included (they are composite); only p itself
-// must stay, and it can lie in a window only when the window starts below 2^32,
-// so those windows (g0 < 2^30) take an exact path with the p^2 rule, and so do
-// masks of 2^27 bits or more.
+// hits are what a wide window pays for: it measured 56 ms against 28.)  The pass
+// marks every multiple of p in the window, those below p^2 included (they are
+// composite); only p itself must stay, and it can lie in a window only when the
+// window starts below 2^32, so those windows (g0 < 2^30) take an exact path with
+// the p^2 rule, and so do masks of 2^27 bits or more.
 #include <cuda_runtime.h>
 
 #include <cstdint>
@@ -95,11 +95,13 @@ __device__ __forceinline__ void win_mark_from(const WinLargeArgs& a, uint32_t w,
   }
 }
 
-// 1/p to a relative error near 2^-47: the single-precision reciprocal (2^-23
-// with the rounding of p to a float) and one Newton step in double precision.
-// The quotient estimate needs x / p * error < 1/8 with x / p < 2^44; a
-// correctly rounded division costs several times more and is paid once per
-// prime, which dominates when few windows share the pass.
+// 1/p to a relative error of 2^-46: the single-precision reciprocal (2^-24 for its
+// own rounding and 2^-24 for p's to a float) and one Newton step in double
+// precision, which squares it.  With g0 / p < 2^42 (p > 2^20 for the windows,
+// masked_bound for ranges) the quotient estimate is then within 2^-4 of exact, and
+// g0's rounding to a double adds 2^-11.  A correctly rounded division costs several
+// times more and is paid once per prime, which dominates when few windows share
+// the pass.
 __device__ __forceinline__ double near_inv(uint32_t p) {
   const double pd = (double)p;
   const double r0 = (double)__frcp_rn((float)p);
@@ -113,10 +115,11 @@ __device__ __forceinline__ double near_inv(uint32_t p) {
 // runs the marking code for one or two lanes at nearly every pair of a wide
 // window.  944 windows of 6e6 n on average near 1e18, 3.0e10 pairs and 1.6e9
 // marks: 27.6 ms; marking at once 86 ms; at once over all windows in one launch
-// (marks missing L2) 57 ms.  What is left is issue: 72% of the slots, about 24
-// instructions a pair, 10 of them arithmetic.  The host launches the pass for groups of windows
-// whose masks stay in L2 (kLargeGroupBytes): a launch over all of them marks a
-// mask of 0.5 GB at random, and every mark reads and writes a sector of HBM.
+// (marks missing L2) 57 ms.  What is left is issue: 77% of the slots, about 24
+// instructions a pair, 10 of them arithmetic.  The host launches the pass for
+// groups of windows whose masks stay in L2 (kLargeGroupBytes): a launch over all
+// of them marks a mask of 0.5 GB at random, and every mark reads and writes a
+// sector of HBM.
 constexpr int kHitRows = 12;  // 48 KB a CTA, 4 CTAs per SM
 struct HitQueue {
   uint4 e[kHitRows][32];  // t1, t5, window, prime index
