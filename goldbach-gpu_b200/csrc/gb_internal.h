@@ -165,7 +165,9 @@ struct CountArgs {
 };
 cudaError_t launch_count_classes(const uint32_t* odd, uint64_t nodd, uint32_t modulus, uint32_t* classes,
                                  uint64_t stride, uint64_t nwords, cudaStream_t s);
-cudaError_t launch_counts(const CountArgs& a, const uint32_t* odd, uint64_t start, uint64_t count, cudaStream_t s);
+// odd: the odd bitset of nodd words, with two words in front and six behind that are cleared here
+cudaError_t launch_counts(const CountArgs& a, uint32_t* odd, uint64_t nodd, uint64_t start, uint64_t count,
+                          cudaStream_t s);
 
 // kernels/range.cu
 size_t range_smem_bytes(const RangeArgs& a);

@@ -1121,10 +1121,8 @@ static gb_status counts_impl(gb_ctx* c, Workspace& w, uint64_t start, uint64_t c
     ca.wps = (std::max(ca.wps, per_task((uint64_t)c->sm_count * 256)) + 223) / 224 * 224;
   }
   ca.splits = (wmax + ca.wps - 1) / ca.wps;
-  // the sieve writes words 2 .. nwords + 1; the padding around them is zero
-  cudaError_t e = cudaMemsetAsync(buf, 0, 8, s);
-  if (e == cudaSuccess) e = cudaMemsetAsync(buf + 2 + nwords, 0, 6 * 4, s);
-  if (e == cudaSuccess) e = launch_sieve_bits(a, s);
+  // the sieve writes words 2 .. nwords + 1; the padding around them is cleared by launch_counts
+  cudaError_t e = launch_sieve_bits(a, s);
   if (ca.modulus > 2) {
     if (e == cudaSuccess) e = cudaMemsetAsync(classes, 0, 16, s);
     const uint64_t nc = ca.modulus == 30 ? 8 : 48;
@@ -1139,9 +1137,7 @@ static gb_status counts_impl(gb_ctx* c, Workspace& w, uint64_t start, uint64_t c
     if (bytes <= kIoBytes) up = std::memcpy(w.h_io, up, bytes);  // pinned
     e = cudaMemcpyAsync(d_pairs, up, bytes, cudaMemcpyHostToDevice, s);
   }
-  if (e == cudaSuccess) e = cudaEventRecord(w.ek0, s);
-  if (e == cudaSuccess) e = launch_counts(ca, buf + 2, start, count, s);
-  if (e == cudaSuccess) e = cudaEventRecord(w.ek1, s);
+  if (e == cudaSuccess) e = launch_counts(ca, buf + 2, nwords, start, count, s);
   if (e == cudaSuccess && !o.on_device) e = cudaMemcpyAsync(counts, d_out, count * 8, cudaMemcpyDeviceToHost, s);
   if (e == cudaSuccess) e = cudaStreamSynchronize(s);
   if (e != cudaSuccess) return cuda_fail(w, e, "partition counts");
