@@ -401,9 +401,9 @@ class Context:
         return w
 
     def autotune_windows(self, starts, counts, phase2_limit=0) -> dict:
-        """gb_autotune_windows: the Miller-Rabin split divisor, chunk, large-prime
-        grid and block shape for this batch (timed on a sample, cached per
-        batch class); the dict carries the choice and the opts to pass on."""
+        """gb_autotune_windows: the split divisor, chunk, large-prime grid and
+        block shape for this batch (timed on a sample, cached per batch class);
+        the dict carries the choice and the opts to pass on."""
         w = self._windows(starts, counts)
         base = WindowsOpts(GB_WINDOWS_PERSISTENT, 0, 0, phase2_limit, 0, None, 0, 0, 0, 0, 0)
         tuned = WindowsOpts()

@@ -3,7 +3,7 @@
 // The reference's big_check (src/big_check.cpp:35-144) sieves the primes up
 // to 1e7 on the host and runs GMP's mpz_probab_prime_p(n - p, 25) on OpenMP
 // threads in batches of 1000 primes, keeping the first success.  Here the
-// candidates come from the resident prime table in batches of kBigBatch:
+// candidates come from the resident prime table in batches sized by n's length:
 // the filter kernel drops q = n - p with a factor below kBigTrialBound (from
 // n mod r, computed here once), the base-2 kernel tests the survivors, the
 // bases kernel runs the other 11 bases on the smallest base-2 passer

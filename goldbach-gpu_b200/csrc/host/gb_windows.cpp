@@ -8,7 +8,8 @@
 // large-prime pass, the narrower ones' from a short sieve and a primality test
 // of every q it leaves (kernels/windows.cu); then range6_kernel in windows
 // mode runs over every (window, chunk) item from one device work counter, and
-// the device Phase 2 over what it leaves.
+// the device Phase 2 over what it leaves.  Windows of a few n, and small batches
+// of narrow ones, go n by n through the single-n kernel instead.
 // GB_WINDOWS_PLAIN runs the same launches window by window (the per-window
 // launch pipeline, kept for comparison).
 #include <algorithm>
@@ -577,8 +578,9 @@ static gb_status windows_sieve_impl(gb_ctx* c, Workspace& ws, Arena* arena, cons
       chk(graph ? cudaEventRecordWithFlags(ev, s, cudaEventRecordExternal) : cudaEventRecord(ev, s));
     };
     if (graph) chk(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
-    // every launch is there in every batch, with a grid of one where it has no
-    // work: another topology would have the graph instantiated anew
+    // every kernel is there in every batch, with a grid of one where it has no
+    // work: another topology would have the graph instantiated anew, as another
+    // number of mask groups does (each of them takes longer than that)
     chk(cudaMemsetAsync(d_lmask, 0xff, std::max<uint64_t>(lwords_sieved, 1) * 4, s));
     mark(ws.ek0);
     size_t r = 0;
@@ -697,9 +699,8 @@ static gb_status windows_sieve_impl(gb_ctx* c, Workspace& ws, Arena* arena, cons
 }
 
 
-// Narrow windows on the Miller-Rabin path: every n of every window through
-// the single-n kernel (minimal p over the resident table, q by the 7-base
-// MR), then one per-window reduction.  Plain mode launches the single-n
+// Windows that go n by n: every n of every window through the single-n kernel
+// (minimal p over the resident table), then one per-window reduction.  Plain mode launches the single-n
 // kernel window by window.
 static gb_status windows_mr_impl(gb_ctx* c, Workspace& ws, Arena* arena, const gb_window* w,
                                  size_t count, const gb_windows_opts& o, uint64_t p_lim,
@@ -757,7 +758,7 @@ static gb_status windows_mr_impl(gb_ctx* c, Workspace& ws, Arena* arena, const g
   chk(cudaMemcpyAsync(agg.data(), d_agg, count * 32, cudaMemcpyDeviceToHost, s));
   if (min_p_concat) chk(cudaMemcpyAsync(pv.data(), d_p, total * 8, cudaMemcpyDeviceToHost, s));
   chk(cudaStreamSynchronize(s));
-  if (e != cudaSuccess) return cuda_fail(ws, e, "windows (Miller-Rabin path)");
+  if (e != cudaSuccess) return cuda_fail(ws, e, "windows (n by n)");
   float ms = 0;
   cudaEventElapsedTime(&ms, ws.ev0, ws.ev1);
   uint64_t fails = 0;
@@ -821,7 +822,8 @@ gb_status windows_impl(gb_ctx* c, Workspace& ws, Arena* arena, const gb_window* 
   for (const gb_window& x : wb) nb += x.count;
   std::vector<uint32_t> ma(min_p_concat ? na : 0), mb(min_p_concat ? nb : 0);
   gb_windows_summary sa{}, sb{};
-  st = windows_mr_impl(c, ws, arena, wa.data(), wa.size(), o, p_lim, ra.data(), min_p_concat ? ma.data() : nullptr, &sa);
+  st = windows_mr_impl(c, ws, arena, wa.data(), wa.size(), o, p_lim, ra.data(),
+                       min_p_concat ? ma.data() : nullptr, &sa);
   if (st == GB_ENOMEM && !o.mr_below && !few) {  // no room for their n (nothing launched yet): the pipeline alone
     ws.err.clear();
     return windows_sieve_impl(c, ws, arena, w, count, opts, res, min_p_concat, sum);

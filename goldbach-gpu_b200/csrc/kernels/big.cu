@@ -133,7 +133,8 @@ struct Big {
   }
   // The carry into this lane, from the lanes that generate one (g) and those
   // that pass one on (p, not g): the carries of the sum of two numbers whose
-  // bits generate and propagate alike.  out: the carry out of the last lane.
+  // bits generate and propagate alike (carry look-ahead by one addition of the two
+  // ballots, a known technique).  out: the carry out of the last lane.
   static __device__ __forceinline__ uint32_t carry_in(bool g, bool p, bool& out) {
     uint32_t gb = __ballot_sync(kAllLanes, g), pb = __ballot_sync(kAllLanes, p && !g);
     if (G < 32) {

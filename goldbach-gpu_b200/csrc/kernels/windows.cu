@@ -377,7 +377,7 @@ cudaError_t launch_win_test(const WinTestArgs& a, int grid, cudaStream_t s) {
   return cudaGetLastError();
 }
 
-// Narrow windows on the Miller-Rabin path: the n of each window, laid out
+// Windows that go n by n: the n of each window, laid out
 // window after window at off[i], for the single-n kernel.
 __global__ void win_expand_kernel(const gb_window* __restrict__ w, const uint64_t* __restrict__ off,
                                   uint32_t nw, uint64_t* __restrict__ n) {
