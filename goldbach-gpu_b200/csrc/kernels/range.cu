@@ -236,10 +236,19 @@ size_t range_smem_bytes(const RangeArgs& a) {
   return range6_smem_words(a.nbw, a.s.minp ? a.chunk_evens : 0) * sizeof(uint32_t);
 }
 
+// The dynamic shared memory that every launch allows its kernel: a block's most
+// (227 KB) less 1 KB for the static variables.  The bound belongs to the
+// function, so a launch that set its own need would lower it under another
+// thread's, whose chunks are wider.
+constexpr int kRange6SmemMost = 226 * 1024;
+static_assert(range6_smem_words(((1u << 17) / 6 + 96) / 32 + 1 + (1u << 20) / 96 + 2 * kTaskWords6 + 8) * 4 <=
+                  kRange6SmemMost,
+              "the widest chunk at the widest halo");
+
 template <typename K>
 static int occupancy(K kernel, size_t smem, int threads) {
   int nb = 0;
-  cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kRange6SmemMost);
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, kernel, threads, smem);
   return nb;
 }
@@ -280,7 +289,7 @@ int range_max_blocks_per_sm(const RangeArgs& a) {
 template <typename K>
 static cudaError_t launch_one(K kernel, const RangeArgs& a, int grid, size_t smem, cudaStream_t st,
                               int threads) {
-  cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kRange6SmemMost);
   if (e != cudaSuccess) return e;
   kernel<<<grid, threads, smem, st>>>(a);
   return cudaGetLastError();
